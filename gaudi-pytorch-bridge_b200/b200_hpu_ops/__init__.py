@@ -32,6 +32,8 @@ def _load():
 
 _load()
 
+_set_sr_seed = torch.ops.b200q.set_sr_seed  # (called once per training step: not looked up again)
+
 from . import abi  # noqa: E402
 from .abi import device_status, launch_count  # noqa: E402
 
@@ -39,7 +41,7 @@ from .abi import device_status, launch_count  # noqa: E402
 def set_sr_seed(seed: int) -> None:
     """Seed of the Philox stream used by stochastic rounding; also rewinds the per-call offset
     (each stochastic cast_to_fp8_v2 call consumes one offset so repeated calls differ)."""
-    torch.ops.b200q.set_sr_seed(int(seed))
+    _set_sr_seed(int(seed))
 
 
 def set_cast_mul_in_fp32(on: bool) -> None:

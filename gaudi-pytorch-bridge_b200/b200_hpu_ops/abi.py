@@ -60,6 +60,7 @@ class SdpaArgs(C.Structure):
         ("d_scale_s_given", C.c_int),
         ("m_out", C.c_void_p), ("linv_out", C.c_void_p), ("amax_s", C.c_void_p), ("amax_o", C.c_void_p),
         ("force_plain", C.c_int), ("stream", C.c_void_p),
+        ("zero_ptr", C.c_void_p * 5), ("zero_bytes", C.c_int * 5),
     ]
 
 

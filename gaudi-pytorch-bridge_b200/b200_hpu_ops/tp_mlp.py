@@ -139,6 +139,9 @@ class TpFp8Mlp:
         dev = shard.w_gate_up.device
         self._xs_inv = torch.tensor(1.0 / self.x_scale, dtype=torch.float32, device=dev)
         self._as_inv = torch.tensor(1.0 / self.act_scale, dtype=torch.float32, device=dev)
+        # the cast's scale as a device scalar: the operator's first overload takes it (a Python float is tried
+        # against that overload, refused and resolved again on every call)
+        self._xs = torch.tensor(self.x_scale, dtype=torch.float32, device=dev) if ops is None else self.x_scale
 
     def _mode(self, tp: int, tokens: int) -> str:
         if tp == 1:
@@ -168,7 +171,7 @@ class TpFp8Mlp:
 
     # -- the three local stages ------------------------------------------------------------
     def gate_up(self, x: torch.Tensor) -> torch.Tensor:
-        x8, _ = self.ops.cast_to_fp8_v2(x, self.x_scale, False, False, E4M3)
+        x8, _ = self.ops.cast_to_fp8_v2(x, self._xs, False, False, E4M3)
         n = self.s.w_gate_up.shape[0]
         return self.ops.fp8_gemm_v2(x8, False, self.s.w_gate_up, True, None, torch.bfloat16, self._xs_inv,
                                     self.s.s_gate_up_inv, None, False, [1, n])
@@ -185,7 +188,7 @@ class TpFp8Mlp:
     def hidden(self, x: torch.Tensor) -> torch.Tensor:
         """e4m3 [tokens, f_local]: this rank's columns of cast(silu(gate) * up)."""
         if self.fused_gate_up:
-            x8, _ = self.ops.cast_to_fp8_v2(x, self.x_scale, False, False, E4M3)
+            x8, _ = self.ops.cast_to_fp8_v2(x, self._xs, False, False, E4M3)
             return torch.ops.b200q.fp8_gemm_swiglu_cast(x8, self.s.w_gate_up, self._xs_inv, self.s.s_gate_up_inv, self.act_scale)
         return self.activation(self.gate_up(x))
 

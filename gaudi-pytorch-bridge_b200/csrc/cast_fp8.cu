@@ -22,7 +22,27 @@ struct CastParams {
   float* amax;
   uint64_t seed, offset, first_index;
   int mul_fp32;
+  int start;  // StartMode
 };
+
+// How a cast is ordered after the kernel in front of it, and where its amax goes.
+enum StartMode {
+  kStartAfter = 0,       // waits for that kernel (or for the memset of the amax word) before its first access
+  kStartBehindClear = 1, // that kernel cleared the amax word and has itself waited: only the atomicMax waits for it
+  kStartCluster = 2,     // waits; the grid is one cluster, which reduces its amax by itself
+};
+__device__ __forceinline__ void cast_begin(int start) {
+  if (start == kStartBehindClear) {
+    pdl_release();
+  } else {
+    pdl_enter();
+    if (start == kStartCluster) cluster_amax_begin();
+  }
+}
+__device__ __forceinline__ void cast_publish_amax(uint32_t amax_bits, float* amax, int start) {
+  if (start == kStartCluster) cluster_amax_store(amax_bits, amax);
+  else if (amax) block_amax_to_global(amax_bits, amax);
+}
 
 template <typename T>
 struct InTraits;
@@ -52,7 +72,7 @@ __device__ __forceinline__ uint32_t nan_byte(float) {
 
 template <typename InT, int FMT, bool SR, int SC>
 __global__ void __launch_bounds__(256) cast_to_fp8_kernel(CastParams p) {
-  pdl_release();
+  cast_begin(p.start);
   constexpr bool BF16 = InTraits<InT>::kIsBf16;
   const InT* __restrict__ in = static_cast<const InT*>(p.in);
   uint8_t* __restrict__ out = static_cast<uint8_t*>(p.out);
@@ -189,7 +209,7 @@ __global__ void __launch_bounds__(256) cast_to_fp8_kernel(CastParams p) {
     out[i] = (uint8_t)b;
   }
 
-  if (p.amax) block_amax_to_global(amax_bits, p.amax);
+  cast_publish_amax(amax_bits, p.amax, p.start);
 }
 
 
@@ -250,7 +270,7 @@ __device__ __forceinline__ uint4 cast16_bf16_rne(const uint4 a, const uint4 b, u
 
 template <int FMT, bool PER_ROW>
 __global__ void __launch_bounds__(256) cast_bf16_rne_fast_kernel(CastParams p) {
-  pdl_release();
+  cast_begin(p.start);
   const __nv_bfloat16* __restrict__ in = static_cast<const __nv_bfloat16*>(p.in);
   uint8_t* __restrict__ out = static_cast<uint8_t*>(p.out);
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -302,7 +322,7 @@ __global__ void __launch_bounds__(256) cast_bf16_rne_fast_kernel(CastParams p) {
     if (y != y) b = 0x7Fu;
     out[i] = (uint8_t)b;
   }
-  if (p.amax) block_amax_to_global(amax_bits, p.amax);
+  cast_publish_amax(amax_bits, p.amax, p.start);
 }
 
 // ------------------------------------------------------------------ bf16 -> fp8, stochastic, fast path
@@ -366,7 +386,7 @@ __device__ __forceinline__ uint4 cast16_bf16_sr(const uint4 a, const uint4 b, ui
 
 template <int FMT, bool PER_ROW>
 __global__ void __launch_bounds__(256) cast_bf16_sr_fast_kernel(CastParams p) {
-  pdl_release();
+  cast_begin(p.start);
   const __nv_bfloat16* __restrict__ in = static_cast<const __nv_bfloat16*>(p.in);
   uint8_t* __restrict__ out = static_cast<uint8_t*>(p.out);
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -421,7 +441,7 @@ __global__ void __launch_bounds__(256) cast_bf16_sr_fast_kernel(CastParams p) {
     if (y != y) b = 0x7Fu;
     out[i] = (uint8_t)b;
   }
-  if (p.amax) block_amax_to_global(amax_bits, p.amax);
+  cast_publish_amax(amax_bits, p.amax, p.start);
 }
 
 // ------------------------------------------------------------------ hybrid cast (e5m2 + e4m3 in one pass)
@@ -437,13 +457,14 @@ struct HybridParams {
   float* amax;
   uint64_t seed, offset, first_index;
   int mul_fp32;
+  int start;  // StartMode
 };
 
 // One read of the input, two fp8 outputs: e5m2 (RNE or stochastic) with its own per-tensor scale
 // and e4m3 (always RNE) with its own.  4 bytes per bf16 element instead of 6 for two casts.
 template <typename InT, bool SR>
 __global__ void __launch_bounds__(256) cast_hybrid_kernel(HybridParams p) {
-  pdl_release();
+  cast_begin(p.start);
   constexpr bool BF16 = InTraits<InT>::kIsBf16;
   const InT* __restrict__ in = static_cast<const InT*>(p.in);
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -533,7 +554,7 @@ __global__ void __launch_bounds__(256) cast_hybrid_kernel(HybridParams p) {
     p.out152[i] = (uint8_t)b5;
     p.out143[i] = (uint8_t)b4;
   }
-  if (p.amax) block_amax_to_global(amax_bits, p.amax);
+  cast_publish_amax(amax_bits, p.amax, p.start);
 }
 
 // ------------------------------------------------------------------ cast_from_fp8
@@ -650,6 +671,7 @@ struct SwigluParams {
 
 
 __global__ void __launch_bounds__(256) swiglu_cast_kernel(SwigluParams p) {
+  pdl_enter();
   const int64_t vec_per_row = p.cols / 16;
   const int64_t nvec = p.rows * vec_per_row;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -757,23 +779,44 @@ int clear_amax(float* amax, cudaStream_t st) {
   return B200Q_OK;
 }
 
-template <typename Params>
-static auto amax_of(const Params& p, int) -> decltype(p.amax) { return p.amax; }
-template <typename Params>
-static float* amax_of(const Params&, long) { return nullptr; }
+// Casts with amax of at most this many elements run as ONE cluster of up to eight blocks that
+// reduces its amax by itself: one launch instead of two, where launches are what such a cast
+// costs.  Eight SMs move 2^18 elements in about 2 us, the time a second launch takes.
+constexpr int64_t kClusterCastMax = 1 << 18;
 
-// overlapped = the kernel may start before its predecessor in the stream has finished: a cast with
-// amax (behind clear_amax_kernel; it waits before its atomicMax only) or a kernel that calls
-// pdl_enter() first thing.  A cast without amax has no such wait and is launched the ordinary way.
-template <typename Kernel, typename Params>
-static void launch_persistent(Kernel kernel, int64_t items, cudaStream_t st, const Params& p, bool one_wave = false,
-                              bool enters = false) {
-  const int grid = grid_for(kernel, items, one_wave);
-  if (enters || amax_of(p, 0) != nullptr) {
-    if (launch_overlapped(kernel, dim3((unsigned)grid), dim3(256), 0, st, p) == cudaSuccess) return;
-    (void)cudaGetLastError();  // fall back to the ordinary launch
+// Up to this many elements a memset clears the amax word, above it clear_amax_kernel: a memset
+// costs the host 0.7 us where a launch costs 2.0, a cast of this size is over before the host has
+// issued the next one, and the launch gap that the clearing kernel hides does not show.
+constexpr int64_t kMemsetCastMax = 1 << 22;
+
+// Decides how a cast starts and clears its amax word where that is needed.
+static int cast_start(float* amax, int64_t n, cudaStream_t st, int* start) {
+  *start = kStartAfter;
+  if (!amax) return B200Q_OK;
+  if (n > kMemsetCastMax) {
+    *start = kStartBehindClear;
+    return clear_amax(amax, st);
   }
-  kernel<<<grid, 256, 0, st>>>(p);
+  if (n > 0 && n <= kClusterCastMax) *start = kStartCluster;
+  else B200Q_CUDA_OK(cudaMemsetAsync(amax, 0, sizeof(float), st));
+  return B200Q_OK;
+}
+template <typename Params>
+static auto start_of(const Params& p, int) -> decltype(p.start) { return p.start; }
+template <typename Params>
+static int start_of(const Params&, long) { return kStartAfter; }
+
+// Every kernel launched here may be set up before its predecessor in the stream has finished (it
+// waits as its StartMode says).
+template <typename Kernel, typename Params>
+static void launch_persistent(Kernel kernel, int64_t items, cudaStream_t st, const Params& p, bool one_wave = false) {
+  if (start_of(p, 0) == kStartCluster) {
+    const int64_t blocks = (items + 255) / 256;
+    const unsigned size = blocks >= 8 ? 8u : blocks >= 4 ? 4u : blocks >= 2 ? 2u : 1u;
+    launch_dependent_cluster(kernel, size, dim3(size), dim3(256), 0, st, p);
+    return;
+  }
+  launch_dependent(kernel, dim3((unsigned)grid_for(kernel, items, one_wave)), dim3(256), 0, st, p);
 }
 
 template <typename InT, int FMT, bool SR>
@@ -810,9 +853,11 @@ int cast_to_fp8_impl(const void* in, int in_dtype, void* out, int out_dtype, con
     if (n) B200Q_CUDA_OK(cudaMemcpyAsync(out, in, (size_t)n, cudaMemcpyDeviceToDevice, st));
     return B200Q_OK;
   }
-  if (amax) { int rc = clear_amax(amax, st); if (rc) return rc; }
+  int start;
+  if (int rc = cast_start(amax, n, st, &start)) return rc;
   if (n == 0) return B200Q_OK;
   CastParams p;
+  p.start = start;
   p.in = in; p.out = out; p.scale = scale; p.scale_host = scale_host;
   p.has_scale = scale_mode != B200Q_BCAST_NONE;
   p.scale_from_dev = scale_mode == B200Q_BCAST_SCALAR_DEV;
@@ -857,10 +902,10 @@ int cast_to_fp8_impl(const void* in, int in_dtype, void* out, int out_dtype, con
 template <typename OutT, int FMT>
 static void launch_uncast_sc(int sc, int64_t items, cudaStream_t st, const UncastParams& p) {
   switch (sc) {
-    case SC_ONE: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_ONE>, items, st, p, false, true); break;
-    case SC_COL: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_COL>, items, st, p, false, true); break;
-    case SC_ROW: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_ROW>, items, st, p, false, true); break;
-    default: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_FULL>, items, st, p, false, true); break;
+    case SC_ONE: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_ONE>, items, st, p); break;
+    case SC_COL: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_COL>, items, st, p); break;
+    case SC_ROW: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_ROW>, items, st, p); break;
+    default: launch_persistent(cast_from_fp8_kernel<OutT, FMT, SC_FULL>, items, st, p); break;
   }
 }
 
@@ -897,7 +942,7 @@ int swiglu_cast_impl(const void* gate, int64_t ld_gate, const void* up, int64_t 
   p.gate = static_cast<const __nv_bfloat16*>(gate); p.up = static_cast<const __nv_bfloat16*>(up);
   p.out = static_cast<uint8_t*>(out); p.ld_gate = ld_gate; p.ld_up = ld_up; p.rows = rows; p.cols = cols;
   p.scale = scale; p.amax = amax;
-  swiglu_cast_kernel<<<grid_for(swiglu_cast_kernel, rows * cols / 16), 256, 0, st>>>(p);
+  launch_dependent(swiglu_cast_kernel, dim3((unsigned)grid_for(swiglu_cast_kernel, rows * cols / 16)), dim3(256), 0, st, p);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }
@@ -905,7 +950,7 @@ int swiglu_cast_impl(const void* gate, int64_t ld_gate, const void* up, int64_t 
 // bf16 input, both outputs rounded to nearest even, product in bf16, everything 16-byte
 // aligned: the packed path of cast_bf16_rne_fast_kernel with two scales and two stores.
 __global__ void __launch_bounds__(256) cast_hybrid_bf16_rne_fast_kernel(HybridParams p) {
-  pdl_release();
+  cast_begin(p.start);
   const __nv_bfloat16* __restrict__ in = static_cast<const __nv_bfloat16*>(p.in);
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
@@ -945,15 +990,17 @@ __global__ void __launch_bounds__(256) cast_hybrid_bf16_rne_fast_kernel(HybridPa
     p.out152[i] = (uint8_t)b5;
     p.out143[i] = (uint8_t)b4;
   }
-  if (p.amax) block_amax_to_global(amax_bits, p.amax);
+  cast_publish_amax(amax_bits, p.amax, p.start);
 }
 
 int cast_hybrid_impl(const void* in, int in_dtype, void* out152, void* out143, const float* s152, float s152_host,
                      int mode152, const float* s143, float s143_host, int mode143, int64_t n, float* amax, int rounding,
                      uint64_t seed, uint64_t offset, uint64_t first_index, int flags, cudaStream_t st) {
-  if (amax) { int rc = clear_amax(amax, st); if (rc) return rc; }
+  int start;
+  if (int rc = cast_start(amax, n, st, &start)) return rc;
   if (n == 0) return B200Q_OK;
   HybridParams p;
+  p.start = start;
   p.in = in; p.out152 = static_cast<uint8_t*>(out152); p.out143 = static_cast<uint8_t*>(out143);
   p.s152 = s152; p.s143 = s143; p.s152_host = s152_host; p.s143_host = s143_host;
   p.has152 = mode152 != B200Q_BCAST_NONE; p.has143 = mode143 != B200Q_BCAST_NONE;

@@ -74,6 +74,29 @@ inline void launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   (void)cudaGetLastError();
   kernel<<<grid, block, smem, st>>>(static_cast<KArgs>(args)...);
 }
+
+// The same for a grid of thread-block clusters of `cluster` blocks along x.
+template <typename... KArgs, typename... Args>
+inline void launch_dependent_cluster(void (*kernel)(KArgs...), unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  if (cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...) == cudaSuccess) return;
+  (void)cudaGetLastError();
+  cfg.numAttrs = 1;  // (an error of this launch is left for the caller's launch check)
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 #endif
 
 // Clears an amax word with a one-thread kernel behind which the kernel that accumulates into it
@@ -212,24 +235,57 @@ __device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
   return v;
 }
 
-// Block-wide max of a non-negative float's bit pattern, then one atomicMax per block.
-// Works on bit patterns so that NaN (pattern above +inf) wins and is propagated.
-__device__ __forceinline__ void block_amax_to_global(uint32_t local_bits, float* amax) {
+// Maximum over the block of a non-negative float's bit pattern, in thread 0.  Works on bit
+// patterns so that NaN (pattern above +inf) wins and is propagated.
+__device__ __forceinline__ uint32_t block_max_u32(uint32_t local_bits) {
   __shared__ uint32_t s_warp[32];
   uint32_t w = warp_max_u32(local_bits);
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) s_warp[wid] = w;
   __syncthreads();
+  uint32_t v = 0u;
   if (wid == 0) {
     int nw = (blockDim.x + 31) >> 5;
-    uint32_t v = lane < nw ? s_warp[lane] : 0u;
+    v = lane < nw ? s_warp[lane] : 0u;
     v = warp_max_u32(v);
-    if (lane == 0 && v != 0u) {
-      // (a kernel launched with programmatic stream serialization behind the kernel that clears
-      // `amax` must not touch it before that kernel is complete; a no-op in an ordinary launch)
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      atomicMax(reinterpret_cast<unsigned int*>(amax), v);
-    }
+  }
+  return v;
+}
+
+// A grid that is one thread-block cluster needs no cleared word and no atomics for its amax: the
+// blocks hand their maxima to the first one through distributed shared memory and it stores the
+// result.  Every thread of the grid calls both functions, cluster_amax_begin() first (a block may
+// only be written to once it runs).
+__device__ __forceinline__ void cluster_amax_begin() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_amax_store(uint32_t local_bits, float* amax) {
+  __shared__ uint32_t s_cta[8];
+  const uint32_t v = block_max_u32(local_bits);
+  uint32_t rank, nranks, dst;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(nranks));
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (threadIdx.x == 0) {
+    const uint32_t own = (uint32_t)__cvta_generic_to_shared(&s_cta[rank]);
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(own));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
+  }
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  if (rank == 0 && threadIdx.x == 0) {
+    uint32_t m = 0u;
+    for (uint32_t i = 0; i < nranks; ++i) m = max(m, s_cta[i]);
+    *amax = __uint_as_float(m);
+  }
+}
+
+// Block-wide max, then one atomicMax per block.
+__device__ __forceinline__ void block_amax_to_global(uint32_t local_bits, float* amax) {
+  const uint32_t v = block_max_u32(local_bits);
+  if (threadIdx.x == 0) {
+    // (a kernel launched with programmatic stream serialization behind the kernel that clears
+    // `amax` must not touch it before that kernel is complete; a no-op in an ordinary launch)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (v != 0u) atomicMax(reinterpret_cast<unsigned int*>(amax), v);
   }
 }
 

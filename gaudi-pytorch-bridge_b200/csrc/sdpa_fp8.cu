@@ -1,8 +1,9 @@
 // FP8 scaled-dot-product attention, forward: out = softmax(q k^T * scale + mask) v with q, k, v in
 // e4m3 and the probabilities re-quantised to e4m3 for the second product.
 //
-// tcgen05 kernel (head dimension 128), one CTA per (batch x head, block of 128 queries), 320 threads:
-//   warp 0    TMA producer: the query tile once, then the key tiles (twice, see below) and value
+// tcgen05 kernel (head dimension 128), persistent, one CTA per SM, 320 threads; a work item is one
+// (batch x head, block of 128 queries):
+//   warp 0    TMA producer: the query tile, then the key tiles (twice, see below) and value
 //             tiles through two shared-memory rings (128-byte swizzle, no multicast)
 //   warp 1    TMEM owner and MMA issuer: S = Q K^T (kind::f8f6f4, 128 x 128 x 32 per instruction)
 //             into one of two score buffers in TMEM, and O += P V with P read from shared memory
@@ -10,9 +11,12 @@
 //   warps 2-9 softmax, two groups of four warps; a group owns one of the two score buffers (it takes
 //             every other key block) and thread = query row: tcgen05.ld of its score row, scale /
 //             mask / exp2, the e4m3 probabilities written into the swizzled P tile for the second
-//             product.  Blocks with nothing to mask take a path of one instruction per score in
-//             the first pass and 3.5 in the second (FFMA, ex2.approx, add, half a convert: the
-//             probability scale is folded into the exponent and divided out of the row sum).
+//             product.
+// The three roles run as one stream of tiles that crosses item boundaries: the scores of tile t + 2
+// are asked for as soon as a group has its 128 scores of tile t in registers (before any of them is
+// used), query tiles and output accumulators are double-buffered, and a group has two P tiles, so
+// that neither product's latency, nor the epilogue of one item, nor the first loads of the next
+// one leave the softmax warps waiting.
 // Two passes over the keys: the first only takes the row maxima, the second recomputes the
 // scores and forms exp(S - max) against the final maximum.  The probabilities are therefore
 // quantised exactly where the CPU restatement quantises them (no running-maximum rescaling of
@@ -23,6 +27,8 @@
 // Every wait is bounded (tcgen05_ptx.cuh); a wait that runs out sets the device status word.
 // Other head dimensions, and anything else the fast path does not take, run a plain CUDA kernel.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05_ptx.cuh"
@@ -64,6 +70,8 @@ struct Params {
   int d_scale_s_given;     // 0: d_scale_s = 1 / q_scale_s
   float softmax_scale;
   int* status;
+  void* zero_ptr[5];       // small buffers to clear (see b200q_sdpa_args)
+  int zero_bytes[5];
   // derived in the kernel (Scales::load)
   float c_log2, q_scale_s, o_scale, q_scale_o;
 };
@@ -77,6 +85,15 @@ __device__ __forceinline__ void load_scales(Params& p) {
   p.q_scale_s = s[3];
   p.q_scale_o = s[4];
   p.o_scale = (p.d_scale_s_given ? s[5] : 1.f / s[3]) * s[2];
+}
+
+// the caller's zero-valued results: cleared by one thread of one block
+__device__ __forceinline__ void clear_zero_list(const Params& p) {
+  if (blockIdx.x != 0 || blockIdx.y != 0 || threadIdx.x != 0) return;
+#pragma unroll
+  for (int i = 0; i < 5; ++i)
+    if (p.zero_ptr[i])
+      for (int b = 0; b < p.zero_bytes[i]; ++b) static_cast<uint8_t*>(p.zero_ptr[i])[b] = 0;
 }
 
 // warp maximum of a non-negative float (bit patterns of non-negative floats order like the values)
@@ -97,58 +114,120 @@ __device__ __forceinline__ float mask_term(const Params& p, int64_t bh, int64_t 
 }
 
 struct Smem {
-  static constexpr int kQ = 0;
-  static constexpr int kK = kQ + kTile;
+  static constexpr int kQ = 0;                            // two query tiles
+  static constexpr int kK = kQ + 2 * kTile;
   static constexpr int kV = kK + kStages * kTile;
-  static constexpr int kP = kV + kStages * kTile;
-  static constexpr int kRowStats = kP + 2 * kTile;        // [2 groups][128 rows] fp32: maxima, then sums
-  static constexpr int kBars = kRowStats + 2 * 128 * 4;
-  // barriers: q_full, k_full[3], k_empty[3], v_full[3], v_empty[3], s_full[2], s_empty[2], p_full[2], p_empty[2], o_full
-  static constexpr int kNumBars = 1 + 4 * kStages + 8 + 1;
+  static constexpr int kP = kV + kStages * kTile;         // two P tiles per group
+  static constexpr int kStats = kP + 4 * kTile;           // [item parity][maxima | sums][2 groups][128 rows] fp32
+  static constexpr int kBars = kStats + 2 * 2 * 2 * 128 * 4;
+  // barriers: {q, o, s}_{full, empty}[2], {k, v}_{full, empty}[3], p_{full, empty}[4]
+  static constexpr int kNumBars = 12 + 4 * kStages + 8;
   static constexpr int kTotal = kBars + kNumBars * 8 + 16;
 };
+
+// Work items in the order of their cost (under a causal mask the last query blocks have the most
+// key blocks), dealt to the CTAs in a snake, so that the CTAs' totals differ by less than an item.
+struct Item {
+  int64_t bh, q0, kv;
+  int nblk;
+};
+__device__ __forceinline__ bool get_item(const Params& p, int round, Item* it) {
+  const int64_t g = gridDim.x, b = blockIdx.x;
+  const int64_t idx = (int64_t)round * g + ((round & 1) ? g - 1 - b : b);
+  const int64_t qblocks = (p.L + kBM - 1) / kBM;
+  if (idx >= qblocks * p.BH) return false;
+  it->bh = idx % p.BH;
+  it->q0 = (qblocks - 1 - idx / p.BH) * kBM;
+  it->kv = it->bh / p.kv_rep;
+  int64_t keys = p.S;  // (causal: keys beyond the block's last query are all masked)
+  if (p.causal && it->q0 + kBM < keys) keys = it->q0 + kBM;
+  it->nblk = (int)((keys + kBN - 1) / kBN);
+  return true;
+}
+
+// Packed fp32 arithmetic: two results per issue slot.
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// First pass over 32 scores: their maximum.
+__device__ __forceinline__ float chunk_max(const uint32_t* r, float m) {
+  float m0 = m, m1 = kMasked;
+#pragma unroll
+  for (int e = 0; e < 32; e += 4) {
+    m0 = max3(m0, __uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+    m1 = max3(m1, __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
+  }
+  return fmaxf(m0, m1);
+}
+// Second pass over 32 scores (keys 32 c ... of the block): exp2(score * mul + off) = probability * q_scale_s,
+// added to the row sums and written as e4m3 into the thread's row of the P tile (two 16-byte
+// pieces, XOR-swizzled by the row).  2.5 issue slots per score: packed FFMA and FADD, ex2, half a convert.
+__device__ __forceinline__ void chunk_exp(const uint32_t* r, int c, uint64_t mul2, uint64_t off2, uint64_t* ls, uint8_t* prow, int row) {
+  uint32_t w[8];
+#pragma unroll
+  for (int e = 0; e < 32; e += 4) {
+    float x[4];
+    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), mul2, off2), x[0], x[1]);
+    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3])), mul2, off2), x[2], x[3]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) x[u] = ex2_approx(x[u]);
+    ls[0] = add_f32x2(ls[0], pack_f32x2(x[0], x[1]));
+    ls[1] = add_f32x2(ls[1], pack_f32x2(x[2], x[3]));
+    // (the conversion saturates at 448: a probability scale beyond that cannot overflow)
+    w[e >> 2] = cvt_fp8x2<B200Q_E4M3>(x[0], x[1]) | (cvt_fp8x2<B200Q_E4M3>(x[2], x[3]) << 16);
+  }
+  *reinterpret_cast<uint4*>(prow + (((2 * c) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4*>(prow + (((2 * c + 1) ^ (row & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+}
 
 __global__ void __launch_bounds__(kThreads, 1)
 sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, const Params p_in) {
-  Params p = p_in;
-  load_scales(p);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::kBars);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Smem::kNumBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile int* sm_stop = reinterpret_cast<volatile int*>(tmem_slot + 2);
   const uint32_t sbase = smem_u32(smem);
   const uint32_t b0 = smem_u32(bars);
-  const uint32_t bar_q = b0, bar_kf = b0 + 8, bar_ke = bar_kf + 8 * kStages, bar_vf = bar_ke + 8 * kStages,
-                 bar_ve = bar_vf + 8 * kStages, bar_sf = bar_ve + 8 * kStages, bar_se = bar_sf + 16, bar_pf = bar_se + 16,
-                 bar_pe = bar_pf + 16, bar_of = bar_pe + 16;
+  const uint32_t bar_qf = b0, bar_qe = b0 + 16, bar_of = b0 + 32, bar_oe = b0 + 48, bar_sf = b0 + 64, bar_se = b0 + 80,
+                 bar_kf = b0 + 96, bar_ke = bar_kf + 8 * kStages, bar_vf = bar_ke + 8 * kStages, bar_ve = bar_vf + 8 * kStages,
+                 bar_pf = bar_ve + 8 * kStages, bar_pe = bar_pf + 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  const int64_t bh = blockIdx.y;
-  // (the last query blocks first: under a causal mask they have the most key blocks, and a long
-  // CTA that starts late is what the kernel ends on)
-  const int64_t q0 = (int64_t)(gridDim.x - 1 - blockIdx.x) * kBM;
-  const int64_t kv = bh / p.kv_rep;
-  // key blocks this query block needs (causal: keys beyond its last query are all masked)
-  int64_t keys = p.S;
-  if (p.causal && q0 + kBM < keys) keys = q0 + kBM;
-  const int nblk = (int)((keys + kBN - 1) / kBN);
-
   if (threadIdx.x == 0) {
-    mbar_init(bar_q, 1);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar_kf + 8 * s, 1); mbar_init(bar_ke + 8 * s, 1);
       mbar_init(bar_vf + 8 * s, 1); mbar_init(bar_ve + 8 * s, 1);
     }
     for (int a = 0; a < 2; ++a) {
-      mbar_init(bar_sf + 8 * a, 1); mbar_init(bar_se + 8 * a, 128);
-      mbar_init(bar_pf + 8 * a, 128); mbar_init(bar_pe + 8 * a, 1);
+      mbar_init(bar_qf + 8 * a, 1); mbar_init(bar_qe + 8 * a, 1);
+      mbar_init(bar_of + 8 * a, 1); mbar_init(bar_oe + 8 * a, 8);  // one arrival per softmax warp
+      mbar_init(bar_sf + 8 * a, 1); mbar_init(bar_se + 8 * a, 4);  // one per warp of the group
     }
-    mbar_init(bar_of, 1);
+    for (int a = 0; a < 4; ++a) { mbar_init(bar_pf + 8 * a, 4); mbar_init(bar_pe + 8 * a, 1); }
     *abort_flag = 0;
-    *sm_stop = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&map_q); tma_prefetch_desc(&map_k); tma_prefetch_desc(&map_v);
@@ -160,26 +239,35 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;  // columns [0,128) S0, [128,256) S1, [256,384) O
+  const uint32_t tmem = *tmem_slot;  // columns [0,128) S0, [128,256) S1, [256,384) O0, [384,512) O1
+  pdl_enter();  // everything above may run under the tail of the kernel in front of this one
+  Params p = p_in;
+  load_scales(p);
+  clear_zero_list(p);
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar_q, kTile);
-      tma_load_3d(sbase + Smem::kQ, &map_q, bar_q, 0, (int)q0, (int)bh);
       uint32_t ks = 0, kph = 0, vs = 0, vph = 0;
+      Item w;
       bool ok = true;
-      for (int t = 0; t < 2 * nblk && ok; ++t) {
-        const int j = t < nblk ? t : t - nblk;
-        if (!mbar_wait(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer)) break;
-        mbar_arrive_expect_tx(bar_kf + 8 * ks, kTile);
-        tma_load_3d(sbase + Smem::kK + ks * kTile, &map_k, bar_kf + 8 * ks, 0, j * kBN, (int)kv);
-        if (++ks == kStages) { ks = 0; kph ^= 1; }
-        if (t >= nblk) {
-          if (!mbar_wait(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer)) { ok = false; break; }
-          mbar_arrive_expect_tx(bar_vf + 8 * vs, kTile);
-          tma_load_3d(sbase + Smem::kV + vs * kTile, &map_v, bar_vf + 8 * vs, 0, j * kBN, (int)kv);
-          if (++vs == kStages) { vs = 0; vph ^= 1; }
+      for (int it = 0; ok && get_item(p, it, &w); ++it) {
+        const uint32_t qb = it & 1;
+        if (!mbar_wait(bar_qe + 8 * qb, ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrProducer)) break;
+        mbar_arrive_expect_tx(bar_qf + 8 * qb, kTile);
+        tma_load_3d(sbase + Smem::kQ + qb * kTile, &map_q, bar_qf + 8 * qb, 0, (int)w.q0, (int)w.bh);
+        for (int t = 0; t < 2 * w.nblk; ++t) {
+          const int j = t < w.nblk ? t : t - w.nblk;
+          if (!mbar_wait(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer)) { ok = false; break; }
+          mbar_arrive_expect_tx(bar_kf + 8 * ks, kTile);
+          tma_load_3d(sbase + Smem::kK + ks * kTile, &map_k, bar_kf + 8 * ks, 0, j * kBN, (int)w.kv);
+          if (++ks == kStages) { ks = 0; kph ^= 1; }
+          if (t >= w.nblk) {
+            if (!mbar_wait(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer)) { ok = false; break; }
+            mbar_arrive_expect_tx(bar_vf + 8 * vs, kTile);
+            tma_load_3d(sbase + Smem::kV + vs * kTile, &map_v, bar_vf + 8 * vs, 0, j * kBN, (int)w.kv);
+            if (++vs == kStages) { vs = 0; vph ^= 1; }
+          }
         }
       }
     }
@@ -188,207 +276,211 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (lane == 0) {
       const uint32_t idesc_s = umma_idesc(0, 0, kBM, kBN);                      // Q, K both K-major e4m3
       const uint32_t idesc_o = umma_idesc_major(0, 0, kBM, kD, 0, 1);           // P K-major, V MN-major
-      const uint64_t qd = smem_desc_k_sw128(sbase + Smem::kQ);
-      uint32_t ks = 0, kph = 0, vs = 0, vph = 0;
-      bool ok = mbar_wait(bar_q, 0, abort_flag, p.status, kErrMma);
-      // O += P_j V_j
-      auto pv = [&](int j) {
-        const uint32_t pb = j & 1, pph = (j >> 1) & 1;
-        if (!mbar_wait(bar_pf + 8 * pb, pph, abort_flag, p.status, kErrMma)) return false;
-        if (!mbar_wait(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma)) return false;
+      // The score stream runs two tiles ahead of the P V stream; st / sit / sw = its next tile.
+      uint32_t ks = 0, kph = 0, vs = 0, vph = 0, sn = 0;   // sn: tiles issued; tile n goes to buffer n & 1
+      int st = 0, sit = 0;
+      Item sw;
+      bool more = get_item(p, 0, &sw), ok = true;
+      auto issue_s = [&]() {  // S of the next tile of the stream
+        const uint32_t sb = sn & 1, qb = sit & 1;
+        if (st == 0 && !mbar_wait(bar_qf + 8 * qb, (sit >> 1) & 1, abort_flag, p.status, kErrMma)) return false;
+        if (!mbar_wait(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma)) return false;
+        if (!mbar_wait(bar_se + 8 * sb, ((sn >> 1) & 1) ^ 1, abort_flag, p.status, kErrMma)) return false;
         tc_fence_after();
-        const uint64_t pd = smem_desc_k_sw128(sbase + Smem::kP + pb * kTile);
-        const uint64_t vd = smem_desc_mn_sw128(sbase + Smem::kV + vs * kTile, 128 * 128, 1024);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f8(tmem + 256, pd + 2 * k, vd + 256 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit(bar_ve + 8 * vs);
-        umma_commit(bar_pe + 8 * pb);
-        if (++vs == kStages) { vs = 0; vph ^= 1; }
-        return true;
-      };
-      for (int t = 0; t < 2 * nblk && ok; ++t) {
-        const uint32_t sb = t & 1, sph = (t >> 1) & 1;
-        if (!mbar_wait(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma)) break;
-        if (!mbar_wait(bar_se + 8 * sb, sph ^ 1, abort_flag, p.status, kErrMma)) break;
-        tc_fence_after();
+        const uint64_t qd = smem_desc_k_sw128(sbase + Smem::kQ + qb * kTile);
         const uint64_t kd = smem_desc_k_sw128(sbase + Smem::kK + ks * kTile);
 #pragma unroll
         for (int k = 0; k < 4; ++k) umma_f8(tmem + sb * 128, qd + 2 * k, kd + 2 * k, idesc_s, k > 0 ? 1u : 0u);
         umma_commit(bar_ke + 8 * ks);
         umma_commit(bar_sf + 8 * sb);
         if (++ks == kStages) { ks = 0; kph ^= 1; }
-        // the second product of the block before: its probabilities are ready by now
-        if (t >= nblk + 1) ok = pv(t - nblk - 1);
+        ++sn;
+        if (++st == 2 * sw.nblk) {
+          umma_commit(bar_qe + 8 * qb);  // the query tile has been read for the last time
+          st = 0;
+          more = get_item(p, ++sit, &sw);
+        }
+        return true;
+      };
+      for (int a = 0; a < 2 && more && ok; ++a) ok = issue_s();
+      uint32_t pc[2] = {0, 0};  // P tiles consumed so far, per group
+      Item w;
+      for (int it = 0; ok && get_item(p, it, &w); ++it) {
+        const uint32_t ob = it & 1, o_tmem = tmem + 256 + 128 * ob;
+        for (int t = 0; t < 2 * w.nblk && ok; ++t) {
+          if (more) ok = issue_s();
+          if (!ok || t < w.nblk) continue;
+          // O += P_j V_j
+          const int j = t - w.nblk, grp = t & 1;
+          const uint32_t pb = 2 * grp + (pc[grp] & 1), pph = (pc[grp] >> 1) & 1;
+          if (j == 0) ok = mbar_wait(bar_oe + 8 * ob, ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrMma);
+          ok = ok && mbar_wait(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma) &&
+               mbar_wait(bar_pf + 8 * pb, pph, abort_flag, p.status, kErrMma);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t pd = smem_desc_k_sw128(sbase + Smem::kP + pb * kTile);
+          const uint64_t vd = smem_desc_mn_sw128(sbase + Smem::kV + vs * kTile, 128 * 128, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f8(o_tmem, pd + 2 * k, vd + 256 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+          umma_commit(bar_ve + 8 * vs);
+          umma_commit(bar_pe + 8 * pb);
+          if (++vs == kStages) { vs = 0; vph ^= 1; }
+          ++pc[grp];
+        }
+        if (ok) umma_commit(bar_of + 8 * ob);
       }
-      if (ok && nblk > 0) ok = pv(nblk - 1);
-      if (ok) umma_commit(bar_of);
     }
   } else {
     // ------------------------------------------------------------ softmax (warps 2..9)
-    const int grp = (warp - 2) >> 2;          // 0 / 1: the score buffer (and key blocks t = grp mod 2) of this group
+    // A wait that runs out sets the abort flag, on which every later wait gives up at once: the
+    // loops below then run to their end on whatever is there, with all barriers among the softmax
+    // warps in place, and nothing is stored.
+    const int grp = (warp - 2) >> 2;          // 0 / 1: the score buffer (and tiles t = grp mod 2) of this group
     const int qtr = warp & 3;                 // TMEM lane quarter of this warp
     const int row = qtr * 32 + lane;          // query row inside the block = TMEM lane
-    const int64_t qi = q0 + row;              // query index
-    const int st = (threadIdx.x - 64) & 127;  // 0..127 inside the group
-    const int bar_id = 1 + grp;               // named barrier of the group; 3 = both groups
     const uint32_t t_lane = tmem + ((uint32_t)(qtr * 32) << 16);
-    float* stats = reinterpret_cast<float*>(smem + Smem::kRowStats);
-    float mx = kMasked;                       // row maximum, log2 domain
-    float off = 0.f;                          // log2(q_scale_s) - mx (second pass)
-    float ls[4] = {0.f, 0.f, 0.f, 0.f};       // partial row sums of the scaled probabilities
+    const uint32_t t_score = t_lane + grp * 128;
+    float* stats = reinterpret_cast<float*>(smem + Smem::kStats);
     const float lq = log2f(p.q_scale_s);
-    bool stop = false;
-    // nothing to mask in a block: no mask tensor, all of its keys exist and (causal) lie at or
-    // before the first query of this block
-    auto block_plain = [&](int j) {
-      const int64_t key0 = (int64_t)j * kBN;
-      return p.mask_kind == 0 && key0 + kBN <= p.S && (!p.causal || key0 + kBN - 1 <= q0);
-    };
-    // One key block of this group: scores -> row maximum (first pass) or e4m3 probabilities and
-    // row sum (second pass).  Returns false when a wait ran out.
-    auto do_tile = [&](int t) {
-      const bool second = t >= nblk;
-      const int j = second ? t - nblk : t;
-      const uint32_t sb = grp, sph = (t >> 1) & 1;
-      mbar_wait(bar_sf + 8 * sb, sph, abort_flag, p.status, kErrSoftmax, 32);
-      if (second && j >= 2) mbar_wait(bar_pe + 8 * (j & 1), ((j >> 1) - 1) & 1, abort_flag, p.status, kErrSoftmax, 32);
-      named_bar_sync(bar_id, 128);
-      if (st == 0) sm_stop[grp] = *abort_flag;
-      named_bar_sync(bar_id, 128);
-      if (sm_stop[grp]) return false;
-      tc_fence_after();
-      const int64_t key0 = (int64_t)j * kBN;
-      const bool plain = block_plain(j);
-      uint8_t* prow = smem + Smem::kP + (j & 1) * kTile + row * 128;
-      // the row in two halves of 64 scores: both loads of a half are in flight together
+    uint32_t sc = 0, pc = 0;                  // tiles of this group so far; P tiles so far
+    Item w;
+    for (int it = 0; get_item(p, it, &w); ++it) {
+      const int64_t qi = w.q0 + row;          // query index
+      float* st_max = stats + (it & 1) * 512;
+      float* st_sum = st_max + 256;
+      float mx = kMasked;                     // row maximum, log2 domain
+      float off = 0.f;                        // log2(q_scale_s) - mx (second pass)
+      uint64_t ls[2] = {0ull, 0ull};          // partial row sums of the scaled probabilities
+
+      // One key block of this group: scores -> row maximum (first pass) or e4m3 probabilities and
+      // row sums (second pass).
+      auto do_tile = [&](int j, auto second_tag) {
+        constexpr bool second = decltype(second_tag)::value;
+        const uint32_t pb = 2 * grp + (pc & 1);
+        const int64_t key0 = (int64_t)j * kBN;
+        uint8_t* prow = smem + Smem::kP + pb * kTile + row * 128;
+        mbar_wait(bar_sf + 8 * grp, sc & 1, abort_flag, p.status, kErrSoftmax);
+        ++sc;
+        if (second) mbar_wait(bar_pe + 8 * pb, ((pc >> 1) & 1) ^ 1, abort_flag, p.status, kErrSoftmax);
+        tc_fence_after();
+        auto release_scores = [&]() {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_se + 8 * grp);
+        };
+        // keys of the block that this row may see: the first `lim` of them
+        int64_t lim64 = (p.causal && qi + 1 < p.S ? qi + 1 : p.S) - key0;
+        const int lim = lim64 > kBN ? kBN : (int)lim64;
+        const uint64_t off2 = pack_f32x2(off, off);
+        if (p.mask_kind == 0) {
+          // the whole row is taken into registers and the score buffer handed back before any use
+          uint32_t r[128];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_score + 32 * c, r + 32 * c);
+          tmem_ld_wait();
+          release_scores();
+          float mul = p.c_log2;
+          // (the test is the same for all rows of the block, so that a warp takes one path)
+          const bool masked = key0 + kBN > p.S || (p.causal && key0 + kBN - 1 > w.q0);
+          if (masked || mul < 0.f) {
+#pragma unroll
+            for (int e = 0; e < 128; ++e) r[e] = __float_as_uint(e < lim ? __uint_as_float(r[e]) * mul : kMasked);
+            mul = 1.f;
+          }
+          if (!second) {
+            float m = kMasked;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) m = chunk_max(r + 32 * c, m);
+            mx = fmaxf(mx, m * mul);
+          } else {
+            const uint64_t mul2 = pack_f32x2(mul, mul);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) chunk_exp(r + 32 * c, c, mul2, off2, ls, prow, row);
+          }
+        } else {
+          const uint64_t one2 = pack_f32x2(1.f, 1.f);
+          const int64_t qm = qi < p.L ? qi : p.L - 1;
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-      uint32_t rr[2][32];
-      tmem_ld_32x32(t_lane + sb * 128 + half * 64, rr[0]);
-      tmem_ld_32x32(t_lane + sb * 128 + half * 64 + 32, rr[1]);
-      tmem_ld_wait();
+          for (int c = 0; c < 4; ++c) {
+            uint32_t r[32];
+            tmem_ld_32x32(t_score + 32 * c, r);
+            tmem_ld_wait();
+            if (c == 3) release_scores();
 #pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c = 2 * half + cc;
-        const uint32_t* r = rr[cc];
-        float x[32];
-        if (plain) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) x[e] = __uint_as_float(r[e]) * p.c_log2;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int64_t key = key0 + c * 32 + e;
-            float v = __uint_as_float(r[e]) * p.c_log2;
-            if (p.mask_kind) v += mask_term(p, bh, qi < p.L ? qi : p.L - 1, key < p.S ? key : p.S - 1);
-            if (key >= p.S || (p.causal && key > qi)) v = kMasked;
-            x[e] = v;
-          }
-        }
-        if (!second) {
-          float m4[4] = {mx, kMasked, kMasked, kMasked};
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            m4[0] = fmaxf(m4[0], x[e]); m4[1] = fmaxf(m4[1], x[e + 1]);
-            m4[2] = fmaxf(m4[2], x[e + 2]); m4[3] = fmaxf(m4[3], x[e + 3]);
-          }
-          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-        } else {
-          uint32_t w[8];
-#pragma unroll
-          for (int e = 0; e < 32; e += 4) {
-            float pr[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              pr[u] = ex2_approx(x[e + u] + off);  // = exp(S - max) * q_scale_s
-              ls[u] += pr[u];
+            for (int e = 0; e < 32; ++e) {
+              const int64_t key = key0 + c * 32 + e;
+              float v = __uint_as_float(r[e]) * p.c_log2 + mask_term(p, w.bh, qm, key < p.S ? key : p.S - 1);
+              r[e] = __float_as_uint(c * 32 + e < lim ? v : kMasked);
             }
-            // (the conversion saturates at 448: a probability scale beyond that cannot overflow)
-            w[e >> 2] = cvt_fp8x2<B200Q_E4M3>(pr[0], pr[1]) | (cvt_fp8x2<B200Q_E4M3>(pr[2], pr[3]) << 16);
+            if (!second) mx = chunk_max(r, mx);
+            else chunk_exp(r, c, one2, off2, ls, prow, row);
           }
-          // 32 keys = two 16-byte pieces (2c, 2c + 1) of the row, XOR-swizzled by the row
-          *reinterpret_cast<uint4*>(prow + (((2 * c) ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-          *reinterpret_cast<uint4*>(prow + (((2 * c + 1) ^ (row & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
         }
-      }
-      }
-      tc_fence_before();
-      mbar_arrive(bar_se + 8 * sb);  // the score buffer may be overwritten
-      if (second) {
-        fence_proxy_async_smem();    // the P tile is read by the tensor core (async proxy)
-        mbar_arrive(bar_pf + 8 * (j & 1));
-      }
-      return true;
-    };
-    // first pass: this group's blocks t = grp, grp + 2, ... < nblk
-    for (int t = grp; t < nblk && !stop; t += 2) stop = !do_tile(t);
-    // between the passes both groups meet (stopped or not, exactly once): the row maximum over
-    // all blocks
-    stats[grp * 128 + row] = mx;
-    named_bar_sync(3, 256);
-    mx = fmaxf(stats[row], stats[128 + row]);
-    off = lq - mx;
-    named_bar_sync(3, 256);
-    // second pass: tiles t = nblk .. 2 nblk - 1 with t = grp (mod 2)
-    for (int t = nblk + ((nblk & 1) == grp ? 0 : 1); t < 2 * nblk && !stop; t += 2) stop = !do_tile(t);
-    // ---- output: O / l, scaled.  The row sums of both groups are added, then group 0 writes the
-    // first 64 output columns of its rows and group 1 the other 64.
-    float lsum = (ls[0] + ls[1]) + (ls[2] + ls[3]);
-    if (!stop && nblk > 0) {
-      mbar_wait(bar_of, 0, abort_flag, p.status, kErrSoftmax, 64);
-      named_bar_sync(bar_id, 128);
-      if (st == 0) sm_stop[grp] = *abort_flag;
-      named_bar_sync(bar_id, 128);
-      stop = sm_stop[grp] != 0;
-    }
-    // (both groups reach these two barriers exactly once, stopped or not)
-    stats[grp * 128 + row] = lsum;
-    named_bar_sync(3, 256);
-    lsum = (stats[row] + stats[128 + row]) / p.q_scale_s;
-    if (!stop) {
+        if (second) {
+          fence_proxy_async_smem();    // the P tile is read by the tensor core (async proxy)
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_pf + 8 * pb);
+          ++pc;
+        }
+      };
+      // first pass: this group's tiles t = grp, grp + 2, ... < nblk
+      for (int t = grp; t < w.nblk; t += 2) do_tile(t, std::false_type{});
+      // between the passes the groups meet: the row maximum over all blocks
+      st_max[grp * 128 + row] = mx;
+      named_bar_sync(1, 256);
+      mx = fmaxf(st_max[row], st_max[128 + row]);
+      off = lq - mx;
+      // second pass: tiles t = nblk ... 2 nblk - 1 with t = grp (mod 2)
+      for (int j = (w.nblk & 1) == grp ? 0 : 1; j < w.nblk; j += 2) do_tile(j, std::true_type{});
+      // ---- output: O / l, scaled.  The row sums of both groups are added, then group 0 writes the
+      // first 64 output columns of its rows and group 1 the other 64.
+      float l4[4];
+      unpack_f32x2(ls[0], l4[0], l4[1]);
+      unpack_f32x2(ls[1], l4[2], l4[3]);
+      st_sum[grp * 128 + row] = (l4[0] + l4[1]) + (l4[2] + l4[3]);
+      named_bar_sync(1, 256);
+      const float lsum = (st_sum[row] + st_sum[128 + row]) / p.q_scale_s;
+      mbar_wait(bar_of + 8 * (it & 1), (it >> 1) & 1, abort_flag, p.status, kErrSoftmax);
       tc_fence_after();
       const float linv = lsum > 0.f ? 1.f / lsum : 0.f;
       const float osc = p.o_scale * linv;
       float amax_o = 0.f;
-      const bool in = qi < p.L;
-#pragma unroll 1
-      for (int c = 2 * grp; c < 2 * grp + 2; ++c) {
-        uint32_t r[32];
-        if (nblk > 0) {
-          tmem_ld_32x32(t_lane + 256 + c * 32, r);
-          tmem_ld_wait();
-        } else {
+      const bool in = qi < p.L && !*abort_flag;
+      uint32_t r[64];
+      const int c0 = 64 * grp;
+      tmem_ld_32x32(t_lane + 256 + 128 * (it & 1) + c0, r);
+      tmem_ld_32x32(t_lane + 256 + 128 * (it & 1) + c0 + 32, r + 32);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_oe + 8 * (it & 1));
+      float o[64];
 #pragma unroll
-          for (int e = 0; e < 32; ++e) r[e] = 0u;
-        }
-        float o[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          o[e] = __uint_as_float(r[e]) * osc;
-          amax_o = fmaxf(amax_o, fabsf(o[e]));
-        }
-        if (in) {
-          if (p.out_fp8) {
-            uint8_t* dst = static_cast<uint8_t*>(p.out) + (bh * p.L + qi) * kD + c * 32;
-            uint32_t w[8];
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              w[e >> 2] = cvt_fp8x2<B200Q_E4M3>(clampf<B200Q_E4M3>(o[e] * p.q_scale_o), clampf<B200Q_E4M3>(o[e + 1] * p.q_scale_o)) |
-                          (cvt_fp8x2<B200Q_E4M3>(clampf<B200Q_E4M3>(o[e + 2] * p.q_scale_o), clampf<B200Q_E4M3>(o[e + 3] * p.q_scale_o)) << 16);
-            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
-            *reinterpret_cast<uint4*>(dst + 16) = make_uint4(w[4], w[5], w[6], w[7]);
-          } else {
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + (bh * p.L + qi) * kD + c * 32;
-#pragma unroll
-            for (int e = 0; e < 32; e += 8)
-              *reinterpret_cast<uint4*>(dst + e) = make_uint4(pack_bf16x2(o[e], o[e + 1]), pack_bf16x2(o[e + 2], o[e + 3]),
-                                                            pack_bf16x2(o[e + 4], o[e + 5]), pack_bf16x2(o[e + 6], o[e + 7]));
-          }
-        }
+      for (int e = 0; e < 64; ++e) {
+        o[e] = __uint_as_float(r[e]) * osc;
+        amax_o = fmaxf(amax_o, fabsf(o[e]));
       }
-      if (in && grp == 0) {
-        if (p.m_out) p.m_out[bh * p.L + qi] = __float2bfloat16_rn(mx / kLog2e);
-        if (p.linv_out) p.linv_out[bh * p.L + qi] = __float2bfloat16_rn(linv);
+      if (in) {
+        if (p.out_fp8) {
+          uint8_t* dst = static_cast<uint8_t*>(p.out) + (w.bh * p.L + qi) * kD + c0;
+          uint32_t b[16];
+#pragma unroll
+          for (int e = 0; e < 64; e += 4)
+            b[e >> 2] = cvt_fp8x2<B200Q_E4M3>(clampf<B200Q_E4M3>(o[e] * p.q_scale_o), clampf<B200Q_E4M3>(o[e + 1] * p.q_scale_o)) |
+                        (cvt_fp8x2<B200Q_E4M3>(clampf<B200Q_E4M3>(o[e + 2] * p.q_scale_o), clampf<B200Q_E4M3>(o[e + 3] * p.q_scale_o)) << 16);
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) *reinterpret_cast<uint4*>(dst + 4 * e) = make_uint4(b[e], b[e + 1], b[e + 2], b[e + 3]);
+        } else {
+          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(p.out) + (w.bh * p.L + qi) * kD + c0;
+#pragma unroll
+          for (int e = 0; e < 64; e += 8)
+            *reinterpret_cast<uint4*>(dst + e) = make_uint4(pack_bf16x2(o[e], o[e + 1]), pack_bf16x2(o[e + 2], o[e + 3]),
+                                                          pack_bf16x2(o[e + 4], o[e + 5]), pack_bf16x2(o[e + 6], o[e + 7]));
+        }
+        if (grp == 0) {
+          if (p.m_out) p.m_out[w.bh * p.L + qi] = __float2bfloat16_rn(mx / kLog2e);
+          if (p.linv_out) p.linv_out[w.bh * p.L + qi] = __float2bfloat16_rn(linv);
+        }
       }
       // amax of the probabilities (1 / l of a row is its largest probability) and of the output
       if (p.amax_s && grp == 0) {
@@ -423,6 +515,7 @@ __global__ void __launch_bounds__(128) sdpa_fp8_plain_kernel(const uint8_t* __re
                                                              const uint8_t* __restrict__ v, int dqk, int dv, const Params p_in) {
   Params p = p_in;
   load_scales(p);
+  clear_zero_list(p);
   __shared__ float s_q[256];
   __shared__ float s_p[128];
   __shared__ float s_red[4];
@@ -530,6 +623,7 @@ int sdpa_fp8_fwd_impl(const b200q_sdpa_args& a, cudaStream_t st) {
   for (int i = 0; i < 6; ++i) { p.scale_dev[i] = devs[i]; p.scale_host[i] = hosts[i]; }
   p.d_scale_s_given = a.d_scale_s_given;
   p.softmax_scale = a.softmax_scale;
+  for (int i = 0; i < 5; ++i) { p.zero_ptr[i] = a.zero_ptr[i]; p.zero_bytes[i] = a.zero_bytes[i]; }
   p.c_log2 = p.q_scale_s = p.o_scale = p.q_scale_o = 0.f;
   p.status = device_status_ptr();
   if (!p.status) return B200Q_ERR_CUDA;
@@ -551,8 +645,9 @@ int sdpa_fp8_fwd_impl(const b200q_sdpa_args& a, cudaStream_t st) {
       B200Q_CUDA_OK(cudaFuncSetAttribute(sdpa::sdpa_fp8_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       configured[dev].store(1, std::memory_order_release);
     }
-    dim3 grid((unsigned)((L + sdpa::kBM - 1) / sdpa::kBM), (unsigned)BH);
-    sdpa::sdpa_fp8_tcgen05_kernel<<<grid, sdpa::kThreads, smem, st>>>(mq, mk, mv, p);
+    const int64_t items = ((L + sdpa::kBM - 1) / sdpa::kBM) * BH;
+    const unsigned grid = (unsigned)(items < kNumSMs ? items : kNumSMs);
+    launch_dependent(sdpa::sdpa_fp8_tcgen05_kernel, dim3(grid), dim3(sdpa::kThreads), smem, st, mq, mk, mv, p);
     B200Q_LAUNCH_CHECK();
     return B200Q_OK;
   }

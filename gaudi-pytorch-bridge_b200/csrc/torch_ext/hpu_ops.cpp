@@ -6,6 +6,7 @@
 // wrappers mirror habana_eager/eager_custom_op_register.cpp:59-322,1272-1306.  All device
 // work goes through the C ABI in b200q.h on the current CUDA stream; there is no fallback.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
@@ -53,6 +54,17 @@ bool is_fp8(at::ScalarType t) { return t == at::kFloat8_e5m2 || t == at::kFloat8
 
 void* current_stream() { return static_cast<void*>(c10::cuda::getCurrentCUDAStream().stream()); }
 
+// The host work of a call sets the pace of everything below about 20 us on the device, and a trip
+// through the dispatcher costs 0.5-1.5 us: outputs come straight from the CUDA allocator, and a
+// conversion that would change nothing is not asked for.
+at::Tensor new_tensor(c10::IntArrayRef sizes, at::ScalarType dtype, const at::Device& dev) {
+  return at::Tensor(at::detail::empty_cuda(sizes, dtype, dev, c10::nullopt));
+}
+at::Tensor on_device_as(const at::Tensor& t, const at::Device& dev, at::ScalarType dtype) {
+  return t.scalar_type() == dtype && t.device() == dev ? t : t.to(dev, dtype);
+}
+at::Tensor on_device(const at::Tensor& t, const at::Device& dev) { return t.device() == dev ? t : t.to(dev); }
+
 int64_t numel_of(c10::IntArrayRef s) {
   int64_t n = 1;
   for (auto d : s) n *= d;
@@ -75,44 +87,50 @@ struct ResolvedScale {
   int mode = B200Q_BCAST_NONE;
   float host = 1.f;
   at::Tensor dev;  // fp32, contiguous, on the problem's device (keeps the storage alive)
-  const float* ptr() const { return dev.defined() ? dev.data_ptr<float>() : nullptr; }
+  const float* ptr() const { return dev.defined() ? dev.const_data_ptr<float>() : nullptr; }
 };
 
-// Scale as an fp32 tensor of its final shape (fp8_ops.cpp:63-96), or undefined for None/float.
-at::Tensor scale_tensor(const ScaleArg& scale, OptShape scale_shape, const at::Device& dev) {
+// A scale as fp32 values in row-major order and the shape they stand for (fp8_ops.cpp:63-96).  Only the
+// pointer and the shape are ever used, so scale_shape needs no reshaped tensor.
+struct ScaleView {
+  at::Tensor t;         // fp32, contiguous; undefined for None / float
+  c10::DimVector dims;
+};
+
+ScaleView scale_view(const ScaleArg& scale, OptShape scale_shape, const at::Device& dev) {
+  ScaleView v;
   if (auto t = std::get_if<at::Tensor>(&scale)) {
-    at::Tensor s = t->to(dev, at::kFloat);
-    if (s.numel() > 1 && scale_shape.has_value() && s.sizes() != *scale_shape) s = s.reshape(*scale_shape);
-    return s;
+    v.t = on_device_as(*t, dev, at::kFloat).contiguous();
+    const bool reshaped = v.t.numel() > 1 && scale_shape.has_value();  // (validate_scale_shape has compared the sizes)
+    const auto dims = reshaped ? *scale_shape : v.t.sizes();
+    v.dims.assign(dims.begin(), dims.end());
+  } else if (auto l = std::get_if<std::vector<double>>(&scale)) {
+    v.t = at::tensor(*l, at::TensorOptions().dtype(at::kDouble)).to(at::kFloat).to(dev);
+    const auto dims = scale_shape.has_value() ? *scale_shape : v.t.sizes();
+    v.dims.assign(dims.begin(), dims.end());
   }
-  if (auto l = std::get_if<std::vector<double>>(&scale)) {
-    at::Tensor s = at::tensor(*l, at::TensorOptions().dtype(at::kDouble)).to(at::kFloat);
-    if (scale_shape.has_value()) s = s.reshape(*scale_shape);
-    return s.to(dev);
-  }
-  return at::Tensor();
+  return v;
 }
 
-// Classify how `s` (already of its final shape) broadcasts against `shape`; on return rows*cols ==
-// numel(shape) and the mode says how s lines up with that 2-D view.
-ResolvedScale classify_against(const at::Tensor& s_in, c10::IntArrayRef shape, int64_t* rows, int64_t* cols,
-                               const char* what) {
+// Classify how the scale broadcasts against `shape`; on return rows*cols == numel(shape) and the
+// mode says how it lines up with that 2-D view.
+ResolvedScale classify_against(const ScaleView& s, c10::IntArrayRef shape, int64_t* rows, int64_t* cols, const char* what) {
   ResolvedScale r;
   const int64_t n = numel_of(shape);
   *rows = 1;
   *cols = n;
-  at::Tensor s = s_in;
-  if (s.numel() == 1) {
+  if (s.t.numel() == 1) {
     r.mode = B200Q_BCAST_SCALAR_DEV;
-    r.dev = s.reshape({1}).contiguous();
+    r.dev = s.t;
     return r;
   }
-  const int64_t rank = (int64_t)shape.size();
-  TORCH_CHECK(s.dim() <= rank, what, " of shape ", s.sizes(), " does not broadcast against ", shape);
-  std::vector<int64_t> ss(rank, 1);
-  for (int64_t i = 0; i < s.dim(); ++i) ss[rank - s.dim() + i] = s.size(i);
+  const int64_t rank = (int64_t)shape.size(), srank = (int64_t)s.dims.size();
+  TORCH_CHECK(srank <= rank, what, " of shape ", c10::IntArrayRef(s.dims), " does not broadcast against ", shape);
+  c10::DimVector ss(rank, 1);
+  for (int64_t i = 0; i < srank; ++i) ss[rank - srank + i] = s.dims[i];
   for (int64_t i = 0; i < rank; ++i)
-    TORCH_CHECK(ss[i] == 1 || ss[i] == shape[i], what, " of shape ", s.sizes(), " does not broadcast against ", shape);
+    TORCH_CHECK(ss[i] == 1 || ss[i] == shape[i], what, " of shape ", c10::IntArrayRef(s.dims), " does not broadcast against ",
+                shape);
   int64_t first_full = rank, last_full = -1;
   bool all_full = true;
   for (int64_t i = 0; i < rank; ++i) {
@@ -123,7 +141,7 @@ ResolvedScale classify_against(const at::Tensor& s_in, c10::IntArrayRef shape, i
   }
   if (all_full) {
     r.mode = B200Q_BCAST_FULL;
-    r.dev = s.contiguous();
+    r.dev = s.t;
     return r;
   }
   // trailing block: ones before first_full, matches from first_full to the end
@@ -139,7 +157,7 @@ ResolvedScale classify_against(const at::Tensor& s_in, c10::IntArrayRef shape, i
     for (int64_t i = first_full; i < rank; ++i) *cols *= shape[i];
     *rows = n / *cols;
     r.mode = B200Q_BCAST_PER_COL;
-    r.dev = s.contiguous().reshape({*cols});
+    r.dev = s.t;
     return r;
   }
   if (leading && last_full >= 0) {
@@ -147,11 +165,11 @@ ResolvedScale classify_against(const at::Tensor& s_in, c10::IntArrayRef shape, i
     for (int64_t i = 0; i <= last_full; ++i) *rows *= shape[i];
     *cols = n / *rows;
     r.mode = B200Q_BCAST_PER_ROW;
-    r.dev = s.contiguous().reshape({*rows});
+    r.dev = s.t;
     return r;
   }
   r.mode = B200Q_BCAST_FULL;  // mixed pattern: materialise
-  r.dev = s.reshape(ss).expand(shape).contiguous();
+  r.dev = s.t.reshape(ss).expand(shape).contiguous();
   return r;
 }
 
@@ -167,7 +185,13 @@ ResolvedScale resolve_cast_scale(const ScaleArg& scale, OptShape scale_shape, co
     r.host = (float)*d;
     return r;
   }
-  return classify_against(scale_tensor(scale, scale_shape, input.device()), input.sizes(), rows, cols, "scale");
+  return classify_against(scale_view(scale, scale_shape, input.device()), input.sizes(), rows, cols, "scale");
+}
+
+// 0-dim fp32 for a requested amax, else the empty [0] tensor
+at::Tensor amax_tensor(bool is_amax, const at::Device& dev) {
+  if (is_amax) return new_tensor({}, at::kFloat, dev);
+  return new_tensor({0}, at::kFloat, dev);
 }
 
 // ------------------------------------------------------------------ cast_to_fp8_v2
@@ -188,8 +212,8 @@ std::tuple<at::Tensor, at::Tensor> cast_to_fp8_v2_common(const at::Tensor& input
   at::Tensor in = input.contiguous();
   int64_t rows, cols;
   ResolvedScale s = resolve_cast_scale(scale, scale_shape, in, &rows, &cols);
-  at::Tensor out = at::empty(in.sizes(), in.options().dtype(dtype));
-  at::Tensor amax = is_amax ? at::empty({}, in.options().dtype(at::kFloat)) : at::empty({0}, in.options().dtype(at::kFloat));
+  at::Tensor out = new_tensor(in.sizes(), dtype, in.device());
+  at::Tensor amax = amax_tensor(is_amax, in.device());
   uint64_t seed = (uint64_t)g_sr_seed.load(), offset = 0;
   if (stochastic_rounding && !fp8_in) offset = (uint64_t)g_sr_offset.fetch_add(1);
   int flags = g_mul_in_fp32.load() ? B200Q_CAST_MUL_IN_FP32 : 0;
@@ -246,7 +270,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> cast_to_fp8_hybrid(const at::Tens
     *mode = B200Q_BCAST_NONE;
     if (!s.has_value() || !s->defined()) return nullptr;
     TORCH_CHECK(s->numel() == 1, "CastToFp8Hybrid scales must have one element, got ", s->sizes());
-    keep = s->to(in.device(), at::kFloat).reshape({1}).contiguous();
+    keep = on_device_as(*s, in.device(), at::kFloat);
     *mode = B200Q_BCAST_SCALAR_DEV;
     return keep.data_ptr<float>();
   };
@@ -254,9 +278,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> cast_to_fp8_hybrid(const at::Tens
   int m152, m143;
   const float* p152 = one_scale(scale_152, k152, &m152);
   const float* p143 = one_scale(scale_143, k143, &m143);
-  at::Tensor o152 = at::empty(in.sizes(), in.options().dtype(at::kFloat8_e5m2));
-  at::Tensor o143 = at::empty(in.sizes(), in.options().dtype(at::kFloat8_e4m3fn));
-  at::Tensor amax = is_amax ? at::empty({}, in.options().dtype(at::kFloat)) : at::empty({0}, in.options().dtype(at::kFloat));
+  at::Tensor o152 = new_tensor(in.sizes(), at::kFloat8_e5m2, in.device());
+  at::Tensor o143 = new_tensor(in.sizes(), at::kFloat8_e4m3fn, in.device());
+  at::Tensor amax = amax_tensor(is_amax, in.device());
   uint64_t seed = (uint64_t)g_sr_seed.load(), offset = 0;
   if (stochastic_rounding) offset = (uint64_t)g_sr_offset.fetch_add(1);
   check_status(b200q_cast_to_fp8_hybrid(in.data_ptr(), to_b200q_dtype(src), o152.data_ptr(), o143.data_ptr(), p152, 1.f, m152,
@@ -279,7 +303,7 @@ at::Tensor cast_from_fp8_common(const at::Tensor& input, const ScaleArg& scale, 
   at::Tensor in = input.contiguous();
   int64_t rows, cols;
   ResolvedScale s = resolve_cast_scale(scale, scale_shape, in, &rows, &cols);
-  at::Tensor out = at::empty(in.sizes(), in.options().dtype(out_dtype));
+  at::Tensor out = new_tensor(in.sizes(), out_dtype, in.device());
   check_status(b200q_cast_from_fp8(in.data_ptr(), to_b200q_dtype(in.scalar_type()), out.data_ptr(),
                                    to_b200q_dtype(out_dtype), s.ptr(), s.host, s.mode, rows, cols, current_stream()),
                "cast_from_fp8");
@@ -313,7 +337,7 @@ at::Tensor convert_from_4bit(const at::Tensor& input, const at::Tensor& scale, c
   const int64_t cols_packed = in.size(-1), cols = cols_packed * 8;
   const int64_t rows = cols_packed ? in.numel() / cols_packed : 0;
   // scale: out_dtype, either the full output shape or [..., K/g, N]
-  at::Tensor sc = scale.to(in.device(), out_dtype).contiguous();
+  at::Tensor sc = on_device_as(scale, in.device(), out_dtype).contiguous();
   int64_t scale_rows = rows;
   if (sc.sizes() != c10::IntArrayRef(out_shape)) {
     bool grouped = sc.dim() == (int64_t)out_shape.size() && sc.dim() >= 2 && sc.size(-1) == cols &&
@@ -329,17 +353,17 @@ at::Tensor convert_from_4bit(const at::Tensor& input, const at::Tensor& scale, c
   if (zero_point.has_value() && zero_point->defined()) {
     if (zero_point->scalar_type() == at::kInt) {
       zp_kind = B200Q_ZP_PACKED;
-      zp = zero_point->to(in.device()).contiguous();
+      zp = on_device(*zero_point, in.device()).contiguous();
       TORCH_CHECK(zp.numel() == scale_rows * cols_packed, "packed zero_point must have the scale's shape with the last "
                   "dimension divided by 8, got ", zp.sizes(), " for scale ", sc.sizes());
     } else {
       zp_kind = B200Q_ZP_FLOAT;
-      zp = zero_point->to(in.device(), out_dtype);
+      zp = on_device_as(*zero_point, in.device(), out_dtype);
       if (zp.numel() != scale_rows * cols) zp = zp.expand(sc.sizes());
       zp = zp.contiguous();
     }
   }
-  at::Tensor out = at::empty(out_shape, in.options().dtype(out_dtype));
+  at::Tensor out = new_tensor(out_shape, out_dtype, in.device());
   check_status(b200q_dequant_int4(in.data_ptr<int32_t>(), sc.data_ptr(), zp.defined() ? zp.data_ptr() : nullptr, zp_kind,
                                   is_signed ? 1 : 0, to_b200q_dtype(out_dtype), out.data_ptr(), rows, cols_packed,
                                   scale_rows, 0, current_stream()),
@@ -361,7 +385,7 @@ at::Tensor dequant_kpacked(const at::Tensor& qweight, const at::Tensor& scales, 
   c10::cuda::CUDAGuard guard(qweight.device());
   at::Tensor q = qweight.contiguous();
   const int64_t K = q.size(0) * 8, N = q.size(1);
-  at::Tensor sc = scales.to(q.device(), out_dtype).contiguous();
+  at::Tensor sc = on_device_as(scales, q.device(), out_dtype).contiguous();
   TORCH_CHECK(sc.dim() == 2 && sc.size(1) == N && K % sc.size(0) == 0, "scales must be [K/g, N]");
   at::Tensor zp;
   int zp_kind = B200Q_ZP_NONE;
@@ -370,7 +394,7 @@ at::Tensor dequant_kpacked(const at::Tensor& qweight, const at::Tensor& scales, 
     TORCH_CHECK(zp.scalar_type() == at::kInt && zp.numel() == sc.size(0) * (N / 8), "qzeros must be int32 [K/g, N/8]");
     zp_kind = B200Q_ZP_PACKED;
   }
-  at::Tensor out = at::empty({K, N}, q.options().dtype(out_dtype));
+  at::Tensor out = new_tensor({K, N}, out_dtype, q.device());
   check_status(b200q_dequant_int4(q.data_ptr<int32_t>(), sc.data_ptr(), zp.defined() ? zp.data_ptr() : nullptr, zp_kind, 0,
                                   to_b200q_dtype(out_dtype), out.data_ptr(), K, N, sc.size(0), 1, current_stream()),
                "dequant_kpacked");
@@ -439,24 +463,23 @@ struct EpiOperand {
 
 // Line a scale / bias tensor up with the output, seen canonically as bshape + [M, N]
 // (has_m / has_n say whether the output really has those dimensions: 1-D operands drop them).
-EpiOperand classify_epi(const at::Tensor& t_in, c10::IntArrayRef bshape, int64_t M, int64_t N, bool has_m, bool has_n,
-                        c10::IntArrayRef out_shape, bool want_float, const char* what) {
-  EpiOperand e;
-  at::Tensor t = want_float ? t_in.to(at::kFloat) : t_in;
+EpiOperand classify_epi(const at::Tensor& t, c10::IntArrayRef dims, c10::IntArrayRef bshape, int64_t M, int64_t N, bool has_m,
+                        bool has_n, c10::IntArrayRef out_shape, const char* what) {
+  EpiOperand e;  // t: contiguous values standing for shape `dims`
   if (t.numel() == 1) {
     e.mode = B200Q_BCAST_SCALAR_DEV;
-    e.t = t.reshape({1}).contiguous();
+    e.t = t;
     return e;
   }
-  const int64_t orank = (int64_t)out_shape.size();
-  TORCH_CHECK(t.dim() <= orank, what, " of shape ", t.sizes(), " does not broadcast against the output ", out_shape);
+  const int64_t orank = (int64_t)out_shape.size(), trank = (int64_t)dims.size();
+  TORCH_CHECK(trank <= orank, what, " of shape ", dims, " does not broadcast against the output ", out_shape);
   // right-align with the output, then insert the dropped M / N dimensions as size 1
-  std::vector<int64_t> ts(orank, 1);
-  for (int64_t i = 0; i < t.dim(); ++i) ts[orank - t.dim() + i] = t.size(i);
+  c10::DimVector ts(orank, 1);
+  for (int64_t i = 0; i < trank; ++i) ts[orank - trank + i] = dims[i];
   for (int64_t i = 0; i < orank; ++i)
-    TORCH_CHECK(ts[i] == 1 || ts[i] == out_shape[i], what, " of shape ", t.sizes(),
-                " does not broadcast against the output ", out_shape);
-  std::vector<int64_t> can(ts.begin(), ts.begin() + (int64_t)bshape.size());
+    TORCH_CHECK(ts[i] == 1 || ts[i] == out_shape[i], what, " of shape ", dims, " does not broadcast against the output ",
+                out_shape);
+  c10::DimVector can(ts.begin(), ts.begin() + (int64_t)bshape.size());
   int64_t pos = (int64_t)bshape.size();
   can.push_back(has_m ? ts[pos++] : 1);
   can.push_back(has_n ? ts[pos++] : 1);
@@ -465,12 +488,12 @@ EpiOperand classify_epi(const at::Tensor& t_in, c10::IntArrayRef bshape, int64_t
   const int64_t tm = can[can.size() - 2], tn = can[can.size() - 1];
   if (batch_ones && tm == 1 && tn == N) {
     e.mode = B200Q_BCAST_PER_COL;
-    e.t = t.reshape({N}).contiguous();
+    e.t = t;
     return e;
   }
   if (batch_ones && tn == 1 && tm == M) {
     e.mode = B200Q_BCAST_PER_ROW;
-    e.t = t.reshape({M}).contiguous();
+    e.t = t;
     return e;
   }
   std::vector<int64_t> full(bshape.begin(), bshape.end());
@@ -517,7 +540,7 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
   const int64_t N = tb ? b.size(-2) : b.size(-1);
   // batch dims
   std::vector<int64_t> bshape;
-  {
+  if (a.dim() > 2 || b.dim() > 2) {
     auto ab = a.sizes().slice(0, a.dim() - 2), bb = b.sizes().slice(0, b.dim() - 2);
     bshape = at::infer_size(ab, bb);
   }
@@ -525,7 +548,7 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
   const bool fused_cast = out8_dtype != at::ScalarType::Undefined;
   at::Tensor out8_scale_keep;
   TORCH_CHECK(!fused_cast || is_fp8(out8_dtype), "fp8_gemm_cast: the output dtype must be float8_e5m2 or float8_e4m3fn");
-  at::Tensor out = at::empty(out_shape, A.options().dtype(fused_cast ? out8_dtype : out_dtype));
+  at::Tensor out = new_tensor(out_shape, fused_cast ? out8_dtype : out_dtype, A.device());
   if (out.numel() == 0) return out;
 
   b200q_gemm_args g{};
@@ -535,7 +558,7 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
     g.out8_scale_host = (float)out8_scale;
     if (out8_scale_dev.has_value() && out8_scale_dev->defined()) {  // a device scalar: no read-back to the host
       TORCH_CHECK(out8_scale_dev->numel() == 1, "the output scale must have one element");
-      out8_scale_keep = out8_scale_dev->to(A.device(), at::kFloat).reshape({1}).contiguous();
+      out8_scale_keep = on_device_as(*out8_scale_dev, A.device(), at::kFloat);
       g.out8_scale = out8_scale_keep.data_ptr<float>();
     }
     if (out8_amax) {
@@ -598,9 +621,9 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
     *mode = B200Q_BCAST_NONE; *dev = nullptr; *host = 1.f;
     if (std::holds_alternative<std::monostate>(s)) return;
     if (auto d = std::get_if<double>(&s)) { *mode = B200Q_BCAST_SCALAR_HOST; *host = (float)*d; return; }
-    at::Tensor t = scale_tensor(s, shape, A.device());
-    EpiOperand e = classify_epi(t, bshape, M, N, has_m, has_n, out_shape, true, "scale");
-    if (folded && e.mode == B200Q_BCAST_PER_ROW) e.t = e.t.repeat({batch});
+    const ScaleView v = scale_view(s, shape, A.device());
+    EpiOperand e = classify_epi(v.t, v.dims, bshape, M, N, has_m, has_n, out_shape, "scale");
+    if (folded && e.mode == B200Q_BCAST_PER_ROW) e.t = e.t.reshape({M}).repeat({batch});
     if (e.mode == B200Q_BCAST_FULL) {
       TORCH_CHECK(folded || batch == 1, "fp8_gemm_v2: an element-wise scale with batched operands is not supported");
     }
@@ -610,22 +633,24 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
   setup_scale(A_scale_inv, c10::nullopt, &g.a_scale, &g.a_scale_host, &g.a_scale_mode);
   setup_scale(B_scale_inv, B_scale_shape, &g.b_scale, &g.b_scale_host, &g.b_scale_mode);
   if (bias.has_value() && bias->defined()) {
-    at::Tensor bt = bias->to(A.device());
+    at::Tensor bt = on_device(*bias, A.device());
     if (bt.scalar_type() != at::kFloat && bt.scalar_type() != at::kBFloat16) bt = bt.to(at::kFloat);
-    EpiOperand e = classify_epi(bt, bshape, M, N, has_m, has_n, out_shape, false, "bias");
+    bt = bt.contiguous();
+    EpiOperand e = classify_epi(bt, bt.sizes(), bshape, M, N, has_m, has_n, out_shape, "bias");
     if (e.mode == B200Q_BCAST_SCALAR_DEV) {  // one value: treat as a per-column vector
-      e.t = e.t.expand({N}).contiguous();
+      e.t = e.t.reshape({1}).expand({N}).contiguous();
       e.mode = B200Q_BCAST_PER_COL;
     }
-    if (folded && e.mode == B200Q_BCAST_PER_ROW) e.t = e.t.repeat({batch});
+    if (folded && e.mode == B200Q_BCAST_PER_ROW) e.t = e.t.reshape({M}).repeat({batch});
     keep.push_back(e.t);
     g.bias = e.t.data_ptr(); g.bias_dtype = to_b200q_dtype(e.t.scalar_type()); g.bias_mode = e.mode;
     g.bias_ld = N; g.bias_batch_stride = folded ? 0 : M * N;
   }
   if (accumulate) {
-    at::Tensor d = D->to(A.device());
+    at::Tensor d = on_device(*D, A.device());
     if (d.scalar_type() != at::kFloat && d.scalar_type() != at::kBFloat16) d = d.to(at::kFloat);
-    d = d.expand(out_shape).contiguous();
+    if (d.sizes() != c10::IntArrayRef(out_shape)) d = d.expand(out_shape);
+    d = d.contiguous();
     keep.push_back(d);
     g.D = d.data_ptr(); g.d_dtype = to_b200q_dtype(d.scalar_type()); g.ldd = N; g.d_batch_stride = folded ? 0 : M * N;
   }
@@ -717,7 +742,7 @@ struct SdpaScale {
 static SdpaScale sdpa_scale(const OptTensor& t, const at::Device& d) {
   SdpaScale s;
   if (t.has_value() && t->defined() && t->numel() > 0) {
-    s.dev = t->to(d, at::kFloat).reshape(-1).slice(0, 0, 1).contiguous();
+    s.dev = on_device_as(*t, d, at::kFloat);  // (its first element is the one that is read)
     s.given = true;
   }
   return s;
@@ -771,14 +796,26 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tenso
   std::vector<int64_t> stat_shape(q.sizes().begin(), q.sizes().end() - 1);
   stat_shape.push_back(1);
   const bool fp8_out = q_o.given;
-  at::Tensor out = at::empty(out_shape, q.options().dtype(fp8_out ? at::kFloat8_e4m3fn : at::kBFloat16));
-  at::Tensor m = requires_backward ? at::empty(stat_shape, q.options().dtype(at::kBFloat16)) : at::zeros({1}, q.options().dtype(at::kBFloat16));
-  at::Tensor linv = requires_backward ? at::empty(stat_shape, q.options().dtype(at::kBFloat16)) : at::zeros({1}, q.options().dtype(at::kBFloat16));
-  at::Tensor seed = at::zeros({1}, q.options().dtype(at::kInt));
-  at::Tensor amax_s = at::zeros({1}, q.options().dtype(at::kFloat)), amax_o = at::zeros({1}, q.options().dtype(at::kFloat));
-  if (out.numel() == 0) return {out, m, linv, seed, amax_s, amax_o};
-
+  const auto dev = q.device();
+  at::Tensor out = new_tensor(out_shape, fp8_out ? at::kFloat8_e4m3fn : at::kBFloat16, dev);
+  const bool empty = out.numel() == 0;
   b200q_sdpa_args a{};
+  int zeros = 0;
+  // a one-element result that is zero: cleared by the attention kernel itself, not by a launch of its own
+  auto zero1 = [&](at::ScalarType t) {
+    if (empty) return at::zeros({1}, q.options().dtype(t));
+    at::Tensor z = new_tensor({1}, t, dev);
+    a.zero_ptr[zeros] = z.data_ptr();
+    a.zero_bytes[zeros++] = (int)z.element_size();
+    return z;
+  };
+  at::Tensor m = requires_backward ? new_tensor(stat_shape, at::kBFloat16, dev) : zero1(at::kBFloat16);
+  at::Tensor linv = requires_backward ? new_tensor(stat_shape, at::kBFloat16, dev) : zero1(at::kBFloat16);
+  at::Tensor seed = zero1(at::kInt);
+  at::Tensor amax_s = is_amax_s ? at::zeros({1}, q.options().dtype(at::kFloat)) : zero1(at::kFloat);
+  at::Tensor amax_o = is_amax_o ? at::zeros({1}, q.options().dtype(at::kFloat)) : zero1(at::kFloat);
+  if (empty) return {out, m, linv, seed, amax_s, amax_o};
+
   a.q = qc.data_ptr(); a.k = kc.data_ptr(); a.v = vc.data_ptr(); a.out = out.data_ptr();
   a.out_dtype = fp8_out ? B200Q_E4M3 : B200Q_BF16;
   a.BH = BH; a.L = L; a.S = S; a.dqk = (int)D; a.dv = (int)Dv; a.kv_rep = kv_rep;
@@ -815,7 +852,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tenso
   float* hosts[6] = {&a.d_scale_q_host, &a.d_scale_k_host, &a.d_scale_v_host, &a.q_scale_s_host, &a.q_scale_o_host, &a.d_scale_s_host};
   for (int i = 0; i < 6; ++i) {
     *hosts[i] = sc[i]->given ? sc[i]->host : 1.f;
-    *devs[i] = sc[i]->dev.defined() ? sc[i]->dev.data_ptr<float>() : nullptr;
+    *devs[i] = sc[i]->dev.defined() ? sc[i]->dev.const_data_ptr<float>() : nullptr;
   }
   a.d_scale_s_given = d_s.given ? 1 : 0;
   if (requires_backward) { a.m_out = m.data_ptr(); a.linv_out = linv.data_ptr(); }
@@ -881,7 +918,7 @@ at::Tensor w4a16_gemm(const at::Tensor& x, const at::Tensor& qweight, const at::
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && x.dim() == 2, "w4a16_gemm: x must be bf16 [M, K]");
   TORCH_CHECK(qweight.scalar_type() == at::kInt && qweight.dim() == 2, "w4a16_gemm: qweight must be int32 2-D");
   c10::cuda::CUDAGuard guard(x.device());
-  at::Tensor xc = x.contiguous(), q = qweight.contiguous(), sc = scales.to(at::kBFloat16).contiguous();
+  at::Tensor xc = x.contiguous(), q = qweight.contiguous(), sc = on_device_as(scales, scales.device(), at::kBFloat16).contiguous();
   const int64_t M = xc.size(0), K = xc.size(1);
   const int64_t N = k_packed ? q.size(1) : q.size(1) * 8;
   TORCH_CHECK((k_packed ? q.size(0) * 8 : q.size(0)) == K, "w4a16_gemm: qweight does not match K = ", K);
@@ -894,7 +931,7 @@ at::Tensor w4a16_gemm(const at::Tensor& x, const at::Tensor& qweight, const at::
     TORCH_CHECK(zp.scalar_type() == at::kInt && zp.numel() == sc.size(0) * (N / 8), "w4a16_gemm: qzeros must be int32 [K/group, N/8]");
     zp_kind = B200Q_ZP_PACKED;
   }
-  at::Tensor out = at::empty({M, N}, xc.options().dtype(out_dtype));
+  at::Tensor out = new_tensor({M, N}, out_dtype, xc.device());
   if (k_packed && M > 16) {
     // The AutoGPTQ layout [K/8, N] is read directly only by the few-token kernel; more tokens go
     // through one repack pass into the operator layout [K, N/8] (a weight-sized copy: callers
@@ -908,7 +945,7 @@ at::Tensor w4a16_gemm(const at::Tensor& x, const at::Tensor& qweight, const at::
   }
   const size_t ws_bytes = b200q_w4a16_workspace_bytes(M, N, K);
   at::Tensor ws;
-  if (ws_bytes) ws = at::empty({(int64_t)ws_bytes}, xc.options().dtype(at::kByte));
+  if (ws_bytes) ws = new_tensor({(int64_t)ws_bytes}, at::kByte, xc.device());
   check_status(b200q_w4a16_gemm(xc.data_ptr(), K, q.data_ptr<int32_t>(), sc.data_ptr(),
                                 zp.defined() ? zp.data_ptr<int32_t>() : nullptr, zp_kind, k_packed ? 1 : 0, M, N, K,
                                 group_size, out.data_ptr(), to_b200q_dtype(out_dtype), N,
@@ -916,8 +953,6 @@ at::Tensor w4a16_gemm(const at::Tensor& x, const at::Tensor& qweight, const at::
                "w4a16_gemm");
   return out;
 }
-
-std::tuple<at::Tensor, at::Tensor> swiglu_cast_fp8(const at::Tensor& gate, const at::Tensor& up, double scale, bool is_amax);
 
 // Gate / up projection GEMM with the SwiGLU + cast in its epilogue.  w_gate_up: e4m3 [2f, d] with
 // gate and up rows interleaved in blocks of 128 (rows [256 b, 256 b + 128) gate, next 128 up, of
@@ -932,7 +967,7 @@ at::Tensor fp8_gemm_swiglu_cast(const at::Tensor& x8, const at::Tensor& w_gate_u
   c10::cuda::CUDAGuard guard(x8.device());
   const int64_t M = x8.size(0), N = w_gate_up.size(0), K = x8.size(1), F = N / 2;
   at::Tensor a = x8.contiguous(), b = w_gate_up.contiguous();
-  at::Tensor out = at::empty({M, F}, x8.options().dtype(at::kFloat8_e4m3fn));
+  at::Tensor out = new_tensor({M, F}, at::kFloat8_e4m3fn, x8.device());
   if (out.numel() == 0) return out;
   b200q_gemm_args g{};
   g.A = a.data_ptr(); g.B = b.data_ptr();
@@ -943,12 +978,12 @@ at::Tensor fp8_gemm_swiglu_cast(const at::Tensor& x8, const at::Tensor& w_gate_u
   at::Tensor sa, sb;
   if (x_scale_inv.has_value() && x_scale_inv->defined()) {
     TORCH_CHECK(x_scale_inv->numel() == 1, "fp8_gemm_swiglu_cast: x_scale_inv must have one element");
-    sa = x_scale_inv->to(at::kFloat).contiguous();
+    sa = on_device_as(*x_scale_inv, x8.device(), at::kFloat).contiguous();
     g.a_scale = sa.data_ptr<float>(); g.a_scale_mode = B200Q_BCAST_SCALAR_DEV;
   }
   if (w_scale_inv.has_value() && w_scale_inv->defined()) {
     TORCH_CHECK(w_scale_inv->numel() == 1 || w_scale_inv->numel() == N, "fp8_gemm_swiglu_cast: w_scale_inv must have 1 or 2f elements");
-    sb = w_scale_inv->to(at::kFloat).contiguous();
+    sb = on_device_as(*w_scale_inv, x8.device(), at::kFloat).contiguous();
     g.b_scale = sb.data_ptr<float>(); g.b_scale_mode = sb.numel() == 1 ? B200Q_BCAST_SCALAR_DEV : B200Q_BCAST_PER_COL;
   }
   g.out8_dtype = B200Q_E4M3; g.out8_scale = nullptr; g.out8_scale_host = (float)act_scale;
@@ -956,13 +991,17 @@ at::Tensor fp8_gemm_swiglu_cast(const at::Tensor& x8, const at::Tensor& w_gate_u
   g.stream = current_stream();
   const int rc = b200q_fp8_gemm(&g);
   if (rc == B200Q_ERR_UNSUPPORTED) {
-    // no fused kernel for this shape: the two operators, on the de-interleaved halves
-    std::vector<int64_t> one_n{1, N};
-    at::Tensor gu = fp8_gemm_v2(a, false, b, true, c10::nullopt, at::kBFloat16, x_scale_inv, w_scale_inv, c10::nullopt, false,
-                                sb.defined() && sb.numel() == N ? OptShape(at::IntArrayRef(one_n)) : OptShape(c10::nullopt));
-    at::Tensor v = gu.view({M, F / 128, 2, 128});
-    at::Tensor gate = v.select(2, 0).reshape({M, F}), up = v.select(2, 1).reshape({M, F});
-    return std::get<0>(swiglu_cast_fp8(gate, up, act_scale, false));
+    // no fused kernel for this shape: the two kernels one after the other.  The interleaved [M, 2f]
+    // result is [M f / 128] rows of 128 gate and 128 up values: the activation kernel reads it as it is.
+    at::Tensor gu = new_tensor({M, N}, at::kBFloat16, x8.device());
+    g.out = gu.data_ptr(); g.ldo = N;
+    g.out8_dtype = 0; g.swiglu = 0;
+    check_status(b200q_fp8_gemm(&g), "fp8_gemm_swiglu_cast (gemm)");
+    const auto* gate = static_cast<const c10::BFloat16*>(gu.const_data_ptr());
+    check_status(b200q_swiglu_cast_fp8(gate, 256, gate + 128, 256, out.data_ptr(), (float)act_scale, M * (F / 128), 128, nullptr,
+                                       current_stream()),
+                 "fp8_gemm_swiglu_cast");
+    return out;
   }
   check_status(rc, "fp8_gemm_swiglu_cast");
   return out;
@@ -974,8 +1013,8 @@ std::tuple<at::Tensor, at::Tensor> swiglu_cast_fp8(const at::Tensor& gate, const
                   gate.sizes() == up.sizes() && gate.stride(1) == 1 && up.stride(1) == 1,
               "swiglu_cast_fp8: gate/up must be bf16 [rows, cols] with unit inner stride");
   c10::cuda::CUDAGuard guard(gate.device());
-  at::Tensor out = at::empty(gate.sizes(), gate.options().dtype(at::kFloat8_e4m3fn));
-  at::Tensor amax = is_amax ? at::empty({}, gate.options().dtype(at::kFloat)) : at::empty({0}, gate.options().dtype(at::kFloat));
+  at::Tensor out = new_tensor(gate.sizes(), at::kFloat8_e4m3fn, gate.device());
+  at::Tensor amax = amax_tensor(is_amax, gate.device());
   check_status(b200q_swiglu_cast_fp8(gate.data_ptr(), gate.stride(0), up.data_ptr(), up.stride(0), out.data_ptr(),
                                      (float)scale, gate.size(0), gate.size(1),
                                      is_amax ? amax.data_ptr<float>() : nullptr, current_stream()),
@@ -995,7 +1034,7 @@ static SoftmaxScale softmax_scale(const OptTensor& t, const at::Tensor& like) {
   if (t.has_value() && t->defined()) {
     TORCH_CHECK(t->scalar_type() == at::kFloat, "Input scale must be of dtype: ", at::kFloat);
     TORCH_CHECK(t->numel() == 1, "softmax_fp8 scales must have one element");
-    s.keep = t->to(like.device()).contiguous();
+    s.keep = on_device(*t, like.device()).contiguous();
     s.dev = s.keep.data_ptr<float>();
     s.given = true;
   }
@@ -1029,7 +1068,7 @@ at::Tensor softmax_fp8_common(const at::Tensor& input, int64_t dim, const Softma
   c10::cuda::CUDAGuard guard(input.device());
   at::Tensor in = input.contiguous();
   const bool fp8_out = in_s.given;
-  at::Tensor out = at::empty(in.sizes(), in.options().dtype(fp8_out ? at::kFloat8_e4m3fn : at::kBFloat16));
+  at::Tensor out = new_tensor(in.sizes(), fp8_out ? at::kFloat8_e4m3fn : at::kBFloat16, in.device());
   at::Tensor fa;
   std::vector<int64_t> lead(in.sizes().begin(), in.sizes().end() - 1), fa_strides(lead.size(), 0);
   if (fused_add.has_value() && fused_add->defined()) {
@@ -1108,9 +1147,9 @@ at::Tensor sum_fp8(const at::Tensor& self, at::OptionalIntArrayRef dim, bool kee
     for (int64_t d : kept) outer *= self.size(d);
     for (int64_t d : reduced) reduce *= self.size(d);
   }
-  at::Tensor out = at::empty(out_shape, self.options().dtype(odt));
+  at::Tensor out = new_tensor(out_shape, odt, self.device());
   const size_t ws_bytes = b200q_sum_fp8_workspace_bytes(outer, reduce, inner);
-  at::Tensor ws = at::empty({(int64_t)((ws_bytes + 3) / 4)}, self.options().dtype(at::kFloat));
+  at::Tensor ws = new_tensor({(int64_t)((ws_bytes + 3) / 4)}, at::kFloat, self.device());
   check_status(b200q_sum_fp8(src.data_ptr(), to_b200q_dtype(self.scalar_type()), out.data_ptr(), to_b200q_dtype(odt), outer, reduce,
                              inner, ws.data_ptr(), ws_bytes, current_stream()),
                "sum_fp8");
@@ -1247,7 +1286,7 @@ at::Tensor amax_op(const at::Tensor& input) {
   TORCH_CHECK(input.scalar_type() == at::kFloat || input.scalar_type() == at::kBFloat16, "amax: input must be float or bfloat16");
   c10::cuda::CUDAGuard guard(input.device());
   at::Tensor in = input.contiguous();
-  at::Tensor amax = at::empty({}, in.options().dtype(at::kFloat));
+  at::Tensor amax = new_tensor({}, at::kFloat, in.device());
   check_status(b200q_amax(in.data_ptr(), to_b200q_dtype(in.scalar_type()), in.numel(), amax.data_ptr<float>(), current_stream()), "amax");
   return amax;
 }

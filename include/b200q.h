@@ -291,6 +291,11 @@ typedef struct b200q_sdpa_args {
   float *amax_s, *amax_o;
   int force_plain;
   void* stream;
+  /* Up to five small device buffers the kernel clears (zero_bytes[i] bytes each; a NULL ends the list): the
+   * statistics of a call that asks for none are returned as zeros and need no launches of their own.
+   * amax_s / amax_o, which are accumulated into, must not be among them. */
+  void* zero_ptr[5];
+  int zero_bytes[5];
 } b200q_sdpa_args;
 
 int b200q_fp8_sdpa_fwd(const b200q_sdpa_args* args);

@@ -340,3 +340,30 @@ def test_hybrid_cast_matches_reference_emulation_and_oracle(ops):
 
 def _c(t):
     return None if t is None else t.cuda()
+
+
+@pytest.mark.parametrize("fill", ["random", "zeros", "nan"])
+@pytest.mark.parametrize("stochastic", [False, True])
+@pytest.mark.parametrize("n", [1, 255, 16 * 256 * 2 + 1, 1 << 18, (1 << 18) + 1, 1 << 22, (1 << 22) + 5])
+def test_amax_launch_forms(ops, n, stochastic, fill):
+    """The three ways an amax is taken -- inside one cluster, behind a memset, behind the clearing kernel --
+    on both sides of the sizes where they change, twice in a row (a word that was not cleared would show)."""
+    g = torch.Generator().manual_seed(n)
+    x = (torch.randn(n, generator=g) * 3).to(torch.bfloat16)
+    if fill == "zeros":
+        x.zero_()
+    elif fill == "nan":
+        x[n // 2] = float("nan")
+    big = (x.float() * 2).to(torch.bfloat16).cuda()
+    xc = x.cuda()
+    for _ in range(2):
+        _, amax_big = torch.ops.hpu.cast_to_fp8_v2(big, None, stochastic, True, torch.float8_e5m2)
+        out, amax = torch.ops.hpu.cast_to_fp8_v2(xc, None, stochastic, True, torch.float8_e5m2)
+        for a, t in ((amax_big, big), (amax, xc)):
+            want = t.abs().max().float()
+            assert torch.equal(a, want) or (fill == "nan" and torch.isnan(a) and torch.isnan(want))
+    if not stochastic:
+        ref, _ = O.cast_to_fp8_v2(x, None, False, False, torch.float8_e5m2)
+        assert torch.equal(out.cpu().view(torch.uint8), ref.view(torch.uint8))
+    o5, o4, am = torch.ops.hpu.cast_to_fp8_hybrid(xc, None, None, stochastic, True)
+    assert torch.equal(am, amax) or (fill == "nan" and torch.isnan(am))
