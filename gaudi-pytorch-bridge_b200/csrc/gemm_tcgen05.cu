@@ -47,7 +47,6 @@ struct TcGemmParams {
   int a_fmt_bits, b_fmt_bits;  // 0 = e4m3, 1 = e5m2 (lane-side, column-side)
   int x_mn, y_mn;              // 1 = that operand is stored MN-major ([K][rows], rows contiguous)
   int* status;                 // device status word (bounded waits report here)
-  int no_probe;                // 1 = the MMA issuer ignores its look-ahead barrier probe (for comparison)
 };
 
 // KPS = k-blocks per ring stage.  A stage is KPS sub-stages [X tile][Y tile] of one k-block each;
@@ -429,7 +428,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * STAGES;
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   // TMEM is allocated in powers of two columns (two accumulators of BN columns each)
   constexpr uint32_t kTmemCols = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
 
@@ -463,134 +462,108 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   // touch global memory before pdl_enter() -- except, in the few-token form with weights that
   // nobody is writing (b_static), the producer's first ring-full of WEIGHT tiles, which it asks
   // for before it waits: the first memory round trip of the launch overlaps the predecessor too.
-  int pre = 0;  // ring stages whose weight tiles were requested before the wait (producer thread only)
-  const bool early_weights = SWAP && p.g.b_static && !p.x_mn && warp == 0 && lane == 0 && (int)blockIdx.x < num_tiles;
+  int pre = 0;  // ring stages whose weight tiles were requested before the wait (producer warp only)
+  const bool early_weights = SWAP && p.g.b_static && !p.x_mn && warp == 0 && (int)blockIdx.x < num_tiles;
   if (early_weights) {
     const int xt = (int)blockIdx.x % p.x_tiles;
     for (int kb0 = 0; kb0 < num_kb && pre < STAGES; kb0 += KPS, ++pre) {
       const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
       const uint32_t full = bar_full + 8 * pre;
-      mbar_arrive_expect_tx(full, nsub * (L::kSubBytes - (kBlockX - p.x_tile_rows) * kBlockK));
+      if (elect_one()) {
+        mbar_arrive_expect_tx(full, nsub * (L::kSubBytes - (kBlockX - p.x_tile_rows) * kBlockK));
 #pragma unroll
-      for (int j = 0; j < KPS; ++j)
-        if (j < nsub)
-          tma_load_2d(smem_base + pre * L::kStageBytes + j * L::kSubBytes, &map_x, full, (kb0 + j) * kBlockK, xt * p.x_tile_rows);
+        for (int j = 0; j < KPS; ++j)
+          if (j < nsub)
+            tma_load_2d(smem_base + pre * L::kStageBytes + j * L::kSubBytes, &map_x, full, (kb0 + j) * kBlockK, xt * p.x_tile_rows);
+      }
     }
   }
   pdl_enter();
 
+  // The producer and the MMA issuer are whole warps that run the same instructions in all lanes
+  // (mbar_wait_uniform); one elected lane issues the copies and the MMAs.
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      int nth = 0;  // stages issued so far
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
-        for (int kb0 = 0; kb0 < num_kb; kb0 += KPS, ++nth) {
-          const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
-          const uint32_t full = bar_full + 8 * stage;
-          if (nth < pre) {
-            // weights already on their way (and the barrier armed): the token tiles follow now
+    uint32_t stage = 0, phase = 0;
+    int nth = 0;  // stages issued so far
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+      const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
+      for (int kb0 = 0; kb0 < num_kb; kb0 += KPS, ++nth) {
+        const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
+        const uint32_t full = bar_full + 8 * stage;
+        if (nth < pre) {
+          // weights already on their way (and the barrier armed): the token tiles follow now
+          if (elect_one()) {
 #pragma unroll
             for (int j = 0; j < KPS; ++j)
               if (j < nsub)
                 tma_load_2d(smem_base + stage * L::kStageBytes + j * L::kSubBytes + L::kXBytes, &map_y, full, (kb0 + j) * kBlockK, yt * BN);
-            if (++stage == STAGES) { stage = 0; phase ^= 1; }
-            continue;
           }
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer)) {
-            ok = false;
-            break;
-          }
-          mbar_arrive_expect_tx(full, nsub * (L::kSubBytes - (kBlockX - p.x_tile_rows) * kBlockK));
-          // K-major operand: box = 128 bytes of k x rows.  MN-major operand (stored [K][rows]):
-          // box = 128 rows (bytes) x 128 k, one box per 128-row block; either way a 128-byte-
-          // swizzled tile of the same size lands in the stage.
-          // (a tile shorter than 128 rows leaves the stage's other rows as they were: the MMA
-          // reads them into accumulator lanes that nobody stores)
+        } else {
+          mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(full, nsub * (L::kSubBytes - (kBlockX - p.x_tile_rows) * kBlockK));
+            // K-major operand: box = 128 bytes of k x rows.  MN-major operand (stored [K][rows]):
+            // box = 128 rows (bytes) x 128 k, one box per 128-row block; either way a 128-byte-
+            // swizzled tile of the same size lands in the stage.
+            // (a tile shorter than 128 rows leaves the stage's other rows as they were: the MMA
+            // reads them into accumulator lanes that nobody stores)
 #pragma unroll
-          for (int j = 0; j < KPS; ++j) {
-            if (j < nsub) {
-              const int kb = kb0 + j;
-              const uint32_t xs = smem_base + stage * L::kStageBytes + j * L::kSubBytes, ys = xs + L::kXBytes;
-              if (!p.x_mn) tma_load_2d(xs, &map_x, full, kb * kBlockK, xt * p.x_tile_rows);
-              else tma_load_2d(xs, &map_x, full, xt * kBlockX, kb * kBlockK);
-              if (!p.y_mn) {
-                tma_load_2d(ys, &map_y, full, kb * kBlockK, yt * BN);
-              } else {
+            for (int j = 0; j < KPS; ++j) {
+              if (j < nsub) {
+                const int kb = kb0 + j;
+                const uint32_t xs = smem_base + stage * L::kStageBytes + j * L::kSubBytes, ys = xs + L::kXBytes;
+                if (!p.x_mn) tma_load_2d(xs, &map_x, full, kb * kBlockK, xt * p.x_tile_rows);
+                else tma_load_2d(xs, &map_x, full, xt * kBlockX, kb * kBlockK);
+                if (!p.y_mn) {
+                  tma_load_2d(ys, &map_y, full, kb * kBlockK, yt * BN);
+                } else {
 #pragma unroll
-                for (int b = 0; b < BN / 128; ++b)
-                  tma_load_2d(ys + b * (kBlockK * 128), &map_y, full, yt * BN + b * 128, kb * kBlockK);
+                  for (int b = 0; b < BN / 128; ++b)
+                    tma_load_2d(ys + b * (kBlockK * 128), &map_y, full, yt * BN + b * 128, kb * kBlockK);
+                }
               }
             }
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = umma_idesc_major(p.a_fmt_bits, p.b_fmt_bits, kBlockX, BN, p.x_mn, p.y_mn);
-      // The issuing thread is a single dependent instruction stream: everything that does not
-      // change per MMA is hoisted.  Descriptors of stage 0 are built once; a stage adds
-      // kStageBytes >> 4 to the address field and a k-step adds 2 (K-major: 32 bytes inside the
-      // 128-byte row) or 256 (MN-major: four 8-k atoms of 1024 bytes; 128-row blocks are a whole
-      // k-block, 16 KB, apart).  The address field is 14 bits of (address >> 4), so the sums
-      // never carry out of it.
-      const uint64_t xd0 = p.x_mn ? smem_desc_mn_sw128(smem_base, kBlockK * 128, 1024) : smem_desc_k_sw128(smem_base);
-      const uint64_t yd0 = p.y_mn ? smem_desc_mn_sw128(smem_base + L::kXBytes, kBlockK * 128, 1024)
-                                  : smem_desc_k_sw128(smem_base + L::kXBytes);
-      const uint32_t xstep = p.x_mn ? (4096u >> 4) : (kUmmaK >> 4), ystep = p.y_mn ? (4096u >> 4) : (kUmmaK >> 4);
-      uint32_t stage = 0, phase = 0, ready = 0;
-      int it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-        const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem)) break;
+    const uint32_t idesc = umma_idesc_major(p.a_fmt_bits, p.b_fmt_bits, kBlockX, BN, p.x_mn, p.y_mn);
+    // Descriptors of stage 0 are built once; a stage adds kStageBytes >> 4 to the address field
+    // and a k-step adds 2 (K-major: 32 bytes inside the 128-byte row) or 256 (MN-major: four 8-k
+    // atoms of 1024 bytes; 128-row blocks are a whole k-block, 16 KB, apart).  The address field
+    // is 14 bits of (address >> 4), so the sums never carry out of it.
+    const uint64_t xd0 = p.x_mn ? smem_desc_mn_sw128(smem_base, kBlockK * 128, 1024) : smem_desc_k_sw128(smem_base);
+    const uint64_t yd0 = p.y_mn ? smem_desc_mn_sw128(smem_base + L::kXBytes, kBlockK * 128, 1024)
+                                : smem_desc_k_sw128(smem_base + L::kXBytes);
+    const uint32_t xstep = p.x_mn ? (4096u >> 4) : (kUmmaK >> 4), ystep = p.y_mn ? (4096u >> 4) : (kUmmaK >> 4);
+    static_assert(kBlockK / kUmmaK == 4, "umma_f8_x4 issues 4 MMAs");
+    uint32_t stage = 0, phase = 0;
+    int it = 0;
+    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
+      const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
+      mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb0 = 0; kb0 < num_kb; kb0 += KPS) {
+        mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb0 = 0; kb0 < num_kb; kb0 += KPS) {
-          if (!ready && !mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
-          uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
-          uint64_t yd = yd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
-          // all but the last k-block of the stage: MMAs only
+        const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
+        const uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
+        const uint64_t yd = yd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
+        if (elect_one()) {
 #pragma unroll
-          for (int j = 0; j + 1 < KPS; ++j) {
-            if (j + 1 < nsub) {
-              umma_f8(d_tmem, xd, yd, idesc, (kb0 + j) != 0);
-#pragma unroll
-              for (int k = 1; k < kBlockK / kUmmaK; ++k) umma_f8(d_tmem, xd + k * xstep, yd + k * ystep, idesc, 1u);
-              xd += (uint32_t)(L::kSubBytes >> 4);
-              yd += (uint32_t)(L::kSubBytes >> 4);
-            }
-          }
-          const int kb = kb0 + nsub - 1;
-          // the last k-block's four MMAs and the stage's commit (the stage is reusable once the
-          // MMAs have read it), with a probe of the next stage's barrier issued before and read
-          // after them
-          const uint32_t nstage = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-          static_assert(kBlockK / kUmmaK == 4, "umma_stage4_probe issues 4 MMAs");
-          if (p.no_probe) {
-            umma_f8(d_tmem, xd, yd, idesc, kb != 0);
-#pragma unroll
-            for (int k = 1; k < kBlockK / kUmmaK; ++k) umma_f8(d_tmem, xd + k * xstep, yd + k * ystep, idesc, 1u);
-            umma_commit(bar_empty + 8 * stage);
-          } else {
-            ready = umma_stage4_probe<false, false>(d_tmem, xd, yd, idesc, kb != 0, bar_empty + 8 * stage,
-                                                    bar_full + 8 * nstage, nphase, xstep, ystep);
-          }
-          stage = nstage;
-          phase = nphase;
+          for (int j = 0; j < KPS; ++j)
+            if (j < nsub)
+              umma_f8_x4(d_tmem, xd + j * (uint32_t)(L::kSubBytes >> 4), yd + j * (uint32_t)(L::kSubBytes >> 4), idesc,
+                         (kb0 + j) != 0, xstep, ystep);
+          umma_commit(bar_empty + 8 * stage);                               // the stage is reusable once the MMAs have read it
+          if (kb0 + KPS >= num_kb) umma_commit(bar_tfull + 8 * acc);        // accumulator complete
         }
-        if (ok) umma_commit(bar_tfull + 8 * acc);  // accumulator complete
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else {
@@ -682,7 +655,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * STAGES;
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   constexpr uint32_t kTmemCols = 2 * BN <= 256 ? 256 : 512;
 
   if (threadIdx.x == 0) {
@@ -718,67 +691,48 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
-        const int x_row = xt * 2 * kBlockX + (int)rank * kBlockX;
-        const int y_row = yt * BN + (int)rank * (BN / 2);
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer)) {
-            ok = false;
-            break;
-          }
+    uint32_t stage = 0, phase = 0;
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+      const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
+      const int x_row = xt * 2 * kBlockX + (int)rank * kBlockX;
+      const int y_row = yt * BN + (int)rank * (BN / 2);
+      for (int kb = 0; kb < num_kb; ++kb) {
+        mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (elect_one()) {
           const uint32_t full_leader = (bar_full + 8 * stage) & kPeerBitMask;
           if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * L::kStageBytes);
           tma_load_2d_pair(smem_base + stage * L::kStageBytes, &map_x, full_leader, kb * kBlockK, x_row);
           tma_load_2d_pair(smem_base + stage * L::kStageBytes + L::kXBytes, &map_y, full_leader, kb * kBlockK, y_row);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = umma_idesc(p.a_fmt_bits, p.b_fmt_bits, 2 * kBlockX, BN);
-      // hoisted descriptors: see the single-CTA kernel
+      // descriptors of stage 0, built once: see the single-CTA kernel
       const uint64_t xd0 = smem_desc_k_sw128(smem_base), yd0 = smem_desc_k_sw128(smem_base + L::kXBytes);
-      uint32_t stage = 0, phase = 0, ready = 0;
-      const bool no_probe = p.no_probe != 0;
+      static_assert(kBlockK / kUmmaK == 4 && (kUmmaK >> 4) == 2, "umma_f8_pair_x4 issues 4 MMAs 32 bytes apart");
+      uint32_t stage = 0, phase = 0;
       int it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++it) {
+      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem)) break;
+        mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!ready && !mbar_wait(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
           tc_fence_after();
           const uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
           const uint64_t yd = yd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
-          // the stage's MMAs and commit, with a probe of the next stage's barrier around them
-          const uint32_t nstage = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-          static_assert(kBlockK / kUmmaK == 4 && (kUmmaK >> 4) == 2, "umma_stage4_probe issues 4 MMAs 32 bytes apart");
-          if (no_probe) {
-            umma_f8_pair(d_tmem, xd, yd, idesc, kb != 0);
-#pragma unroll
-            for (int k = 1; k < kBlockK / kUmmaK; ++k)
-              umma_f8_pair(d_tmem, xd + k * (kUmmaK >> 4), yd + k * (kUmmaK >> 4), idesc, 1u);
+          if (elect_one()) {
+            umma_f8_pair_x4(d_tmem, xd, yd, idesc, kb != 0, 2, 2);
             umma_commit_pair_both(bar_empty + 8 * stage);
-          } else {
-            ready = umma_stage4_probe<false, true>(d_tmem, xd, yd, idesc, kb != 0, bar_empty + 8 * stage,
-                                                   bar_full + 8 * nstage, nphase, 2, 2);
+            if (kb + 1 == num_kb) umma_commit_pair_both(bar_tfull + 8 * acc);
           }
-          stage = nstage;
-          phase = nphase;
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_pair_both(bar_tfull + 8 * acc);
       }
     }
   } else {
@@ -938,8 +892,6 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
 
   TcGemmParams tp;
   tp.g = g;
-  static const bool no_probe = std::getenv("B200Q_GEMM_NO_PROBE") != nullptr;
-  tp.no_probe = no_probe;
   tp.status = device_status_ptr();
   if (!tp.status) return B200Q_ERR_CUDA;
   tp.num_kb = (int)((g.K + kBlockK - 1) / kBlockK);

@@ -1,22 +1,32 @@
 // FP8 scaled-dot-product attention, forward: out = softmax(q k^T * scale + mask) v with q, k, v in
 // e4m3 and the probabilities re-quantised to e4m3 for the second product.
 //
-// tcgen05 kernel (head dimension 128), persistent, one CTA per SM, 320 threads; a work item is one
-// (batch x head, block of 128 queries):
-//   warp 0    TMA producer: the query tile, then the key tiles (twice, see below) and value
-//             tiles through two shared-memory rings (128-byte swizzle, no multicast)
-//   warp 1    TMEM owner and MMA issuer: S = Q K^T (kind::f8f6f4, 128 x 128 x 32 per instruction)
-//             into one of two score buffers in TMEM, and O += P V with P read from shared memory
-//             (K-major) and V through an MN-major descriptor (V is stored [key][d]: no transpose)
-//   warps 2-9 softmax, two groups of four warps; a group owns one of the two score buffers (it takes
-//             every other key block) and thread = query row: tcgen05.ld of its score row, scale /
-//             mask / exp2, the e4m3 probabilities written into the swizzled P tile for the second
-//             product.
-// The three roles run as one stream of tiles that crosses item boundaries: the scores of tile t + 2
-// are asked for as soon as a group has its 128 scores of tile t in registers (before any of them is
-// used), query tiles and output accumulators are double-buffered, and a group has two P tiles, so
-// that neither product's latency, nor the epilogue of one item, nor the first loads of the next
-// one leave the softmax warps waiting.
+// tcgen05 kernel (head dimension 128), persistent, one CTA per SM, 352 threads; a work item is one
+// (batch x head, block of 128 queries), a step 256 keys, and group g of the softmax warps takes keys
+// [128 g, 128 g + 128) of every step:
+//   warp 0    TMA producer: query tiles, key tiles (twice, see below) and value tiles through
+//             shared-memory rings (128-byte swizzle, no multicast)
+//   warp 1    TMEM owner, issuer of S = Q K^T (kind::f8f6f4): in the first pass one product of
+//             128 x 256 x 128 for both groups, in the second one per group, so that the groups need
+//             not run in step
+//   warps 2-9 softmax, two groups of four warps; thread = query row: tcgen05.ld of its score row,
+//             scale / mask / exp2, the e4m3 probabilities written into the group's swizzled P tile
+//   warp 10   issuer of O += P V, with P read from shared memory (K-major) and V through an MN-major
+//             descriptor (V is stored [key][d]: no transpose)
+// The roles run as one stream of steps that crosses item boundaries: the scores of the next step are
+// asked for as soon as a group has its scores of this one in registers (before any of them is
+// used), query tiles are double-buffered, and the next item's first scores are computed under the
+// epilogue.  TMEM: columns [0, 256) = score region A (128 columns per group), [256, 512) = region B,
+// the odd steps of the first pass; in the second pass its first 128 columns are the accumulator O.
+//
+// What bounds it: ex2 on the SFU, 16 a clock and SM: 1024 cycles per 128 x 128 scores, of which the
+// tensor core is busy for 768.  Measured on the way here (causal, 16 heads x 8192 tokens): 583 us
+// with one lane issuing both products of 128 keys and a CTA per item; 422 us as one stream; 326 us
+// with the issuing roles run by whole warps (a lane spends 200 cycles per wait on addresses that a
+// converged warp keeps in uniform registers); 274 us with 256 keys per
+// step; 262 us with the two products issued by two warps and the groups out of step.  What did not
+// help: part of the exponentials as polynomials on the FMA pipe (the issue slots they take are as
+// scarce), sixteen softmax warps with half a row each, a strict alternation of the groups' exponentials.
 // Two passes over the keys: the first only takes the row maxima, the second recomputes the
 // scores and forms exp(S - max) against the final maximum.  The probabilities are therefore
 // quantised exactly where the CPU restatement quantises them (no running-maximum rescaling of
@@ -42,10 +52,11 @@ namespace sdpa {
 
 constexpr int kD = 128;        // head dimension of the tcgen05 path (bytes per row)
 constexpr int kBM = 128;       // queries per CTA
-constexpr int kBN = 128;       // keys per block
-constexpr int kStages = 3;     // key / value ring depth
-constexpr int kTile = 128 * 128;  // bytes of every tile here
-constexpr int kThreads = 320;   // producer warp, MMA warp, two softmax warpgroups
+constexpr int kBN = 128;       // keys per group and step
+constexpr int kKSteps = 3;     // depth of the key ring, in steps (256 keys)
+constexpr int kVTiles = 3;     // depth of the value ring, in tiles (128 keys)
+constexpr int kTile = 128 * 128;  // bytes of 128 rows of any operand
+constexpr int kThreads = 352;   // producer warp, two MMA warps, two softmax warpgroups
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMasked = -1.0e30f;
 
@@ -115,13 +126,14 @@ __device__ __forceinline__ float mask_term(const Params& p, int64_t bh, int64_t 
 
 struct Smem {
   static constexpr int kQ = 0;                            // two query tiles
-  static constexpr int kK = kQ + 2 * kTile;
-  static constexpr int kV = kK + kStages * kTile;
-  static constexpr int kP = kV + kStages * kTile;         // two P tiles per group
-  static constexpr int kStats = kP + 4 * kTile;           // [item parity][maxima | sums][2 groups][128 rows] fp32
+  static constexpr int kK = kQ + 2 * kTile;               // key ring
+  static constexpr int kV = kK + kKSteps * 2 * kTile;     // value ring
+  static constexpr int kP = kV + kVTiles * kTile;         // a P tile per group
+  static constexpr int kStats = kP + 2 * kTile;           // [item parity][maxima | sums][2 groups][128 rows] fp32
   static constexpr int kBars = kStats + 2 * 2 * 2 * 128 * 4;
-  // barriers: {q, o, s}_{full, empty}[2], {k, v}_{full, empty}[3], p_{full, empty}[4]
-  static constexpr int kNumBars = 12 + 4 * kStages + 8;
+  // barriers: q_{full, empty}[2], s_{full, empty}[region][group], p_{full, empty}[group], o_{full, empty},
+  // k_{full, empty}[kKSteps], v_{full, empty}[kVTiles]
+  static constexpr int kNumBars = 4 + 8 + 4 + 2 + 2 * kKSteps + 2 * kVTiles;
   static constexpr int kTotal = kBars + kNumBars * 8 + 16;
 };
 
@@ -129,7 +141,8 @@ struct Smem {
 // key blocks), dealt to the CTAs in a snake, so that the CTAs' totals differ by less than an item.
 struct Item {
   int64_t bh, q0, kv;
-  int nblk;
+  int nblk;   // blocks of 128 keys
+  int steps;  // pairs of them; the last one may hold one block only
 };
 __device__ __forceinline__ bool get_item(const Params& p, int round, Item* it) {
   const int64_t g = gridDim.x, b = blockIdx.x;
@@ -142,8 +155,30 @@ __device__ __forceinline__ bool get_item(const Params& p, int round, Item* it) {
   int64_t keys = p.S;  // (causal: keys beyond the block's last query are all masked)
   if (p.causal && it->q0 + kBM < keys) keys = it->q0 + kBM;
   it->nblk = (int)((keys + kBN - 1) / kBN);
+  it->steps = (it->nblk + 1) / 2;
   return true;
 }
+
+// The score steps of all work items of this CTA as one stream (item by item: the first pass over its
+// keys, then the second), which the producer and the score issuer walk ahead of the softmax warps.
+struct ScoreStream {
+  Item w;
+  int it = 0, t = 0;
+  bool more;
+  __device__ __forceinline__ explicit ScoreStream(const Params& p) { more = get_item(p, 0, &w); }
+  __device__ __forceinline__ bool first() const { return t == 0; }
+  __device__ __forceinline__ bool last() const { return t + 1 == 2 * w.steps; }
+  __device__ __forceinline__ bool second() const { return t >= w.steps; }
+  __device__ __forceinline__ int step() const { return t < w.steps ? t : t - w.steps; }
+  __device__ __forceinline__ void next(const Params& p) {
+    if (++t == 2 * w.steps) {
+      t = 0;
+      more = get_item(p, ++it, &w);
+    }
+  }
+};
+// whether step j of the item has a second block of keys
+__device__ __forceinline__ bool two_blocks(const Item& w, int j) { return 2 * j + 1 < w.nblk; }
 
 // Packed fp32 arithmetic: two results per issue slot.
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
@@ -182,18 +217,20 @@ __device__ __forceinline__ float chunk_max(const uint32_t* r, float m) {
 }
 // Second pass over 32 scores (keys 32 c ... of the block): exp2(score * mul + off) = probability * q_scale_s,
 // added to the row sums and written as e4m3 into the thread's row of the P tile (two 16-byte
-// pieces, XOR-swizzled by the row).  2.5 issue slots per score: packed FFMA and FADD, ex2, half a convert.
+// pieces, XOR-swizzled by the row).
 __device__ __forceinline__ void chunk_exp(const uint32_t* r, int c, uint64_t mul2, uint64_t off2, uint64_t* ls, uint8_t* prow, int row) {
   uint32_t w[8];
 #pragma unroll
   for (int e = 0; e < 32; e += 4) {
     float x[4];
-    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), mul2, off2), x[0], x[1]);
-    unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[e + 2]), __uint_as_float(r[e + 3])), mul2, off2), x[2], x[3]);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) x[u] = ex2_approx(x[u]);
-    ls[0] = add_f32x2(ls[0], pack_f32x2(x[0], x[1]));
-    ls[1] = add_f32x2(ls[1], pack_f32x2(x[2], x[3]));
+    for (int h = 0; h < 2; ++h) {
+      const uint64_t y2 = fma_f32x2(pack_f32x2(__uint_as_float(r[e + 2 * h]), __uint_as_float(r[e + 2 * h + 1])), mul2, off2);
+      unpack_f32x2(y2, x[2 * h], x[2 * h + 1]);
+      x[2 * h] = ex2_approx(x[2 * h]);
+      x[2 * h + 1] = ex2_approx(x[2 * h + 1]);
+      ls[h] = add_f32x2(ls[h], pack_f32x2(x[2 * h], x[2 * h + 1]));
+    }
     // (the conversion saturates at 448: a probability scale beyond that cannot overflow)
     w[e >> 2] = cvt_fp8x2<B200Q_E4M3>(x[0], x[1]) | (cvt_fp8x2<B200Q_E4M3>(x[2], x[3]) << 16);
   }
@@ -211,22 +248,21 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const uint32_t sbase = smem_u32(smem);
   const uint32_t b0 = smem_u32(bars);
-  const uint32_t bar_qf = b0, bar_qe = b0 + 16, bar_of = b0 + 32, bar_oe = b0 + 48, bar_sf = b0 + 64, bar_se = b0 + 80,
-                 bar_kf = b0 + 96, bar_ke = bar_kf + 8 * kStages, bar_vf = bar_ke + 8 * kStages, bar_ve = bar_vf + 8 * kStages,
-                 bar_pf = bar_ve + 8 * kStages, bar_pe = bar_pf + 32;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // s_full / s_empty of region r and group g: + 8 * (2 r + g)
+  const uint32_t bar_qf = b0, bar_qe = b0 + 16, bar_sf = b0 + 32, bar_se = b0 + 64, bar_pf = b0 + 96, bar_pe = b0 + 112,
+                 bar_of = b0 + 128, bar_oe = b0 + 136, bar_kf = b0 + 144, bar_ke = bar_kf + 8 * kKSteps,
+                 bar_vf = bar_ke + 8 * kKSteps, bar_ve = bar_vf + 8 * kVTiles;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(bar_kf + 8 * s, 1); mbar_init(bar_ke + 8 * s, 1);
-      mbar_init(bar_vf + 8 * s, 1); mbar_init(bar_ve + 8 * s, 1);
+    for (int i = 0; i < kKSteps; ++i) { mbar_init(bar_kf + 8 * i, 1); mbar_init(bar_ke + 8 * i, 1); }
+    for (int i = 0; i < kVTiles; ++i) { mbar_init(bar_vf + 8 * i, 1); mbar_init(bar_ve + 8 * i, 1); }
+    for (int i = 0; i < 4; ++i) { mbar_init(bar_sf + 8 * i, 1); mbar_init(bar_se + 8 * i, 4); }  // one arrival per warp of the group
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_qf + 8 * i, 1); mbar_init(bar_qe + 8 * i, 1);
+      mbar_init(bar_pf + 8 * i, 4); mbar_init(bar_pe + 8 * i, 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(bar_qf + 8 * a, 1); mbar_init(bar_qe + 8 * a, 1);
-      mbar_init(bar_of + 8 * a, 1); mbar_init(bar_oe + 8 * a, 8);  // one arrival per softmax warp
-      mbar_init(bar_sf + 8 * a, 1); mbar_init(bar_se + 8 * a, 4);  // one per warp of the group
-    }
-    for (int a = 0; a < 4; ++a) { mbar_init(bar_pf + 8 * a, 4); mbar_init(bar_pe + 8 * a, 1); }
+    mbar_init(bar_of, 1); mbar_init(bar_oe, 8);
     *abort_flag = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -239,7 +275,7 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;  // columns [0,128) S0, [128,256) S1, [256,384) O0, [384,512) O1
+  const uint32_t tmem = *tmem_slot;  // score regions A, B; O is the first half of B
   pdl_enter();  // everything above may run under the tail of the kernel in front of this one
   Params p = p_in;
   load_scales(p);
@@ -247,102 +283,130 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
-      uint32_t ks = 0, kph = 0, vs = 0, vph = 0;
-      Item w;
-      bool ok = true;
-      for (int it = 0; ok && get_item(p, it, &w); ++it) {
-        const uint32_t qb = it & 1;
-        if (!mbar_wait(bar_qe + 8 * qb, ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrProducer)) break;
-        mbar_arrive_expect_tx(bar_qf + 8 * qb, kTile);
-        tma_load_3d(sbase + Smem::kQ + qb * kTile, &map_q, bar_qf + 8 * qb, 0, (int)w.q0, (int)w.bh);
-        for (int t = 0; t < 2 * w.nblk; ++t) {
-          const int j = t < w.nblk ? t : t - w.nblk;
-          if (!mbar_wait(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer)) { ok = false; break; }
-          mbar_arrive_expect_tx(bar_kf + 8 * ks, kTile);
-          tma_load_3d(sbase + Smem::kK + ks * kTile, &map_k, bar_kf + 8 * ks, 0, j * kBN, (int)w.kv);
-          if (++ks == kStages) { ks = 0; kph ^= 1; }
-          if (t >= w.nblk) {
-            if (!mbar_wait(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer)) { ok = false; break; }
+    uint32_t ks = 0, kph = 0, vs = 0, vph = 0;
+    ScoreStream ss(p);
+    auto load_k = [&]() {
+      if (ss.first()) {
+        const uint32_t qb = ss.it & 1;
+        mbar_wait_uniform(bar_qe + 8 * qb, ((ss.it >> 1) & 1) ^ 1, abort_flag, p.status, kErrProducer);
+        if (elect_one()) {
+          mbar_arrive_expect_tx(bar_qf + 8 * qb, kTile);
+          tma_load_3d(sbase + Smem::kQ + qb * kTile, &map_q, bar_qf + 8 * qb, 0, (int)ss.w.q0, (int)ss.w.bh);
+        }
+      }
+      mbar_wait_uniform(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer);
+      if (elect_one()) {
+        const uint32_t dst = sbase + Smem::kK + ks * (2 * kTile), full = bar_kf + 8 * ks;
+        const bool two = two_blocks(ss.w, ss.step());
+        mbar_arrive_expect_tx(full, two ? 2 * kTile : kTile);
+        tma_load_3d(dst, &map_k, full, 0, ss.step() * (2 * kBN), (int)ss.w.kv);
+        if (two) tma_load_3d(dst + kTile, &map_k, full, 0, ss.step() * (2 * kBN) + kBN, (int)ss.w.kv);
+      }
+      if (++ks == kKSteps) { ks = 0; kph ^= 1; }
+      ss.next(p);
+    };
+    // (keys run two steps ahead of values: a key tile is wanted when its group still works on the step before)
+    for (int a = 0; a < 2 && ss.more; ++a) load_k();
+    Item w;
+    for (int it = 0; get_item(p, it, &w); ++it)
+      for (int t = 0; t < 2 * w.steps; ++t) {
+        if (ss.more) load_k();
+        for (int b = 2 * (t - w.steps); b >= 0 && b < 2 * (t - w.steps) + 2 && b < w.nblk; ++b) {
+          mbar_wait_uniform(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer);
+          if (elect_one()) {
             mbar_arrive_expect_tx(bar_vf + 8 * vs, kTile);
-            tma_load_3d(sbase + Smem::kV + vs * kTile, &map_v, bar_vf + 8 * vs, 0, j * kBN, (int)w.kv);
-            if (++vs == kStages) { vs = 0; vph ^= 1; }
+            tma_load_3d(sbase + Smem::kV + vs * kTile, &map_v, bar_vf + 8 * vs, 0, b * kBN, (int)w.kv);
           }
+          if (++vs == kVTiles) { vs = 0; vph ^= 1; }
         }
       }
-    }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc_s = umma_idesc(0, 0, kBM, kBN);                      // Q, K both K-major e4m3
-      const uint32_t idesc_o = umma_idesc_major(0, 0, kBM, kD, 0, 1);           // P K-major, V MN-major
-      // The score stream runs two tiles ahead of the P V stream; st / sit / sw = its next tile.
-      uint32_t ks = 0, kph = 0, vs = 0, vph = 0, sn = 0;   // sn: tiles issued; tile n goes to buffer n & 1
-      int st = 0, sit = 0;
-      Item sw;
-      bool more = get_item(p, 0, &sw), ok = true;
-      auto issue_s = [&]() {  // S of the next tile of the stream
-        const uint32_t sb = sn & 1, qb = sit & 1;
-        if (st == 0 && !mbar_wait(bar_qf + 8 * qb, (sit >> 1) & 1, abort_flag, p.status, kErrMma)) return false;
-        if (!mbar_wait(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma)) return false;
-        if (!mbar_wait(bar_se + 8 * sb, ((sn >> 1) & 1) ^ 1, abort_flag, p.status, kErrMma)) return false;
+    // ------------------------------------------------------------ issuer of the scores
+    const uint32_t idesc2 = umma_idesc(0, 0, kBM, 2 * kBN), idesc1 = umma_idesc(0, 0, kBM, kBN);  // Q, K both K-major e4m3
+    const uint64_t qd0 = smem_desc_k_sw128(sbase + Smem::kQ), kd0 = smem_desc_k_sw128(sbase + Smem::kK);
+    constexpr uint32_t kTileStep = kTile >> 4;  // (the address field of a descriptor never carries out)
+    uint32_t ks = 0, kph = 0;
+    uint32_t eph = 0xFu;  // bit 2 r + g: parity of the next wait for that score buffer to be free
+    for (ScoreStream ss(p); ss.more; ss.next(p)) {
+      const uint32_t qb = ss.it & 1;
+      const bool two = two_blocks(ss.w, ss.step());
+      const uint64_t qd = qd0 + qb * kTileStep, kd = kd0 + ks * (2 * kTileStep);
+      if (ss.first()) mbar_wait_uniform(bar_qf + 8 * qb, (ss.it >> 1) & 1, abort_flag, p.status, kErrMma);
+      mbar_wait_uniform(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma);
+      if (!ss.second()) {
+        const uint32_t reg = ss.step() & 1;
+        // region B holds the accumulator of the item before until its epilogue has read it
+        if (ss.step() == 1 && ss.it > 0) mbar_wait_uniform(bar_oe, (ss.it - 1) & 1, abort_flag, p.status, kErrMma);
+        mbar_wait_uniform(bar_se + 16 * reg, (eph >> (2 * reg)) & 1, abort_flag, p.status, kErrMma);
+        if (two) mbar_wait_uniform(bar_se + 16 * reg + 8, (eph >> (2 * reg + 1)) & 1, abort_flag, p.status, kErrMma);
         tc_fence_after();
-        const uint64_t qd = smem_desc_k_sw128(sbase + Smem::kQ + qb * kTile);
-        const uint64_t kd = smem_desc_k_sw128(sbase + Smem::kK + ks * kTile);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) umma_f8(tmem + sb * 128, qd + 2 * k, kd + 2 * k, idesc_s, k > 0 ? 1u : 0u);
-        umma_commit(bar_ke + 8 * ks);
-        umma_commit(bar_sf + 8 * sb);
-        if (++ks == kStages) { ks = 0; kph ^= 1; }
-        ++sn;
-        if (++st == 2 * sw.nblk) {
-          umma_commit(bar_qe + 8 * qb);  // the query tile has been read for the last time
-          st = 0;
-          more = get_item(p, ++sit, &sw);
+        if (elect_one()) {
+          umma_f8_x4(tmem + reg * 256, qd, kd, two ? idesc2 : idesc1, 0u, 2, 2);
+          umma_commit(bar_sf + 16 * reg);
+          if (two) umma_commit(bar_sf + 16 * reg + 8);
+          umma_commit(bar_ke + 8 * ks);
         }
-        return true;
-      };
-      for (int a = 0; a < 2 && more && ok; ++a) ok = issue_s();
-      uint32_t pc[2] = {0, 0};  // P tiles consumed so far, per group
-      Item w;
-      for (int it = 0; ok && get_item(p, it, &w); ++it) {
-        const uint32_t ob = it & 1, o_tmem = tmem + 256 + 128 * ob;
-        for (int t = 0; t < 2 * w.nblk && ok; ++t) {
-          if (more) ok = issue_s();
-          if (!ok || t < w.nblk) continue;
-          // O += P_j V_j
-          const int j = t - w.nblk, grp = t & 1;
-          const uint32_t pb = 2 * grp + (pc[grp] & 1), pph = (pc[grp] >> 1) & 1;
-          if (j == 0) ok = mbar_wait(bar_oe + 8 * ob, ((it >> 1) & 1) ^ 1, abort_flag, p.status, kErrMma);
-          ok = ok && mbar_wait(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma) &&
-               mbar_wait(bar_pf + 8 * pb, pph, abort_flag, p.status, kErrMma);
-          if (!ok) break;
+        eph ^= (two ? 3u : 1u) << (2 * reg);
+      } else {
+        mbar_wait_uniform(bar_se, eph & 1, abort_flag, p.status, kErrMma);
+        tc_fence_after();
+        if (elect_one()) {
+          umma_f8_x4(tmem, qd, kd, idesc1, 0u, 2, 2);
+          umma_commit(bar_sf);
+        }
+        eph ^= 1u;
+        if (two) {
+          mbar_wait_uniform(bar_se + 8, (eph >> 1) & 1, abort_flag, p.status, kErrMma);
           tc_fence_after();
-          const uint64_t pd = smem_desc_k_sw128(sbase + Smem::kP + pb * kTile);
-          const uint64_t vd = smem_desc_mn_sw128(sbase + Smem::kV + vs * kTile, 128 * 128, 1024);
-#pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f8(o_tmem, pd + 2 * k, vd + 256 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-          umma_commit(bar_ve + 8 * vs);
-          umma_commit(bar_pe + 8 * pb);
-          if (++vs == kStages) { vs = 0; vph ^= 1; }
-          ++pc[grp];
+          if (elect_one()) {
+            umma_f8_x4(tmem + 128, qd, kd + kTileStep, idesc1, 0u, 2, 2);
+            umma_commit(bar_sf + 8);
+          }
+          eph ^= 2u;
         }
-        if (ok) umma_commit(bar_of + 8 * ob);
+        if (elect_one()) {
+          umma_commit(bar_ke + 8 * ks);
+          if (ss.last()) umma_commit(bar_qe + 8 * qb);  // the query tile has been read for the last time
+        }
       }
+      if (++ks == kKSteps) { ks = 0; kph ^= 1; }
     }
+  } else if (warp == 10) {
+    // ------------------------------------------------------------ issuer of O += P V
+    // (Its first product of an item may overwrite region B: both groups have met between the passes,
+    // so the scores of the first pass are in registers and the item before has been stored.)
+    const uint32_t idesc_o = umma_idesc_major(0, 0, kBM, kD, 0, 1);           // P K-major, V MN-major
+    const uint64_t pd0 = smem_desc_k_sw128(sbase + Smem::kP), vd0 = smem_desc_mn_sw128(sbase + Smem::kV, 128 * 128, 1024);
+    constexpr uint32_t kTileStep = kTile >> 4;
+    uint32_t vs = 0, vph = 0, pph = 0;  // pph bit g: parity of group g's next P tile
+    Item w;
+    for (int it = 0; get_item(p, it, &w); ++it)
+      for (int b = 0; b < w.nblk; ++b) {
+        const uint32_t g = b & 1;
+        mbar_wait_uniform(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma);
+        mbar_wait_uniform(bar_pf + 8 * g, (pph >> g) & 1, abort_flag, p.status, kErrMma);
+        tc_fence_after();
+        if (elect_one()) {
+          umma_f8_x4(tmem + 256, pd0 + g * kTileStep, vd0 + vs * kTileStep, idesc_o, b > 0 ? 1u : 0u, 2, 256);
+          umma_commit(bar_pe + 8 * g);
+          umma_commit(bar_ve + 8 * vs);
+          if (b + 1 == w.nblk) umma_commit(bar_of);
+        }
+        pph ^= 1u << g;
+        if (++vs == kVTiles) { vs = 0; vph ^= 1; }
+      }
   } else {
     // ------------------------------------------------------------ softmax (warps 2..9)
     // A wait that runs out sets the abort flag, on which every later wait gives up at once: the
     // loops below then run to their end on whatever is there, with all barriers among the softmax
     // warps in place, and nothing is stored.
-    const int grp = (warp - 2) >> 2;          // 0 / 1: the score buffer (and tiles t = grp mod 2) of this group
+    const int grp = (warp - 2) >> 2;          // 0 / 1: which 128 keys of a step
     const int qtr = warp & 3;                 // TMEM lane quarter of this warp
     const int row = qtr * 32 + lane;          // query row inside the block = TMEM lane
     const uint32_t t_lane = tmem + ((uint32_t)(qtr * 32) << 16);
-    const uint32_t t_score = t_lane + grp * 128;
     float* stats = reinterpret_cast<float*>(smem + Smem::kStats);
     const float lq = log2f(p.q_scale_s);
-    uint32_t sc = 0, pc = 0;                  // tiles of this group so far; P tiles so far
+    uint32_t fph = 0, pph = 1;                // parities: bit r of the next score tile in region r, of the P tile to be free
     Item w;
     for (int it = 0; get_item(p, it, &w); ++it) {
       const int64_t qi = w.q0 + row;          // query index
@@ -352,22 +416,23 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       float off = 0.f;                        // log2(q_scale_s) - mx (second pass)
       uint64_t ls[2] = {0ull, 0ull};          // partial row sums of the scaled probabilities
 
-      // One key block of this group: scores -> row maximum (first pass) or e4m3 probabilities and
+      // This group's keys of step j: scores -> row maximum (first pass) or e4m3 probabilities and
       // row sums (second pass).
-      auto do_tile = [&](int j, auto second_tag) {
+      auto do_step = [&](int j, auto second_tag) {
         constexpr bool second = decltype(second_tag)::value;
-        const uint32_t pb = 2 * grp + (pc & 1);
-        const int64_t key0 = (int64_t)j * kBN;
-        uint8_t* prow = smem + Smem::kP + pb * kTile + row * 128;
-        mbar_wait(bar_sf + 8 * grp, sc & 1, abort_flag, p.status, kErrSoftmax);
-        ++sc;
-        if (second) mbar_wait(bar_pe + 8 * pb, ((pc >> 1) & 1) ^ 1, abort_flag, p.status, kErrSoftmax);
+        const uint32_t reg = second ? 0u : (uint32_t)(j & 1);
+        const uint32_t t_score = t_lane + 256 * reg + 128 * grp, bar = 16 * reg + 8 * grp;
+        const int64_t key0 = (int64_t)(2 * j + grp) * kBN;
+        uint8_t* prow = smem + Smem::kP + grp * kTile + row * 128;
+        mbar_wait_uniform(bar_sf + bar, (fph >> reg) & 1, abort_flag, p.status, kErrSoftmax);
+        fph ^= 1u << reg;
         tc_fence_after();
         auto release_scores = [&]() {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar_se + 8 * grp);
+          if (lane == 0) mbar_arrive(bar_se + bar);
         };
+        auto wait_p_free = [&]() { mbar_wait_uniform(bar_pe + 8 * grp, pph, abort_flag, p.status, kErrSoftmax); };
         // keys of the block that this row may see: the first `lim` of them
         int64_t lim64 = (p.causal && qi + 1 < p.S ? qi + 1 : p.S) - key0;
         const int lim = lim64 > kBN ? kBN : (int)lim64;
@@ -394,12 +459,14 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             mx = fmaxf(mx, m * mul);
           } else {
             const uint64_t mul2 = pack_f32x2(mul, mul);
+            wait_p_free();
 #pragma unroll
             for (int c = 0; c < 4; ++c) chunk_exp(r + 32 * c, c, mul2, off2, ls, prow, row);
           }
         } else {
           const uint64_t one2 = pack_f32x2(1.f, 1.f);
           const int64_t qm = qi < p.L ? qi : p.L - 1;
+          if (second) wait_p_free();
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t r[32];
@@ -419,19 +486,17 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         if (second) {
           fence_proxy_async_smem();    // the P tile is read by the tensor core (async proxy)
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar_pf + 8 * pb);
-          ++pc;
+          if (lane == 0) mbar_arrive(bar_pf + 8 * grp);
+          pph ^= 1;
         }
       };
-      // first pass: this group's tiles t = grp, grp + 2, ... < nblk
-      for (int t = grp; t < w.nblk; t += 2) do_tile(t, std::false_type{});
+      for (int j = 0; 2 * j + grp < w.nblk; ++j) do_step(j, std::false_type{});
       // between the passes the groups meet: the row maximum over all blocks
       st_max[grp * 128 + row] = mx;
       named_bar_sync(1, 256);
       mx = fmaxf(st_max[row], st_max[128 + row]);
       off = lq - mx;
-      // second pass: tiles t = nblk ... 2 nblk - 1 with t = grp (mod 2)
-      for (int j = (w.nblk & 1) == grp ? 0 : 1; j < w.nblk; j += 2) do_tile(j, std::true_type{});
+      for (int j = 0; 2 * j + grp < w.nblk; ++j) do_step(j, std::true_type{});
       // ---- output: O / l, scaled.  The row sums of both groups are added, then group 0 writes the
       // first 64 output columns of its rows and group 1 the other 64.
       float l4[4];
@@ -440,7 +505,7 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       st_sum[grp * 128 + row] = (l4[0] + l4[1]) + (l4[2] + l4[3]);
       named_bar_sync(1, 256);
       const float lsum = (st_sum[row] + st_sum[128 + row]) / p.q_scale_s;
-      mbar_wait(bar_of + 8 * (it & 1), (it >> 1) & 1, abort_flag, p.status, kErrSoftmax);
+      mbar_wait_uniform(bar_of, it & 1, abort_flag, p.status, kErrSoftmax);
       tc_fence_after();
       const float linv = lsum > 0.f ? 1.f / lsum : 0.f;
       const float osc = p.o_scale * linv;
@@ -448,12 +513,12 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       const bool in = qi < p.L && !*abort_flag;
       uint32_t r[64];
       const int c0 = 64 * grp;
-      tmem_ld_32x32(t_lane + 256 + 128 * (it & 1) + c0, r);
-      tmem_ld_32x32(t_lane + 256 + 128 * (it & 1) + c0 + 32, r + 32);
+      tmem_ld_32x32(t_lane + 256 + c0, r);
+      tmem_ld_32x32(t_lane + 256 + c0 + 32, r + 32);
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_oe + 8 * (it & 1));
+      if (lane == 0) mbar_arrive(bar_oe);
       float o[64];
 #pragma unroll
       for (int e = 0; e < 64; ++e) {

@@ -92,6 +92,37 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
+// The form for roles that a whole warp runs: control flow that is the same for all 32 lanes, with
+// nothing depending on the outcome of a wait, lets the compiler keep addresses and descriptors in
+// uniform registers; a single-lane role spends some 200 cycles per wait and 60 per MMA on getting
+// them there.  A wait that runs out sets the flag, on which every later wait gives up at once: the
+// role then runs to its end on whatever is in the buffers (nothing of it is stored) and the CTA
+// ends in the ordinary way.
+__device__ __forceinline__ void mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (mbar_try_wait(bar, parity)) return;
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+    if ((i & 63u) == 0u && *abort_flag) return;
+    if (mbar_try_wait(bar, parity)) return;
+    if (i > 4096u) __nanosleep(64);
+  }
+  *abort_flag = 1;
+  atomicCAS(status, 0, code);
+}
+// The index of the calling warp, known to be the same in all its lanes.
+__device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
+// True in one lane of a converged warp (always the same one).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "elect.sync _|p, 0xFFFFFFFF;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(e));
+  return e != 0;
+}
+
 // ---- TMA: 2-D tiled load global -> shared, completion on an mbarrier (never multicast) ----
 __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
@@ -146,6 +177,23 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
       "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Four kind::f8f6f4 MMAs whose operand descriptors advance by astep / bstep (16-byte units), as one
+// instruction sequence; only the first one may start a new accumulator.
+__device__ __forceinline__ void umma_f8_x4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                           uint32_t astep, uint32_t bstep) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.b32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %5, %6, %3, t;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %7, %8, %3, t;\n"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %9, %10, %3, t;\n"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "l"(adesc + astep), "l"(bdesc + bstep),
+      "l"(adesc + 2 * astep), "l"(bdesc + 2 * bstep), "l"(adesc + 3 * astep), "l"(bdesc + 3 * bstep)
+      : "memory");
+}
 // Arrive on an mbarrier once every previously issued MMA of this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -193,6 +241,22 @@ __device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t adesc, ui
       "setp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
       "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// umma_f8_x4 for a CTA pair.
+__device__ __forceinline__ void umma_f8_pair_x4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                uint32_t astep, uint32_t bstep) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.b32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %5, %6, %3, t;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %7, %8, %3, t;\n"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %9, %10, %3, t;\n"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "l"(adesc + astep), "l"(bdesc + bstep),
+      "l"(adesc + 2 * astep), "l"(bdesc + 2 * bstep), "l"(adesc + 3 * astep), "l"(bdesc + 3 * bstep)
       : "memory");
 }
 // One ring stage in a single instruction sequence: a non-blocking probe of the NEXT stage's
