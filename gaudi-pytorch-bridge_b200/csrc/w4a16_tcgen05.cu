@@ -170,7 +170,7 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
   const uint32_t bar_raw_full = smem_u32(bars), bar_raw_empty = bar_raw_full + 8 * RS;
   const uint32_t bar_w_ready = bar_raw_empty + 8 * RS, bar_w_empty = bar_w_ready + 8 * WS;
   const uint32_t bar_tfull = bar_w_empty + 8 * WS, bar_tempty = bar_tfull + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   enum { kProducer, kProducerMeta, kProducerAct, kMma, kEpilogue, kExpander, kIdle };
   // expander warp index (valid when that role): warps off scheduler 0 first, then 20, 24, 28
   const int ewarp = (warp & 3) != 0 ? ((warp - 5) >> 2) * 3 + ((warp & 3) - 1) : C::kOffS0 + ((warp - 20) >> 2);
@@ -235,23 +235,21 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     //   warp 0   packed weights
     //   warp 12  scales and zero points; every k-block carries them because consecutive
     //            k-blocks go to different expander warps
-    if (lane == 0) {
-      const bool meta = role == kProducerMeta;
-      uint32_t slot = 0, phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        int xt, yt, kb0, kb1, split;
-        decode(w, xt, yt, kb0, kb1, split);
-        const int n0 = yt * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer)) {
-            ok = false;
-            break;
-          }
-          const uint32_t sbase = raw_base + slot * C::kRawSlotBytes;
-          const uint32_t full = bar_raw_full + 8 * slot;
+    // (The issuing roles are whole warps that elect a lane for the copies and MMAs; see
+    // mbar_wait_uniform.)
+    const bool meta = role == kProducerMeta;
+    uint32_t slot = 0, phase = 0;
+    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+      int xt, yt, kb0, kb1, split;
+      decode(w, xt, yt, kb0, kb1, split);
+      const int n0 = yt * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        const uint32_t sbase = raw_base + slot * C::kRawSlotBytes;
+        const uint32_t full = bar_raw_full + 8 * slot;
+        const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
+        if (elect_one()) {
           if (meta) {
-            const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
             mbar_arrive_expect_tx(full, C::kScaleBytes + (p.zp ? C::kZpBytes : 0));
             tma_load_2d(sbase + C::kMetaOffset, &map_scale, full, n0, grp);
             if (p.zp) tma_load_2d(sbase + C::kZpOffset, &map_zp, full, n0 / 8, grp);
@@ -259,73 +257,58 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
             mbar_arrive_expect_tx(full, C::kRawBytes);
             tma_load_2d(sbase, &map_raw, full, n0 / 8, kb * kK);
           }
-          if (++slot == RS) { slot = 0; phase ^= 1; }
         }
+        if (++slot == RS) { slot = 0; phase ^= 1; }
       }
     }
   } else if (role == kProducerAct) {
     // ------------------------------------------------------------ activation producer (work ring)
-    if (lane == 0) {
-      uint32_t slot = 0, phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        int xt, yt, kb0, kb1, split;
-        decode(w, xt, yt, kb0, kb1, split);
-        const int act_row0 = xt * 128;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(bar_w_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer)) {
-            ok = false;
-            break;
-          }
+    uint32_t slot = 0, phase = 0;
+    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+      int xt, yt, kb0, kb1, split;
+      decode(w, xt, yt, kb0, kb1, split);
+      const int act_row0 = xt * 128;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait_uniform(bar_w_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (elect_one()) {
           mbar_arrive_expect_tx(bar_w_ready + 8 * slot, C::kActBytes);
           tma_load_2d(smem_base + slot * C::kWorkSlotBytes, &map_act, bar_w_ready + 8 * slot, kb * kK, act_row0);
-          if (++slot == WS) { slot = 0; phase ^= 1; }
         }
+        if (++slot == WS) { slot = 0; phase ^= 1; }
       }
     }
   } else if (role == kMma) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // bf16 x bf16; the expanded weights are the MN-major B operand
-      const uint32_t idesc = umma_idesc_major(1u, 1u, 128, BN, 0u, 1u);
-      const uint64_t da0 = smem_desc_k_sw128(smem_base);
-      const uint64_t dw0 = smem_desc_mn_sw128(smem_base + C::kWOffset, (kK / 8) * 1024, 1024);
-      uint32_t stage = 0, phase = 0, ready = 0;  // work-ring slot
-      constexpr int STAGES = WS;
-      uint32_t rslot = 0;
-      int it = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++it) {
-        int xt, yt, kb0, kb1, split;
-        decode(w, xt, yt, kb0, kb1, split);
-        const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem)) break;
+    // bf16 x bf16; the expanded weights are the MN-major B operand
+    const uint32_t idesc = umma_idesc_major(1u, 1u, 128, BN, 0u, 1u);
+    const uint64_t da0 = smem_desc_k_sw128(smem_base);
+    const uint64_t dw0 = smem_desc_mn_sw128(smem_base + C::kWOffset, (kK / 8) * 1024, 1024);
+    uint32_t stage = 0, phase = 0;  // work-ring slot
+    uint32_t rslot = 0;
+    int it = 0;
+    for (int w = blockIdx.x; w < num_work; w += gridDim.x, ++it) {
+      int xt, yt, kb0, kb1, split;
+      decode(w, xt, yt, kb0, kb1, split);
+      const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
+      mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        mbar_wait_uniform(bar_w_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!ready && !mbar_wait(bar_w_ready + 8 * stage, phase, abort_flag, p.status, kErrMma)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          // activations: K-major, 32 bytes per k-step inside the 128-byte row; weights: MN-major,
-          // two 8-k atoms (2048 bytes) per k-step, column blocks 8 atoms apart (descriptors of
-          // slot 0 are hoisted out of the loop).  Four MMAs and the commit in one sequence, with
-          // a probe of the next slot's barrier issued before and read after them.
-          const uint64_t soff = (uint64_t)(stage * (uint32_t)(C::kWorkSlotBytes >> 4));
-          const uint64_t da = da0 + soff, dw = dw0 + soff;
-          const uint32_t nstage = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-          static_assert(kK / 16 == 4, "umma_stage4_probe issues 4 MMAs");
-          constexpr uint64_t kActStep = kUmmaKBytes >> 4, kWStep = 2048 >> 4;
-          ready = umma_stage4_probe<true, false>(d_tmem, da, dw, idesc, kb != kb0, bar_w_empty + 8 * stage,
-                                                 bar_w_ready + 8 * nstage, nphase, kActStep, kWStep);
+        // activations: K-major, 32 bytes per k-step inside the 128-byte row; weights: MN-major,
+        // two 8-k atoms (2048 bytes) per k-step, column blocks 8 atoms apart (descriptors of
+        // slot 0 are hoisted out of the loop)
+        const uint64_t soff = (uint64_t)(stage * (uint32_t)(C::kWorkSlotBytes >> 4));
+        static_assert(kK / 16 == 4, "umma_x4 issues 4 MMAs");
+        if (elect_one()) {
+          umma_f16_x4(d_tmem, da0 + soff, dw0 + soff, idesc, kb != kb0, kUmmaKBytes >> 4, 2048 >> 4);
+          umma_commit(bar_w_empty + 8 * stage);
           umma_commit(bar_raw_empty + 8 * rslot);  // the expanders read raw slot rslot before they arrived on w_ready
-          if (++rslot == RS) rslot = 0;
-          stage = nstage;
-          phase = nphase;
+          if (kb + 1 == kb1) umma_commit(bar_tfull + 8 * acc);
         }
-        if (ok) umma_commit(bar_tfull + 8 * acc);
+        if (++rslot == RS) rslot = 0;
+        if (++stage == WS) { stage = 0; phase ^= 1; }
       }
     }
   } else if (role == kEpilogue) {
@@ -436,8 +419,7 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     advance(rslot, rphase, my_group, RS);
     advance(wslot, wphase, my_group, WS);
     int lead = my_group;  // k-blocks of the next work item that belong to other groups before ours
-    bool ok = true;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
+    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
       int xt, yt, kb0, kb1, split;
       decode(w, xt, yt, kb0, kb1, split);
       GroupRegs g;
@@ -446,11 +428,8 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
       for (; kb < kb1; kb += C::kExpandGroups) {
         {
           // the packed weights have landed and the work slot's previous tile has been consumed
-          if (!mbar_wait(bar_raw_full + 8 * rslot, rphase, abort_flag, p.status, kErrExpand) ||
-              !mbar_wait(bar_w_empty + 8 * wslot, wphase ^ 1, abort_flag, p.status, kErrExpand)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_uniform(bar_raw_full + 8 * rslot, rphase, abort_flag, p.status, kErrExpand);
+          mbar_wait_uniform(bar_w_empty + 8 * wslot, wphase ^ 1, abort_flag, p.status, kErrExpand);
           const uint32_t rbase = raw_base + rslot * C::kRawSlotBytes;
           const uint32_t wbase = smem_base + wslot * C::kWorkSlotBytes;
           const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
@@ -566,7 +545,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t bar_ready = smem_u32(bars), bar_empty = bar_ready + 8 * STAGES, bar_raw = bar_empty + 8 * STAGES;
   const uint32_t bar_tfull = bar_raw + 8 * STAGES, bar_tempty = bar_tfull + 16;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   enum { kProducer, kMma, kEpilogue, kExpander, kIdle };
   const int ewarp = ((warp - 5) >> 2) * 3 + ((warp & 3) - 1);  // expander warp index (valid when that role)
   const int role = warp == 0 ? kProducer
@@ -611,21 +590,17 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
 
   if (role == kProducer) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      const uint32_t meta_bytes = C::kScaleBytes + (p.zp ? C::kZpBytes : 0);
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
-        const int act_row0 = xt * 256 + (int)rank * 128;
-        const int n0 = yt * BN + (int)rank * kUnit;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer)) {
-            ok = false;
-            break;
-          }
-          const uint32_t sbase = smem_base + stage * C::kStageBytes;
-          const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
+    uint32_t stage = 0, phase = 0;
+    const uint32_t meta_bytes = C::kScaleBytes + (p.zp ? C::kZpBytes : 0);
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+      const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
+      const int act_row0 = xt * 256 + (int)rank * 128;
+      const int n0 = yt * BN + (int)rank * kUnit;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        const uint32_t sbase = smem_base + stage * C::kStageBytes;
+        const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
+        if (elect_one()) {
           // packed weights and scales first: the expanders are the longer chain
           const uint32_t rawb = bar_raw + 8 * stage;
           mbar_arrive_expect_tx(rawb, C::kRawBytes + meta_bytes);
@@ -635,43 +610,34 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
           // activations of both CTAs complete on the even CTA's barrier
           if (rank == 0) mbar_arrive_expect_tx(bar_ready + 8 * stage, 2 * C::kActBytes);
           tma_load_2d_pair(sbase, &map_act, (bar_ready + 8 * stage) & kPeerBitMask, kb * kK, act_row0);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (role == kMma) {
     // ------------------------------------------------------------ MMA issuer (even CTA)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = umma_idesc_major(1u, 1u, 256, BN, 0u, 1u);
       const uint64_t da0 = smem_desc_k_sw128(smem_base);
       const uint64_t dw0 = smem_desc_mn_sw128(smem_base + C::kWOffset, (kK / 8) * 1024, 1024);
-      uint32_t stage = 0, phase = 0, ready = 0;
+      uint32_t stage = 0, phase = 0;
       int it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++it) {
+      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem)) break;
+        mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!ready && !mbar_wait(bar_ready + 8 * stage, phase, abort_flag, p.status, kErrMma)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_uniform(bar_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
           tc_fence_after();
           const uint64_t soff = (uint64_t)(stage * (uint32_t)(C::kStageBytes >> 4));
-          const uint64_t da = da0 + soff, dw = dw0 + soff;
-          // four MMAs and the commit in one sequence, with a probe of the next stage's barrier
-          // issued before and read after them
-          const uint32_t nstage = stage + 1 == STAGES ? 0 : stage + 1;
-          const uint32_t nphase = nstage == 0 ? phase ^ 1 : phase;
-          static_assert(kK / 16 == 4, "umma_stage4_probe issues 4 MMAs");
-          ready = umma_stage4_probe<true, true>(d_tmem, da, dw, idesc, kb != 0, bar_empty + 8 * stage,
-                                                bar_ready + 8 * nstage, nphase, kUmmaKBytes >> 4, 2048 >> 4);
-          stage = nstage;
-          phase = nphase;
+          if (elect_one()) {
+            umma_f16_pair_x4(d_tmem, da0 + soff, dw0 + soff, idesc, kb != 0, kUmmaKBytes >> 4, 2048 >> 4);
+            umma_commit_pair_both(bar_empty + 8 * stage);
+            if (kb + 1 == num_kb) umma_commit_pair_both(bar_tfull + 8 * acc);
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_pair_both(bar_tfull + 8 * acc);
       }
     }
   } else if (role == kEpilogue) {
@@ -752,16 +718,12 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const uint32_t wt_off = C::kWOffset + ((ngl >> 3) * (kK / 8) + (kr >> 3)) * 1024 + krow * 128 + (((ngl & 7) ^ krow) << 4);
     uint32_t stage = 0, phase = 0;
     int turn = 0;  // whose stage this is
-    bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       GroupRegs g;
       int g_cur = -1;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (turn == my_group) {
-          if (!mbar_wait(bar_raw + 8 * stage, phase, abort_flag, p.status, kErrExpand)) {
-            ok = false;
-            break;
-          }
+          mbar_wait_uniform(bar_raw + 8 * stage, phase, abort_flag, p.status, kErrExpand);
           const uint32_t sbase = smem_base + stage * C::kStageBytes;
           const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
           if (grp != g_cur) {
