@@ -108,6 +108,26 @@ __device__ __forceinline__ void mbar_wait_uniform(uint32_t bar, uint32_t parity,
   *abort_flag = 1;
   atomicCAS(status, 0, code);
 }
+// The same for two barriers at once: the two polls are in flight together (a poll of a completed phase takes
+// about a hundred cycles).
+__device__ __forceinline__ void mbar_wait2_uniform(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
+                                                   volatile int* abort_flag, int* status, int code) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n"
+      "and.pred p, p, q;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
+      : "memory");
+  if (ok) return;
+  mbar_wait_uniform(bar0, parity0, abort_flag, status, code);
+  mbar_wait_uniform(bar1, parity1, abort_flag, status, code);
+}
 // The index of the calling warp, known to be the same in all its lanes.
 __device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
 // True in one lane of a converged warp (always the same one).
@@ -201,6 +221,24 @@ B200Q_UMMA_X4(umma_f16_x4, "1", "f16")
 B200Q_UMMA_X4(umma_f8_pair_x4, "2", "f8f6f4")  // (over both CTAs of a pair; issued by one thread of the even CTA)
 B200Q_UMMA_X4(umma_f16_pair_x4, "2", "f16")
 #undef B200Q_UMMA_X4
+// Four kind::f16 MMAs whose A operand is in tensor memory (128 lanes, two bf16 per 32-bit column: 8 columns per
+// K = 16 step): the TMEM address advances by astep columns, the B descriptor by bstep 16-byte units.
+__device__ __forceinline__ void umma_f16_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                               uint32_t astep, uint32_t bstep) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p, t;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "setp.eq.b32 t, 0, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%5], %6, %3, t;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%7], %8, %3, t;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%9], %10, %3, t;\n"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(a_tmem + astep), "l"(bdesc + bstep), "r"(a_tmem + 2 * astep),
+      "l"(bdesc + 2 * bstep), "r"(a_tmem + 3 * astep), "l"(bdesc + 3 * bstep)
+      : "memory");
+}
 // Arrive on an mbarrier once every previously issued MMA of this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -319,6 +357,16 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
+// Stores: thread t of the warp writes 16 columns of lane (base lane + t).
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+      "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Named barrier among a subset of the CTA's warps.

@@ -21,10 +21,10 @@
 //     columns), always in the same order: no global scratch, no second kernel, the same bits on
 //     every run.
 //
-// Two weight layouts: the operator's [K][N/8] (a word = 8 neighbouring columns of one k; k-pairs
-// for the MMA operand are built with two byte permutes per four weights) and AutoGPTQ's [K/8][N]
-// (a word = 8 consecutive k of one column; a word's nibble pairs are used as k-pairs directly and
-// the activations are permuted to match, which costs nothing per weight).
+// Takes the operator's layout [K][N/8] (a word = 8 neighbouring columns of one k; k-pairs for the MMA
+// operand are built with two byte permutes per four weights) with groups of 16 or 32 rows; groups of whole
+// 64-row blocks, and AutoGPTQ's layout, go to w4a16_tmem.cu (16 tokens, K = N = 8192, group 128:
+// 22.4 us here, 19.0 there).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -126,18 +126,13 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t ra
   return v;
 }
 
-// MT = token blocks of 8 (M <= 8 * MT).  KP = 0: operator layout [K][N/8]; 1: AutoGPTQ layout [K/8][N].
+// MT = token blocks of 8 (M <= 8 * MT).
 //
 // Thread (g = lane / 4, q = lane % 4) owns 8 of its warp's 64 columns and feeds 4 MMAs per k-step
 // whose 16 operand rows are output columns:
-//   KP = 0  step = 16 k-rows; the thread's word column g (columns 8g .. 8g + 7) of k-rows
+//   step = 16 k-rows; the thread's word column g (columns 8g .. 8g + 7) of k-rows
 //           {2q, 2q+1, 2q+8, 2q+9}; MMA i: operand row g = column 8g + i, row g + 8 = column 8g + i + 4
-//   KP = 1  step = 64 k-rows = 8 word-rows; columns g + 8j (j = 0..7) of word-rows q and q + 4; MMA
-//           i of accumulator a takes its k labels (2q, 2q+1) from nibbles (i, i+4) of word-row q
-//           and (2q+8, 2q+9) from the same nibbles of word-row q + 4 -- over q and i every nibble
-//           of the 8 word-rows once -- with the activation fragment gathered the same way;
-//           accumulator a = columns g + 16a (operand row g) and g + 16a + 8 (row g + 8)
-template <int MT, int KP>
+template <int MT>
 __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) w4a16_smallm_kernel(const Params p) {
   extern __shared__ __align__(16) uint8_t smem[];
   pdl_enter();  // launched under the tail of the kernel in front of it
@@ -146,32 +141,27 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
   const uint32_t crank = cluster_rank();
   const int cg = blockIdx.x / kCluster;
   const int64_t n0 = (int64_t)cg * kCols + strip * kStrip;  // first column of this warp's strip
-  constexpr int kStepRows = KP ? 64 : 16;
-  constexpr int kStageBytes = 2048;                 // KP = 1: a ring stage is one k-step
-  constexpr int kDepth = kRingBytes / kStageBytes;  // 4 steps in flight
+  constexpr int kStepRows = 16;
   const int64_t rows_per_slice = p.K / kSlices;
   const int64_t k_begin = ((int64_t)crank * kParts + khalf) * rows_per_slice;
   const int steps = (int)(rows_per_slice / kStepRows);
-  const int64_t nw = KP ? p.N : p.N / 8;  // words per row of the packed matrix
+  const int64_t nw = p.N / 8;  // words per row of the packed matrix
   uint8_t* ring = smem + warp * kRingBytes;
   const uint32_t ring_u = smem_addr(ring);
 
-  // One k-step in the ring.  KP = 0: 16 rows x 8 words, one 16-byte copy per lane (row
+  // One k-step in the ring: 16 rows x 8 words, one 16-byte copy per lane (row
   // lane / 2, words 4 (lane % 2) ..); rows are stored in the order [load L = (row & 1) + 2 (row >> 3)]
   // [(row >> 1) & 3] so that load L of thread (g, q) -- word g of row 2q (+1, +8, +9) -- is
-  // conflict-free.  KP = 1: 8 word-rows x 64 columns, 16-byte pieces XOR-swizzled by word-row so
-  // that the column-strided reads are conflict-free.
+  // conflict-free.
   // this lane's source of the next step to be issued, and where its copy goes inside a stage
   const int32_t* w_src;
   uint32_t w_dst = 0;
-  if (KP == 0) {
+  {
     const int row = lane >> 1, hf = lane & 1;
     w_dst = (((row & 1) + 2 * (row >> 3)) * 4 + ((row >> 1) & 3)) * 32 + hf * 16;
     w_src = p.qw + (k_begin + row) * nw + n0 / 8 + 4 * hf;
-  } else {
-    w_src = p.qw + (k_begin / 8) * nw + n0 + (lane & 15) * 4;  // (word-row offsets are added per copy)
   }
-  // KP = 0: k-steps 4t .. 4t + 3 (those that exist) into slot t % kSlots, as one group -- committed
+  // k-steps 4t .. 4t + 3 (those that exist) into slot t % kSlots, as one group -- committed
   // even when empty, so that the number of groups that may stay pending is the same at every t
   auto issue_batch = [&](int t) {
     const uint32_t dst = ring_u + (t & (kSlots - 1)) * kSlotBytes + w_dst;
@@ -181,20 +171,9 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
     w_src += (int64_t)kBatch * 16 * nw;
     cp_async_commit();
   };
-  auto issue = [&](int s) {  // KP = 1: one k-step into stage s % kDepth
-    const uint32_t dst = ring_u + (s & (kDepth - 1)) * kStageBytes;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int id = c * 32 + lane, w = id >> 4, piece = id & 15;
-      cp_async16(dst + w * 256 + ((piece * 16) ^ ((w & 3) * 32)), w_src + (int64_t)w * nw);
-    }
-    w_src += 8 * nw;
-    cp_async_commit();
-  };
   // The activations of k-rows [k_begin + 512 c, + 512) of this k-part, copied by its 4 warps (8
-  // pieces of 16 bytes per thread) in fragment order.  KP = 0: per step of 16 rows
-  // [k half][token][16 bytes]; KP = 1: per step of 64 rows [token][128 bytes] with the 16-byte
-  // pieces XOR-swizzled by token parity.  Tokens beyond M read the last real token's row.
+  // pieces of 16 bytes per thread) in fragment order: per step of 16 rows [k half][token][16 bytes].
+  // Tokens beyond M read the last real token's row.
   const uint32_t xs_u = smem_addr(smem + kXOffset + khalf * kXBytes);
   const uint8_t* xs = smem + kXOffset + khalf * kXBytes;
   auto stage_x = [&](int chunk) {
@@ -205,30 +184,15 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
 #pragma unroll
     for (int c = 0; c < kXBytes / 16 / (32 * kStrips); ++c) {
       const int id = c * (32 * kStrips) + tid;  // 16-byte piece of the chunk
-      if (KP == 0) {
-        const int step = id >> 5, tok = (id & 31) >> 1, hf = id & 1;
-        if (step * 16 < rows)
-          cp_async16(xs_u + step * 512 + hf * 256 + tok * 16, p.x + (tok < p.M ? tok : p.M - 1) * p.ldx + kc + step * 16 + 8 * hf);
-      } else {
-        const int step = id >> 7, tok = (id & 127) >> 3, piece = id & 7;
-        if (step * 64 < rows)
-          cp_async16(xs_u + step * 2048 + tok * 128 + ((piece ^ ((tok & 1) << 2)) * 16),
-                     p.x + (tok < p.M ? tok : p.M - 1) * p.ldx + kc + step * 64 + 8 * piece);
-      }
+      const int step = id >> 5, tok = (id & 31) >> 1, hf = id & 1;
+      if (step * 16 < rows)
+        cp_async16(xs_u + step * 512 + hf * 256 + tok * 16, p.x + (tok < p.M ? tok : p.M - 1) * p.ldx + kc + step * 16 + 8 * hf);
     }
     cp_async_commit();
   };
-  constexpr int kStepsPerChunk = kXChunkRows / kStepRows;
 
   stage_x(0);
-  if (KP == 0) {
-    for (int t = 0; t < kSlots - 1; ++t) issue_batch(t);
-  } else {
-    for (int t = 0; t < kDepth - 1; ++t) {
-      if (t < steps) issue(t);
-      else cp_async_commit();
-    }
-  }
+  for (int t = 0; t < kSlots - 1; ++t) issue_batch(t);
 
   float acc[4][MT][4];
 #pragma unroll
@@ -243,182 +207,105 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
   int64_t cur_grp = k_begin / p.group;
   const int steps_per_group = p.group / kStepRows;
   int to_next_group = steps_per_group - (int)((k_begin % p.group) / kStepRows) + 1;
-  if (KP == 0) {
-    // scales and 128 + zero point of the thread's 8 columns, each twice in a register: lo[i] column
-    // 8g + i, hi[i] column 8g + i + 4 (an operand register holds two k of one column)
-    uint32_t slo[4], shi[4], zlo[4], zhi[4];
-    // The scales and zero points of a group are fetched one group ahead: a load that is consumed at
-    // once comes back behind the cp.async traffic this warp has queued, i.e. after a full memory
-    // latency, once per group.
-    uint4 nsv;
-    uint32_t nz;
-    const int64_t last_grp = (p.K - 1) / p.group;
-    auto fetch_group = [&](int64_t grp) {
-      if (grp > last_grp) grp = last_grp;  // (never used then)
-      nsv = __ldg(reinterpret_cast<const uint4*>(p.scale + grp * p.N + n0 + 8 * g));
-      nz = p.zp ? (uint32_t)__ldg(p.zp + grp * (p.N / 8) + n0 / 8 + g) : 0u;
-    };
-    auto load_group = [&](int64_t grp) {  // takes what fetch_group(grp) asked for, asks for grp + 1
-      const uint4 sv = nsv;
-      const uint32_t z = nz;
-      fetch_group(grp + 1);
-      slo[0] = __byte_perm(sv.x, 0u, 0x1010); slo[1] = __byte_perm(sv.x, 0u, 0x3232);
-      slo[2] = __byte_perm(sv.y, 0u, 0x1010); slo[3] = __byte_perm(sv.y, 0u, 0x3232);
-      shi[0] = __byte_perm(sv.z, 0u, 0x1010); shi[1] = __byte_perm(sv.z, 0u, 0x3232);
-      shi[2] = __byte_perm(sv.w, 0u, 0x1010); shi[3] = __byte_perm(sv.w, 0u, 0x3232);
+  // scales and 128 + zero point of the thread's 8 columns, each twice in a register: lo[i] column
+  // 8g + i, hi[i] column 8g + i + 4 (an operand register holds two k of one column)
+  uint32_t slo[4], shi[4], zlo[4], zhi[4];
+  // The scales and zero points of a group are fetched one group ahead: a load that is consumed at
+  // once comes back behind the cp.async traffic this warp has queued, i.e. after a full memory
+  // latency, once per group.
+  uint4 nsv;
+  uint32_t nz;
+  const int64_t last_grp = (p.K - 1) / p.group;
+  auto fetch_group = [&](int64_t grp) {
+    if (grp > last_grp) grp = last_grp;  // (never used then)
+    nsv = __ldg(reinterpret_cast<const uint4*>(p.scale + grp * p.N + n0 + 8 * g));
+    nz = p.zp ? (uint32_t)__ldg(p.zp + grp * (p.N / 8) + n0 / 8 + g) : 0u;
+  };
+  auto load_group = [&](int64_t grp) {  // takes what fetch_group(grp) asked for, asks for grp + 1
+    const uint4 sv = nsv;
+    const uint32_t z = nz;
+    fetch_group(grp + 1);
+    slo[0] = __byte_perm(sv.x, 0u, 0x1010); slo[1] = __byte_perm(sv.x, 0u, 0x3232);
+    slo[2] = __byte_perm(sv.y, 0u, 0x1010); slo[3] = __byte_perm(sv.y, 0u, 0x3232);
+    shi[0] = __byte_perm(sv.z, 0u, 0x1010); shi[1] = __byte_perm(sv.z, 0u, 0x3232);
+    shi[2] = __byte_perm(sv.w, 0u, 0x1010); shi[3] = __byte_perm(sv.w, 0u, 0x3232);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        zlo[i] = (((z >> (4 * i)) & 15u) * 0x00010001u) | 0x43004300u;
-        zhi[i] = (((z >> (4 * i + 16)) & 15u) * 0x00010001u) | 0x43004300u;
-      }
-    };
-    // One k-step: the lane's four packed words (word g of k-rows 2q, 2q + 1, 2q + 8, 2q + 9) are
-    // transposed while still packed -- two byte permutes per pair of rows put the same four
-    // columns of both rows into one word -- so that a nibble pair (i, i + 4) of such a word is
-    // one column at two consecutive k: the operand register the MMA wants, with nothing to
-    // shuffle after the expansion.
-    auto k_step = [&](const uint8_t* wp, const uint8_t* xp) {
-      uint32_t b[MT][2];
-#pragma unroll
-      for (int tk = 0; tk < MT; ++tk) {
-        b[tk][0] = *reinterpret_cast<const uint32_t*>(xp + tk * 128);
-        b[tk][1] = *reinterpret_cast<const uint32_t*>(xp + 256 + tk * 128);
-      }
-      uint32_t w[4];
-#pragma unroll
-      for (int L = 0; L < 4; ++L) w[L] = *reinterpret_cast<const uint32_t*>(wp + L * 128);
-      const uint32_t m0 = __byte_perm(w[0], w[1], 0x5410), m1 = __byte_perm(w[0], w[1], 0x7632);
-      const uint32_t m2 = __byte_perm(w[2], w[3], 0x5410), m3 = __byte_perm(w[2], w[3], 0x7632);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t a0 = bf2_mul(bf2_sub(nib_pair(m0, i), zlo[i]), slo[i]);
-        const uint32_t a1 = bf2_mul(bf2_sub(nib_pair(m1, i), zhi[i]), shi[i]);
-        const uint32_t a2 = bf2_mul(bf2_sub(nib_pair(m2, i), zlo[i]), slo[i]);
-        const uint32_t a3 = bf2_mul(bf2_sub(nib_pair(m3, i), zhi[i]), shi[i]);
-#pragma unroll
-        for (int tk = 0; tk < MT; ++tk) mma_bf16(acc[i][tk], a0, a1, a2, a3, b[tk][0], b[tk][1]);
-      }
-    };
-    fetch_group(cur_grp);
-    load_group(cur_grp);  // before the first wait: its latency hides under the weights'
-    // A ring slot holds kBatch k-steps: per slot one wait, one warp barrier (which also says that
-    // every lane is done with the slot before), one refill of that slot and one set of addresses;
-    // per k-step only 4 + 2 MT shared loads, the expansion and the MMAs (plus the group countdown
-    // in a slot that a group boundary or the end of the slice cuts).
-    constexpr int kBatchesPerChunk = kXChunkRows / (16 * kBatch);
-    const int batches = (steps + kBatch - 1) / kBatch;
-    for (int t = 0; t < batches; ++t) {
-      if ((t & (kBatchesPerChunk - 1)) == 0) {
-        // a new chunk of activations: the first one was issued before the weights (it is the
-        // oldest group), a later one is issued here, after every warp of the k-half is done
-        // with the old chunk, and waited for at once
-        if (t > 0) {
-          named_bar(1 + khalf, 32 * kStrips);
-          stage_x(t / kBatchesPerChunk);
-          cp_async_wait(0);
-        } else {
-          asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");  // all but the weights: the chunk
-        }
-        named_bar(1 + khalf, 32 * kStrips);
-      }
-      asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 2) : "memory");
-      __syncwarp();
-      issue_batch(t + kSlots - 1);
-      const uint8_t* sl = ring + (t & (kSlots - 1)) * kSlotBytes + q * 32 + g * 4;
-      const uint8_t* xb = xs + (t & (kBatchesPerChunk - 1)) * (kBatch * 512) + g * 16 + 4 * q;
-      const int nst = steps - t * kBatch;
-      if (to_next_group == 1) {  // a group begins with this slot's first step
-        to_next_group = steps_per_group + 1;
-        load_group(++cur_grp);
-      }
-      if (nst >= kBatch && to_next_group > kBatch) {  // a whole slot inside one group: nothing to test per step
-        to_next_group -= kBatch;
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j) k_step(sl + j * 512, xb + j * 512);
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < kBatch && j < nst; ++j) {
-          if (--to_next_group == 0) {  // (a division per step costs more than the step's arithmetic)
-            to_next_group = steps_per_group;
-            load_group(++cur_grp);
-          }
-          k_step(sl + j * 512, xb + j * 512);
-        }
-      }
+    for (int i = 0; i < 4; ++i) {
+      zlo[i] = (((z >> (4 * i)) & 15u) * 0x00010001u) | 0x43004300u;
+      zhi[i] = (((z >> (4 * i + 16)) & 15u) * 0x00010001u) | 0x43004300u;
     }
-  } else {
-    // per accumulator a the two columns g + 16a and g + 16a + 8: scale and 128 + zero point, each
-    // twice in a register (an operand register holds two k of one column), set up once per group
-    uint32_t sc2[4][2], zc2[4][2];
-    auto load_group = [&](int64_t grp) {
+  };
+  // One k-step: the lane's four packed words (word g of k-rows 2q, 2q + 1, 2q + 8, 2q + 9) are
+  // transposed while still packed -- two byte permutes per pair of rows put the same four
+  // columns of both rows into one word -- so that a nibble pair (i, i + 4) of such a word is
+  // one column at two consecutive k: the operand register the MMA wants, with nothing to
+  // shuffle after the expansion.
+  auto k_step = [&](const uint8_t* wp, const uint8_t* xp) {
+    uint32_t b[MT][2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        sc2[j >> 1][j & 1] = (uint32_t)__bfloat16_as_ushort(p.scale[grp * p.N + n0 + g + 8 * j]) * 0x00010001u;
-        // column n0 + g + 8j is nibble g of zero-point word n0 / 8 + j
-        const uint32_t z = p.zp ? ((uint32_t)__ldg(p.zp + grp * (p.N / 8) + n0 / 8 + j) >> (4 * g)) & 15u : 0u;
-        zc2[j >> 1][j & 1] = (z * 0x00010001u) | 0x43004300u;
-      }
-    };
-    load_group(cur_grp);
-    // A stage is refilled one step after it was read (after the warp barrier of the next step),
-    // so its words are loaded where they are used instead of all in front of the refill; every
-    // step commits a group, an empty one past the end, so that the wait is the same at every step.
-    auto issue_or_empty = [&](int s) {
-      if (s < steps) issue(s);
-      else cp_async_commit();
-    };
-    const uint32_t lane_off = q * 256 + g * 4, q32 = q * 32;
-    for (int s = 0; s < steps; ++s) {
-      if ((s & (kStepsPerChunk - 1)) == 0) {
-        if (s > 0) {
-          named_bar(1 + khalf, 32 * kStrips);
-          stage_x(s / kStepsPerChunk);
-          cp_async_wait(0);
-        } else {
-          asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");  // all but the weights: the chunk
-        }
+    for (int tk = 0; tk < MT; ++tk) {
+      b[tk][0] = *reinterpret_cast<const uint32_t*>(xp + tk * 128);
+      b[tk][1] = *reinterpret_cast<const uint32_t*>(xp + 256 + tk * 128);
+    }
+    uint32_t w[4];
+#pragma unroll
+    for (int L = 0; L < 4; ++L) w[L] = *reinterpret_cast<const uint32_t*>(wp + L * 128);
+    const uint32_t m0 = __byte_perm(w[0], w[1], 0x5410), m1 = __byte_perm(w[0], w[1], 0x7632);
+    const uint32_t m2 = __byte_perm(w[2], w[3], 0x5410), m3 = __byte_perm(w[2], w[3], 0x7632);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t a0 = bf2_mul(bf2_sub(nib_pair(m0, i), zlo[i]), slo[i]);
+      const uint32_t a1 = bf2_mul(bf2_sub(nib_pair(m1, i), zhi[i]), shi[i]);
+      const uint32_t a2 = bf2_mul(bf2_sub(nib_pair(m2, i), zlo[i]), slo[i]);
+      const uint32_t a3 = bf2_mul(bf2_sub(nib_pair(m3, i), zhi[i]), shi[i]);
+#pragma unroll
+      for (int tk = 0; tk < MT; ++tk) mma_bf16(acc[i][tk], a0, a1, a2, a3, b[tk][0], b[tk][1]);
+    }
+  };
+  fetch_group(cur_grp);
+  load_group(cur_grp);  // before the first wait: its latency hides under the weights'
+  // A ring slot holds kBatch k-steps: per slot one wait, one warp barrier (which also says that
+  // every lane is done with the slot before), one refill of that slot and one set of addresses;
+  // per k-step only 4 + 2 MT shared loads, the expansion and the MMAs (plus the group countdown
+  // in a slot that a group boundary or the end of the slice cuts).
+  constexpr int kBatchesPerChunk = kXChunkRows / (16 * kBatch);
+  const int batches = (steps + kBatch - 1) / kBatch;
+  for (int t = 0; t < batches; ++t) {
+    if ((t & (kBatchesPerChunk - 1)) == 0) {
+      // a new chunk of activations: the first one was issued before the weights (it is the
+      // oldest group), a later one is issued here, after every warp of the k-half is done
+      // with the old chunk, and waited for at once
+      if (t > 0) {
         named_bar(1 + khalf, 32 * kStrips);
+        stage_x(t / kBatchesPerChunk);
+        cp_async_wait(0);
+      } else {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");  // all but the weights: the chunk
       }
-      asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 2) : "memory");
-      __syncwarp();  // step s has landed for every lane, and every lane is done with the stage of step s - 1
-      issue_or_empty(s + kDepth - 1);
-      if (--to_next_group == 0) {
-        to_next_group = steps_per_group;
-        load_group(++cur_grp);
-      }
-      // [token block][word-row q / q + 4][nibble pair i]: (x[k_i], x[k_{i+4}]) of that word-row's 8 k
-      uint32_t bx[MT][2][4];
-      const uint8_t* xf = xs + (s & (kStepsPerChunk - 1)) * 2048;
+      named_bar(1 + khalf, 32 * kStrips);
+    }
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 2) : "memory");
+    __syncwarp();
+    issue_batch(t + kSlots - 1);
+    const uint8_t* sl = ring + (t & (kSlots - 1)) * kSlotBytes + q * 32 + g * 4;
+    const uint8_t* xb = xs + (t & (kBatchesPerChunk - 1)) * (kBatch * 512) + g * 16 + 4 * q;
+    const int nst = steps - t * kBatch;
+    if (to_next_group == 1) {  // a group begins with this slot's first step
+      to_next_group = steps_per_group + 1;
+      load_group(++cur_grp);
+    }
+    if (nst >= kBatch && to_next_group > kBatch) {  // a whole slot inside one group: nothing to test per step
+      to_next_group -= kBatch;
 #pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const int tok = 8 * t + g;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const uint4 xv = *reinterpret_cast<const uint4*>(xf + tok * 128 + (((q + 4 * h) ^ ((tok & 1) << 2)) * 16));
-          bx[t][h][0] = __byte_perm(xv.x, xv.z, 0x5410);
-          bx[t][h][1] = __byte_perm(xv.x, xv.z, 0x7632);
-          bx[t][h][2] = __byte_perm(xv.y, xv.w, 0x5410);
-          bx[t][h][3] = __byte_perm(xv.y, xv.w, 0x7632);
+      for (int j = 0; j < kBatch; ++j) k_step(sl + j * 512, xb + j * 512);
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < kBatch && j < nst; ++j) {
+        if (--to_next_group == 0) {  // (a division per step costs more than the step's arithmetic)
+          to_next_group = steps_per_group;
+          load_group(++cur_grp);
         }
-      }
-      // word (word-row wr, column g + 8j) sits at wr * 256 + ((g + 8j) * 4 ^ (wr & 3) * 32); with wr = q or
-      // q + 4 that is lane_off (+ 1024) + 32 (j ^ q)
-      const uint8_t* st = ring + (s & (kDepth - 1)) * kStageBytes + lane_off;
-#pragma unroll
-      for (int a = 0; a < 4; ++a) {
-        const uint32_t o0 = (uint32_t)(64 * a) ^ q32, o1 = (uint32_t)(64 * a + 32) ^ q32;
-        const uint32_t w00 = *reinterpret_cast<const uint32_t*>(st + o0), w01 = *reinterpret_cast<const uint32_t*>(st + o1);
-        const uint32_t w10 = *reinterpret_cast<const uint32_t*>(st + 1024 + o0),
-                       w11 = *reinterpret_cast<const uint32_t*>(st + 1024 + o1);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t a0 = bf2_mul(bf2_sub(nib_pair(w00, i), zc2[a][0]), sc2[a][0]);
-          const uint32_t a1 = bf2_mul(bf2_sub(nib_pair(w01, i), zc2[a][1]), sc2[a][1]);
-          const uint32_t a2 = bf2_mul(bf2_sub(nib_pair(w10, i), zc2[a][0]), sc2[a][0]);
-          const uint32_t a3 = bf2_mul(bf2_sub(nib_pair(w11, i), zc2[a][1]), sc2[a][1]);
-#pragma unroll
-          for (int t = 0; t < MT; ++t) mma_bf16(acc[a][t], a0, a1, a2, a3, bx[t][0][i], bx[t][1][i]);
-        }
+        k_step(sl + j * 512, xb + j * 512);
       }
     }
   }
@@ -431,7 +318,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
   float* red = reinterpret_cast<float*>(ring);
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const int col_lo = KP ? g + 16 * a : 8 * g + a, col_hi = KP ? col_lo + 8 : col_lo + 4;
+    const int col_lo = 8 * g + a, col_hi = col_lo + 4;
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
       const int tok = 8 * t + 2 * q;
@@ -469,9 +356,9 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
   cluster_sync();  // no CTA leaves while another may still read its partial tile
 }
 
-template <int MT, int KP>
+template <int MT>
 static int launch(const Params& p, cudaStream_t st) {
-  auto kern = w4a16_smallm_kernel<MT, KP>;
+  auto kern = w4a16_smallm_kernel<MT>;
   static std::atomic<int> configured[kMaxDevices];
   const int dev = current_device_index();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -490,9 +377,9 @@ static int launch(const Params& p, cudaStream_t st) {
 
 }  // namespace w4s
 
-// Whether the few-token kernel takes this problem: M <= 16, whole 256-column blocks, K divisible
-// into 16 slices of whole k-steps (16 rows; 64 for the AutoGPTQ layout), groups that k-steps do
-// not straddle.
+// Whether this is a few-token problem that needs no scratch: M <= 16, whole 256-column blocks, K divisible
+// into 16 slices of whole k-steps (16 rows; 64 for the AutoGPTQ layout, which w4a16_tmem.cu reads), groups that
+// k-steps do not straddle.
 bool w4a16_smallm_eligible(int64_t M, int64_t N, int64_t K, int64_t group, int k_packed) {
   const int64_t step = k_packed ? 64 : 16;
   return M >= 1 && M <= 16 && N >= w4s::kCols && N % w4s::kCols == 0 && K >= w4s::kSlices * step &&
@@ -502,7 +389,7 @@ bool w4a16_smallm_eligible(int64_t M, int64_t N, int64_t K, int64_t group, int k
 int w4a16_smallm_launch(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp,
                         int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out, int out_dtype,
                         int64_t ldo, cudaStream_t st) {
-  if (!w4a16_smallm_eligible(M, N, K, group, k_packed)) return B200Q_ERR_UNSUPPORTED;
+  if (k_packed || !w4a16_smallm_eligible(M, N, K, group, 0)) return B200Q_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(qweight) | reinterpret_cast<uintptr_t>(scale)) & 15)
     return B200Q_ERR_UNSUPPORTED;
   if (ldx % 8) return B200Q_ERR_UNSUPPORTED;
@@ -510,8 +397,7 @@ int w4a16_smallm_launch(const void* x, int64_t ldx, const int32_t* qweight, cons
   p.qw = qweight; p.scale = static_cast<const __nv_bfloat16*>(scale); p.zp = zp;
   p.x = static_cast<const __nv_bfloat16*>(x); p.out = out;
   p.M = M; p.N = N; p.K = K; p.ldx = ldx; p.ldo = ldo; p.group = (int)group; p.out_dtype = out_dtype;
-  if (k_packed) return M <= 8 ? w4s::launch<1, 1>(p, st) : w4s::launch<2, 1>(p, st);
-  return M <= 8 ? w4s::launch<1, 0>(p, st) : w4s::launch<2, 0>(p, st);
+  return M <= 8 ? w4s::launch<1>(p, st) : w4s::launch<2>(p, st);
 }
 
 }  // namespace b200q

@@ -15,11 +15,9 @@
 //                 pairs come out as columns (i, i+4); they are stored in that order and the
 //                 epilogue undoes the permutation when it writes the output columns.
 //   warp 1        MMA issuer: tcgen05.mma.kind::f16 (bf16 x bf16 -> fp32 in TMEM)
-//   warps 2..5    epilogue: tcgen05.ld, convert, store (or fp32 partials for split-K)
+//   warps 2..5    epilogue: tcgen05.ld, convert, store
 //
-// Lanes <- 128 tokens, columns <- BN weight columns.  Small M (<= 128): only AR token rows are
-// loaded (see Cfg), K is split over several CTAs per tile so that every SM streams weights, and
-// the fp32 partial tiles are summed by a second kernel (deterministic: no atomics).
+// Lanes <- 128 tokens, columns <- BN weight columns; for more than 128 tokens (w4a16_tmem.cu has the others).
 #include <cuda.h>
 
 #include <cstdlib>
@@ -45,12 +43,11 @@ enum { kErrProducer = 201, kErrMma = 202, kErrMmaTmem = 203, kErrEpilogue = 204,
 struct Params {
   const __nv_bfloat16* scale;  // [K/group][N]
   const int32_t* zp;           // [K/group][N/8] or null
-  void* out;                   // [M][N] out_dtype (splits == 1)
-  float* partial;              // [splits][M][N] fp32 (splits > 1)
+  void* out;                   // [M][N] out_dtype
   int64_t M, N, K, ldo;
   int group, out_dtype;
   int group_shift;  // log2(group / 64) when that is a power of two, else -1 (the kernels then divide)
-  int x_tiles, y_tiles, num_kb, splits, kb_per_split;
+  int x_tiles, y_tiles, num_kb;
   int* status;
 };
 
@@ -62,15 +59,10 @@ struct Params {
 //   work ring (WS slots)  activations (bf16, K-major, 128-byte swizzle) + the expanded bf16
 //                         tile (MN-major, 128-byte swizzle).  Large (16 KB per 128 columns) and
 //                         live only from the expansion to the MMAs that read it: few slots.
-template <int BN, int RS, int WS, int GROUPS, int AR = 0, int EW = 0>
+template <int BN, int RS, int WS, int GROUPS>
 struct Cfg {
   static constexpr int kUnits = BN / kUnit;
-  // Activation rows held per work slot.  The MMA always reads 128 rows through its descriptor;
-  // with AR < 128 the rows beyond AR are whatever follows in the slot (the expanded tile).  Each
-  // output row depends on its own operand row only, and rows >= M are never stored, so for
-  // M <= AR nothing needs to be there.
-  static constexpr int kActRows = AR ? AR : 128;
-  static_assert(AR == 0 || (AR <= 128 && AR % 8 == 0), "narrow activation tile: a multiple of 8 rows");
+  static constexpr int kActRows = 128;
   static constexpr int kActBytes = kActRows * 128;
   static constexpr int kWCols = kUnits * kUnit;
   // work slot
@@ -90,7 +82,7 @@ struct Cfg {
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
   // 8 expander warps per 128 weight columns and k-block (4 packed words per thread), in GROUPS
   // groups that take alternate k-blocks
-  static constexpr int kExpandWarps = EW ? EW : 8 * kUnits;
+  static constexpr int kExpandWarps = 8 * kUnits;
   static constexpr int kExpandGroups = GROUPS;
   // Warp roles are placed by scheduler (warp % 4): the three producers (warps 0, 12, 16) and the
   // MMA issuer (warp 4) have scheduler 0 to themselves; their per-k-block instruction chains
@@ -147,11 +139,11 @@ __device__ __forceinline__ void make_group(GroupRegs& g, uint4 s, uint32_t zw, b
   for (int i = 0; i < 4; ++i) g.zr[i] = has_zp ? nib_pair(zw, i) : 0x43004300u;
 }
 
-template <int BN, int RS, int WS, int GROUPS, int AR = 0, int EW = 0>
-__global__ void __launch_bounds__((Cfg<BN, RS, WS, GROUPS, AR, EW>::kThreads), 1)
+template <int BN, int RS, int WS, int GROUPS>
+__global__ void __launch_bounds__((Cfg<BN, RS, WS, GROUPS>::kThreads), 1)
 w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_raw,
              const __grid_constant__ CUtensorMap map_scale, const __grid_constant__ CUtensorMap map_zp, const Params p) {
-  using C = Cfg<BN, RS, WS, GROUPS, AR, EW>;
+  using C = Cfg<BN, RS, WS, GROUPS>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kBarOffset);
@@ -214,19 +206,13 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
   const uint32_t tmem_base = *tmem_slot;
   pdl_enter();  // everything above overlaps the tail of the kernel in front; global memory is touched from here on
 
-  const int num_work = p.x_tiles * p.y_tiles * p.splits;
-  // work item -> (lane-side tile, column-side tile, k range).  Consecutive items (CTAs that run
-  // at the same time) are neighbouring tiles of the same k range: together they read whole rows
-  // of the packed weight matrix, which keeps the DRAM pages they open fully used.
-  auto decode = [&](int w, int& xt, int& yt, int& kb0, int& kb1, int& split) {
-    const int tiles = p.x_tiles * p.y_tiles;
-    split = w / tiles;
-    const int tile = w % tiles;
-    xt = tile % p.x_tiles;
-    yt = tile / p.x_tiles;
-    kb0 = split * p.kb_per_split;
-    kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+  const int num_work = p.x_tiles * p.y_tiles;
+  // work item -> (lane-side tile, column-side tile)
+  auto decode = [&](int w, int& xt, int& yt) {
+    xt = w % p.x_tiles;
+    yt = w / p.x_tiles;
   };
+  const int num_kb = p.num_kb;
 
   if (role == kProducer || role == kProducerMeta) {
     // ------------------------------------------------------------ raw-ring producers
@@ -240,10 +226,10 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     const bool meta = role == kProducerMeta;
     uint32_t slot = 0, phase = 0;
     for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
-      int xt, yt, kb0, kb1, split;
-      decode(w, xt, yt, kb0, kb1, split);
+      int xt, yt;
+      decode(w, xt, yt);
       const int n0 = yt * BN;
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
         const uint32_t sbase = raw_base + slot * C::kRawSlotBytes;
         const uint32_t full = bar_raw_full + 8 * slot;
@@ -265,10 +251,10 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     // ------------------------------------------------------------ activation producer (work ring)
     uint32_t slot = 0, phase = 0;
     for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
-      int xt, yt, kb0, kb1, split;
-      decode(w, xt, yt, kb0, kb1, split);
+      int xt, yt;
+      decode(w, xt, yt);
       const int act_row0 = xt * 128;
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait_uniform(bar_w_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
         if (elect_one()) {
           mbar_arrive_expect_tx(bar_w_ready + 8 * slot, C::kActBytes);
@@ -287,13 +273,13 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     uint32_t rslot = 0;
     int it = 0;
     for (int w = blockIdx.x; w < num_work; w += gridDim.x, ++it) {
-      int xt, yt, kb0, kb1, split;
-      decode(w, xt, yt, kb0, kb1, split);
+      int xt, yt;
+      decode(w, xt, yt);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * BN;
-      for (int kb = kb0; kb < kb1; ++kb) {
+      for (int kb = 0; kb < num_kb; ++kb) {
         mbar_wait_uniform(bar_w_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
         tc_fence_after();
         // activations: K-major, 32 bytes per k-step inside the 128-byte row; weights: MN-major,
@@ -302,10 +288,10 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
         const uint64_t soff = (uint64_t)(stage * (uint32_t)(C::kWorkSlotBytes >> 4));
         static_assert(kK / 16 == 4, "umma_x4 issues 4 MMAs");
         if (elect_one()) {
-          umma_f16_x4(d_tmem, da0 + soff, dw0 + soff, idesc, kb != kb0, kUmmaKBytes >> 4, 2048 >> 4);
+          umma_f16_x4(d_tmem, da0 + soff, dw0 + soff, idesc, kb != 0, kUmmaKBytes >> 4, 2048 >> 4);
           umma_commit(bar_w_empty + 8 * stage);
           umma_commit(bar_raw_empty + 8 * rslot);  // the expanders read raw slot rslot before they arrived on w_ready
-          if (kb + 1 == kb1) umma_commit(bar_tfull + 8 * acc);
+          if (kb + 1 == num_kb) umma_commit(bar_tfull + 8 * acc);
         }
         if (++rslot == RS) rslot = 0;
         if (++stage == WS) { stage = 0; phase ^= 1; }
@@ -317,8 +303,8 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     const int et = q * 32 + lane;
     int it = 0;
     for (int w = blockIdx.x; w < num_work; w += gridDim.x, ++it) {
-      int xt, yt, kb0, kb1, split;
-      decode(w, xt, yt, kb0, kb1, split);
+      int xt, yt;
+      decode(w, xt, yt);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
       mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
       named_bar_sync(1, kEpiThreads);
@@ -349,18 +335,7 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
         }
         const int64_t n0 = y0 + c0;
         if (m < p.M) {
-          if (p.splits > 1) {
-            float* o = p.partial + ((int64_t)split * p.M + m) * p.N + n0;
-            if (n0 + CW <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-#pragma unroll
-              for (int j = 0; j < CW; j += 4)
-                *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < CW; ++j)
-                if (n0 + j < p.N) o[j] = __uint_as_float(r[j]);
-            }
-          } else if (p.out_dtype == B200Q_BF16) {
+          if (p.out_dtype == B200Q_BF16) {
             __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + m * p.ldo + n0;
             if (n0 + CW <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
 #pragma unroll
@@ -420,12 +395,12 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     advance(wslot, wphase, my_group, WS);
     int lead = my_group;  // k-blocks of the next work item that belong to other groups before ours
     for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
-      int xt, yt, kb0, kb1, split;
-      decode(w, xt, yt, kb0, kb1, split);
+      int xt, yt;
+      decode(w, xt, yt);
       GroupRegs g;
       int g_cur = -1;
-      int kb = kb0 + lead;
-      for (; kb < kb1; kb += C::kExpandGroups) {
+      int kb = lead;
+      for (; kb < num_kb; kb += C::kExpandGroups) {
         {
           // the packed weights have landed and the work slot's previous tile has been consumed
           mbar_wait_uniform(bar_raw_full + 8 * rslot, rphase, abort_flag, p.status, kErrExpand);
@@ -463,7 +438,7 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
         advance(rslot, rphase, C::kExpandGroups, RS);
         advance(wslot, wphase, C::kExpandGroups, WS);
       }
-      lead = kb - kb1;  // how far the stride overshot this work item's range
+      lead = kb - num_kb;  // how far the stride overshot this work item's range
     }
   }
 
@@ -807,48 +782,15 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mr, const CUten
   return B200Q_OK;
 }
 
-// Sum the fp32 partial tiles of a split-K run (in split order) and round once to the output dtype.
-// VEC = 4: four neighbouring columns per thread (N and ldo multiples of 4, 16-byte aligned
-// pointers): 16-byte loads of the partials, one division per four outputs, an 8- or 16-byte
-// store.  Launched under the tail of the GEMM kernel; it waits for that grid before it reads.
-template <int VEC>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ partial, void* out, int out_dtype,
-                                                            int64_t M, int64_t N, int64_t ldo, int splits) {
-  pdl_enter();
-  const int64_t total = M * N / VEC;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = i * VEC, m = e / N, n = e - m * N;
-    if (VEC == 4) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int s = 0; s < splits; ++s) {
-        const float4 t = __ldcs(reinterpret_cast<const float4*>(partial + (int64_t)s * M * N + e));
-        v.x += t.x, v.y += t.y, v.z += t.z, v.w += t.w;
-      }
-      if (out_dtype == B200Q_BF16) {
-        __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-        *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + m * ldo + n) =
-            make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-      } else {
-        *reinterpret_cast<float4*>(static_cast<float*>(out) + m * ldo + n) = v;
-      }
-    } else {
-      float v = 0.f;
-      for (int s = 0; s < splits; ++s) v += partial[(int64_t)s * M * N + e];
-      if (out_dtype == B200Q_BF16) static_cast<__nv_bfloat16*>(out)[m * ldo + n] = __float2bfloat16_rn(v);
-      else static_cast<float*>(out)[m * ldo + n] = v;
-    }
-  }
-}
-
-template <int BN, int RS, int WS, int GROUPS, int AR = 0, int EW = 0>
+template <int BN, int RS, int WS, int GROUPS>
 static int launch(const CUtensorMap& ma, const CUtensorMap& mr, const CUtensorMap& ms, const CUtensorMap& mz, const Params& p,
                   cudaStream_t st) {
-  using C = Cfg<BN, RS, WS, GROUPS, AR, EW>;
+  using C = Cfg<BN, RS, WS, GROUPS>;
   constexpr int smem = C::kTotal + 1024;
   static_assert(smem <= 227 * 1024, "shared memory budget");
   // TMEM: CTAs that share an SM must never ask for more than 512 columns together
   static_assert(C::kTmemCols * (227 * 1024 / smem) <= 512, "TMEM over-subscription");
-  auto kern = w4a16_kernel<BN, RS, WS, GROUPS, AR, EW>;
+  auto kern = w4a16_kernel<BN, RS, WS, GROUPS>;
   static std::atomic<int> configured[kMaxDevices];
   const int dev = current_device_index();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -856,7 +798,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mr, const CUtensorMa
     B200Q_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured[dev].store(1, std::memory_order_release);
   }
-  int work = p.x_tiles * p.y_tiles * p.splits;
+  int work = p.x_tiles * p.y_tiles;
   int per_sm = 227 * 1024 / smem;
   int grid = work < kNumSMs * per_sm ? work : kNumSMs * per_sm;
   if (launch_overlapped(kern, dim3((unsigned)grid), dim3(C::kThreads), (size_t)smem, st, ma, mr, ms, mz, p) != cudaSuccess) {
@@ -869,8 +811,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mr, const CUtensorMa
 
 }  // namespace w4
 
-// Number of K splits the small-M path uses (every split gets at least one k-block), and the
-// fp32 workspace that goes with it.
+// The workspace that the entry asks for at 17 - 128 tokens: fp32 partial tiles of this many K splits.  The
+// kernel that now takes these shapes adds its splits inside clusters and needs none; the size stays what callers
+// and the limit of the allocation-free entry know.
 static int w4a16_splits(int64_t M, int64_t N, int64_t K) {
   if (M > 128) return 1;
   // 128-token x 256-column tiles; the split count that minimises the busiest CTA's k-blocks
@@ -895,6 +838,10 @@ int w4a16_smallm_launch(const void* x, int64_t ldx, const int32_t* qweight, cons
                         int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out, int out_dtype,
                         int64_t ldo, cudaStream_t st);
 
+// up to 128 tokens (w4a16_tmem.cu)
+int w4a16_tmem_launch(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp, int k_packed,
+                      int64_t M, int64_t N, int64_t K, int64_t group, void* out, int out_dtype, int64_t ldo, cudaStream_t st);
+
 size_t w4a16_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0 || K % w4::kK || N % 32) return 0;  // shapes the fused kernel does not take
   if (w4a16_smallm_eligible(M, N, K, w4::kK, 0)) return 0;  // reduced inside its clusters: no scratch
@@ -913,6 +860,9 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
   }
   // a handful of tokens: the streaming kernel (either weight layout)
   if (w4a16_smallm_eligible(M, N, K, group, k_packed)) {
+    const int rt = w4a16_tmem_launch(x, ldx, qweight, scale, zp_kind == B200Q_ZP_PACKED ? zp : nullptr, k_packed, M, N, K, group,
+                                     out, out_dtype, ldo, st);
+    if (rt != B200Q_ERR_UNSUPPORTED) return rt;
     const int rc = w4a16_smallm_launch(x, ldx, qweight, scale, zp_kind == B200Q_ZP_PACKED ? zp : nullptr, k_packed, M, N, K,
                                        group, out, out_dtype, ldo, st);
     if (rc != B200Q_ERR_UNSUPPORTED) return rc;
@@ -925,7 +875,7 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
   w4::Params p;
   p.scale = static_cast<const __nv_bfloat16*>(scale);
   p.zp = zp_kind == B200Q_ZP_PACKED ? zp : nullptr;
-  p.out = out; p.partial = nullptr; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.group = (int)group;
+  p.out = out; p.M = M; p.N = N; p.K = K; p.ldo = ldo; p.group = (int)group;
   {
     const int64_t gk = group / w4::kK;
     p.group_shift = -1;
@@ -935,17 +885,13 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
   p.out_dtype = out_dtype; p.num_kb = (int)(K / w4::kK);
   p.status = device_status_ptr();
   if (!p.status) return B200Q_ERR_CUDA;
-  const bool small_m = M <= 128;
-  p.splits = small_m ? w4a16_splits(M, N, K) : 1;
-  p.kb_per_split = (p.num_kb + p.splits - 1) / p.splits;
-  if (p.splits > 1) {
-    const size_t need = (size_t)p.splits * (size_t)M * (size_t)N * sizeof(float);
-    if (!workspace || workspace_bytes < need) return B200Q_ERR_BAD_ARGUMENT;
-    p.partial = static_cast<float*>(workspace);
-  }
+  const size_t need = w4a16_workspace_bytes_impl(M, N, K);  // (the contract of the entry; no kernel uses it any more)
+  if (need && (!workspace || workspace_bytes < need)) return B200Q_ERR_BAD_ARGUMENT;
+  if (p.zp && (reinterpret_cast<uintptr_t>(p.zp) & 15)) return B200Q_ERR_UNSUPPORTED;
+  if (M <= 128) return w4a16_tmem_launch(x, ldx, qweight, scale, p.zp, 0, M, N, K, group, out, out_dtype, ldo, st);
   CUtensorMap ma, mr;
   int rc = 0;
-  const int bn_w = (!small_m && N > 128) ? 256 : 128;  // weight columns per stage tile
+  const int bn_w = N > 128 ? 256 : 128;  // weight columns per stage tile
   rc = make_tma_map_2d(&mr, qweight, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, N / 8, K, (N / 8) * 4, bn_w / 8, w4::kK,
                        CU_TENSOR_MAP_SWIZZLE_NONE);
   if (rc) return rc;
@@ -983,60 +929,13 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
     rc = w4::launch_pair<6, 2>(ma, mr1, ms1, mz1, pp, st);
     if (rc != B200Q_ERR_UNSUPPORTED) return rc;
   }
-  if (!small_m) {
-    p.x_tiles = (int)((M + 127) / 128);
-    const int bn = bn_w;
-    p.y_tiles = (int)((N + bn - 1) / bn);
-    rc = make_tma_map_2d(&ma, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, w4::kK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    if (bn == 256) rc = w4::launch<256, 8, 3, 1>(ma, mr, ms, mz, p, st);
-    else rc = w4::launch<128, 12, 4, 2>(ma, mr, ms, mz, p, st);
-  } else {
-    // small M, token-major with a narrow activation tile: 128 x 256 MMAs cover twice the weight
-    // columns per instruction of the weight-major form, whose issue rate is what bounds it
-    p.x_tiles = 1;
-    p.y_tiles = (int)((N + 255) / 256);
-    CUtensorMap mr2, ms2, mz2;
-    rc = make_tma_map_2d(&mr2, qweight, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, N / 8, K, (N / 8) * 4, 32, w4::kK,
-                         CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
-    rc = make_tma_map_2d(&ms2, scale, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K / group, N * 2, 256, 1, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (rc) return rc;
-    mz2 = ms2;
-    if (p.zp) {
-      rc = make_tma_map_2d(&mz2, p.zp, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, N / 8, K / group, (N / 8) * 4, 32, 1,
-                           CU_TENSOR_MAP_SWIZZLE_NONE);
-      if (rc) return rc;
-    }
-    const int ar = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
-    rc = make_tma_map_2d(&ma, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, w4::kK, ar, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (rc) return rc;
-    // three expander groups over four work slots (24 expander warps, 32 warps in all): the
-    // expand -> MMA -> release round trip of a work slot is what paces small M
-    switch (ar) {
-      case 16: rc = w4::launch<256, 8, 4, 3, 16, 8>(ma, mr2, ms2, mz2, p, st); break;
-      case 32: rc = w4::launch<256, 8, 4, 3, 32, 8>(ma, mr2, ms2, mz2, p, st); break;
-      case 64: rc = w4::launch<256, 6, 4, 3, 64, 8>(ma, mr2, ms2, mz2, p, st); break;
-      default: rc = w4::launch<256, 7, 3, 3, 0, 8>(ma, mr2, ms2, mz2, p, st); break;
-    }
-  }
+  p.x_tiles = (int)((M + 127) / 128);
+  p.y_tiles = (int)((N + bn_w - 1) / bn_w);
+  rc = make_tma_map_2d(&ma, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, w4::kK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
   if (rc) return rc;
-  if (p.splits > 1) {
-    const int esz = out_dtype == B200Q_BF16 ? 2 : 4;
-    const bool vec4 = (N % 4) == 0 && (ldo % 4) == 0 && (reinterpret_cast<uintptr_t>(out) % (4 * esz)) == 0 &&
-                      (reinterpret_cast<uintptr_t>(p.partial) & 15) == 0;
-    const int64_t total = vec4 ? M * N / 4 : M * N;
-    int grid = (int)((total + 255) / 256);
-    if (grid > kNumSMs * 8) grid = kNumSMs * 8;
-    auto kern = vec4 ? w4::splitk_reduce_kernel<4> : w4::splitk_reduce_kernel<1>;
-    if (launch_overlapped(kern, dim3((unsigned)grid), dim3(256), 0, st, (const float*)p.partial, out, out_dtype, M, N, ldo,
-                          p.splits) != cudaSuccess) {
-      (void)cudaGetLastError();
-      kern<<<grid, 256, 0, st>>>(p.partial, out, out_dtype, M, N, ldo, p.splits);
-    }
-    B200Q_LAUNCH_CHECK();
-  }
-  return B200Q_OK;
+  if (bn_w == 256) rc = w4::launch<256, 8, 3, 1>(ma, mr, ms, mz, p, st);
+  else rc = w4::launch<128, 12, 4, 2>(ma, mr, ms, mz, p, st);
+  return rc;
 }
 
 // ------------------------------------------------------------------------ allocation-free variant
@@ -1075,8 +974,6 @@ int w4a16_gemm_noalloc_impl(const void* x, int64_t ldx, const int32_t* qweight, 
   float* scratch = nullptr;
   int rc = static_scratch_ptr(&scratch);
   if (rc) return rc;
-  // Nothing in the scratch has to start at zero: every (split, row, column) cell that the
-  // reduction reads is written by exactly one CTA of this call first.
   return w4a16_gemm_impl(x, ldx, qweight, scale, zp, zp_kind, k_packed, M, N, K, group, out, out_dtype, ldo, scratch,
                          kStaticScratchBytes, st);
 }

@@ -330,9 +330,8 @@ int b200q_tp_reduce_bcast(const void* stage, void* const* out_ptrs_host, int tp,
  * scale    bf16 [K/group][N];  zp: NONE or PACKED int32 [K/group][N/8]
  * out      out_dtype F32/BF16 [M][N], row stride ldo
  * workspace  caller-owned device scratch of at least b200q_w4a16_workspace_bytes(M, N, K) bytes
- *            (0 for M > 128): for small M the K dimension is split over several CTAs per
- *            output tile and the fp32 partial tiles are summed by a second kernel.  May be
- *            NULL when the required size is 0.  Needs 16-byte alignment; contents are scratch.
+ *            (0 for M > 128).  May be NULL when the required size is 0.  Needs 16-byte alignment;
+ *            contents are scratch (the present kernels add their K splits on chip and leave it alone).
  * The fused kernel takes k_packed = 0 with K % 64 == 0, group % 64 == 0, K % group == 0,
  * N % 32 == 0 and 16-byte aligned bases; other cases return B200Q_ERR_UNSUPPORTED.
  */

@@ -280,3 +280,28 @@ def test_w4a16_kpacked_many_tokens_goes_through_repack(ops):
     a = torch.ops.b200q.w4a16_gemm(x.cuda(), _pack_k(w).cuda(), scale.cuda(), zp.cuda(), group, True, torch.bfloat16)
     b = torch.ops.b200q.w4a16_gemm(x.cuda(), O.pack_nibbles(w).cuda(), scale.cuda(), zp.cuda(), group, False, torch.bfloat16)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 63, 65, 96, 97, 128])
+@pytest.mark.parametrize("N,K,group", [(256, 64 * 61, 64), (96, 64 * 33, 64 * 33), (1024, 8192, 128)])
+@pytest.mark.parametrize("k_packed", [False, True])
+def test_w4a16_weights_in_tensor_memory(ops, M, N, K, group, k_packed):
+    """The kernel for up to 128 tokens at the edges of its dispatch: token counts around a change of the
+    number of expander groups, an odd number of k-blocks (also inside a cluster's share), columns that end inside a
+    tile, one group over all of K and one per k-block.  fp32 output against the fp64 product of the bf16 weights: sums
+    of up to 8192 fp32 terms in some order, 2e-5 as for the other forms."""
+    if k_packed and (M > 16 or N % 256 or K % 1024):
+        pytest.skip("the AutoGPTQ layout is taken up to 16 tokens, with N % 256 == 0 and K % 1024 == 0")
+    g = torch.Generator().manual_seed(M * 7 + N + K)
+    w = torch.randint(0, 16, (K, N), generator=g)
+    scale = (torch.rand(K // group, N, generator=g) * 0.015 + 0.005).to(torch.bfloat16)
+    zp = O.pack_nibbles(torch.randint(0, 16, (K // group, N), generator=g))
+    x = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    wdq = O.convert_from_uint4(O.pack_nibbles(w), scale, zp, torch.bfloat16)
+    e = x.double() @ wdq.double()
+    qw = (_pack_k(w) if k_packed else O.pack_nibbles(w)).cuda()
+    for dt, tol in ((torch.float32, 2e-5), (torch.bfloat16, 4e-3)):
+        r = torch.ops.b200q.w4a16_gemm(x.cuda(), qw, scale.cuda(), zp.cuda(), group, k_packed, dt)
+        assert O.rel_frobenius(r, e.float()) <= tol
+        assert torch.equal(r, torch.ops.b200q.w4a16_gemm(x.cuda(), qw, scale.cuda(), zp.cuda(), group, k_packed, dt))
+    assert ops.device_status() == 0
