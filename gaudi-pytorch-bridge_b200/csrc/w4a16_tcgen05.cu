@@ -473,7 +473,11 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
 // saw empty[s] and refilled the stage.  The MMA issuer waits on one barrier per stage, and
 // commits once.  Expander warps come in kExpandGroups groups that take alternate stages: the
 // chain wait -> load -> expand -> store -> fence -> arrive of one stage is several times
-// longer than the tensor-core time of a stage, so several stages are expanded concurrently.
+// longer than the tensor-core time of a stage, so several stages are expanded concurrently.  Most of that
+// chain is latency that does not grow with the words a thread expands, so few warps per stage and many
+// stages at once are the better split: three groups of four warps against two of eight, 2048 x 8192 x 8192
+// 240 -> 199 us, 300 x 4096 x 14336 78 -> 61, 1000 x 5120 x 2560 48 -> 38 (two groups of four: 220, 67, 42).
+// The number of groups divides the number of stages, so that a stage is always the same group's.
 template <int STAGES, int GROUPS>
 struct PairCfg {
   static constexpr int kActBytes = 128 * 128;
@@ -488,7 +492,7 @@ struct PairCfg {
   static constexpr int kBarOffset = STAGES * kStageBytes;
   static constexpr int kNumBars = 3 * STAGES + 4;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
-  static constexpr int kExpandWarps = 8;  // per stage
+  static constexpr int kExpandWarps = 4;  // per stage (see the head of this form)
   static constexpr int kExpandGroups = GROUPS;
   // Warp roles are placed by scheduler (warp % 4): the producer (warp 0) and the MMA issuer
   // (warp 4) share scheduler 0 with no expander warp; their per-stage instruction chains
@@ -499,6 +503,7 @@ struct PairCfg {
   static constexpr int kLastExpander = kExpandWarps * kExpandGroups - 1;
   static constexpr int kWarps = 5 + (kLastExpander / 3) * 4 + kLastExpander % 3 + 1;
   static_assert(kWarps <= 32, "too many expander warps for one CTA");
+  static_assert(STAGES % GROUPS == 0, "a stage belongs to one group");
   static constexpr int kThreads = 32 * kWarps;
   static_assert(kWOffset % 1024 == 0 && kStageBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
 };
@@ -680,7 +685,7 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     }
   } else if (role == kExpander) {
     // ------------------------------------------------------------ expanders
-    // this CTA's 128 columns: 8 warps per stage, 4 packed words per thread
+    // this CTA's 128 columns: 4 warps per stage, 8 packed words per thread
     const int et = (ewarp % C::kExpandWarps) * 32 + lane;
     const int my_group = ewarp / C::kExpandWarps;
     constexpr int W = 16;
@@ -926,7 +931,7 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
     }
     rc = make_tma_map_2d(&ma, x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, K, M, ldx * 2, w4::kK, 128, CU_TENSOR_MAP_SWIZZLE_128B);
     if (rc) return rc;
-    rc = w4::launch_pair<6, 2>(ma, mr1, ms1, mz1, pp, st);
+    rc = w4::launch_pair<6, 3>(ma, mr1, ms1, mz1, pp, st);
     if (rc != B200Q_ERR_UNSUPPORTED) return rc;
   }
   p.x_tiles = (int)((M + 127) / 128);
