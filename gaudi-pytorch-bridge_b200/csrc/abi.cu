@@ -38,22 +38,52 @@ int* device_status_ptr() {
   return static_cast<int*>(addr);
 }
 
-// Self-test of the bounded-wait mechanism: one warp waits on an mbarrier that nothing ever
-// arrives at, with a short poll limit.  The wait must give up, record `code` in the status
-// word and let the kernel finish normally -- the same path a production kernel takes when a
-// producer or a peer never shows up.
+// Self-test of the bounded waits with a short poll limit, in the two forms the kernels use.  Warp 0 waits
+// on an mbarrier that nothing ever arrives at (mbar_wait): the wait must give up, record `code` in the
+// status word and let the kernel finish normally -- the path a production kernel takes when a producer or a
+// peer never shows up.  Warps 1 and 2 are a producer and a consumer of a two-slot ring in the form of the
+// whole-warp roles (mbar_wait_uniform), between which no data ever arrives: the producer must arm each
+// slot once and leave its loop instead of arming a slot again whose phase has not completed, the consumer must
+// release nothing, and both must come to the end.  -code in the status word means that they did not.
 __global__ void wait_timeout_selftest_kernel(int* status, int code, uint32_t limit) {
-  __shared__ uint64_t bar;
-  __shared__ int abort_flag;
-  const uint32_t b = ptx::smem_u32(&bar);
+  __shared__ uint64_t bar, full[2], empty[2];
+  __shared__ int abort_flag, ring_abort, ring_status, armed, released;
+  const uint32_t b = ptx::smem_u32(&bar), f = ptx::smem_u32(full), e = ptx::smem_u32(empty);
   if (threadIdx.x == 0) {
     ptx::mbar_init(b, 1);
-    abort_flag = 0;
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(f + 8 * i, 1);
+      ptx::mbar_init(e + 8 * i, 1);
+    }
+    abort_flag = ring_abort = ring_status = armed = released = 0;
     ptx::fence_barrier_init();
   }
   __syncthreads();
-  ptx::mbar_wait(b, 0, &abort_flag, status, code, 0, limit);  // phase 0 never completes
+  const int warp = ptx::uniform_warp_index();
+  uint32_t slot = 0, phase = 0;
+  if (warp == 0) {
+    ptx::mbar_wait(b, 0, &abort_flag, status, code, 0, limit);  // phase 0 never completes
+  } else if (warp == 1) {
+    for (int i = 0; i < 64; ++i) {
+      if (!ptx::mbar_wait_uniform(e + 8 * slot, phase ^ 1, &ring_abort, &ring_status, code, limit)) break;
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive_expect_tx(f + 8 * slot, 16);  // (for a copy that is never made)
+        ++armed;
+      }
+      if (++slot == 2) { slot = 0; phase ^= 1; }
+    }
+  } else {
+    for (int i = 0; i < 64; ++i) {
+      if (!ptx::mbar_wait_uniform(f + 8 * slot, phase, &ring_abort, &ring_status, code, limit)) break;
+      if (ptx::elect_one()) {
+        ptx::mbar_arrive(e + 8 * slot);
+        ++released;
+      }
+      if (++slot == 2) { slot = 0; phase ^= 1; }
+    }
+  }
   __syncthreads();
+  if (threadIdx.x == 0 && (armed != 2 || released != 0 || ring_abort == 0 || ring_status != code)) atomicExch(status, -code);
 }
 
 int cast_to_fp8_impl(const void*, int, void*, int, const float*, float, int, int64_t, int64_t, float*, int, uint64_t,
@@ -137,7 +167,7 @@ int b200q_selftest_wait_timeout(int code, void* stream) {
   int* status = device_status_ptr();
   if (!status) return B200Q_ERR_CUDA;
   if (code == 0) return B200Q_ERR_BAD_ARGUMENT;
-  wait_timeout_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(status, code, 1u << 12);
+  wait_timeout_selftest_kernel<<<1, 96, 0, static_cast<cudaStream_t>(stream)>>>(status, code, 1u << 12);
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
 }

@@ -486,7 +486,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     // ------------------------------------------------------------ TMA producer
     uint32_t stage = 0, phase = 0;
     int nth = 0;  // stages issued so far
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
       for (int kb0 = 0; kb0 < num_kb; kb0 += KPS, ++nth) {
         const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
@@ -500,7 +501,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 tma_load_2d(smem_base + stage * L::kStageBytes + j * L::kSubBytes + L::kXBytes, &map_y, full, (kb0 + j) * kBlockK, yt * BN);
           }
         } else {
-          mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+          ok = mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+          if (!ok) break;
           if (elect_one()) {
             mbar_arrive_expect_tx(full, nsub * (L::kSubBytes - (kBlockX - p.x_tile_rows) * kBlockK));
             // K-major operand: box = 128 bytes of k x rows.  MN-major operand (stored [K][rows]):
@@ -543,13 +545,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     static_assert(kBlockK / kUmmaK == 4, "umma_f8_x4 issues 4 MMAs");
     uint32_t stage = 0, phase = 0;
     int it = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-      mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      ok = mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * BN;
       for (int kb0 = 0; kb0 < num_kb; kb0 += KPS) {
-        mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
+        ok = mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
+        if (!ok) break;  // (the accumulator is not published)
         tc_fence_after();
         const int nsub = num_kb - kb0 < KPS ? num_kb - kb0 : KPS;
         const uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
@@ -598,7 +603,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   }
 
   // ---------------------------------------------------------------- teardown
-  __syncwarp();  // lanes 1..31 of the single-thread roles rejoin lane 0 here
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
@@ -692,12 +697,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
     uint32_t stage = 0, phase = 0;
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
       const int x_row = xt * 2 * kBlockX + (int)rank * kBlockX;
       const int y_row = yt * BN + (int)rank * (BN / 2);
       for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        ok = mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (!ok) break;
         if (elect_one()) {
           const uint32_t full_leader = (bar_full + 8 * stage) & kPeerBitMask;
           if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * L::kStageBytes);
@@ -716,13 +723,18 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       static_assert(kBlockK / kUmmaK == 4 && (kUmmaK >> 4) == 2, "umma_f8_pair_x4 issues 4 MMAs 32 bytes apart");
       uint32_t stage = 0, phase = 0;
       int it = 0;
-      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+        ok = mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
+          // (on a wait that runs out the accumulator is published to neither CTA: the peer's epilogue, which
+          // knows only its own CTA's flag, must not take it for complete; its wait runs out in turn)
+          ok = mbar_wait_uniform(bar_full + 8 * stage, phase, abort_flag, p.status, kErrMma);
+          if (!ok) break;
           tc_fence_after();
           const uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
           const uint64_t yd = yd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));

@@ -285,16 +285,19 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // ------------------------------------------------------------ producer
     uint32_t ks = 0, kph = 0, vs = 0, vph = 0;
     ScoreStream ss(p);
+    bool ok = true;
     auto load_k = [&]() {
       if (ss.first()) {
         const uint32_t qb = ss.it & 1;
-        mbar_wait_uniform(bar_qe + 8 * qb, ((ss.it >> 1) & 1) ^ 1, abort_flag, p.status, kErrProducer);
+        ok = mbar_wait_uniform(bar_qe + 8 * qb, ((ss.it >> 1) & 1) ^ 1, abort_flag, p.status, kErrProducer);
+        if (!ok) return;
         if (elect_one()) {
           mbar_arrive_expect_tx(bar_qf + 8 * qb, kTile);
           tma_load_3d(sbase + Smem::kQ + qb * kTile, &map_q, bar_qf + 8 * qb, 0, (int)ss.w.q0, (int)ss.w.bh);
         }
       }
-      mbar_wait_uniform(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer);
+      ok = mbar_wait_uniform(bar_ke + 8 * ks, kph ^ 1, abort_flag, p.status, kErrProducer);
+      if (!ok) return;
       if (elect_one()) {
         const uint32_t dst = sbase + Smem::kK + ks * (2 * kTile), full = bar_kf + 8 * ks;
         const bool two = two_blocks(ss.w, ss.step());
@@ -306,13 +309,14 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       ss.next(p);
     };
     // (keys run two steps ahead of values: a key tile is wanted when its group still works on the step before)
-    for (int a = 0; a < 2 && ss.more; ++a) load_k();
+    for (int a = 0; a < 2 && ss.more && ok; ++a) load_k();
     Item w;
-    for (int it = 0; get_item(p, it, &w); ++it)
-      for (int t = 0; t < 2 * w.steps; ++t) {
+    for (int it = 0; ok && get_item(p, it, &w); ++it)
+      for (int t = 0; t < 2 * w.steps && ok; ++t) {
         if (ss.more) load_k();
-        for (int b = 2 * (t - w.steps); b >= 0 && b < 2 * (t - w.steps) + 2 && b < w.nblk; ++b) {
-          mbar_wait_uniform(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer);
+        for (int b = 2 * (t - w.steps); ok && b >= 0 && b < 2 * (t - w.steps) + 2 && b < w.nblk; ++b) {
+          ok = mbar_wait_uniform(bar_ve + 8 * vs, vph ^ 1, abort_flag, p.status, kErrProducer);
+          if (!ok) break;
           if (elect_one()) {
             mbar_arrive_expect_tx(bar_vf + 8 * vs, kTile);
             tma_load_3d(sbase + Smem::kV + vs * kTile, &map_v, bar_vf + 8 * vs, 0, b * kBN, (int)w.kv);
@@ -331,14 +335,14 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       const uint32_t qb = ss.it & 1;
       const bool two = two_blocks(ss.w, ss.step());
       const uint64_t qd = qd0 + qb * kTileStep, kd = kd0 + ks * (2 * kTileStep);
-      if (ss.first()) mbar_wait_uniform(bar_qf + 8 * qb, (ss.it >> 1) & 1, abort_flag, p.status, kErrMma);
-      mbar_wait_uniform(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma);
+      if (ss.first() && !mbar_wait_uniform(bar_qf + 8 * qb, (ss.it >> 1) & 1, abort_flag, p.status, kErrMma)) break;
+      if (!mbar_wait_uniform(bar_kf + 8 * ks, kph, abort_flag, p.status, kErrMma)) break;
       if (!ss.second()) {
         const uint32_t reg = ss.step() & 1;
         // region B holds the accumulator of the item before until its epilogue has read it
-        if (ss.step() == 1 && ss.it > 0) mbar_wait_uniform(bar_oe, (ss.it - 1) & 1, abort_flag, p.status, kErrMma);
-        mbar_wait_uniform(bar_se + 16 * reg, (eph >> (2 * reg)) & 1, abort_flag, p.status, kErrMma);
-        if (two) mbar_wait_uniform(bar_se + 16 * reg + 8, (eph >> (2 * reg + 1)) & 1, abort_flag, p.status, kErrMma);
+        if (ss.step() == 1 && ss.it > 0 && !mbar_wait_uniform(bar_oe, (ss.it - 1) & 1, abort_flag, p.status, kErrMma)) break;
+        if (!mbar_wait_uniform(bar_se + 16 * reg, (eph >> (2 * reg)) & 1, abort_flag, p.status, kErrMma)) break;
+        if (two && !mbar_wait_uniform(bar_se + 16 * reg + 8, (eph >> (2 * reg + 1)) & 1, abort_flag, p.status, kErrMma)) break;
         tc_fence_after();
         if (elect_one()) {
           umma_f8_x4(tmem + reg * 256, qd, kd, two ? idesc2 : idesc1, 0u, 2, 2);
@@ -348,7 +352,7 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         eph ^= (two ? 3u : 1u) << (2 * reg);
       } else {
-        mbar_wait_uniform(bar_se, eph & 1, abort_flag, p.status, kErrMma);
+        if (!mbar_wait_uniform(bar_se, eph & 1, abort_flag, p.status, kErrMma)) break;
         tc_fence_after();
         if (elect_one()) {
           umma_f8_x4(tmem, qd, kd, idesc1, 0u, 2, 2);
@@ -356,7 +360,7 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         eph ^= 1u;
         if (two) {
-          mbar_wait_uniform(bar_se + 8, (eph >> 1) & 1, abort_flag, p.status, kErrMma);
+          if (!mbar_wait_uniform(bar_se + 8, (eph >> 1) & 1, abort_flag, p.status, kErrMma)) break;
           tc_fence_after();
           if (elect_one()) {
             umma_f8_x4(tmem + 128, qd, kd + kTileStep, idesc1, 0u, 2, 2);
@@ -380,11 +384,13 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     constexpr uint32_t kTileStep = kTile >> 4;
     uint32_t vs = 0, vph = 0, pph = 0;  // pph bit g: parity of group g's next P tile
     Item w;
-    for (int it = 0; get_item(p, it, &w); ++it)
+    bool ok = true;
+    for (int it = 0; ok && get_item(p, it, &w); ++it)
       for (int b = 0; b < w.nblk; ++b) {
         const uint32_t g = b & 1;
-        mbar_wait_uniform(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma);
-        mbar_wait_uniform(bar_pf + 8 * g, (pph >> g) & 1, abort_flag, p.status, kErrMma);
+        ok = mbar_wait_uniform(bar_vf + 8 * vs, vph, abort_flag, p.status, kErrMma) &&
+             mbar_wait_uniform(bar_pf + 8 * g, (pph >> g) & 1, abort_flag, p.status, kErrMma);
+        if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
           umma_f8_x4(tmem + 256, pd0 + g * kTileStep, vd0 + vs * kTileStep, idesc_o, b > 0 ? 1u : 0u, 2, 256);
@@ -397,9 +403,9 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       }
   } else {
     // ------------------------------------------------------------ softmax (warps 2..9)
-    // A wait that runs out sets the abort flag, on which every later wait gives up at once: the
-    // loops below then run to their end on whatever is there, with all barriers among the softmax
-    // warps in place, and nothing is stored.
+    // A warp whose wait ran out (ok = false) hands nothing on any more -- no P tile, so that no accumulator of
+    // this or a later item is completed and no warp stores one -- and goes through its items only for the two
+    // barriers among the softmax warps.
     const int grp = (warp - 2) >> 2;          // 0 / 1: which 128 keys of a step
     const int qtr = warp & 3;                 // TMEM lane quarter of this warp
     const int row = qtr * 32 + lane;          // query row inside the block = TMEM lane
@@ -407,6 +413,7 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     float* stats = reinterpret_cast<float*>(smem + Smem::kStats);
     const float lq = log2f(p.q_scale_s);
     uint32_t fph = 0, pph = 1;                // parities: bit r of the next score tile in region r, of the P tile to be free
+    bool ok = true;
     Item w;
     for (int it = 0; get_item(p, it, &w); ++it) {
       const int64_t qi = w.q0 + row;          // query index
@@ -424,7 +431,8 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const uint32_t t_score = t_lane + 256 * reg + 128 * grp, bar = 16 * reg + 8 * grp;
         const int64_t key0 = (int64_t)(2 * j + grp) * kBN;
         uint8_t* prow = smem + Smem::kP + grp * kTile + row * 128;
-        mbar_wait_uniform(bar_sf + bar, (fph >> reg) & 1, abort_flag, p.status, kErrSoftmax);
+        ok = mbar_wait_uniform(bar_sf + bar, (fph >> reg) & 1, abort_flag, p.status, kErrSoftmax);
+        if (!ok) return;
         fph ^= 1u << reg;
         tc_fence_after();
         auto release_scores = [&]() {
@@ -432,7 +440,10 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           __syncwarp();
           if (lane == 0) mbar_arrive(bar_se + bar);
         };
-        auto wait_p_free = [&]() { mbar_wait_uniform(bar_pe + 8 * grp, pph, abort_flag, p.status, kErrSoftmax); };
+        auto wait_p_free = [&]() {
+          ok = mbar_wait_uniform(bar_pe + 8 * grp, pph, abort_flag, p.status, kErrSoftmax);
+          return ok;
+        };
         // keys of the block that this row may see: the first `lim` of them
         int64_t lim64 = (p.causal && qi + 1 < p.S ? qi + 1 : p.S) - key0;
         const int lim = lim64 > kBN ? kBN : (int)lim64;
@@ -459,14 +470,14 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             mx = fmaxf(mx, m * mul);
           } else {
             const uint64_t mul2 = pack_f32x2(mul, mul);
-            wait_p_free();
+            if (!wait_p_free()) return;
 #pragma unroll
             for (int c = 0; c < 4; ++c) chunk_exp(r + 32 * c, c, mul2, off2, ls, prow, row);
           }
         } else {
           const uint64_t one2 = pack_f32x2(1.f, 1.f);
           const int64_t qm = qi < p.L ? qi : p.L - 1;
-          if (second) wait_p_free();
+          if (second && !wait_p_free()) return;
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
             uint32_t r[32];
@@ -490,13 +501,13 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           pph ^= 1;
         }
       };
-      for (int j = 0; 2 * j + grp < w.nblk; ++j) do_step(j, std::false_type{});
+      for (int j = 0; ok && 2 * j + grp < w.nblk; ++j) do_step(j, std::false_type{});
       // between the passes the groups meet: the row maximum over all blocks
       st_max[grp * 128 + row] = mx;
       named_bar_sync(1, 256);
       mx = fmaxf(st_max[row], st_max[128 + row]);
       off = lq - mx;
-      for (int j = 0; 2 * j + grp < w.nblk; ++j) do_step(j, std::true_type{});
+      for (int j = 0; ok && 2 * j + grp < w.nblk; ++j) do_step(j, std::true_type{});
       // ---- output: O / l, scaled.  The row sums of both groups are added, then group 0 writes the
       // first 64 output columns of its rows and group 1 the other 64.
       float l4[4];
@@ -505,12 +516,13 @@ sdpa_fp8_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       st_sum[grp * 128 + row] = (l4[0] + l4[1]) + (l4[2] + l4[3]);
       named_bar_sync(1, 256);
       const float lsum = (st_sum[row] + st_sum[128 + row]) / p.q_scale_s;
-      mbar_wait_uniform(bar_of, it & 1, abort_flag, p.status, kErrSoftmax);
+      ok = ok && mbar_wait_uniform(bar_of, it & 1, abort_flag, p.status, kErrSoftmax);
+      if (!ok) continue;
       tc_fence_after();
       const float linv = lsum > 0.f ? 1.f / lsum : 0.f;
       const float osc = p.o_scale * linv;
       float amax_o = 0.f;
-      const bool in = qi < p.L && !*abort_flag;
+      const bool in = qi < p.L;
       uint32_t r[64];
       const int c0 = 64 * grp;
       tmem_ld_32x32(t_lane + 256 + c0, r);

@@ -92,26 +92,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return false;
 }
 
-// The form for roles that a whole warp runs: control flow that is the same for all 32 lanes, with
-// nothing depending on the outcome of a wait, lets the compiler keep addresses and descriptors in
-// uniform registers; a single-lane role spends some 200 cycles per wait and 60 per MMA on getting
-// them there.  A wait that runs out sets the flag, on which every later wait gives up at once: the
-// role then runs to its end on whatever is in the buffers (nothing of it is stored) and the CTA
-// ends in the ordinary way.
-__device__ __forceinline__ void mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (mbar_try_wait(bar, parity)) return;
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    if ((i & 63u) == 0u && *abort_flag) return;
-    if (mbar_try_wait(bar, parity)) return;
+// The form for roles that a whole warp runs: control flow that is the same for all 32 lanes lets the
+// compiler keep addresses and descriptors in uniform registers; a single-lane role spends some 200
+// cycles per wait and 60 per MMA on getting them there.  The outcome is a vote, so it is the same for
+// all lanes too.  False when the wait ran out or another role's has: the role must then neither
+// arrive, commit, copy nor issue anything more -- a barrier whose phase has not completed takes no
+// further arrivals -- and leave its loops (or go through them for the named barriers it shares with
+// other warps only), so that the CTA ends in the ordinary way with one ring of copies in flight at most.
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait_uniform(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                                int code, uint32_t limit = kWaitLimit) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  for (uint32_t i = 0; i < limit; ++i) {
+    if ((i & 63u) == 0u && __any_sync(0xFFFFFFFFu, *abort_flag)) return false;
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
     if (i > 4096u) __nanosleep(64);
   }
   *abort_flag = 1;
   atomicCAS(status, 0, code);
+  return false;
 }
 // The same for two barriers at once: the two polls are in flight together (a poll of a completed phase takes
 // about a hundred cycles).
-__device__ __forceinline__ void mbar_wait2_uniform(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
-                                                   volatile int* abort_flag, int* status, int code) {
+[[nodiscard]] __device__ __forceinline__ bool mbar_wait2_uniform(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
+                                                                 volatile int* abort_flag, int* status, int code) {
   uint32_t ok;
   asm volatile(
       "{\n"
@@ -124,9 +127,8 @@ __device__ __forceinline__ void mbar_wait2_uniform(uint32_t bar0, uint32_t parit
       : "=r"(ok)
       : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
       : "memory");
-  if (ok) return;
-  mbar_wait_uniform(bar0, parity0, abort_flag, status, code);
-  mbar_wait_uniform(bar1, parity1, abort_flag, status, code);
+  if (__all_sync(0xFFFFFFFFu, ok)) return true;
+  return mbar_wait_uniform(bar0, parity0, abort_flag, status, code) && mbar_wait_uniform(bar1, parity1, abort_flag, status, code);
 }
 // The index of the calling warp, known to be the same in all its lanes.
 __device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }

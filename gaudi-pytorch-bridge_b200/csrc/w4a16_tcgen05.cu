@@ -225,12 +225,14 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     // mbar_wait_uniform.)
     const bool meta = role == kProducerMeta;
     uint32_t slot = 0, phase = 0;
-    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
       int xt, yt;
       decode(w, xt, yt);
       const int n0 = yt * BN;
       for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        ok = mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (!ok) break;
         const uint32_t sbase = raw_base + slot * C::kRawSlotBytes;
         const uint32_t full = bar_raw_full + 8 * slot;
         const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
@@ -250,12 +252,14 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
   } else if (role == kProducerAct) {
     // ------------------------------------------------------------ activation producer (work ring)
     uint32_t slot = 0, phase = 0;
-    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
       int xt, yt;
       decode(w, xt, yt);
       const int act_row0 = xt * 128;
       for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait_uniform(bar_w_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        ok = mbar_wait_uniform(bar_w_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (!ok) break;
         if (elect_one()) {
           mbar_arrive_expect_tx(bar_w_ready + 8 * slot, C::kActBytes);
           tma_load_2d(smem_base + slot * C::kWorkSlotBytes, &map_act, bar_w_ready + 8 * slot, kb * kK, act_row0);
@@ -272,15 +276,18 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     uint32_t stage = 0, phase = 0;  // work-ring slot
     uint32_t rslot = 0;
     int it = 0;
-    for (int w = blockIdx.x; w < num_work; w += gridDim.x, ++it) {
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++it) {
       int xt, yt;
       decode(w, xt, yt);
       const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-      mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      ok = mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+      if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + acc * BN;
       for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait_uniform(bar_w_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
+        ok = mbar_wait_uniform(bar_w_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
+        if (!ok) break;  // (the accumulator is not published)
         tc_fence_after();
         // activations: K-major, 32 bytes per k-step inside the 128-byte row; weights: MN-major,
         // two 8-k atoms (2048 bytes) per k-step, column blocks 8 atoms apart (descriptors of
@@ -394,7 +401,8 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
     advance(rslot, rphase, my_group, RS);
     advance(wslot, wphase, my_group, WS);
     int lead = my_group;  // k-blocks of the next work item that belong to other groups before ours
-    for (int w = blockIdx.x; w < num_work; w += gridDim.x) {
+    bool ok = true;
+    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
       int xt, yt;
       decode(w, xt, yt);
       GroupRegs g;
@@ -403,8 +411,9 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
       for (; kb < num_kb; kb += C::kExpandGroups) {
         {
           // the packed weights have landed and the work slot's previous tile has been consumed
-          mbar_wait_uniform(bar_raw_full + 8 * rslot, rphase, abort_flag, p.status, kErrExpand);
-          mbar_wait_uniform(bar_w_empty + 8 * wslot, wphase ^ 1, abort_flag, p.status, kErrExpand);
+          ok = mbar_wait_uniform(bar_raw_full + 8 * rslot, rphase, abort_flag, p.status, kErrExpand) &&
+               mbar_wait_uniform(bar_w_empty + 8 * wslot, wphase ^ 1, abort_flag, p.status, kErrExpand);
+          if (!ok) break;
           const uint32_t rbase = raw_base + rslot * C::kRawSlotBytes;
           const uint32_t wbase = smem_base + wslot * C::kWorkSlotBytes;
           const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
@@ -572,12 +581,14 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     // ------------------------------------------------------------ TMA producer
     uint32_t stage = 0, phase = 0;
     const uint32_t meta_bytes = C::kScaleBytes + (p.zp ? C::kZpBytes : 0);
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
       const int act_row0 = xt * 256 + (int)rank * 128;
       const int n0 = yt * BN + (int)rank * kUnit;
       for (int kb = 0; kb < num_kb; ++kb) {
-        mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        ok = mbar_wait_uniform(bar_empty + 8 * stage, phase ^ 1, abort_flag, p.status, kErrProducer);
+        if (!ok) break;
         const uint32_t sbase = smem_base + stage * C::kStageBytes;
         const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
         if (elect_one()) {
@@ -602,13 +613,16 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
       const uint64_t dw0 = smem_desc_mn_sw128(smem_base + C::kWOffset, (kK / 8) * 1024, 1024);
       uint32_t stage = 0, phase = 0;
       int it = 0;
-      for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++it) {
         const uint32_t acc = it & 1, acc_phase = (it >> 1) & 1;
-        mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+        ok = mbar_wait_uniform(bar_tempty + 8 * acc, acc_phase ^ 1, abort_flag, p.status, kErrMmaTmem);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          mbar_wait_uniform(bar_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
+          ok = mbar_wait_uniform(bar_ready + 8 * stage, phase, abort_flag, p.status, kErrMma);
+          if (!ok) break;  // (the accumulator is published to neither CTA)
           tc_fence_after();
           const uint64_t soff = (uint64_t)(stage * (uint32_t)(C::kStageBytes >> 4));
           if (elect_one()) {
@@ -698,12 +712,14 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const uint32_t wt_off = C::kWOffset + ((ngl >> 3) * (kK / 8) + (kr >> 3)) * 1024 + krow * 128 + (((ngl & 7) ^ krow) << 4);
     uint32_t stage = 0, phase = 0;
     int turn = 0;  // whose stage this is
-    for (int tile = pair; tile < num_tiles; tile += num_pairs) {
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       GroupRegs g;
       int g_cur = -1;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (turn == my_group) {
-          mbar_wait_uniform(bar_raw + 8 * stage, phase, abort_flag, p.status, kErrExpand);
+          ok = mbar_wait_uniform(bar_raw + 8 * stage, phase, abort_flag, p.status, kErrExpand);
+          if (!ok) break;
           const uint32_t sbase = smem_base + stage * C::kStageBytes;
           const int grp = p.group_shift >= 0 ? (kb >> p.group_shift) : (kb * kK) / p.group;
           if (grp != g_cur) {

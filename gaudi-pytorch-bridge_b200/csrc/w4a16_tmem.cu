@@ -193,7 +193,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ------------------------------------------------------------ packed words
     uint32_t slot = 0, phase = 0;
     for (int st = 0; st < stages; ++st) {
-      mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrRaw);
+      if (!mbar_wait_uniform(bar_raw_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrRaw)) break;
       if (elect_one()) {
         const uint32_t full = bar_raw_full + 8 * slot, dst = base + slot * 2 * kUnitBytes;
         const int kb = kb0 + st * kStageKb;
@@ -215,7 +215,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     // ------------------------------------------------------------ activations
     uint32_t slot = 0, phase = 0;
     for (int st = 0; st < stages; ++st) {
-      mbar_wait_uniform(bar_x_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrAct);
+      if (!mbar_wait_uniform(bar_x_empty + 8 * slot, phase ^ 1, abort_flag, p.status, kErrAct)) break;
       if (elect_one()) {
         const uint32_t full = bar_x_full + 8 * slot, dst = base + kXOffset + slot * x_slot_bytes;
         const int i = st * kStageKb;
@@ -234,8 +234,10 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const uint32_t d = tmem + j * acc_cols;
     constexpr int kStep = TC == 1 ? 2 : 1;
     uint32_t xs = TC == 1 ? j : 0, xphase = 0, as = xs, aphase = 0;
+    bool ok = true;
     for (int st = TC == 1 ? (int)j : 0; st < stages; st += kStep) {
-      mbar_wait2_uniform(bar_x_full + 8 * xs, xphase, bar_a_full + 8 * as, aphase, abort_flag, p.status, kErrMma);
+      ok = mbar_wait2_uniform(bar_x_full + 8 * xs, xphase, bar_a_full + 8 * as, aphase, abort_flag, p.status, kErrMma);
+      if (!ok) break;
       tc_fence_after();
       const uint64_t xd = xd0 + (uint64_t)(xs * (x_slot_bytes >> 4));
       const uint32_t a = a_col + as * 64;
@@ -254,7 +256,7 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
       as += kStep;
       if (as >= (uint32_t)groups) { as -= groups; aphase ^= 1; }
     }
-    if (elect_one()) umma_commit(bar_d_full);
+    if (ok && elect_one()) umma_commit(bar_d_full);
   } else {
     // ------------------------------------------------------------ expanders
     const int qtr = warp & 3, grp = (warp - kExpWarp0) >> 2;
@@ -298,6 +300,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     const uint32_t sel0 = hfirst ? sel_hi : sel_lo, sel1 = hfirst ? sel_lo : sel_hi;
     const uint32_t blk_ld = oct * 512 + ng * 4 + swap * 64, blk_st = oct * 512 + ng * 32;
     const int pair_step = swap ? -64 : 64;
+    // (after a wait that ran out the warps of a group still meet at their barrier, which no limit ends)
+    bool ok = true;
     for (int st = grp < groups ? grp : stages; st < stages; st += groups) {
       const bool two = TC == 2 || 2 * st + 1 < kbn;
       uint32_t s2[2], z2[2];
@@ -306,7 +310,11 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         s2[h] = sn[h] * 0x00010001u;
         z2[h] = (((zn[h] >> (4 * ((h ? nb : na) & 7))) & 15u) * 0x00010001u) | 0x43004300u;
       }
-      mbar_wait_uniform(bar_raw_full + 8 * slot, phase, abort_flag, p.status, kErrExpand);
+      ok = ok && mbar_wait_uniform(bar_raw_full + 8 * slot, phase, abort_flag, p.status, kErrExpand);
+      if (!ok) {
+        if (!KP) named_bar_sync(1 + grp, 128);
+        continue;
+      }
       fetch(st + groups);
       const uint32_t raw = base + slot * 2 * kUnitBytes;
       if (!KP) {
@@ -336,7 +344,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
         for (int o = 0; o < 8; ++o) w[h][o] = lds32(raw + h * kUnitBytes + o * 512 + col * 4);
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_raw_empty + 8 * slot);
-      mbar_wait_uniform(bar_a_empty + 8 * as, aphase ^ 1, abort_flag, p.status, kErrExpand);
+      ok = mbar_wait_uniform(bar_a_empty + 8 * as, aphase ^ 1, abort_flag, p.status, kErrExpand);
+      if (!ok) continue;
       tc_fence_after();
       const uint32_t a = a_col + ((uint32_t)(qtr * 32) << 16) + as * 64;
 #pragma unroll
@@ -366,9 +375,8 @@ w4a16_tmem_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_consta
     }
     // accumulators -> fp32 tile [tc][token][128 columns] over the rings (every copy has landed and
     // been read when the last MMA retires)
-    mbar_wait_uniform(bar_d_full, 0, abort_flag, p.status, kErrEpilogue);
-    tc_fence_after();
-    if (!*abort_flag) {
+    if (ok && mbar_wait_uniform(bar_d_full, 0, abort_flag, p.status, kErrEpilogue)) {
+      tc_fence_after();
       for (int c = grp; c < TC * (nt >> 4); c += kMaxGroups) {
         const int ct = TC == 1 ? 0 : c & 1, t0 = (TC == 1 ? c : c >> 1) * 16;
         uint32_t d[16];

@@ -66,9 +66,9 @@ const char* b200q_last_cuda_error(void);
 /* Synchronises the current device, reads and clears the device status word.
  * 0 = every bounded wait completed; otherwise a kernel-specific code. */
 int b200q_device_status(int* code_out);
-/* Launches a one-warp kernel whose only wait can never be satisfied and has a short poll limit:
- * the wait gives up, stores `code` (non-zero) in the device status word and the kernel ends
- * normally.  b200q_device_status() then reports B200Q_ERR_DEVICE_TIMEOUT with that code and the
+/* Launches a small kernel whose waits can never be satisfied and have a short poll limit: the
+ * waits give up, `code` (non-zero) is stored in the device status word and the kernel ends
+ * normally (-code: the roles of a ring did not stop at the wait that ran out).  b200q_device_status() then reports B200Q_ERR_DEVICE_TIMEOUT with that code and the
  * context stays usable.  Exercises the path every tcgen05 kernel here takes when a barrier is
  * never signalled (the reference maps device errors to exceptions in
  * backend/synapse_helpers/synapse_error.h). */

@@ -20,6 +20,17 @@ def test_bounded_wait_reports_and_context_survives():
     assert abi.lib.b200q_selftest_wait_timeout(0, None) == -1
 
 
+def test_roles_stop_at_the_wait_that_runs_out():
+    """A producer and a consumer of a ring between which nothing arrives: a slot whose phase has not completed is not
+    armed a second time, nothing is released, and both end (the kernel reports -code otherwise)."""
+    import b200_hpu_ops
+    from b200_hpu_ops import abi
+    for code in (17, 18, 19):
+        assert abi.lib.b200q_selftest_wait_timeout(code, abi.stream_ptr()) == 0
+        assert b200_hpu_ops.device_status() == code
+    assert b200_hpu_ops.device_status() == 0
+
+
 def test_status_codes_have_text():
     from b200_hpu_ops import abi
     assert b"bounded wait" in abi.lib.b200q_strerror(-5)
