@@ -513,6 +513,26 @@ ScaleArg to_scale_arg(const OptTensor& t) {
   return s;
 }
 
+// K not a multiple of 16 with an operand stored [rows][K]: its row pitch is not 16-byte granular and
+// the tensor-core kernels (TMA) cannot take it; the CUDA-core kernel that can is two to three orders
+// of magnitude slower.  For problems large enough to matter both operands are copied into
+// buffers with K rounded up to 16, the extra k filled with zeros (fp8 0x00 = +0 adds nothing).
+// Returns the K of the operands as they are then.
+int64_t pad_k_for_tma(at::Tensor& a, bool ta, at::Tensor& b, bool tb, int64_t M, int64_t N, int64_t K) {
+  if ((K % 16) == 0 || (ta && !tb) || (double)M * (double)N * (double)K < (double)(1 << 26)) return K;
+  const int64_t Kk = (K + 15) / 16 * 16;
+  auto pad_k = [&](at::Tensor& t, int64_t kdim) {
+    auto sizes = t.sizes().vec();
+    sizes[t.dim() + kdim] = Kk;
+    at::Tensor padded = at::zeros(sizes, t.options().dtype(at::kByte));
+    padded.narrow(kdim, 0, K).copy_(t.view(at::kByte));
+    t = padded.view(t.scalar_type());
+  };
+  pad_k(a, ta ? -2 : -1);
+  pad_k(b, tb ? -1 : -2);
+  return Kk;
+}
+
 // out8_dtype / out8_scale: fused output cast (b200q::fp8_gemm_cast); Undefined = plain fp8_gemm_v2.
 at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tensor& B, bool trans_B, const OptTensor& D,
                               at::ScalarType out_dtype, const ScaleArg& A_scale_inv, const ScaleArg& B_scale_inv,
@@ -586,23 +606,7 @@ at::Tensor fp8_gemm_v2_common(const at::Tensor& A, bool trans_A, const at::Tenso
   };
   as_matrix(a);
   as_matrix(b);
-  // K not a multiple of 16 with an operand stored [rows][K]: its row pitch is not 16-byte granular and
-  // the tensor-core kernels (TMA) cannot take it; the CUDA-core kernel that can is two to three orders
-  // of magnitude slower.  For problems large enough to matter both operands are copied into
-  // buffers with K rounded up to 16, the extra k filled with zeros (fp8 0x00 = +0 adds nothing).
-  int64_t Kk = K;
-  if ((K % 16) != 0 && (!ta || tb) && (double)Mk * (double)N * (double)K >= (double)(1 << 26)) {
-    Kk = (K + 15) / 16 * 16;
-    auto pad_k = [&](at::Tensor& t, int64_t kdim) {
-      auto sizes = t.sizes().vec();
-      sizes[t.dim() + kdim] = Kk;
-      at::Tensor padded = at::zeros(sizes, t.options().dtype(at::kByte));
-      padded.narrow(kdim, 0, K).copy_(t.view(at::kByte));
-      t = padded.view(t.scalar_type());
-    };
-    pad_k(a, ta ? -2 : -1);
-    pad_k(b, tb ? -1 : -2);
-  }
+  const int64_t Kk = pad_k_for_tma(a, ta, b, tb, Mk, N, K);
   const int64_t kbatch = folded ? 1 : batch;
   g.A = a.data_ptr(); g.B = b.data_ptr();
   g.a_dtype = to_b200q_dtype(a.scalar_type()); g.b_dtype = to_b200q_dtype(b.scalar_type());
@@ -969,11 +973,12 @@ at::Tensor fp8_gemm_swiglu_cast(const at::Tensor& x8, const at::Tensor& w_gate_u
   at::Tensor a = x8.contiguous(), b = w_gate_up.contiguous();
   at::Tensor out = new_tensor({M, F}, at::kFloat8_e4m3fn, x8.device());
   if (out.numel() == 0) return out;
+  const int64_t Kk = pad_k_for_tma(a, false, b, true, M, N, K);
   b200q_gemm_args g{};
   g.A = a.data_ptr(); g.B = b.data_ptr();
   g.a_dtype = to_b200q_dtype(a.scalar_type()); g.b_dtype = to_b200q_dtype(b.scalar_type());
   g.trans_a = 0; g.trans_b = 1;
-  g.M = M; g.N = N; g.K = K; g.lda = K; g.ldb = K; g.batch = 1;
+  g.M = M; g.N = N; g.K = Kk; g.lda = Kk; g.ldb = Kk; g.batch = 1;
   g.out = out.data_ptr(); g.out_dtype = B200Q_BF16; g.ldo = F;
   at::Tensor sa, sb;
   if (x_scale_inv.has_value() && x_scale_inv->defined()) {

@@ -62,6 +62,26 @@ def test_fused_gate_up_swiglu_is_bit_identical(T):
     assert b200_hpu_ops.device_status() == 0
 
 
+@pytest.mark.parametrize("T,d,f", [(300, 1000, 512), (64, 4104, 3584), (129, 1025, 256), (129, 100, 128)])
+def test_fused_gate_up_swiglu_with_a_ragged_inner_dimension(T, d, f):
+    """d not a multiple of 16, which TMA cannot address: from 2^26 products on the operands are padded, as in fp8_gemm_v2,
+    and the tensor-core kernels run (one fused launch from 129 tokens on).  The bytes of the two operators."""
+    import b200_hpu_ops
+    g = torch.Generator().manual_seed(T + d)
+    x8 = (torch.randn(T, d, generator=g) * 40).to(torch.float8_e4m3fn).cuda()
+    w8 = (torch.randn(2 * f, d, generator=g) * 40).to(torch.float8_e4m3fn).cuda()
+    xs, ws = torch.tensor(0.01, device="cuda"), (torch.rand(2 * f, generator=g) * 2e-3).cuda()
+    n0 = b200_hpu_ops.launch_count()
+    h = torch.ops.b200q.fp8_gemm_swiglu_cast(x8, w8, xs, ws, 20.0)
+    launches = b200_hpu_ops.launch_count() - n0
+    assert launches == (1 if T > 128 and T * 2 * f * d >= 1 << 26 else 2)
+    gu = torch.ops.hpu.fp8_gemm_v2(x8, False, w8, True, None, torch.bfloat16, xs, ws, None, False, [1, 2 * f])
+    gu = gu.view(T, f // 128, 2, 128)
+    ref, _ = torch.ops.b200q.swiglu_cast_fp8(gu[:, :, 0].reshape(T, f), gu[:, :, 1].reshape(T, f), 20.0, False)
+    assert torch.equal(h.view(torch.uint8), ref.view(torch.uint8))
+    assert b200_hpu_ops.device_status() == 0
+
+
 def _free_port():
     s = socket.socket()
     s.bind(("127.0.0.1", 0))
