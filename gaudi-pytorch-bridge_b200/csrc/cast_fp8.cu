@@ -787,26 +787,64 @@ int clear_amax(float* amax, cudaStream_t st) {
   return B200Q_OK;
 }
 
-// Casts with amax of at most this many elements run as ONE cluster of up to eight blocks that
-// reduces its amax by itself: one launch instead of two, where launches are what such a cast
-// costs.  Eight SMs move 2^18 elements in about 2 us, the time a second launch takes.
-constexpr int64_t kClusterCastMax = 1 << 18;
+static int scale_class(int mode) {
+  switch (mode) {
+    case B200Q_BCAST_PER_COL: return SC_COL;
+    case B200Q_BCAST_PER_ROW: return SC_ROW;
+    case B200Q_BCAST_FULL: return SC_FULL;
+    default: return SC_ONE;
+  }
+}
 
-// Up to this many elements a memset clears the amax word, above it clear_amax_kernel: a memset
-// costs the host 0.7 us where a launch costs 2.0, a cast of this size is over before the host has
-// issued the next one, and the launch gap that the clearing kernel hides does not show.
-constexpr int64_t kMemsetCastMax = 1 << 22;
+// A cast with amax takes one of three forms, by its number of elements:
+//   one cluster of up to eight blocks, which reduces its amax by itself: one launch, but eight SMs only;
+//   behind a memset of the amax word: 1.4 us less of host time than a clearing kernel, but 3.5 us of
+//     idle device, since nothing is set up across a memset;
+//   behind clear_amax_kernel.
+// So the first two end where eight SMs, or the idle time, last longer than the host takes to issue
+// the call, which comes the sooner the more a cast does per element.  us per call of the forms, launched back to
+// back (in brackets: in a graph, where the host costs nothing and the memset is never the best):
+//                                     2^15 elements          2^17                        2^18                   2^21
+//   vectors, to nearest               7.0 / 8.2 / 9.9        7.2 / 8.3 (2.7 / 6.0 / 2.6) 7.3 / 8.2 / 9.8        8.2 / 9.8
+//   the same, scale per column        8.0 / 9.2 / 10.9       8.0 / 9.1 (5.9 / 6.2 / 3.3) 10.5 / 9.2 / 10.8      9.2 / 10.6
+//   vectors, stochastic, bf16 -> e5m2 7.0 / 8.3 / 10.1       7.2 / 8.2                   7.3 / 8.3 / 9.8        8.2 / 9.6
+//   the same to e4m3                  7.0 / 8.2 / 9.7        7.3 / 8.3 (6.7 / 8.1 / 4.7) 12.1 / 8.2 / 9.8       9.9 / 9.7
+//   vectors, stochastic, otherwise    7.0 / 8.2 / 9.8        8.7 / 8.2 (8.0 / 6.2 / 3.6) 14.6 / 8.3 / 9.8       9.9 / 9.7
+//   element by element, to nearest    7.0 / 8.2 / 10.0       14.7 / 8.4 (14.1 / 8.2 / 5.3) 27 / 8.4 / 9.9       9.4 / 9.7
+//   the same, scale per row           8.6 / 11.5 / 10.7      28 / 12.4 (27 / 12.3 / 9.5) 52 / 12.4 / 10.4       14.4 / 11.0
+//   the same, stochastic              12.8 / 15.6 / 13.0     45 / 16.5 (44 / 16.4 / 13.7) 87 / 16.6 / 14.3      24 / 21
+// (packed: the kernels that round pairs of bf16 as they are.  To e4m3 a stochastic cast meets more values below the
+// smallest normal, which it rounds one by one.  Element by element: as the kernels go where pointers or row lengths rule vectors out; up to 2^15
+// elements the other forms have no more than eight blocks either).
+struct AmaxForms {
+  int64_t cluster, memset;  // up to how many elements
+};
+static AmaxForms amax_forms(bool vectors, bool stochastic, bool packed, int out_dtype, int sc) {
+  if (!vectors) return {1 << 15, stochastic || sc != SC_ONE ? 0 : 1 << 20};
+  if (stochastic && packed) return out_dtype == B200Q_E5M2 ? AmaxForms{1 << 18, 1 << 21} : AmaxForms{1 << 17, 1 << 20};
+  if (stochastic) return {1 << 16, 1 << 20};
+  if (sc == SC_COL || sc == SC_FULL) return {1 << 17, 1 << 21};
+  return {1 << 18, 1 << 22};
+}
 
 // Decides how a cast starts and clears its amax word where that is needed.
-static int cast_start(float* amax, int64_t n, cudaStream_t st, int* start) {
+static int cast_start(float* amax, int64_t n, AmaxForms forms, cudaStream_t st, int* start) {
   *start = kStartAfter;
   if (!amax) return B200Q_OK;
-  if (n > kMemsetCastMax) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
+  if (capture != cudaStreamCaptureStatusNone) {
+    forms.cluster >>= 2;
+    forms.memset = 0;
+  }
+  if (n > 0 && n <= forms.cluster) {
+    *start = kStartCluster;
+  } else if (n <= forms.memset || n == 0) {
+    B200Q_CUDA_OK(cudaMemsetAsync(amax, 0, sizeof(float), st));
+  } else {
     *start = kStartBehindClear;
     return clear_amax(amax, st);
   }
-  if (n > 0 && n <= kClusterCastMax) *start = kStartCluster;
-  else B200Q_CUDA_OK(cudaMemsetAsync(amax, 0, sizeof(float), st));
   return B200Q_OK;
 }
 template <typename Params>
@@ -843,15 +881,6 @@ static void launch_cast_sr(bool sr, int sc, int64_t items, cudaStream_t st, cons
   else launch_cast_sc<InT, FMT, false>(sc, items, st, p);
 }
 
-static int scale_class(int mode) {
-  switch (mode) {
-    case B200Q_BCAST_PER_COL: return SC_COL;
-    case B200Q_BCAST_PER_ROW: return SC_ROW;
-    case B200Q_BCAST_FULL: return SC_FULL;
-    default: return SC_ONE;
-  }
-}
-
 int cast_to_fp8_impl(const void* in, int in_dtype, void* out, int out_dtype, const float* scale,
                      float scale_host, int scale_mode, int64_t rows, int64_t cols, float* amax, int rounding,
                      uint64_t seed, uint64_t offset, uint64_t first_index, int flags, cudaStream_t st) {
@@ -861,8 +890,17 @@ int cast_to_fp8_impl(const void* in, int in_dtype, void* out, int out_dtype, con
     if (n) B200Q_CUDA_OK(cudaMemcpyAsync(out, in, (size_t)n, cudaMemcpyDeviceToDevice, st));
     return B200Q_OK;
   }
+  const int sc = scale_class(scale_mode);
+  const bool sr = rounding == B200Q_ROUND_STOCHASTIC;
+  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  // (as the kernels decide it)
+  const bool vectors = aligned && ((sc != SC_FULL && sc != SC_COL) || (reinterpret_cast<uintptr_t>(scale) & 15) == 0) &&
+                       ((sc != SC_COL && sc != SC_ROW) || cols % 16 == 0) && (!sr || (first_index & 15) == 0);
+  // fast path: bf16 input, product in bf16, one scale per 16-element chunk, aligned pointers
+  const bool fast = in_dtype == B200Q_BF16 && !(flags & B200Q_CAST_MUL_IN_FP32) && aligned &&
+                    (sc == SC_ONE || (sc == SC_ROW && cols % 16 == 0)) && (!sr || (first_index & 15) == 0);
   int start;
-  if (int rc = cast_start(amax, n, st, &start)) return rc;
+  if (int rc = cast_start(amax, n, amax_forms(vectors, sr, fast, out_dtype, sc), st, &start)) return rc;
   if (n == 0) return B200Q_OK;
   CastParams p;
   p.start = start;
@@ -871,13 +909,7 @@ int cast_to_fp8_impl(const void* in, int in_dtype, void* out, int out_dtype, con
   p.scale_from_dev = scale_mode == B200Q_BCAST_SCALAR_DEV;
   p.n = n; p.cols = cols; p.amax = amax; p.seed = seed; p.offset = offset; p.first_index = first_index;
   p.mul_fp32 = (flags & B200Q_CAST_MUL_IN_FP32) ? 1 : 0;
-  const int sc = scale_class(scale_mode);
   const int64_t items = (n + 15) / 16;
-  const bool sr = rounding == B200Q_ROUND_STOCHASTIC;
-  // fast path: bf16 input, RNE, product in bf16, one scale per 16-element chunk, aligned pointers
-  const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  const bool fast = in_dtype == B200Q_BF16 && !p.mul_fp32 && aligned &&
-                    (sc == SC_ONE || (sc == SC_ROW && cols % 16 == 0)) && (!sr || (first_index & 15) == 0);
   if (fast && sr) {
     const int64_t half = (items + 1) / 2;
     if (out_dtype == B200Q_E4M3) {
@@ -1004,8 +1036,11 @@ __global__ void __launch_bounds__(256) cast_hybrid_bf16_rne_fast_kernel(HybridPa
 int cast_hybrid_impl(const void* in, int in_dtype, void* out152, void* out143, const float* s152, float s152_host,
                      int mode152, const float* s143, float s143_host, int mode143, int64_t n, float* amax, int rounding,
                      uint64_t seed, uint64_t offset, uint64_t first_index, int flags, cudaStream_t st) {
+  const bool sr = rounding == B200Q_ROUND_STOCHASTIC;
+  const bool all_aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out152) |
+                             reinterpret_cast<uintptr_t>(out143)) & 15) == 0;
   int start;
-  if (int rc = cast_start(amax, n, st, &start)) return rc;
+  if (int rc = cast_start(amax, n, amax_forms(all_aligned && (first_index & 15) == 0, sr, false, 0, SC_ONE), st, &start)) return rc;
   if (n == 0) return B200Q_OK;
   HybridParams p;
   p.start = start;
@@ -1016,9 +1051,6 @@ int cast_hybrid_impl(const void* in, int in_dtype, void* out152, void* out143, c
   p.n = n; p.amax = amax; p.seed = seed; p.offset = offset; p.first_index = first_index;
   p.mul_fp32 = (flags & B200Q_CAST_MUL_IN_FP32) ? 1 : 0;
   const int64_t items = (n + 15) / 16;
-  const bool sr = rounding == B200Q_ROUND_STOCHASTIC;
-  const bool all_aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out152) |
-                             reinterpret_cast<uintptr_t>(out143)) & 15) == 0;
   if (in_dtype == B200Q_BF16 && !sr && !p.mul_fp32 && all_aligned) {
     launch_persistent(cast_hybrid_bf16_rne_fast_kernel, items, st, p, true);
   } else if (in_dtype == B200Q_BF16) {
