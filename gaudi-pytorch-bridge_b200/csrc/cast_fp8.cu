@@ -35,7 +35,7 @@ __device__ __forceinline__ void cast_begin(int start) {
   if (start == kStartBehindClear) {
     pdl_release();
   } else {
-    pdl_enter();
+    pdl_enter_spread();
     if (start == kStartCluster) cluster_amax_begin();
   }
 }
@@ -626,7 +626,7 @@ constexpr int kUncastUnroll = 8;
 
 template <typename OutT, int FMT, int SC>
 __global__ void __launch_bounds__(256) cast_from_fp8_kernel(UncastParams p) {
-  pdl_enter();
+  pdl_enter_spread();
   constexpr bool BF16 = InTraits<OutT>::kIsBf16;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
