@@ -70,8 +70,14 @@ __device__ __forceinline__ uint32_t nan_byte(float) {
   return 0x7Fu;
 }
 
+// Blocks per SM that the registers must leave room for (0: whatever the compiler takes; a stated 1 makes it take
+// more).  Stochastic: four (64 registers), without which two of the fp32 forms take 68: row scales, 2^26 elements, 100 -> 92 us,
+// element by element 565 -> 456.  bf16 with column scales: five (48), without which it takes 54: 60 -> 55 us.
+template <typename InT, bool SR, int SC>
+constexpr int cast_blocks_per_sm() { return SR ? 4 : InTraits<InT>::kIsBf16 && SC == SC_COL ? 5 : 0; }
+
 template <typename InT, int FMT, bool SR, int SC>
-__global__ void __launch_bounds__(256) cast_to_fp8_kernel(CastParams p) {
+__global__ void __launch_bounds__(256, cast_blocks_per_sm<InT, SR, SC>()) cast_to_fp8_kernel(CastParams p) {
   cast_begin(p.start);
   constexpr bool BF16 = InTraits<InT>::kIsBf16;
   const InT* __restrict__ in = static_cast<const InT*>(p.in);
@@ -329,9 +335,9 @@ __global__ void __launch_bounds__(256) cast_bf16_rne_fast_kernel(CastParams p) {
 // Same frame as the RNE fast path.  In the normal range a bf16 product needs only its low
 // g = 4 (e4m3) or 5 (e5m2) mantissa bits resolved, so stochastic rounding is a packed integer
 // add of g random bits to both halves of a bf16x2 word; one Philox block (16 random bytes) serves a
-// 16-element chunk (2^26 elements to e5m2 44.8 -> 44.4 us against masks, shifts and conversions; a third
-// fewer logic instructions gave so little that the pipe is not what bounds it, and five blocks per SM
-// instead of three, with 48 registers, spill: 53 us).  Chunks that hold a value below the smallest
+// 16-element chunk (2^26 elements to e5m2 45.4 -> 42.2 us against masks, shifts and conversions).  What bounds it
+// are the integer multiplications of Philox as much as latency at three blocks per SM (80 registers; row scales
+// without the bound 94 and two blocks: 109 -> 103 us to e4m3); five, with 48, spill: 53 us.  Chunks that hold a value below the smallest
 // normal, an infinity or a NaN take the general per-element routine instead (same definition).
 template <int FMT>
 __device__ __forceinline__ uint4 cast16_bf16_sr(const uint4 a, const uint4 b, uint32_t s2, bool has_scale,
@@ -393,7 +399,7 @@ __device__ __forceinline__ uint4 cast16_bf16_sr(const uint4 a, const uint4 b, ui
 }
 
 template <int FMT, bool PER_ROW>
-__global__ void __launch_bounds__(256) cast_bf16_sr_fast_kernel(CastParams p) {
+__global__ void __launch_bounds__(256, 3) cast_bf16_sr_fast_kernel(CastParams p) {
   cast_begin(p.start);
   const __nv_bfloat16* __restrict__ in = static_cast<const __nv_bfloat16*>(p.in);
   uint8_t* __restrict__ out = static_cast<uint8_t*>(p.out);
@@ -471,7 +477,7 @@ struct HybridParams {
 // One read of the input, two fp8 outputs: e5m2 (RNE or stochastic) with its own per-tensor scale
 // and e4m3 (always RNE) with its own.  4 bytes per bf16 element instead of 6 for two casts.
 template <typename InT, bool SR>
-__global__ void __launch_bounds__(256) cast_hybrid_kernel(HybridParams p) {
+__global__ void __launch_bounds__(256, SR ? 3 : 0) cast_hybrid_kernel(HybridParams p) {
   cast_begin(p.start);
   constexpr bool BF16 = InTraits<InT>::kIsBf16;
   const InT* __restrict__ in = static_cast<const InT*>(p.in);
