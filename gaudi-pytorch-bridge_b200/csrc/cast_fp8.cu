@@ -826,7 +826,7 @@ struct AmaxForms {
   int64_t cluster, memset;  // up to how many elements
 };
 static AmaxForms amax_forms(bool vectors, bool stochastic, bool packed, int out_dtype, int sc) {
-  if (!vectors) return {1 << 15, stochastic || sc != SC_ONE ? 0 : 1 << 20};
+  if (!vectors) return {1 << 15, stochastic || sc != SC_ONE ? 0 : 1 << 21};
   if (stochastic && packed) return out_dtype == B200Q_E5M2 ? AmaxForms{1 << 18, 1 << 21} : AmaxForms{1 << 17, 1 << 20};
   if (stochastic) return {1 << 16, 1 << 20};
   if (sc == SC_COL || sc == SC_FULL) return {1 << 17, 1 << 21};
@@ -837,11 +837,11 @@ static AmaxForms amax_forms(bool vectors, bool stochastic, bool packed, int out_
 static int cast_start(float* amax, int64_t n, AmaxForms forms, cudaStream_t st, int* start) {
   *start = kStartAfter;
   if (!amax) return B200Q_OK;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
-  if (capture != cudaStreamCaptureStatusNone) {
-    forms.cluster >>= 2;
-    forms.memset = 0;
+  const AmaxForms captured = {forms.cluster / 4, 0};
+  if (n > captured.cluster && (n <= forms.cluster || n <= forms.memset)) {  // (asking costs the host 0.1 us)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) forms = captured;
   }
   if (n > 0 && n <= forms.cluster) {
     *start = kStartCluster;
