@@ -155,3 +155,94 @@ def test_fp8_sdpa_long_sequence_both_kernels_agree(monkeypatch):
         outs.append(out)
     torch.cuda.synchronize()
     assert O.rel_frobenius(outs[0], outs[1]) <= 5e-3
+
+
+def _both_kernels(BH, L, S, causal, mask=None, softmax_scale=None, fp8_out=False, seed=0):
+    """The tcgen05 kernel (twice) and the plain kernel through the C ABI: [out, m, 1/l, amax_s, amax_o] each."""
+    import ctypes as C
+    from b200_hpu_ops import abi
+    D = 128
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    q8, k8, v8 = (torch.randn(BH, n, D, device="cuda", generator=g).mul(40).to(E4M3) for n in (L, S, S))
+    res = []
+    for plain in (0, 0, 1):
+        out = torch.empty(BH, L, D, device="cuda", dtype=E4M3 if fp8_out else torch.bfloat16)
+        m, linv = (torch.empty(BH, L, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+        amax = torch.zeros(2, device="cuda")
+        a = abi.SdpaArgs()
+        a.q, a.k, a.v, a.out, a.out_dtype = q8.data_ptr(), k8.data_ptr(), v8.data_ptr(), out.data_ptr(), abi.E4M3 if fp8_out else abi.BF16
+        a.BH, a.L, a.S, a.dqk, a.dv, a.kv_rep, a.causal = BH, L, S, D, D, 1, causal
+        if mask is not None:  # [BH or 1, L or 1, S]
+            a.mask, a.mask_kind = mask.data_ptr(), {torch.bfloat16: 1, torch.float32: 2, torch.uint8: 3}[mask.dtype]
+            a.mask_sb = mask.stride(0) if mask.size(0) > 1 else 0
+            a.mask_sl = mask.stride(1) if mask.size(1) > 1 else 0
+        a.softmax_scale = softmax_scale if softmax_scale is not None else 1.0 / math.sqrt(D)
+        a.d_scale_q_host = a.d_scale_k_host = a.d_scale_v_host = 1.0 / 40
+        a.q_scale_s_host, a.q_scale_o_host, a.d_scale_s_host = 256.0, 100.0, 1.0
+        a.m_out, a.linv_out, a.amax_s, a.amax_o = m.data_ptr(), linv.data_ptr(), amax.data_ptr(), amax.data_ptr() + 4
+        a.force_plain = plain
+        a.stream = torch.cuda.current_stream().cuda_stream
+        abi.check(abi.lib.b200q_fp8_sdpa_fwd(C.byref(a)), "b200q_fp8_sdpa_fwd")
+        res.append((out, m, linv, amax))
+    torch.cuda.synchronize()
+    return res
+
+
+def _check_both(res, fp8_out=False):
+    first, second, plain = res
+    for x, y in zip(first, second):
+        assert torch.equal(x.view(torch.uint8), y.view(torch.uint8))  # the same bits on every run
+    for x in first[:3]:
+        assert not torch.isnan(x.float()).any()
+    # one e4m3 step of a probability or of the output where a value sits on a tie: as in the tests above
+    assert O.rel_frobenius(first[0].float(), plain[0].float()) <= (4e-2 if fp8_out else 5e-3)
+    assert torch.allclose(first[1].float(), plain[1].float(), atol=2e-2, rtol=1e-2)
+    assert torch.allclose(first[2].float(), plain[2].float(), atol=1e-3, rtol=2e-2)
+    assert torch.allclose(first[3], plain[3], rtol=2e-2)
+
+
+def _mask(kind, heads, rows, S, offset, g):
+    """[heads, rows, S] of the kind, `offset` elements behind an aligned base; key 0 is always kept."""
+    keep = torch.rand(heads, rows, S, device="cuda", generator=g) < 0.6
+    keep[..., 0] = True
+    flat = torch.empty(offset + keep.numel(), device="cuda", dtype=kind)
+    m = flat[offset:].view(keep.shape)
+    if kind == torch.uint8:
+        return m.copy_(keep)
+    m.copy_(torch.randn(keep.shape, device="cuda", generator=g) * 2)
+    return m.masked_fill_(~keep, torch.finfo(kind).min if heads > 1 else -float("inf"))
+
+
+# heads, rows: 1 = the same for all.  Pitches that are whole 16-byte pieces, odd ones, bases one element off
+@pytest.mark.parametrize("kind", [torch.uint8, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("BH,L,S,heads,rows,offset,causal", [
+    (30, 700, 640, 30, 700, 0, 0), (30, 700, 333, 30, 700, 0, 0), (50, 300, 301, 1, 300, 1, 1), (170, 100, 37, 170, 100, 3, 0),
+    (200, 128, 128, 1, 128, 0, 1), (40, 520, 1000, 40, 1, 1, 0), (160, 64, 15, 160, 64, 1, 0)])
+def test_masks_by_pitch_and_alignment(kind, BH, L, S, heads, rows, offset, causal):
+    """More items than CTAs, masks read in aligned pieces and (at the mask's ends) element by element."""
+    g = torch.Generator(device="cuda").manual_seed(S)
+    _check_both(_both_kernels(BH, L, S, causal, _mask(kind, heads, rows, S, offset, g), seed=L))
+
+
+def test_row_dependent_mask_costs_a_few_times_the_unmasked_kernel():
+    """64 heads of 1100 queries and keys: a mask read element by element took nine times as long as none."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q8, k8, v8 = (torch.randn(1, 64, 1100, 128, device="cuda", generator=g).mul(40).to(E4M3) for _ in range(3))
+    t = lambda v: torch.tensor([v], device="cuda")  # noqa: E731
+    keep = torch.rand(1, 1, 1100, 1100, device="cuda", generator=g) < 0.5
+    keep[..., 0] = True
+    us = []
+    for mask in (None, keep, keep.float()):
+        best = float("inf")
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            for _ in range(5):
+                torch.ops.hpu.fp8_sdpa_recomp_fwd(q8, k8, v8, mask, 0.0, 0.1, False, False, "None", t(0.025), t(0.025), t(0.025), t(256.0),
+                                                  None, t(1 / 256), False, False, None, "left")
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 1e3 / 5)
+        us.append(best)
+    assert us[1] <= 5.5 * us[0] and us[2] <= 5.5 * us[0], us
