@@ -305,3 +305,34 @@ def test_w4a16_weights_in_tensor_memory(ops, M, N, K, group, k_packed):
         assert O.rel_frobenius(r, e.float()) <= tol
         assert torch.equal(r, torch.ops.b200q.w4a16_gemm(x.cuda(), qw, scale.cuda(), zp.cuda(), group, k_packed, dt))
     assert ops.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,group,k_packed", [
+    # two column tiles per CTA: six, five and four expander groups; a partly empty second tile (N % 256 = 128 + 32); an
+    # odd number of k-blocks
+    (1, 18976, 512, 64, False), (64, 18976, 576, 64, False), (65, 18976, 576, 192, False), (96, 18976, 512, 512, False),
+    (97, 18976, 576, 64, False), (128, 18976, 512, 128, False),
+    # the same over a cluster of two and four, and more tiles than fit at once
+    (97, 9632, 1088, 1088, False), (77, 8192, 8192, 128, False), (128, 8192, 8192, 128, False),
+    (33, 38144, 1024, 128, False), (77, 38144, 1024, 64, False), (128, 38144, 1024, 128, False),
+    # AutoGPTQ words
+    (1, 19200, 1024, 128, True), (16, 19200, 2048, 64, True), (16, 38400, 1024, 128, True),
+])
+def test_w4a16_two_column_tiles_per_cta(ops, M, N, K, group, k_packed):
+    """fp32 output against the fp64 product with the weights that convert_from_uint4 gives (itself checked bit by bit):
+    sums of up to 8192 fp32 terms in some order, 2e-5 as for the other forms."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    words = lambda *s: torch.randint(-2 ** 31, 2 ** 31 - 1, s, device="cuda", dtype=torch.int32, generator=g)  # noqa: E731
+    qw, zp = words(K // 8, N) if k_packed else words(K, N // 8), words(K // group, N // 8)
+    scale = (torch.rand(K // group, N, device="cuda", generator=g) * 0.015 + 0.005).to(torch.bfloat16)
+    x = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    if k_packed:
+        w = torch.ops.b200q.dequant_kpacked(qw, scale, zp, torch.bfloat16)
+    else:
+        w = torch.ops.hpu.convert_from_uint4(qw, scale, zp, torch.bfloat16)
+    e = torch.cat([x.double() @ w[:, n:n + 4096].double() for n in range(0, N, 4096)], dim=1)
+    for dt, tol in ((torch.float32, 2e-5), (torch.bfloat16, 4e-3)):
+        r = torch.ops.b200q.w4a16_gemm(x, qw, scale, zp, group, k_packed, dt)
+        assert O.rel_frobenius(r.double(), e) <= tol
+        assert torch.equal(r, torch.ops.b200q.w4a16_gemm(x, qw, scale, zp, group, k_packed, dt))
+    assert ops.device_status() == 0

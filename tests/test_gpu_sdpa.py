@@ -246,3 +246,31 @@ def test_row_dependent_mask_costs_a_few_times_the_unmasked_kernel():
             best = min(best, a.elapsed_time(b) * 1e3 / 5)
         us.append(best)
     assert us[1] <= 5.5 * us[0] and us[2] <= 5.5 * us[0], us
+
+
+@pytest.mark.parametrize("fp8_out", [False, True])
+@pytest.mark.parametrize("BH,L,S,causal,sign", [
+    (64, 1100, 1100, 1, 1),   # 576 items, odd and even numbers of key blocks, ragged ends
+    (500, 128, 128, 0, 1),    # one block per item: the second group of softmax warps has none
+    (470, 100, 200, 0, 1),    # two blocks, one item per head
+    (75, 513, 127, 0, -1),    # a negative scale; the last query block holds one row
+    (40, 900, 1500, 1, -1),   # more keys than queries, long items next to short ones
+])
+def test_many_items_per_cta(BH, L, S, causal, sign, fp8_out):
+    """Three and more items per CTA (148 CTAs at most): query tiles, accumulator, row statistics and rings carried from item
+    to item."""
+    scale = sign / math.sqrt(128)
+    _check_both(_both_kernels(BH, L, S, causal, None, scale, fp8_out, seed=S), fp8_out)
+
+
+@pytest.mark.parametrize("D", [128, 64])
+def test_outputs_that_are_not_asked_for_are_zero(D):
+    """All five one-element results, over memory that held something else (the kernels clear them)."""
+    q8 = torch.randn(1, 2, 40, D, device="cuda").to(E4M3)
+    for _ in range(3):
+        dirty = [torch.full((1,), 7, device="cuda", dtype=dt) for dt in (torch.bfloat16, torch.bfloat16, torch.int32, torch.float32, torch.float32)]
+        torch.cuda.synchronize()
+        del dirty
+        r = torch.ops.hpu.fp8_sdpa_recomp_fwd(q8, q8, q8, None, 0.0, 0.1, True, False, "None", None, None, None, None, None, None, False,
+                                              False, None, "left")
+        assert [t.shape for t in r[1:]] == [(1,)] * 5 and [t.item() for t in r[1:]] == [0] * 5
