@@ -3,9 +3,9 @@
 // Persistent, warp-specialised kernel, one CTA per SM:
 //   warp 0    TMA producer: 128-byte-swizzled K-major tiles of both operands into a
 //             shared-memory ring (no multicast), completion on "full" mbarriers
-//   warp 1    TMEM owner and MMA issuer: one thread issues tcgen05.mma.kind::f8f6f4
-//             (128 x BN x 32 per instruction), tcgen05.commit releases ring stages
-//             and publishes finished accumulators
+//   warp 1    TMEM owner and MMA issuer: tcgen05.mma.kind::f8f6f4 (128 x BN x 32 per
+//             instruction), tcgen05.commit releases ring stages and publishes finished
+//             accumulators (both roles are run by the whole warp, which elects a lane to issue)
 //   warps 2-5 epilogue: tcgen05.ld the fp32 accumulator (each warp its 32 TMEM lanes),
 //             apply (acc * sa) * sb + bias + D, round once, store
 // The accumulator is double-buffered in TMEM (2 x BN columns) so the epilogue of tile i
@@ -622,7 +622,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 // ------------------------------------------------------------------------ CTA-pair kernel
 // Large-M form: two CTAs of a cluster (one per SM of a TPC) share a 256 x BN output tile.  Each
 // CTA loads its own 128 rows of A and its own BN/2 rows of B per ring stage (no multicast: every
-// byte is fetched by exactly one CTA), the even CTA's MMA thread issues
+// byte is fetched by exactly one CTA), the even CTA's MMA warp issues
 // tcgen05.mma.cta_group::2 (M = 256), which reads both CTAs' shared memory and writes 128
 // accumulator rows into each CTA's TMEM.  Per flop the pair moves a third less data from L2
 // into shared memory than two independent 128 x BN tiles, which is what bounds the
@@ -917,11 +917,12 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
     tp.x_mn = a_mn; tp.y_mn = b_mn;
     tp.x_tiles = (int)((g.M + kBlockX - 1) / kBlockX);
     tp.x_tile_rows = kBlockX;
-    // Column-tile width: the one that minimises (waves over the 148 SMs) x (tile cost).  Measured
-    // on 4096 x 14336 x 4096: a wave of 224-column tiles takes 96 % of the time of a wave of
-    // 256-column tiles (the k-block time is dominated by operand traffic that does not shrink with
-    // the width), i.e. a tile costs about (width + 590) units; narrower tiles only win when they
-    // remove a whole wave.
+    // Column-tile width: the one that minimises (waves over the 148 SMs) x (tile cost), with a tile at
+    // (width + kTileOverheadCols), so that narrower tiles are taken only where they remove a whole wave.  The overhead
+    // was fitted when a wait cost the issuing roles some 200 cycles (a wave of 224-column tiles took 96 % of one of 256);
+    // since the roles are whole warps a wave costs nearly its width: one wave of 256, 224 and 192 columns on CTA pairs (512 rows)
+    // 19.8, 17.4 and 15.8 us at K = 4096, 55.6, 47.8 and 42.4 at K = 14336.  4096 x 14336 x 4096, whose waves are 12.1, 13.8
+    // and 16.2: 167, 177 and 178 us.
     // An MN-major B operand comes in 128-column blocks: 256 or 128 only.
     static const int kWidths[] = {256, 224, 192, 160, 128};
     int bn = 128;
@@ -986,6 +987,7 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
   // beyond the tile read whatever the stage holds and are not stored.  Heights are multiples of 8
   // (the swizzle atom) from 32 up (a stage shorter than that keeps too few bytes in flight); the
   // cost of a round has a height-independent part (pipeline fill, accumulator drain) of about 24 rows.
+  // 16 tokens, against 128 rows always, us: K = 4096, N = 14336 11.6 / 11.7; K = 14336, N = 4096 17.1 / 17.8.
   int rows = kBlockX;
   if (!b_mn) {
     static const bool fixed_height = std::getenv("B200Q_GEMM_SWAP_128") != nullptr;  // comparison switch
@@ -1002,15 +1004,13 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
   if (rc) return rc;
   rc = make_operand_map(&my, g.A, g.M, g.K, g.lda, bn);
   if (rc) return rc;
-  // Few tokens: neither the bytes nor the MMAs set the pace here -- measured, a k-block costs a CTA
-  // 0.25-0.3 us whatever the tile height (32 or 128 rows), with one MMA or none in place of four,
-  // with or without the token tile's load, with 7 ring stages or 10 -- so the per-stage work of
-  // the two single-thread roles (barrier round trips, commit) is spread over two k-blocks
-  // (-6 % at K = 4096, -16 % at K = 14336).
+  // Few tokens: the per-stage work of the two issuing roles (barrier round trips, commit) is spread over two
+  // k-blocks: 16 tokens, one / two k-blocks a stage, us: K = 4096, N = 14336 12.1 / 11.6; K = 14336, N = 4096
+  // 23.6 / 18.3; K = 2048, N = 5120 6.0 / 5.2; 128 tokens, K = 4096, N = 14336 16.0 / 16.2.
   static const bool one_kb = std::getenv("B200Q_GEMM_SWAP_KPS1") != nullptr;  // comparison switch
   if (!b_mn && !one_kb) {
     switch (bn) {
-      case 16:  // long K: four k-blocks per stage (measured: 27 against 30 us at K = 14336; no gain at 4096)
+      case 16:  // long K: four k-blocks per stage (K = 14336, N = 4096 17.1 against 18.3 us; no difference at 4096)
         if (tp.num_kb >= 64) return launch_cfg<16, 3, true, 4>(mx, my, tp, st);
         return launch_cfg<16, 5, true, 2>(mx, my, tp, st);
       case 32: return launch_cfg<32, 5, true, 2>(mx, my, tp, st);

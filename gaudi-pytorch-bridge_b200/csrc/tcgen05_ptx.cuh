@@ -42,35 +42,6 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
   return ok;
 }
 
-// try_wait with a suspend-time hint (nanoseconds): the hardware may park the thread for up to
-// that long while the phase is incomplete, instead of returning to a polling loop that takes
-// issue slots from the other warps of its scheduler.
-__device__ __forceinline__ uint32_t mbar_try_wait_hint(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok;
-}
-__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                 int code, uint32_t hint_ns, uint32_t limit = 1u << 22) {
-  for (uint32_t i = 0; i < limit; ++i) {
-    if (mbar_try_wait_hint(bar, parity, hint_ns)) return true;
-    if ((i & 63u) == 63u) {
-      if (*abort_flag) return false;
-    }
-  }
-  *abort_flag = 1;
-  atomicCAS(status, 0, code);
-  return false;
-}
-
 // Bounded wait.  `abort_flag` is a shared-memory word any role may set; the wait gives up
 // when it is set or after kWaitLimit polls (seconds of wall time), and then sets it itself.
 // `backoff_ns` > 0 makes a waiter that is not on the critical path (an epilogue warp waiting
@@ -177,30 +148,10 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]; one thread issues.  kind::f8f6f4: K = 32 per instruction.
-__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// kind::f16 (bf16 / fp16 operands): K = 16 per instruction.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Four MMAs whose operand descriptors advance by astep / bstep (16-byte units), as one instruction
-// sequence; only the first one may start a new accumulator.
+// Four MMAs, D[tmem] (+)= A[smem] * B[smem], whose operand descriptors advance by astep / bstep (16-byte units), as one
+// instruction sequence that one thread issues; only the first one may start a new accumulator.  kind::f8f6f4: K = 32
+// each; kind::f16 (bf16 or fp16 operands): K = 16.  The pair forms multiply 256 rows over both CTAs' shared
+// memory and TMEM.
 #define B200Q_UMMA_X4(NAME, G, KIND)                                                                                        \
   __device__ __forceinline__ void NAME(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, \
                                        uint32_t astep, uint32_t bstep) {                                                    \
@@ -278,42 +229,6 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t smem_dst, const CUtens
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
       : "memory");
-}
-// 256 x N x 32 MMA over both CTAs' shared memory and TMEM; issued by one thread of the even CTA.
-__device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Bounded wait on a barrier that threads of the peer CTA arrive on (cluster-scope acquire, so
-// that what they wrote to their shared memory before arriving is ordered before what follows).
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                  int code) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u) {
-      if (*abort_flag) return false;
-      if (i > 4096u) __nanosleep(64);
-    }
-  }
-  *abort_flag = 1;
-  atomicCAS(status, 0, code);
-  return false;
 }
 // Completion of the pair's MMAs signalled on the barrier at the same offset in both CTAs.
 __device__ __forceinline__ void umma_commit_pair_both(uint32_t bar) {

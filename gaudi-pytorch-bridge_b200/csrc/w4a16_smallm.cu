@@ -61,34 +61,11 @@ struct Params {
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait(int pending) {  // the count must be an immediate
-  switch (pending) {
-    case 0: asm volatile("cp.async.wait_group 0;" ::: "memory"); break;
-    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
-    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
-    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
-    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
-    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
-    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
-    case 7: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
-    case 8: asm volatile("cp.async.wait_group 8;" ::: "memory"); break;
-    case 9: asm volatile("cp.async.wait_group 9;" ::: "memory"); break;
-    case 10: asm volatile("cp.async.wait_group 10;" ::: "memory"); break;
-    case 11: asm volatile("cp.async.wait_group 11;" ::: "memory"); break;
-    case 12: asm volatile("cp.async.wait_group 12;" ::: "memory"); break;
-    case 13: asm volatile("cp.async.wait_group 13;" ::: "memory"); break;
-    case 14: asm volatile("cp.async.wait_group 14;" ::: "memory"); break;
-    case 15: asm volatile("cp.async.wait_group 15;" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 16;" ::: "memory"); break;
-  }
-}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
   asm volatile(
@@ -278,7 +255,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
       if (t > 0) {
         named_bar(1 + khalf, 32 * kStrips);
         stage_x(t / kBatchesPerChunk);
-        cp_async_wait(0);
+        cp_async_wait_all();
       } else {
         asm volatile("cp.async.wait_group %0;" ::"n"(kSlots - 1) : "memory");  // all but the weights: the chunk
       }
@@ -313,7 +290,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads, 1) 
   // ---------------------------------------------------------------- reduction
   // warp partial tile -> this warp's ring (all of its copies have landed and been read):
   // red[warp][token 0..15][column 0..63] fp32 = 4 KB
-  cp_async_wait(0);
+  cp_async_wait_all();
   __syncwarp();
   float* red = reinterpret_cast<float*>(ring);
 #pragma unroll
@@ -377,9 +354,10 @@ static int launch(const Params& p, cudaStream_t st) {
 
 }  // namespace w4s
 
-// Whether this is a few-token problem that needs no scratch: M <= 16, whole 256-column blocks, K divisible
-// into 16 slices of whole k-steps (16 rows; 64 for the AutoGPTQ layout, which w4a16_tmem.cu reads), groups that
-// k-steps do not straddle.
+// Whether this is a few-token problem: M <= 16, whole 256-column blocks, K divisible into 16 slices of whole k-steps
+// (16 rows), groups that k-steps do not straddle.  The same rule with steps of 64 rows is what the entry takes of
+// AutoGPTQ words, and for what shapes the workspace query answers 0: limits of the interface, wider than which
+// w4a16_tmem.cu, which runs those words, could go.
 bool w4a16_smallm_eligible(int64_t M, int64_t N, int64_t K, int64_t group, int k_packed) {
   const int64_t step = k_packed ? 64 : 16;
   return M >= 1 && M <= 16 && N >= w4s::kCols && N % w4s::kCols == 0 && K >= w4s::kSlices * step &&

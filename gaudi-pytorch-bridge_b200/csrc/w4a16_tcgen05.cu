@@ -325,28 +325,26 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
       // the registers read from TMEM are renamed into column order below.
       const int64_t m = (int64_t)xt * 128 + q * 32 + lane;  // this thread's token
       const int64_t y0 = (int64_t)yt * BN;
-      constexpr int CW = (BN % 32 == 0) ? 32 : 16;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t r[32];
-        if (BN % 32 == 0) tmem_ld_32x32(t_row + c0, r);
-        else tmem_ld_32x16(t_row + c0, r);
+        tmem_ld_32x32(t_row + c0, r);
         tmem_ld_wait();
         // registers are in tile-position order: rename them into column order (free: all static)
         {
           uint32_t t[32];
 #pragma unroll
-          for (int j = 0; j < CW; ++j) t[(j & ~7) + ((j & 7) >> 1) + 4 * (j & 1)] = r[j];
+          for (int j = 0; j < 32; ++j) t[(j & ~7) + ((j & 7) >> 1) + 4 * (j & 1)] = r[j];
 #pragma unroll
-          for (int j = 0; j < CW; ++j) r[j] = t[j];
+          for (int j = 0; j < 32; ++j) r[j] = t[j];
         }
         const int64_t n0 = y0 + c0;
         if (m < p.M) {
           if (p.out_dtype == B200Q_BF16) {
             __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + m * p.ldo + n0;
-            if (n0 + CW <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+            if (n0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
 #pragma unroll
-              for (int j = 0; j < CW; j += 8)
+              for (int j = 0; j < 32; j += 8)
                 *reinterpret_cast<uint4*>(o + j) = make_uint4(
                     pack_bf16x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])),
                     pack_bf16x2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
@@ -354,18 +352,18 @@ w4a16_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_constant_
                     pack_bf16x2(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7])));
             } else {
 #pragma unroll
-              for (int j = 0; j < CW; ++j)
+              for (int j = 0; j < 32; ++j)
                 if (n0 + j < p.N) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
             }
           } else {
             float* o = static_cast<float*>(p.out) + m * p.ldo + n0;
-            if (n0 + CW <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+            if (n0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
 #pragma unroll
-              for (int j = 0; j < CW; j += 4)
+              for (int j = 0; j < 32; j += 4)
                 *reinterpret_cast<uint4*>(o + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
             } else {
 #pragma unroll
-              for (int j = 0; j < CW; ++j)
+              for (int j = 0; j < 32; ++j)
                 if (n0 + j < p.N) o[j] = __uint_as_float(r[j]);
             }
           }
@@ -703,8 +701,8 @@ w4a16_pair_kernel(const __grid_constant__ CUtensorMap map_act, const __grid_cons
     const int et = (ewarp % C::kExpandWarps) * 32 + lane;
     const int my_group = ewarp / C::kExpandWarps;
     constexpr int W = 16;
-    constexpr int kRowsPerPass = C::kExpandWarps * 32 / W;  // 16
-    constexpr int kPasses = kK / kRowsPerPass;              // 4
+    constexpr int kRowsPerPass = C::kExpandWarps * 32 / W;  // 8
+    constexpr int kPasses = kK / kRowsPerPass;              // 8
     const int ngl = et % W, kr = et / W;
     const bool has_zp = p.zp != nullptr;
     const uint32_t krow = kr & 7;
@@ -832,9 +830,9 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mr, const CUtensorMa
 
 }  // namespace w4
 
-// The workspace that the entry asks for at 17 - 128 tokens: fp32 partial tiles of this many K splits.  The
-// kernel that now takes these shapes adds its splits inside clusters and needs none; the size stays what callers
-// and the limit of the allocation-free entry know.
+// b200q_w4a16_workspace_bytes() is part of the interface: at 17 - 128 tokens it asks for fp32 partial tiles of this many
+// K splits, b200q_w4a16_gemm() refuses less, and the allocation-free entry refuses what would need more than 8 MiB.  The
+// kernels add their splits inside clusters and use none of it.
 static int w4a16_splits(int64_t M, int64_t N, int64_t K) {
   if (M > 128) return 1;
   // 128-token x 256-column tiles; the split count that minimises the busiest CTA's k-blocks
@@ -870,9 +868,10 @@ size_t w4a16_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
 }
 
-int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp,
-                    int zp_kind, int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out,
-                    int out_dtype, int64_t ldo, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+// workspace: what the caller has stated, in bytes (see above)
+static int w4a16_dispatch(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp,
+                          int zp_kind, int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out,
+                          int out_dtype, int64_t ldo, size_t workspace, cudaStream_t st) {
   if (K == 0) {
     // an empty contraction: the result is all zeros (rows may be strided)
     const size_t esz = out_dtype == B200Q_BF16 ? 2 : 4;
@@ -906,8 +905,7 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
   p.out_dtype = out_dtype; p.num_kb = (int)(K / w4::kK);
   p.status = device_status_ptr();
   if (!p.status) return B200Q_ERR_CUDA;
-  const size_t need = w4a16_workspace_bytes_impl(M, N, K);  // (the contract of the entry; no kernel uses it any more)
-  if (need && (!workspace || workspace_bytes < need)) return B200Q_ERR_BAD_ARGUMENT;
+  if (workspace < w4a16_workspace_bytes_impl(M, N, K)) return B200Q_ERR_BAD_ARGUMENT;
   if (p.zp && (reinterpret_cast<uintptr_t>(p.zp) & 15)) return B200Q_ERR_UNSUPPORTED;
   if (M <= 128) return w4a16_tmem_launch(x, ldx, qweight, scale, p.zp, 0, M, N, K, group, out, out_dtype, ldo, st);
   CUtensorMap ma, mr;
@@ -959,49 +957,21 @@ int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const vo
   return rc;
 }
 
-// ------------------------------------------------------------------------ allocation-free variant
-// Scratch for b200q_w4a16_gemm_noalloc: it lives in the library image, so every GPU that loads
-// the library carries these 8 MiB until the process exits, and the caller never has to hand in
-// (or allocate) a workspace.  Only device code may use the name directly; host code must ask the
-// runtime for the device address (below).
-constexpr size_t kStaticScratchBytes = size_t(8) << 20;
-static __device__ __align__(256) float g_w4a16_static_scratch[kStaticScratchBytes / sizeof(float)];
-
-// Device address of the static scratch on the current device.  In host code the array's name
-// is only a stand-in for the symbol, not a pointer the GPU can follow, so the address is
-// looked up with cudaGetSymbolAddress -- once per device, with that device current -- and kept.
-static int static_scratch_ptr(float** out) {
-  static std::atomic<float*> cache[kMaxDevices];
-  const int dev = current_device_index();
-  if (dev < 0) return B200Q_ERR_CUDA;
-  float* p = cache[dev].load(std::memory_order_acquire);
-  if (!p) {
-    void* addr = nullptr;
-    B200Q_CUDA_OK(cudaGetSymbolAddress(&addr, g_w4a16_static_scratch));
-    p = static_cast<float*>(addr);
-    cache[dev].store(p, std::memory_order_release);
-  }
-  *out = p;
-  return B200Q_OK;
+int w4a16_gemm_impl(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp,
+                    int zp_kind, int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out,
+                    int out_dtype, int64_t ldo, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  return w4a16_dispatch(x, ldx, qweight, scale, zp, zp_kind, k_packed, M, N, K, group, out, out_dtype, ldo,
+                        workspace ? workspace_bytes : 0, st);
 }
 
+// The allocation-free entry, with its limit.  (Shapes the kernels reject report a zero workspace here and are refused, with
+// their own code, by the checks of the dispatch.)
 int w4a16_gemm_noalloc_impl(const void* x, int64_t ldx, const int32_t* qweight, const void* scale, const int32_t* zp,
                             int zp_kind, int k_packed, int64_t M, int64_t N, int64_t K, int64_t group, void* out,
                             int out_dtype, int64_t ldo, cudaStream_t st) {
-  // (shapes the fused kernel rejects report a zero workspace here and are refused, with their
-  // own code, by the argument checks of w4a16_gemm_impl)
-  const size_t need = w4a16_workspace_bytes_impl(M, N, K);
-  if (need > kStaticScratchBytes) return B200Q_ERR_TOO_LARGE;
-  float* scratch = nullptr;
-  int rc = static_scratch_ptr(&scratch);
-  if (rc) return rc;
-  return w4a16_gemm_impl(x, ldx, qweight, scale, zp, zp_kind, k_packed, M, N, K, group, out, out_dtype, ldo, scratch,
-                         kStaticScratchBytes, st);
+  constexpr size_t kLimit = size_t(8) << 20;
+  if (w4a16_workspace_bytes_impl(M, N, K) > kLimit) return B200Q_ERR_TOO_LARGE;
+  return w4a16_dispatch(x, ldx, qweight, scale, zp, zp_kind, k_packed, M, N, K, group, out, out_dtype, ldo, kLimit, st);
 }
 
-size_t w4a16_noalloc_max_bytes_impl() { return kStaticScratchBytes; }
-
 }  // namespace b200q
-
-
-

@@ -1,11 +1,10 @@
 """b200q_w4a16_gemm_noalloc: the W4A16 GEMM for callers that may not allocate device memory
 (a serving loop with a frozen memory plan, a plug-in inside another framework's callback, a host
-binding without an allocator).  Its split-K scratch is a static array inside the library, so the
-caller passes inputs and output only.
+binding without an allocator): the caller passes inputs and output only.
 
 Checked through the C ABI against b200q_w4a16_gemm with a caller-provided workspace: the two
 entry points run the same kernels in the same order, so the results must be identical; the
-check is repeated on a second call because the static scratch keeps the first call's contents.
+check is repeated on a second call, which must not depend on what the first one left behind.
 This file sorts last on purpose: a run that stops at the first failure has then already run
 every other test."""
 import ctypes as C
