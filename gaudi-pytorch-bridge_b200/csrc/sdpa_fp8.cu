@@ -24,7 +24,8 @@
 // with one lane issuing both products of 128 keys and a CTA per item; 422 us as one stream; 326 us
 // with the issuing roles run by whole warps (a lane spends 200 cycles per wait on addresses that a
 // converged warp keeps in uniform registers); 274 us with 256 keys per
-// step; 262 us with the two products issued by two warps and the groups out of step.  What did not
+// step; 262 us with the two products issued by two warps and the groups out of step; 250 us with waits whose outcome
+// is a vote.  What did not
 // help: part of the exponentials as polynomials on the FMA pipe (the issue slots they take are as
 // scarce), sixteen softmax warps with half a row each, a strict alternation of the groups' exponentials.
 // Two passes over the keys: the first only takes the row maxima, the second recomputes the
