@@ -840,8 +840,8 @@ static int cast_start(float* amax, int64_t n, AmaxForms forms, cudaStream_t st, 
   const AmaxForms captured = {forms.cluster / 4, 0};
   if (n > captured.cluster && (n <= forms.cluster || n <= forms.memset)) {  // (asking costs the host 0.1 us)
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
-    if (capture != cudaStreamCaptureStatusNone) forms = captured;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();  // (capture is not set then)
+    else if (capture != cudaStreamCaptureStatusNone) forms = captured;
   }
   if (n > 0 && n <= forms.cluster) {
     *start = kStartCluster;
