@@ -708,8 +708,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         if (elect_one()) {
           const uint32_t full_leader = (bar_full + 8 * stage) & kPeerBitMask;
           if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * L::kStageBytes);
-          tma_load_2d_pair(smem_base + stage * L::kStageBytes, &map_x, full_leader, kb * kBlockK, x_row);
-          tma_load_2d_pair(smem_base + stage * L::kStageBytes + L::kXBytes, &map_y, full_leader, kb * kBlockK, y_row);
+          const int k0 = kb * kBlockK;
+          tma_load_2d_pair(smem_base + stage * L::kStageBytes, &map_x, full_leader, p.x_mn ? x_row : k0, p.x_mn ? k0 : x_row);
+          tma_load_2d_pair(smem_base + stage * L::kStageBytes + L::kXBytes, &map_y, full_leader, p.y_mn ? y_row : k0,
+                           p.y_mn ? k0 : y_row);
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
@@ -717,10 +719,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA only)
     if (rank == 0) {
-      const uint32_t idesc = umma_idesc(p.a_fmt_bits, p.b_fmt_bits, 2 * kBlockX, BN);
-      // descriptors of stage 0, built once: see the single-CTA kernel
-      const uint64_t xd0 = smem_desc_k_sw128(smem_base), yd0 = smem_desc_k_sw128(smem_base + L::kXBytes);
-      static_assert(kBlockK / kUmmaK == 4 && (kUmmaK >> 4) == 2, "umma_f8_pair_x4 issues 4 MMAs 32 bytes apart");
+      const uint32_t idesc = umma_idesc_major(p.a_fmt_bits, p.b_fmt_bits, 2 * kBlockX, BN, p.x_mn, p.y_mn);
+      // descriptors of stage 0, built once, and the step between their MMAs: see the single-CTA kernel.  (The pair's
+      // MN-major tiles are one 128-row block per CTA, so that no block step is needed.)
+      const uint64_t xd0 = p.x_mn ? smem_desc_mn_sw128(smem_base, kBlockK * 128, 1024) : smem_desc_k_sw128(smem_base);
+      const uint64_t yd0 = p.y_mn ? smem_desc_mn_sw128(smem_base + L::kXBytes, kBlockK * 128, 1024)
+                                  : smem_desc_k_sw128(smem_base + L::kXBytes);
+      const uint32_t xstep = p.x_mn ? (4096u >> 4) : (kUmmaK >> 4), ystep = p.y_mn ? (4096u >> 4) : (kUmmaK >> 4);
+      static_assert(kBlockK / kUmmaK == 4, "umma_f8_pair_x4 issues 4 MMAs");
       uint32_t stage = 0, phase = 0;
       int it = 0;
       bool ok = true;
@@ -739,7 +745,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
           const uint64_t xd = xd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
           const uint64_t yd = yd0 + (uint64_t)(stage * (uint32_t)(L::kStageBytes >> 4));
           if (elect_one()) {
-            umma_f8_pair_x4(d_tmem, xd, yd, idesc, kb != 0, 2, 2);
+            umma_f8_pair_x4(d_tmem, xd, yd, idesc, kb != 0, xstep, ystep);
             umma_commit_pair_both(bar_empty + 8 * stage);
             if (kb + 1 == num_kb) umma_commit_pair_both(bar_tfull + 8 * acc);
           }
@@ -937,25 +943,27 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
     tp.y_tiles = (int)((g.N + bn - 1) / bn);
     int rc = make_map(&mx, g.A, g.M, g.K, g.lda, a_mn, kBlockX);
     if (rc) return rc;
-    // CTA pairs (256-row tiles) when there are enough rows to fill them (K-major operands)
+    // CTA pairs (256-row tiles) when there are enough rows to fill them.  An MN-major operand is a box of 128 rows x
+    // 128 k in each CTA, so an MN-major B takes 256 columns.  Both products of the backward pass of a linear layer (8000
+    // tokens, 4096 x 4096: B MN-major, then both; 64 MB of fp32 accumulated): 268 us on single CTAs, 244 on pairs.
     static const bool no_pairs = std::getenv("B200Q_GEMM_NO_PAIRS") != nullptr;
-    if (g.M > 128 && g.N > 128 && !no_pairs && !a_mn && !b_mn) {
+    if (g.M > 128 && g.N > 128 && !no_pairs) {
       TcGemmParams pp = tp;
       pp.x_tiles = (int)((g.M + 2 * kBlockX - 1) / (2 * kBlockX));
       int bp = 256;
       double bestp = 1e30;
       static const int kPairWidths[] = {256, 224, 192};
       for (int w : kPairWidths) {
-        if (routed && (w % 64)) continue;
+        if ((routed && (w % 64)) || (b_mn && w != 256)) continue;
         const int64_t tiles = (int64_t)pp.x_tiles * ((g.N + w - 1) / w);
         const double cost = (double)((tiles + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (w + kTileOverheadCols);
         if (cost < bestp) { bestp = cost; bp = w; }
       }
       static const int forced = std::getenv("B200Q_GEMM_PAIR_BN") ? std::atoi(std::getenv("B200Q_GEMM_PAIR_BN")) : 0;
-      if ((forced == 256 || forced == 224 || forced == 192) && !(routed && (forced % 64))) bp = forced;
+      if ((forced == 256 || forced == 224 || forced == 192) && !(routed && (forced % 64)) && !b_mn) bp = forced;
       if (g.swiglu) bp = 256;  // gate and up halves of a tile
       pp.y_tiles = (int)((g.N + bp - 1) / bp);
-      rc = make_operand_map(&my, g.B, g.N, g.K, g.ldb, bp / 2);
+      rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, bp / 2);
       if (rc) return rc;
       switch (bp) {
         case 256: rc = launch_pair<256, 6>(mx, my, pp, st); break;

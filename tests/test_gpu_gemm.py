@@ -368,6 +368,20 @@ def test_tcgen05_mn_major_operands(ops, tA, tB, M, N, K):
     assert torch.equal(r.cpu(), ref)
 
 
+@pytest.mark.parametrize("tA,tB", [(True, False), (True, True), (False, False)])
+@pytest.mark.parametrize("M,N,K", [(144, 144, 16), (272, 528, 2064), (5120, 2064, 144)])
+def test_mn_major_operands_on_cta_pairs(ops, tA, tB, M, N, K):
+    """Partial tiles of one k-block, the stage ring wrapped, several tiles for each pair; accumulated into fp32.
+    Small integers, whose sums are exact (below 2^24), so that the result is the same to the bit."""
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randint(-4, 5, (K, M) if tA else (M, K), generator=g).float()
+    B = torch.randint(-4, 5, (N, K) if tB else (K, N), generator=g).float()
+    D = torch.randint(-9, 10, (M, N), generator=g).float()
+    r = torch.ops.hpu.fp8_gemm_v2(A.to(torch.float8_e5m2).cuda(), tA, B.to(torch.float8_e4m3fn).cuda(), tB, D.cuda(), torch.float32,
+                                  None, None, None, True)
+    assert torch.equal(r.cpu(), (A.t() if tA else A) @ (B.t() if tB else B) + D)
+
+
 def test_tcgen05_mn_major_k_not_multiple_of_16(ops):
     g = torch.Generator().manual_seed(77)
     M, N, K = 256, 384, 200   # both operands MN-major: K needs no alignment
