@@ -33,7 +33,6 @@ constexpr int kBlockK = 128;  // bytes (= fp8 elements) of K per ring stage: one
 constexpr int kUmmaK = 32;
 constexpr int kThreads = 192;
 constexpr int kEpiThreads = 128;
-constexpr int kTileOverheadCols = 590;  // width-independent part of a tile's cost, in columns (see the width choice)
 
 enum { kErrProducer = 101, kErrMma = 102, kErrMmaTmem = 103, kErrEpilogue = 104 };
 
@@ -46,6 +45,7 @@ struct TcGemmParams {
   int x_tile_rows;
   int a_fmt_bits, b_fmt_bits;  // 0 = e4m3, 1 = e5m2 (lane-side, column-side)
   int x_mn, y_mn;              // 1 = that operand is stored MN-major ([K][rows], rows contiguous)
+  int whole_rows;              // 1 = the output leaves through epi_drain_rows()
   int* status;                 // device status word (bounded waits report here)
 };
 
@@ -60,7 +60,9 @@ struct SmemLayout {
   static_assert(kSubBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;  // per accumulator: col scale A, col scale B, col bias
-  static constexpr int kBarOffset = kRing + kEpiFloats * 4;
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 4 epilogue warps x 4 KB (whole-row output)
+  static constexpr int kPatchBytes = BN >= 128 && KPS == 1 ? 4 * 4096 : 0;
+  static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
 };
@@ -359,6 +361,98 @@ __device__ __forceinline__ void epi_drain_routed(const GemmParams& g, uint32_t t
   }
 }
 
+// fp32 output, with or without an fp32 accumulate input, or bf16 output without one, in whole 128-byte row segments:
+// what a thread computes for its row goes through a 4 KB patch of its warp as in the routed form, so that a load or
+// store instruction covers four rows of 128 bytes instead of 16 bytes of 32 rows.  The accumulate input of the next 32
+// columns is on its way while a group is finished.  (whole_rows_output() says for which outputs.)
+template <int BN>
+__device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
+                                               const float* cA, const float* cB, const float* cBias, uint4* patch, int lane) {
+  const EpiFlags f = epi_flags<false>(g);
+  const int prow = lane >> 3, piece = lane & 7;  // a lane's rows of the patch: prow + 4 k
+  if (g.out_dtype == B200Q_F32) {
+    float* out = static_cast<float*>(g.out) + (row0 + prow) * g.ldo + y0 + 4 * piece;
+    const float* acc = static_cast<const float*>(g.D) + (row0 + prow) * g.ldd + y0 + 4 * piece;
+    float4 d[8];
+    auto load_acc = [&](int c0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (row0 + prow + 4 * k < g.M && y0 + c0 + 4 * piece < g.N)
+          d[k] = __ldg(reinterpret_cast<const float4*>(acc + (int64_t)(4 * k) * g.ldd + c0));
+    };
+    if (g.D) load_acc(0);
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += 32) {
+      uint32_t r[32];
+      tmem_ld_32x32(t_row + c0, r);
+      tmem_ld_wait();
+      float v[32];
+      epi_values<32>(r, c0, e, cA, cB, cBias, f, v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        patch[lane * 8 + (k ^ (lane & 7))] = make_uint4(__float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]),
+                                                        __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int row = prow + 4 * k;
+        const uint4 w = patch[row * 8 + (piece ^ (row & 7))];
+        float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+        if (row0 + row < g.M && y0 + c0 + 4 * piece < g.N) {
+          if (g.D) o.x += d[k].x, o.y += d[k].y, o.z += d[k].z, o.w += d[k].w;
+          *reinterpret_cast<float4*>(out + (int64_t)(4 * k) * g.ldo + c0) = o;
+        }
+      }
+      if (g.D && c0 + 32 < BN) load_acc(c0 + 32);
+      __syncwarp();
+    }
+  } else {
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + (row0 + prow) * g.ldo + y0 + 8 * piece;
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += 64) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (c0 + 32 * h >= BN) break;
+        uint32_t r[32];
+        tmem_ld_32x32(t_row + c0 + 32 * h, r);
+        tmem_ld_wait();
+        float v[32];
+        epi_values<32>(r, c0 + 32 * h, e, cA, cB, cBias, f, v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          patch[lane * 8 + ((4 * h + k) ^ (lane & 7))] =
+              make_uint4(pack_bf16x2(v[8 * k], v[8 * k + 1]), pack_bf16x2(v[8 * k + 2], v[8 * k + 3]),
+                         pack_bf16x2(v[8 * k + 4], v[8 * k + 5]), pack_bf16x2(v[8 * k + 6], v[8 * k + 7]));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int row = prow + 4 * k;
+        const uint4 w = patch[row * 8 + (piece ^ (row & 7))];
+        if (row0 + row < g.M && c0 + 8 * piece < BN && y0 + c0 + 8 * piece < g.N)
+          *reinterpret_cast<uint4*>(out + (int64_t)(4 * k) * g.ldo + c0) = w;
+      }
+      __syncwarp();
+    }
+  }
+}
+// The accumulate input of a warp's 32 rows and BN columns is asked for as far as L2 while the tile is still being multiplied.
+template <int BN>
+__device__ __forceinline__ void epi_prefetch_acc(const GemmParams& g, int64_t row, int64_t y0) {
+  if (row >= g.M) return;
+  const float* acc = static_cast<const float*>(g.D) + row * g.ldd + y0;
+#pragma unroll
+  for (int c = 0; c < BN; c += 32)
+    if (y0 + c < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(acc + c));
+}
+// Outputs that epi_drain_rows() takes: 16-byte aligned rows of whole 16-byte pieces.
+static bool whole_rows_output(const GemmParams& g) {
+  if (g.out8_dtype || g.swiglu || g.route_count > 0 || g.bias_mode == B200Q_BCAST_FULL || (reinterpret_cast<uintptr_t>(g.out) & 15)) return false;
+  if (g.out_dtype == B200Q_BF16) return !g.D && g.N % 8 == 0 && g.ldo % 8 == 0;
+  return g.N % 4 == 0 && g.ldo % 4 == 0 &&
+         (!g.D || (g.d_dtype == B200Q_F32 && g.ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(g.D) & 15) == 0));
+}
+
 // Fused SwiGLU epilogue of a 256-column tile whose columns [0, 128) are gate and [128, 256) up
 // projections of the same 128 hidden units (GemmParams::swiglu): both halves get the GEMM's
 // scale / bias epilogue and its rounding to bf16, then silu(gate) * up -> bf16 -> * scale -> bf16
@@ -587,6 +681,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       float* cB = cA + BN;
       float* cBias = cB + BN;
       const EpiRow er = epi_stage_operands<BN, SWAP>(g, x_end, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
+      if (!SWAP && p.whole_rows && g.D) epi_prefetch_acc<BN>(g, x0 + q * 32 + lane, y0);
       // The wait can give up for some threads only; the decision to stop must be the same for
       // all 128 epilogue threads because they meet at named barriers: one thread samples the
       // abort flag between two barriers and everybody follows that sample.
@@ -596,7 +691,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       named_bar_sync(1, kEpiThreads);
       if (*epi_stop) break;
       tc_fence_after();
-      epi_drain<BN, SWAP>(g, tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN, er, y0, cA, cB, cBias);
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      if constexpr (!SWAP) {
+        if (p.whole_rows)
+          epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+        else
+          epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias);
+      } else {
+        epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias);
+      }
       tc_fence_before();
       mbar_arrive(bar_tempty + 8 * acc);
     }
@@ -636,8 +739,8 @@ struct PairSmem {
   static constexpr int kStageBytes = kXBytes + kYBytes;
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 4 epilogue warps x 4 KB (routed output)
-  static constexpr int kPatchBytes = (BN % 64 == 0) ? 4 * 4096 : 0;
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 4 epilogue warps x 4 KB (routed and whole-row output)
+  static constexpr int kPatchBytes = 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
@@ -767,6 +870,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       float* cB = cA + BN;
       float* cBias = cB + BN;
       const EpiRow er = epi_stage_operands<BN, false>(g, p.x_rows, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
+      if (p.whole_rows && g.D) epi_prefetch_acc<BN>(g, x0 + q * 32 + lane, y0);
       mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
       named_bar_sync(1, kEpiThreads);
       if (et == 0) *epi_stop = *abort_flag;
@@ -780,6 +884,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
         if constexpr (BN % 64 == 0)
           epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
                                reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+      } else if (p.whole_rows) {
+        epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
       } else {
         epi_drain<BN, false>(g, t_row, er, y0, cA, cB, cBias);
       }
@@ -885,6 +991,22 @@ static int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K,
   return make_tma_map_2d(map, base, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, rows, K, ld, 128, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// Estimated time of an M x N output in tiles of `rows` x `w`, on `units` SMs or SM pairs, per k and in columns: rounds of
+// tiles, each as long as its width and a width-independent part.  A grid of many rounds is limited by power and by L2,
+// not by its last round: an idle SM leaves its share to the others, so that it counts with its fraction.  us of pair
+// tiles of 256 / 224 / 192 / 160 / 128 / 96 / 64 columns, then of single tiles:
+//   256 x 4096 x 4096    16.9 / 15.3 / 13.9 / 12.2 / 11.1 / 10.6 / 10.1, 12.3    (M x N x K)
+//   256 x 8192 x 28672   71.5 / 66.5 / 64.0 / 60.7 / 56.6 / 80.7 / 75.9, 64.3
+//   300 x 14336 x 4096   33.8 / 30.0 / 35.1 / 31.8 / 35.5 / 34.9 / 40.8, 23.8
+//   700 x 2048 x 8192    26.7 / 24.1 / 21.3 / 19.7 / 17.0 / 15.6 / 23.3, 20.1
+//   1024 x 14336 x 4096  52.1 / 51.1 / 53.2 / 51.7 / 56.0 / 63.3 / 81.9, 57.0
+//   4096 x 14336 x 4096   167 / 182 / 210 / 219 / 242 / 275 / 323, 199
+static double tiling_cost(int64_t M, int64_t N, int rows, int w, int units) {
+  const int64_t tiles = (M + rows - 1) / rows * ((N + w - 1) / w);
+  const double rounds = (double)((tiles + units - 1) / units), spread = 1.1 * (double)tiles / units;
+  return (rounds > spread ? rounds : spread) * (w + 60);
+}
+
 int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
   // eligibility: TMA-compatible strides and bases, one problem per launch.  A is K-major when
   // stored [M][K] (trans_a = 0), B when stored [N][K] (trans_b = 1); the other storage orders
@@ -913,6 +1035,7 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
   tp.status = device_status_ptr();
   if (!tp.status) return B200Q_ERR_CUDA;
   tp.num_kb = (int)((g.K + kBlockK - 1) / kBlockK);
+  tp.whole_rows = whole_rows_output(g);
   // small M: weights on the lanes, tokens on the columns -- unless the tokens are MN-major (their
   // column tile would be narrower than the 128-byte MN-major row)
   const bool swap = g.M <= 128 && g.N >= 128 && !a_mn;
@@ -923,21 +1046,13 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
     tp.x_mn = a_mn; tp.y_mn = b_mn;
     tp.x_tiles = (int)((g.M + kBlockX - 1) / kBlockX);
     tp.x_tile_rows = kBlockX;
-    // Column-tile width: the one that minimises (waves over the 148 SMs) x (tile cost), with a tile at
-    // (width + kTileOverheadCols), so that narrower tiles are taken only where they remove a whole wave.  The overhead
-    // was fitted when a wait cost the issuing roles some 200 cycles (a wave of 224-column tiles took 96 % of one of 256);
-    // since the roles are whole warps a wave costs nearly its width: one wave of 256, 224 and 192 columns on CTA pairs (512 rows)
-    // 19.8, 17.4 and 15.8 us at K = 4096, 55.6, 47.8 and 42.4 at K = 14336.  4096 x 14336 x 4096, whose waves are 12.1, 13.8
-    // and 16.2: 167, 177 and 178 us.
-    // An MN-major B operand comes in 128-column blocks: 256 or 128 only.
+    // Column-tile width: the cheapest one.  (An MN-major B operand comes in 128-column blocks: 256 or 128 only.)
     static const int kWidths[] = {256, 224, 192, 160, 128};
     int bn = 128;
     double best = 1e30;
     for (int w : kWidths) {
-      if (w > 128 && g.N <= 128) continue;
-      if (b_mn && (w % 128)) continue;
-      const int64_t tiles = (int64_t)tp.x_tiles * ((g.N + w - 1) / w);
-      const double cost = (double)((tiles + kNumSMs - 1) / kNumSMs) * (w + kTileOverheadCols);
+      if (w > 128 && (g.N <= 128 || (b_mn && w % 128))) continue;
+      const double cost = 1.1 * tiling_cost(g.M, g.N, kBlockX, w, kNumSMs);  // (more L2 traffic than a pair's tile)
       if (cost < best) { best = cost; bn = w; }
     }
     tp.y_tiles = (int)((g.N + bn - 1) / bn);
@@ -950,25 +1065,30 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
     if (g.M > 128 && g.N > 128 && !no_pairs) {
       TcGemmParams pp = tp;
       pp.x_tiles = (int)((g.M + 2 * kBlockX - 1) / (2 * kBlockX));
-      int bp = 256;
-      double bestp = 1e30;
-      static const int kPairWidths[] = {256, 224, 192};
+      int bp = 0;  // 0: single CTAs are cheaper, for instance where a last 256-row tile would be half empty
+      static const int kPairWidths[] = {256, 224, 192, 160, 128, 96, 64};
+      static const int forced = std::getenv("B200Q_GEMM_PAIR_BN") ? std::atoi(std::getenv("B200Q_GEMM_PAIR_BN")) : 0;
+      if (routed) best = 1e30;  // (only the pair kernel has that epilogue)
       for (int w : kPairWidths) {
         if ((routed && (w % 64)) || (b_mn && w != 256)) continue;
-        const int64_t tiles = (int64_t)pp.x_tiles * ((g.N + w - 1) / w);
-        const double cost = (double)((tiles + kNumSMs / 2 - 1) / (kNumSMs / 2)) * (w + kTileOverheadCols);
-        if (cost < bestp) { bestp = cost; bp = w; }
+        const double cost = w == forced ? 0. : tiling_cost(g.M, g.N, 2 * kBlockX, w, kNumSMs / 2);
+        if (cost < best) { best = cost; bp = w; }
       }
-      static const int forced = std::getenv("B200Q_GEMM_PAIR_BN") ? std::atoi(std::getenv("B200Q_GEMM_PAIR_BN")) : 0;
-      if ((forced == 256 || forced == 224 || forced == 192) && !(routed && (forced % 64)) && !b_mn) bp = forced;
       if (g.swiglu) bp = 256;  // gate and up halves of a tile
-      pp.y_tiles = (int)((g.N + bp - 1) / bp);
-      rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, bp / 2);
-      if (rc) return rc;
+      if (bp) {
+        pp.y_tiles = (int)((g.N + bp - 1) / bp);
+        rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, bp / 2);
+        if (rc) return rc;
+      }
       switch (bp) {
         case 256: rc = launch_pair<256, 6>(mx, my, pp, st); break;
-        case 224: rc = launch_pair<224, 7>(mx, my, pp, st); break;
-        default: rc = launch_pair<192, 7>(mx, my, pp, st); break;
+        case 224: rc = launch_pair<224, 6>(mx, my, pp, st); break;
+        case 192: rc = launch_pair<192, 7>(mx, my, pp, st); break;
+        case 160: rc = launch_pair<160, 7>(mx, my, pp, st); break;
+        case 128: rc = launch_pair<128, 8>(mx, my, pp, st); break;
+        case 96: rc = launch_pair<96, 9>(mx, my, pp, st); break;
+        case 64: rc = launch_pair<64, 10>(mx, my, pp, st); break;
+        default: rc = B200Q_ERR_UNSUPPORTED;
       }
       if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     }
@@ -977,9 +1097,9 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
     if (rc) return rc;
     switch (bn) {
       case 256: return launch_cfg<256, 4, false>(mx, my, tp, st);
-      case 224: return launch_cfg<224, 5, false>(mx, my, tp, st);
+      case 224: return launch_cfg<224, 4, false>(mx, my, tp, st);
       case 192: return launch_cfg<192, 5, false>(mx, my, tp, st);
-      case 160: return launch_cfg<160, 6, false>(mx, my, tp, st);
+      case 160: return launch_cfg<160, 5, false>(mx, my, tp, st);
       default: return launch_cfg<128, 6, false>(mx, my, tp, st);
     }
   }

@@ -368,6 +368,20 @@ def test_tcgen05_mn_major_operands(ops, tA, tB, M, N, K):
     assert torch.equal(r.cpu(), ref)
 
 
+@pytest.mark.parametrize("M,N", [(129, 136), (700, 2056), (500, 4104), (1000, 2600), (760, 4088), (512, 8200), (300, 11016)])
+@pytest.mark.parametrize("K", [48, 1424])
+def test_tile_widths(ops, M, N, K):
+    """Pair tiles of 64, 96, 128, 160, 192 and 224 columns and single tiles of 160, with partial tiles in both directions, below
+    and beyond one filling of the stage rings; small integers, whose sums are exact."""
+    g = torch.Generator().manual_seed(M + N + K)
+    A = torch.randint(-4, 5, (M, K), generator=g).float()
+    B = torch.randint(-4, 5, (N, K), generator=g).float()
+    bias = torch.randint(-9, 10, (N,), generator=g).float()
+    r = torch.ops.hpu.fp8_gemm_v2(A.to(torch.float8_e4m3fn).cuda(), False, B.to(torch.float8_e4m3fn).cuda(), True, None, torch.float32,
+                                  None, None, bias.cuda())
+    assert torch.equal(r.cpu(), A @ B.t() + bias)
+
+
 @pytest.mark.parametrize("tA,tB", [(True, False), (True, True), (False, False)])
 @pytest.mark.parametrize("M,N,K", [(144, 144, 16), (272, 528, 2064), (5120, 2064, 144)])
 def test_mn_major_operands_on_cta_pairs(ops, tA, tB, M, N, K):
