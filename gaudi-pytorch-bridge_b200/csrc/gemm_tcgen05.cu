@@ -6,7 +6,7 @@
 //   warp 1    TMEM owner and MMA issuer: tcgen05.mma.kind::f8f6f4 (128 x BN x 32 per
 //             instruction), tcgen05.commit releases ring stages and publishes finished
 //             accumulators (both roles are run by the whole warp, which elects a lane to issue)
-//   warps 2-5 epilogue: tcgen05.ld the fp32 accumulator (each warp its 32 TMEM lanes),
+//   warps 2-9 epilogue: tcgen05.ld the fp32 accumulator (each warp its 32 TMEM lanes),
 //             apply (acc * sa) * sb + bias + D, round once, store
 // The accumulator is double-buffered in TMEM (2 x BN columns) so the epilogue of tile i
 // overlaps the main loop of tile i+1.
@@ -31,8 +31,9 @@ using namespace ptx;
 constexpr int kBlockX = 128;  // rows of the lane-side operand per tile (UMMA M)
 constexpr int kBlockK = 128;  // bytes (= fp8 elements) of K per ring stage: one swizzle row
 constexpr int kUmmaK = 32;
-constexpr int kThreads = 192;
-constexpr int kEpiThreads = 128;
+// Epilogue warps: two for each quarter of the TMEM lanes, which take turns with 32-column groups of a tile (few-token form:
+// one, its tiles have few columns).
+constexpr int epi_threads(bool swap) { return swap ? 128 : 256; }
 
 enum { kErrProducer = 101, kErrMma = 102, kErrMmaTmem = 103, kErrEpilogue = 104 };
 
@@ -60,7 +61,7 @@ struct SmemLayout {
   static_assert(kSubBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;  // per accumulator: col scale A, col scale B, col bias
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 4 epilogue warps x 4 KB (whole-row output)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 8 epilogue warps x 2 KB (whole-row output)
   static constexpr int kPatchBytes = BN >= 128 && KPS == 1 ? 4 * 4096 : 0;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
@@ -83,7 +84,7 @@ __device__ __forceinline__ EpiRow epi_stage_operands(const GemmParams& g, int64_
   // which output dimension the columns are: n (normal) or m (swapped)
   const int col_mode = SWAP ? B200Q_BCAST_PER_ROW : B200Q_BCAST_PER_COL;
   const int row_mode = SWAP ? B200Q_BCAST_PER_COL : B200Q_BCAST_PER_ROW;
-  for (int c = et; c < BN; c += kEpiThreads) {
+  for (int c = et; c < BN; c += epi_threads(SWAP)) {
     const int64_t y = y0 + c;
     const bool in = y < y_rows;
     cA[c] = (g.a_scale_mode == col_mode && in) ? __ldg(g.a_scale + y) : 1.f;
@@ -295,11 +296,11 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& g, const uint32_t* r
 // TMEM accumulator (this warp's 32 lanes, BN columns from t_row) -> scaled, biased, rounded, stored.
 template <int BN, bool SWAP>
 __device__ __forceinline__ void epi_drain(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t y0,
-                                          const float* cA, const float* cB, const float* cBias) {
+                                          const float* cA, const float* cB, const float* cBias, int half) {
   const EpiFlags f = epi_flags<SWAP>(g);
   uint32_t code_max = 0;  // fused output cast: largest magnitude code (fp8 byte & 0x7F) this thread wrote, per byte lane
 #pragma unroll 1
-  for (int c0 = 0; c0 < BN; c0 += 32) {
+  for (int c0 = 32 * half; c0 < BN; c0 += SWAP ? 32 : 64) {
     uint32_t r[32];
     if (BN % 32 == 0) {
       tmem_ld_32x32(t_row + c0, r);
@@ -361,89 +362,85 @@ __device__ __forceinline__ void epi_drain_routed(const GemmParams& g, uint32_t t
   }
 }
 
-// fp32 output, with or without an fp32 accumulate input, or bf16 output without one, in whole 128-byte row segments:
-// what a thread computes for its row goes through a 4 KB patch of its warp as in the routed form, so that a load or
-// store instruction covers four rows of 128 bytes instead of 16 bytes of 32 rows.  The accumulate input of the next 32
-// columns is on its way while a group is finished.  (whole_rows_output() says for which outputs.)
+// fp32 output, with or without an fp32 accumulate input, or bf16 output without one, in 64-byte row segments: what a
+// thread computes for its row goes through a 2 KB patch of its warp (four 16-byte pieces per row, XOR-swizzled so that
+// neither side has bank conflicts), so that a load or store instruction covers eight rows of 64 bytes instead of 16 bytes
+// of 32 rows.  The accumulate input of the warp's next 32 columns is on its way while a group is finished.  Of few k it is
+// the epilogue that sets the pace; accumulated 4352 x 4992 x 498 (M x N x K) / plain fp32 8192 x 8192 x 640, us: 82 / - with 16-byte
+// pieces of 32 rows, 61 / 99 with four warps and 128-byte segments, 55 / 79 with eight warps.  Asking for the accumulate
+// input's lines of the next tile as far as L2 did not help (71).  (whole_rows_output() says for which outputs.)
 template <int BN>
 __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
-                                               const float* cA, const float* cB, const float* cBias, uint4* patch, int lane) {
+                                               const float* cA, const float* cB, const float* cBias, uint4* patch, int lane, int half) {
   const EpiFlags f = epi_flags<false>(g);
-  const int prow = lane >> 3, piece = lane & 7;  // a lane's rows of the patch: prow + 4 k
+  const int prow = lane >> 2, piece = lane & 3;  // a lane's rows of the patch: prow + 8 k
+  uint4* put = patch + lane * 4;
+  const int put_x = (lane >> 1) & 3;
+  const uint4* take = patch + prow * 4 + (piece ^ ((prow >> 1) & 3));  // (rows 8 apart are swizzled alike)
   if (g.out_dtype == B200Q_F32) {
     float* out = static_cast<float*>(g.out) + (row0 + prow) * g.ldo + y0 + 4 * piece;
     const float* acc = static_cast<const float*>(g.D) + (row0 + prow) * g.ldd + y0 + 4 * piece;
     float4 d[8];
     auto load_acc = [&](int c0) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (row0 + prow + 4 * k < g.M && y0 + c0 + 4 * piece < g.N)
-          d[k] = __ldg(reinterpret_cast<const float4*>(acc + (int64_t)(4 * k) * g.ldd + c0));
+      for (int k = 0; k < 8; ++k) {
+        const int c = c0 + 16 * (k >> 2);
+        if (row0 + prow + 8 * (k & 3) < g.M && y0 + c + 4 * piece < g.N)
+          d[k] = __ldg(reinterpret_cast<const float4*>(acc + (int64_t)(8 * (k & 3)) * g.ldd + c));
+      }
     };
-    if (g.D) load_acc(0);
+    if (g.D) load_acc(32 * half);
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
+    for (int c0 = 32 * half; c0 < BN; c0 += 64) {
       uint32_t r[32];
       tmem_ld_32x32(t_row + c0, r);
       tmem_ld_wait();
       float v[32];
       epi_values<32>(r, c0, e, cA, cB, cBias, f, v);
 #pragma unroll
-      for (int k = 0; k < 8; ++k)
-        patch[lane * 8 + (k ^ (lane & 7))] = make_uint4(__float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]),
-                                                        __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
-      __syncwarp();
+      for (int h = 0; h < 2; ++h) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int row = prow + 4 * k;
-        const uint4 w = patch[row * 8 + (piece ^ (row & 7))];
-        float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
-        if (row0 + row < g.M && y0 + c0 + 4 * piece < g.N) {
-          if (g.D) o.x += d[k].x, o.y += d[k].y, o.z += d[k].z, o.w += d[k].w;
-          *reinterpret_cast<float4*>(out + (int64_t)(4 * k) * g.ldo + c0) = o;
+        for (int k = 0; k < 4; ++k) {
+          const float* w = v + 16 * h + 4 * k;
+          put[k ^ put_x] = make_uint4(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), __float_as_uint(w[3]));
         }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint4 w = take[32 * k];
+          float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
+          const int c = c0 + 16 * h;
+          if (row0 + prow + 8 * k < g.M && y0 + c + 4 * piece < g.N) {
+            if (g.D) o.x += d[4 * h + k].x, o.y += d[4 * h + k].y, o.z += d[4 * h + k].z, o.w += d[4 * h + k].w;
+            *reinterpret_cast<float4*>(out + (int64_t)(8 * k) * g.ldo + c) = o;
+          }
+        }
+        __syncwarp();
       }
-      if (g.D && c0 + 32 < BN) load_acc(c0 + 32);
-      __syncwarp();
+      if (g.D && c0 + 64 < BN) load_acc(c0 + 64);
     }
   } else {
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + (row0 + prow) * g.ldo + y0 + 8 * piece;
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 64) {
+    for (int c0 = 32 * half; c0 < BN; c0 += 64) {
+      uint32_t r[32];
+      tmem_ld_32x32(t_row + c0, r);
+      tmem_ld_wait();
+      float v[32];
+      epi_values<32>(r, c0, e, cA, cB, cBias, f, v);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (c0 + 32 * h >= BN) break;
-        uint32_t r[32];
-        tmem_ld_32x32(t_row + c0 + 32 * h, r);
-        tmem_ld_wait();
-        float v[32];
-        epi_values<32>(r, c0 + 32 * h, e, cA, cB, cBias, f, v);
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          patch[lane * 8 + ((4 * h + k) ^ (lane & 7))] =
-              make_uint4(pack_bf16x2(v[8 * k], v[8 * k + 1]), pack_bf16x2(v[8 * k + 2], v[8 * k + 3]),
-                         pack_bf16x2(v[8 * k + 4], v[8 * k + 5]), pack_bf16x2(v[8 * k + 6], v[8 * k + 7]));
-      }
+      for (int k = 0; k < 4; ++k)
+        put[k ^ put_x] = make_uint4(pack_bf16x2(v[8 * k], v[8 * k + 1]), pack_bf16x2(v[8 * k + 2], v[8 * k + 3]),
+                                    pack_bf16x2(v[8 * k + 4], v[8 * k + 5]), pack_bf16x2(v[8 * k + 6], v[8 * k + 7]));
       __syncwarp();
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int row = prow + 4 * k;
-        const uint4 w = patch[row * 8 + (piece ^ (row & 7))];
-        if (row0 + row < g.M && c0 + 8 * piece < BN && y0 + c0 + 8 * piece < g.N)
-          *reinterpret_cast<uint4*>(out + (int64_t)(4 * k) * g.ldo + c0) = w;
+      for (int k = 0; k < 4; ++k) {
+        const uint4 w = take[32 * k];
+        if (row0 + prow + 8 * k < g.M && y0 + c0 + 8 * piece < g.N) *reinterpret_cast<uint4*>(out + (int64_t)(8 * k) * g.ldo + c0) = w;
       }
       __syncwarp();
     }
   }
-}
-// The accumulate input of a warp's 32 rows and BN columns is asked for as far as L2 while the tile is still being multiplied.
-template <int BN>
-__device__ __forceinline__ void epi_prefetch_acc(const GemmParams& g, int64_t row, int64_t y0) {
-  if (row >= g.M) return;
-  const float* acc = static_cast<const float*>(g.D) + row * g.ldd + y0;
-#pragma unroll
-  for (int c = 0; c < BN; c += 32)
-    if (y0 + c < g.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(acc + c));
 }
 // Outputs that epi_drain_rows() takes: 16-byte aligned rows of whole 16-byte pieces.
 static bool whole_rows_output(const GemmParams& g) {
@@ -459,14 +456,14 @@ static bool whole_rows_output(const GemmParams& g) {
 // -> e4m3, with the same device functions as swiglu_cast_kernel so that the bytes are those of
 // the unfused pair of operators.  128 bytes per row and tile instead of 512 + a second pass.
 __device__ __forceinline__ void epi_drain_swiglu(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t y0,
-                                                 const float* cA, const float* cB, const float* cBias) {
+                                                 const float* cA, const float* cB, const float* cBias, int half) {
   const int64_t m = e.x;
   const float rA = e.rA, rB = e.rB, rBias = e.rBias;
   const float s_act = round_to_bf16(out8_scale_value(g));
   const int64_t f0 = (y0 >> 8) << 7;  // first hidden unit of the tile
   const int64_t F = g.N >> 1;
 #pragma unroll 1
-  for (int c0 = 0; c0 < 128; c0 += 32) {
+  for (int c0 = 32 * half; c0 < 128; c0 += 64) {
     uint32_t rg[32], ru[32];
     tmem_ld_32x32(t_row + c0, rg);
     tmem_ld_32x32(t_row + 128 + c0, ru);
@@ -506,7 +503,7 @@ __device__ __forceinline__ void epi_drain_swiglu(const GemmParams& g, uint32_t t
 }
 
 template <int BN, int STAGES, bool SWAP, int KPS = 1>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(64 + epi_threads(SWAP), 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const TcGemmParams p) {
   using L = SmemLayout<BN, STAGES, KPS>;
@@ -524,6 +521,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   // TMEM is allocated in powers of two columns (two accumulators of BN columns each)
+  constexpr int kEpiThreads = epi_threads(SWAP);
   constexpr uint32_t kTmemCols = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
 
   if (threadIdx.x == 0) {
@@ -533,7 +531,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(bar_tfull + 8 * a, 1);
-      mbar_init(bar_tempty + 8 * a, kEpiThreads);
+      mbar_init(bar_tempty + 8 * a, kEpiThreads / 32);  // (a warp arrives once)
     }
     *abort_flag = 0;
     *epi_stop = 0;
@@ -666,10 +664,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..9, few-token form 2..5)
     const GemmParams& g = p.g;
     const int q = warp & 3;              // TMEM lane quarter this warp may read
-    const int et = threadIdx.x - 64;     // 0..127
+    const int half = (warp - 2) >> 2;    // which of its two warps this is
+    const int et = threadIdx.x - 64;
     int it = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
       const int xt = tile % p.x_tiles, yt = tile / p.x_tiles;
@@ -681,9 +680,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       float* cB = cA + BN;
       float* cBias = cB + BN;
       const EpiRow er = epi_stage_operands<BN, SWAP>(g, x_end, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
-      if (!SWAP && p.whole_rows && g.D) epi_prefetch_acc<BN>(g, x0 + q * 32 + lane, y0);
       // The wait can give up for some threads only; the decision to stop must be the same for
-      // all 128 epilogue threads because they meet at named barriers: one thread samples the
+      // all epilogue threads because they meet at named barriers: one thread samples the
       // abort flag between two barriers and everybody follows that sample.
       mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
       named_bar_sync(1, kEpiThreads);
@@ -694,14 +692,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       if constexpr (!SWAP) {
         if (p.whole_rows)
-          epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+          epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+                             reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
         else
-          epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias);
+          epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias, half);
       } else {
-        epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias);
+        epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias, 0);
       }
       tc_fence_before();
-      mbar_arrive(bar_tempty + 8 * acc);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_tempty + 8 * acc);
     }
   }
 
@@ -739,7 +739,7 @@ struct PairSmem {
   static constexpr int kStageBytes = kXBytes + kYBytes;
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 4 epilogue warps x 4 KB (routed and whole-row output)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 8 epilogue warps x 2 KB (whole-row output; routed output: 4 x 4 KB)
   static constexpr int kPatchBytes = 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
@@ -747,7 +747,7 @@ struct PairSmem {
 };
 
 template <int BN, int STAGES>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + epi_threads(false), 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                          const TcGemmParams p) {
   using L = PairSmem<BN, STAGES>;
@@ -764,6 +764,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * STAGES;
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+  constexpr int kEpiThreads = epi_threads(false);
   constexpr uint32_t kTmemCols = 2 * BN <= 256 ? 256 : 512;
 
   if (threadIdx.x == 0) {
@@ -773,7 +774,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(bar_tfull + 8 * a, 1);
-      mbar_init(bar_tempty + 8 * a, 2 * kEpiThreads);  // used in the even CTA only
+      mbar_init(bar_tempty + 8 * a, 2 * kEpiThreads / 32);  // used in the even CTA only; a warp arrives once
     }
     *abort_flag = 0;
     *epi_stop = 0;
@@ -857,9 +858,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
+    // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
     const GemmParams& g = p.g;
-    const int q = warp & 3;
+    const int q = warp & 3, half = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;
     int it = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++it) {
@@ -870,7 +871,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       float* cB = cA + BN;
       float* cBias = cB + BN;
       const EpiRow er = epi_stage_operands<BN, false>(g, p.x_rows, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
-      if (p.whole_rows && g.D) epi_prefetch_acc<BN>(g, x0 + q * 32 + lane, y0);
       mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
       named_bar_sync(1, kEpiThreads);
       if (et == 0) *epi_stop = *abort_flag;
@@ -879,18 +879,23 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       if (BN == 256 && g.swiglu) {
-        epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias);
+        epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias, half);
       } else if (BN % 64 == 0 && g.route_count > 0) {
         if constexpr (BN % 64 == 0)
-          epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
-                               reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+          if (half == 0)  // (with the patches of both warps)
+            epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+                                 reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
       } else if (p.whole_rows) {
-        epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+        epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+                           reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
       } else {
-        epi_drain<BN, false>(g, t_row, er, y0, cA, cB, cBias);
+        epi_drain<BN, false>(g, t_row, er, y0, cA, cB, cBias, half);
       }
       tc_fence_before();
-      mbar_arrive_cluster((bar_tempty + 8 * acc) & kPeerBitMask);  // the even CTA's barrier
+      __syncwarp();
+      // the even CTA's barrier (a release of CTA scope: what it says is that tensor memory has been read; of cluster
+      // scope and from every thread, it held the accumulator back by 1 us per tile)
+      if (lane == 0) mbar_arrive_remote((bar_tempty + 8 * acc) & kPeerBitMask);
     }
   }
 
@@ -911,7 +916,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
 template <int BN, int STAGES>
 static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = PairSmem<BN, STAGES>;
-  constexpr int smem = L::kTotal + 1024;
+  constexpr int smem = L::kTotal + 1024, kPairThreads = 64 + epi_threads(false);
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
   auto kern = gemm_tcgen05_pair_kernel<BN, STAGES>;
@@ -925,7 +930,7 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGem
     B200Q_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kNumSMs, 1, 1);
-    cfg.blockDim = dim3(kThreads, 1, 1);
+    cfg.blockDim = dim3(kPairThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaError_t oe = cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg);
@@ -939,9 +944,9 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGem
   int tiles = tp.x_tiles * tp.y_tiles;
   int pairs = tiles < clusters ? tiles : clusters;
   static const bool no_pdl = std::getenv("B200Q_GEMM_NO_PDL") != nullptr;  // comparison switch
-  if (no_pdl || launch_overlapped(kern, dim3((unsigned)(2 * pairs)), dim3(kThreads), smem, st, mx, my, tp) != cudaSuccess) {
+  if (no_pdl || launch_overlapped(kern, dim3((unsigned)(2 * pairs)), dim3(kPairThreads), smem, st, mx, my, tp) != cudaSuccess) {
     if (!no_pdl) (void)cudaGetLastError();
-    kern<<<2 * pairs, kThreads, smem, st>>>(mx, my, tp);
+    kern<<<2 * pairs, kPairThreads, smem, st>>>(mx, my, tp);
   }
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
@@ -958,6 +963,7 @@ int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k
 template <int BN, int STAGES, bool SWAP, int KPS = 1>
 static int launch_cfg(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = SmemLayout<BN, STAGES, KPS>;
+  constexpr int kThreads = 64 + epi_threads(SWAP);
   constexpr int smem = L::kTotal + 1024;  // slack for the manual 1024-byte alignment
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
@@ -1071,7 +1077,9 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
       if (routed) best = 1e30;  // (only the pair kernel has that epilogue)
       for (int w : kPairWidths) {
         if ((routed && (w % 64)) || (b_mn && w != 256)) continue;
-        const double cost = w == forced ? 0. : tiling_cost(g.M, g.N, 2 * kBlockX, w, kNumSMs / 2);
+        // (a cluster's launch and its barriers take about 1 us more: 678 x 5504 x 1536 in a round of either 10.2 us on
+        // pairs, 9.1 on single CTAs; 2000 x 4096 x 1024 12.6, 11.5)
+        const double cost = w == forced ? 0. : tiling_cost(g.M, g.N, 2 * kBlockX, w, kNumSMs / 2) + 140e3 / (double)g.K;
         if (cost < best) { best = cost; bp = w; }
       }
       if (g.swiglu) bp = 256;  // gate and up halves of a tile
