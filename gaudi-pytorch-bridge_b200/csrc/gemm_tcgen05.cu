@@ -6,7 +6,7 @@
 //   warp 1    TMEM owner and MMA issuer: tcgen05.mma.kind::f8f6f4 (128 x BN x 32 per
 //             instruction), tcgen05.commit releases ring stages and publishes finished
 //             accumulators (both roles are run by the whole warp, which elects a lane to issue)
-//   warps 2-9 epilogue: tcgen05.ld the fp32 accumulator (each warp its 32 TMEM lanes),
+//   warps 2-5 or 2-9 epilogue: tcgen05.ld the fp32 accumulator (each warp its 32 TMEM lanes),
 //             apply (acc * sa) * sb + bias + D, round once, store
 // The accumulator is double-buffered in TMEM (2 x BN columns) so the epilogue of tile i
 // overlaps the main loop of tile i+1.
@@ -31,9 +31,10 @@ using namespace ptx;
 constexpr int kBlockX = 128;  // rows of the lane-side operand per tile (UMMA M)
 constexpr int kBlockK = 128;  // bytes (= fp8 elements) of K per ring stage: one swizzle row
 constexpr int kUmmaK = 32;
-// Epilogue warps: two for each quarter of the TMEM lanes, which take turns with 32-column groups of a tile (few-token form:
-// one, its tiles have few columns).
-constexpr int epi_threads(bool swap) { return swap ? 128 : 256; }
+// Epilogue warps, EW: one or two for each quarter of the TMEM lanes; two take turns with 32-column groups of a tile.  fp32
+// outputs have two, since of few k their epilogue sets the pace (linear layer's backward pass, 8000 x 4096 x 4096: 238 -> 231
+// us; see epi_drain_rows()), the others one: a gate/up GEMM of 8192 x 57344 x 8192, limited by power, took 3195 us with
+// two and 3110 with one.
 
 enum { kErrProducer = 101, kErrMma = 102, kErrMmaTmem = 103, kErrEpilogue = 104 };
 
@@ -61,7 +62,7 @@ struct SmemLayout {
   static_assert(kSubBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;  // per accumulator: col scale A, col scale B, col bias
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 8 epilogue warps x 2 KB (whole-row output)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // epilogue warps x 2 KB (whole-row output)
   static constexpr int kPatchBytes = BN >= 128 && KPS == 1 ? 4 * 4096 : 0;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
@@ -78,13 +79,13 @@ struct EpiRow {
   bool x_in;
 };
 
-template <int BN, bool SWAP>
+template <int BN, bool SWAP, int EW>
 __device__ __forceinline__ EpiRow epi_stage_operands(const GemmParams& g, int64_t x_rows, int64_t y_rows, int64_t x,
                                                      int64_t y0, int et, float* cA, float* cB, float* cBias) {
   // which output dimension the columns are: n (normal) or m (swapped)
   const int col_mode = SWAP ? B200Q_BCAST_PER_ROW : B200Q_BCAST_PER_COL;
   const int row_mode = SWAP ? B200Q_BCAST_PER_COL : B200Q_BCAST_PER_ROW;
-  for (int c = et; c < BN; c += epi_threads(SWAP)) {
+  for (int c = et; c < BN; c += 32 * EW) {
     const int64_t y = y0 + c;
     const bool in = y < y_rows;
     cA[c] = (g.a_scale_mode == col_mode && in) ? __ldg(g.a_scale + y) : 1.f;
@@ -294,13 +295,13 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& g, const uint32_t* r
 }
 
 // TMEM accumulator (this warp's 32 lanes, BN columns from t_row) -> scaled, biased, rounded, stored.
-template <int BN, bool SWAP>
+template <int BN, bool SWAP, int EW>
 __device__ __forceinline__ void epi_drain(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t y0,
                                           const float* cA, const float* cB, const float* cBias, int half) {
   const EpiFlags f = epi_flags<SWAP>(g);
   uint32_t code_max = 0;  // fused output cast: largest magnitude code (fp8 byte & 0x7F) this thread wrote, per byte lane
 #pragma unroll 1
-  for (int c0 = 32 * half; c0 < BN; c0 += SWAP ? 32 : 64) {
+  for (int c0 = 32 * half; c0 < BN; c0 += 8 * EW) {
     uint32_t r[32];
     if (BN % 32 == 0) {
       tmem_ld_32x32(t_row + c0, r);
@@ -369,7 +370,7 @@ __device__ __forceinline__ void epi_drain_routed(const GemmParams& g, uint32_t t
 // the epilogue that sets the pace; accumulated 4352 x 4992 x 498 (M x N x K) / plain fp32 8192 x 8192 x 640, us: 82 / - with 16-byte
 // pieces of 32 rows, 61 / 99 with four warps and 128-byte segments, 55 / 79 with eight warps.  Asking for the accumulate
 // input's lines of the next tile as far as L2 did not help (71).  (whole_rows_output() says for which outputs.)
-template <int BN>
+template <int BN, int EW>
 __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
                                                const float* cA, const float* cB, const float* cBias, uint4* patch, int lane, int half) {
   const EpiFlags f = epi_flags<false>(g);
@@ -391,7 +392,7 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
     };
     if (g.D) load_acc(32 * half);
 #pragma unroll 1
-    for (int c0 = 32 * half; c0 < BN; c0 += 64) {
+    for (int c0 = 32 * half; c0 < BN; c0 += 8 * EW) {
       uint32_t r[32];
       tmem_ld_32x32(t_row + c0, r);
       tmem_ld_wait();
@@ -417,12 +418,12 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
         }
         __syncwarp();
       }
-      if (g.D && c0 + 64 < BN) load_acc(c0 + 64);
+      if (g.D && c0 + 8 * EW < BN) load_acc(c0 + 8 * EW);
     }
   } else {
     __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + (row0 + prow) * g.ldo + y0 + 8 * piece;
 #pragma unroll 1
-    for (int c0 = 32 * half; c0 < BN; c0 += 64) {
+    for (int c0 = 32 * half; c0 < BN; c0 += 8 * EW) {
       uint32_t r[32];
       tmem_ld_32x32(t_row + c0, r);
       tmem_ld_wait();
@@ -456,14 +457,14 @@ static bool whole_rows_output(const GemmParams& g) {
 // -> e4m3, with the same device functions as swiglu_cast_kernel so that the bytes are those of
 // the unfused pair of operators.  128 bytes per row and tile instead of 512 + a second pass.
 __device__ __forceinline__ void epi_drain_swiglu(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t y0,
-                                                 const float* cA, const float* cB, const float* cBias, int half) {
+                                                 const float* cA, const float* cB, const float* cBias) {
   const int64_t m = e.x;
   const float rA = e.rA, rB = e.rB, rBias = e.rBias;
   const float s_act = round_to_bf16(out8_scale_value(g));
   const int64_t f0 = (y0 >> 8) << 7;  // first hidden unit of the tile
   const int64_t F = g.N >> 1;
 #pragma unroll 1
-  for (int c0 = 32 * half; c0 < 128; c0 += 64) {
+  for (int c0 = 0; c0 < 128; c0 += 32) {
     uint32_t rg[32], ru[32];
     tmem_ld_32x32(t_row + c0, rg);
     tmem_ld_32x32(t_row + 128 + c0, ru);
@@ -502,8 +503,8 @@ __device__ __forceinline__ void epi_drain_swiglu(const GemmParams& g, uint32_t t
   }
 }
 
-template <int BN, int STAGES, bool SWAP, int KPS = 1>
-__global__ void __launch_bounds__(64 + epi_threads(SWAP), 1)
+template <int BN, int STAGES, bool SWAP, int KPS, int EW>
+__global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const TcGemmParams p) {
   using L = SmemLayout<BN, STAGES, KPS>;
@@ -521,7 +522,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   // TMEM is allocated in powers of two columns (two accumulators of BN columns each)
-  constexpr int kEpiThreads = epi_threads(SWAP);
+  constexpr int kEpiThreads = 32 * EW;
   constexpr uint32_t kTmemCols = 2 * BN <= 32 ? 32 : 2 * BN <= 64 ? 64 : 2 * BN <= 128 ? 128 : 2 * BN <= 256 ? 256 : 512;
 
   if (threadIdx.x == 0) {
@@ -534,7 +535,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       mbar_init(bar_tempty + 8 * a, kEpiThreads / 32);  // (a warp arrives once)
     }
     *abort_flag = 0;
-    *epi_stop = 0;
+    epi_stop[0] = epi_stop[1] = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&map_x);
@@ -664,7 +665,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9, few-token form 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..5 or 2..9)
     const GemmParams& g = p.g;
     const int q = warp & 3;              // TMEM lane quarter this warp may read
     const int half = (warp - 2) >> 2;    // which of its two warps this is
@@ -679,25 +680,27 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       float* cA = epi_f + acc * 3 * BN;
       float* cB = cA + BN;
       float* cBias = cB + BN;
-      const EpiRow er = epi_stage_operands<BN, SWAP>(g, x_end, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
-      // The wait can give up for some threads only; the decision to stop must be the same for
-      // all epilogue threads because they meet at named barriers: one thread samples the
-      // abort flag between two barriers and everybody follows that sample.
-      mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
+      const EpiRow er = epi_stage_operands<BN, SWAP, EW>(g, x_end, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
+      // One warp waits for the accumulator (polling costs power and issue slots) and says whether to stop; the others meet it at the barrier, behind which the
+      // operands staged above can be read too.  A word per accumulator: a warp has read one before it lets the next
+      // but one be written.
+      if (et < 32) {
+        mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
+        __syncwarp();
+        if (et == 0) epi_stop[acc] = *abort_flag;
+      }
       named_bar_sync(1, kEpiThreads);
-      if (et == 0) *epi_stop = *abort_flag;
-      named_bar_sync(1, kEpiThreads);
-      if (*epi_stop) break;
+      if (epi_stop[acc]) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       if constexpr (!SWAP) {
         if (p.whole_rows)
-          epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+          epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
                              reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
         else
-          epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias, half);
+          epi_drain<BN, SWAP, EW>(g, t_row, er, y0, cA, cB, cBias, half);
       } else {
-        epi_drain<BN, SWAP>(g, t_row, er, y0, cA, cB, cBias, 0);
+        epi_drain<BN, SWAP, EW>(g, t_row, er, y0, cA, cB, cBias, 0);
       }
       tc_fence_before();
       __syncwarp();
@@ -739,15 +742,15 @@ struct PairSmem {
   static constexpr int kStageBytes = kXBytes + kYBytes;
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 8 epilogue warps x 2 KB (whole-row output; routed output: 4 x 4 KB)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // epilogue warps x 2 KB (whole-row output; routed output: 4 x 4 KB)
   static constexpr int kPatchBytes = 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
 };
 
-template <int BN, int STAGES>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + epi_threads(false), 1)
+template <int BN, int STAGES, int EW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                          const TcGemmParams p) {
   using L = PairSmem<BN, STAGES>;
@@ -764,7 +767,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * STAGES;
   const uint32_t bar_tfull = bar_empty + 8 * STAGES, bar_tempty = bar_tfull + 16;
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
-  constexpr int kEpiThreads = epi_threads(false);
+  constexpr int kEpiThreads = 32 * EW;
   constexpr uint32_t kTmemCols = 2 * BN <= 256 ? 256 : 512;
 
   if (threadIdx.x == 0) {
@@ -777,7 +780,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       mbar_init(bar_tempty + 8 * a, 2 * kEpiThreads / 32);  // used in the even CTA only; a warp arrives once
     }
     *abort_flag = 0;
-    *epi_stop = 0;
+    epi_stop[0] = epi_stop[1] = 0;
     fence_barrier_init();
     fence_proxy_async_smem();
     tma_prefetch_desc(&map_x);
@@ -858,7 +861,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
+    // ------------------------------------------------------------ epilogue (warps 2..5 or 2..9, both CTAs)
     const GemmParams& g = p.g;
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;
@@ -870,26 +873,27 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       float* cA = epi_f + acc * 3 * BN;
       float* cB = cA + BN;
       float* cBias = cB + BN;
-      const EpiRow er = epi_stage_operands<BN, false>(g, p.x_rows, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
-      mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
+      const EpiRow er = epi_stage_operands<BN, false, EW>(g, p.x_rows, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
+      if (et < 32) {  // (one warp waits for all: see the single-CTA kernel)
+        mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
+        __syncwarp();
+        if (et == 0) epi_stop[acc] = *abort_flag;
+      }
       named_bar_sync(1, kEpiThreads);
-      if (et == 0) *epi_stop = *abort_flag;
-      named_bar_sync(1, kEpiThreads);
-      if (*epi_stop) break;
+      if (epi_stop[acc]) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       if (BN == 256 && g.swiglu) {
-        epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias, half);
+        epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias);
       } else if (BN % 64 == 0 && g.route_count > 0) {
         if constexpr (BN % 64 == 0)
-          if (half == 0)  // (with the patches of both warps)
-            epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
-                                 reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+          epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+                               reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
       } else if (p.whole_rows) {
-        epi_drain_rows<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
+        epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
                            reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
       } else {
-        epi_drain<BN, false>(g, t_row, er, y0, cA, cB, cBias, half);
+        epi_drain<BN, false, EW>(g, t_row, er, y0, cA, cB, cBias, half);
       }
       tc_fence_before();
       __syncwarp();
@@ -913,13 +917,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   }
 }
 
-template <int BN, int STAGES>
-static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
+template <int BN, int STAGES, int EW>
+static int launch_pair_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = PairSmem<BN, STAGES>;
-  constexpr int smem = L::kTotal + 1024, kPairThreads = 64 + epi_threads(false);
+  constexpr int smem = L::kTotal + 1024, kPairThreads = 64 + 32 * EW;
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
-  auto kern = gemm_tcgen05_pair_kernel<BN, STAGES>;
+  auto kern = gemm_tcgen05_pair_kernel<BN, STAGES, EW>;
   // per device, once: raise the dynamic shared-memory limit and ask how many CTA pairs can be
   // resident at once (a pair needs both SMs of a TPC); -1 = pairs not available on this device
   static std::atomic<int> resident_pairs[kMaxDevices];
@@ -952,6 +956,11 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGem
   return B200Q_OK;
 }
 
+template <int BN, int STAGES>
+static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
+  return tp.g.out_dtype == B200Q_F32 ? launch_pair_ew<BN, STAGES, 8>(mx, my, tp, st) : launch_pair_ew<BN, STAGES, 4>(mx, my, tp, st);
+}
+
 // ------------------------------------------------------------------------ host side
 // 2-D map over a row-major byte matrix [rows][kbytes] with row stride ld bytes; box = 128 bytes x box_rows.
 int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t kbytes, int64_t ld_bytes,
@@ -960,14 +969,14 @@ int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k
                          CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-template <int BN, int STAGES, bool SWAP, int KPS = 1>
-static int launch_cfg(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
+template <int BN, int STAGES, bool SWAP, int KPS, int EW>
+static int launch_cfg_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = SmemLayout<BN, STAGES, KPS>;
-  constexpr int kThreads = 64 + epi_threads(SWAP);
+  constexpr int kThreads = 64 + 32 * EW;
   constexpr int smem = L::kTotal + 1024;  // slack for the manual 1024-byte alignment
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, SWAP, KPS>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SWAP, KPS, EW>;
   static std::atomic<int> configured[kMaxDevices];
   const int dev = current_device_index();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -986,6 +995,13 @@ static int launch_cfg(const CUtensorMap& mx, const CUtensorMap& my, const TcGemm
   }
   B200Q_LAUNCH_CHECK();
   return B200Q_OK;
+}
+
+template <int BN, int STAGES, bool SWAP, int KPS = 1>
+static int launch_cfg(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
+  if constexpr (!SWAP)
+    if (tp.g.out_dtype == B200Q_F32) return launch_cfg_ew<BN, STAGES, SWAP, KPS, 8>(mx, my, tp, st);
+  return launch_cfg_ew<BN, STAGES, SWAP, KPS, 4>(mx, my, tp, st);
 }
 
 static inline int fmt_bits(int dtype) { return dtype == B200Q_E5M2 ? 1 : 0; }

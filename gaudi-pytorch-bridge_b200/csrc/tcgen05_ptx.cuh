@@ -240,13 +240,9 @@ __device__ __forceinline__ void umma_commit_pair_both(uint32_t bar) {
       "}\n" ::"r"(bar)
       : "memory");
 }
-// Arrive on a barrier addressed in the cluster window (own CTA or the peer).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same with the default (CTA-scope) release: no cluster-wide fence is executed, which on
-// B200 costs about a thousand cycles per arrival.  Enough when what the arrival publishes is
-// this CTA's own shared memory, already made visible to the async proxy by
+// Arrive on a barrier addressed in the cluster window (own CTA or the peer), with the default (CTA-scope) release: no
+// cluster-wide fence is executed, which on B200 costs about a thousand cycles per arrival.  Enough when what the arrival
+// publishes is that tensor memory has been read, or this CTA's own shared memory, already made visible to the async proxy by
 // fence.proxy.async, and read there by the tensor core of this same SM.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
