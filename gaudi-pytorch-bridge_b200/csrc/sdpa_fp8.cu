@@ -27,7 +27,8 @@
 // step; 262 us with the two products issued by two warps and the groups out of step; 250 us with waits whose outcome
 // is a vote.  What did not
 // help: part of the exponentials as polynomials on the FMA pipe (the issue slots they take are as
-// scarce), sixteen softmax warps with half a row each, a strict alternation of the groups' exponentials.
+// scarce), sixteen softmax warps with half a row each, a strict alternation of the groups' exponentials, a third group of
+// warps that takes the row maxima of the next item meanwhile (16 heads x 8192 269 -> 252, but 8 x 4096 38 -> 43).
 // Two passes over the keys: the first only takes the row maxima, the second recomputes the
 // scores and forms exp(S - max) against the final maximum.  The probabilities are therefore
 // quantised exactly where the CPU restatement quantises them (no running-maximum rescaling of
