@@ -2,7 +2,8 @@
 lib/b200_hpu_ops_ext.so (the C++ torch extension that registers the hpu::* operators).
 
 Usage: python build.py [--force] [--verbose-ptxas]
-Objects are rebuilt only when a source or header is newer.
+Objects are rebuilt only when a source or header is newer.  What ptxas says of each kernel (registers, spills, shared memory) is
+kept beside the object as build/<source>.ptxas.
 """
 import glob
 import os
@@ -43,12 +44,15 @@ def build_kernels(force=False, ptxas_verbose=False):
     for src in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
         obj = os.path.join(OBJ, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
-        if force or _newer(obj, [src] + headers):
-            cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
+        report = obj[:-2] + ".ptxas"
+        if force or _newer(obj, [src] + headers) or not os.path.exists(report):
+            cmd = [NVCC, *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xptxas", "-v",
                    "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c", src, "-o", obj]
+            text = _run(cmd)
+            with open(report, "w") as f:
+                f.write(text)
             if ptxas_verbose:
-                cmd[1:1] = ["-Xptxas", "-v"]
-            log += _run(cmd)
+                log += text
     so = os.path.join(LIB, "libb200q.so")
     if force or _newer(so, objs):
         _run([NVCC, *ARCH, "-shared", "-o", so, *objs])

@@ -154,7 +154,17 @@ __device__ __forceinline__ void epi_values(const uint32_t* r, int c0, const EpiR
   }
 }
 
-template <int BN, bool SWAP>
+// Whether the GEMM's result is bf16 (else fp32).  The kernels with the rows of A on the lanes have it at compile time:
+// launch_cfg() and launch_pair() pick EW by it.  Instances that carried the other type's code and the bf16-only epilogues
+// as well spilled (fp32: 16 to 96 bytes stored per thread) or took 234 to 255 registers instead of 190 to 240; without, us:
+// fp32 7538 x 17744 x 640 with both operands MN-major 178 -> 160, 1817 x 21368 x 128 54 -> 50, the others 1 to 2 % less.
+template <bool SWAP, int EW>
+__device__ __forceinline__ bool bf16_output(const GemmParams& g) {
+  if constexpr (SWAP) return g.out_dtype == B200Q_BF16;
+  return EW == 4;
+}
+
+template <int BN, bool SWAP, int EW>
 __device__ __forceinline__ void epi_chunk(const GemmParams& g, const uint32_t* r, int c0, const EpiRow& e, int64_t y0,
                                           const float* cA, const float* cB, const float* cBias, const EpiFlags& f,
                                           uint32_t& code_max) {
@@ -224,7 +234,7 @@ __device__ __forceinline__ void epi_chunk(const GemmParams& g, const uint32_t* r
               code_max = max(code_max, (w[j / 4] >> (8 * (j & 3))) & 0x7Fu);
             }
         }
-      } else if (g.out_dtype == B200Q_BF16) {
+      } else if (bf16_output<SWAP, EW>(g)) {
         __nv_bfloat16* o = static_cast<__nv_bfloat16*>(g.out) + m * g.ldo + n0;
         if (n0 + CW <= g.N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
 #pragma unroll
@@ -309,7 +319,7 @@ __device__ __forceinline__ void epi_drain(const GemmParams& g, uint32_t t_row, c
       tmem_ld_32x16(t_row + c0, r);  // BN == 16
     }
     tmem_ld_wait();
-    epi_chunk<BN, SWAP>(g, r, c0, e, y0, cA, cB, cBias, f, code_max);
+    epi_chunk<BN, SWAP, EW>(g, r, c0, e, y0, cA, cB, cBias, f, code_max);
   }
   if (g.out8_amax) {
     uint32_t m = max(max(code_max & 0xFFu, (code_max >> 8) & 0xFFu), max((code_max >> 16) & 0xFFu, code_max >> 24));
@@ -375,18 +385,22 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
                                                const float* cA, const float* cB, const float* cBias, uint4* patch, int lane, int half) {
   const EpiFlags f = epi_flags<false>(g);
   const int prow = lane >> 2, piece = lane & 3;  // a lane's rows of the patch: prow + 8 k
+  constexpr int kPiece = EW == 8 ? 4 : 8;        // columns in 16 bytes
+  // the lane's rows and columns inside the output, counted from its own first ones (in 32 bits: the fp32 form has no register to spare)
+  const int rows = (int)(g.M - row0 < 32 ? g.M - row0 : 32) - prow;
+  const int cols = (int)(g.N - y0 < BN ? g.N - y0 : BN) - kPiece * piece;
   uint4* put = patch + lane * 4;
   const int put_x = (lane >> 1) & 3;
   const uint4* take = patch + prow * 4 + (piece ^ ((prow >> 1) & 3));  // (rows 8 apart are swizzled alike)
-  if (g.out_dtype == B200Q_F32) {
-    float* out = static_cast<float*>(g.out) + (row0 + prow) * g.ldo + y0 + 4 * piece;
-    const float* acc = static_cast<const float*>(g.D) + (row0 + prow) * g.ldd + y0 + 4 * piece;
+  if constexpr (EW == 8) {
+    float* out = static_cast<float*>(g.out) + (row0 + prow) * g.ldo + y0 + kPiece * piece;
+    const float* acc = static_cast<const float*>(g.D) + (row0 + prow) * g.ldd + y0 + kPiece * piece;
     float4 d[8];
     auto load_acc = [&](int c0) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int c = c0 + 16 * (k >> 2);
-        if (row0 + prow + 8 * (k & 3) < g.M && y0 + c + 4 * piece < g.N)
+        if (8 * (k & 3) < rows && c < cols)
           d[k] = __ldg(reinterpret_cast<const float4*>(acc + (int64_t)(8 * (k & 3)) * g.ldd + c));
       }
     };
@@ -411,7 +425,7 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
           const uint4 w = take[32 * k];
           float4 o = make_float4(__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w));
           const int c = c0 + 16 * h;
-          if (row0 + prow + 8 * k < g.M && y0 + c + 4 * piece < g.N) {
+          if (8 * k < rows && c < cols) {
             if (g.D) o.x += d[4 * h + k].x, o.y += d[4 * h + k].y, o.z += d[4 * h + k].z, o.w += d[4 * h + k].w;
             *reinterpret_cast<float4*>(out + (int64_t)(8 * k) * g.ldo + c) = o;
           }
@@ -421,7 +435,7 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
       if (g.D && c0 + 8 * EW < BN) load_acc(c0 + 8 * EW);
     }
   } else {
-    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + (row0 + prow) * g.ldo + y0 + 8 * piece;
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(g.out) + (row0 + prow) * g.ldo + y0 + kPiece * piece;
 #pragma unroll 1
     for (int c0 = 32 * half; c0 < BN; c0 += 8 * EW) {
       uint32_t r[32];
@@ -437,7 +451,7 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const uint4 w = take[32 * k];
-        if (row0 + prow + 8 * k < g.M && y0 + c0 + 8 * piece < g.N) *reinterpret_cast<uint4*>(out + (int64_t)(8 * k) * g.ldo + c0) = w;
+        if (8 * k < rows && c0 < cols) *reinterpret_cast<uint4*>(out + (int64_t)(8 * k) * g.ldo + c0) = w;
       }
       __syncwarp();
     }
@@ -883,15 +897,15 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       if (epi_stop[acc]) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
-      if (BN == 256 && g.swiglu) {
+      uint4* patch = reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256;
+      // (SwiGLU and routed output are bf16 epilogues: four warps, so that a quarter's 4 KB patch is one warp's)
+      if (EW == 4 && BN == 256 && g.swiglu) {
         epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias);
-      } else if (BN % 64 == 0 && g.route_count > 0) {
-        if constexpr (BN % 64 == 0)
-          epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
-                               reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256, lane);
+      } else if (EW == 4 && BN % 64 == 0 && g.route_count > 0) {
+        if constexpr (EW == 4 && BN % 64 == 0)
+          epi_drain_routed<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, patch, lane);
       } else if (p.whole_rows) {
-        epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
-                           reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
+        epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, patch + half * 128, lane, half);
       } else {
         epi_drain<BN, false, EW>(g, t_row, er, y0, cA, cB, cBias, half);
       }

@@ -140,3 +140,15 @@ def test_w4a16_workspace_query_below_one_k_block(K):
         assert abi.lib.b200q_w4a16_workspace_bytes(M, 64, K) == 0
     assert abi.lib.b200q_w4a16_workspace_bytes(64, 8192, 8192) > 0   # split-K path
     assert abi.lib.b200q_w4a16_workspace_bytes(16, 8192, 8192) == 0  # few-token kernel: reduced inside its clusters
+
+
+def test_fp8_gemm_kernels_keep_their_registers():
+    """No instance of the FP8 GEMM kernels spills (its epilogue sets the pace of products with few k)."""
+    path = os.path.join(ROOT, "gaudi-pytorch-bridge_b200", "build", "gemm_tcgen05.ptxas")
+    if not os.path.exists(path):
+        pytest.skip("the kernels were not built in this tree")
+    with open(path) as f:
+        report = f.read()
+    kernels = re.findall(r"Compiling entry function '(\S*gemm_tcgen05\S*)'.*?\n.*?\n\s*(\d+) bytes stack frame, (\d+) bytes spill stores", report)
+    assert len(kernels) == len(set(k[0] for k in kernels)) > 0
+    assert [k for k in kernels if k[1:] != ("0", "0")] == []
