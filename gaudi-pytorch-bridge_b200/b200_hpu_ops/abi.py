@@ -12,11 +12,12 @@ F32, BF16, E4M3, E5M2 = 0, 1, 2, 3
 BCAST_NONE, BCAST_SCALAR_HOST, BCAST_SCALAR_DEV, BCAST_PER_COL, BCAST_PER_ROW, BCAST_FULL = range(6)
 ROUND_RNE, ROUND_STOCHASTIC = 0, 1
 ZP_NONE, ZP_PACKED, ZP_FLOAT = 0, 1, 2
+GEMM_GENERIC, GEMM_FEW_TOKENS, GEMM_SINGLE, GEMM_PAIRS = range(4)
 CAST_MUL_IN_FP32 = 1
 
 EXPORTS = [
     "b200q_strerror", "b200q_last_cuda_error", "b200q_device_status", "b200q_selftest_wait_timeout", "b200q_launch_count", "b200q_sizeof_args",
-    "b200q_cast_to_fp8", "b200q_cast_to_fp8_hybrid", "b200q_cast_from_fp8", "b200q_dequant_int4", "b200q_gptq_repack", "b200q_fp8_gemm", "b200q_tp_reduce_bcast", "b200q_fp8_sdpa_fwd",
+    "b200q_cast_to_fp8", "b200q_cast_to_fp8_hybrid", "b200q_cast_from_fp8", "b200q_dequant_int4", "b200q_gptq_repack", "b200q_fp8_gemm", "b200q_fp8_gemm_plan", "b200q_tp_reduce_bcast", "b200q_fp8_sdpa_fwd",
     "b200q_w4a16_gemm", "b200q_w4a16_workspace_bytes", "b200q_w4a16_gemm_noalloc", "b200q_swiglu_cast_fp8",
     "b200q_amax", "b200q_scale_from_amax", "b200q_amax_history_update",
     "b200q_softmax_fp8", "b200q_sum_fp8_workspace_bytes", "b200q_sum_fp8", "b200q_in_place_interleave", "b200q_im2col_fp8",
@@ -44,6 +45,7 @@ class GemmArgs(C.Structure):
         ("swiglu", C.c_int),
         ("route_out", C.c_void_p * 8), ("route_count", C.c_int), ("route_rows", C.c_int64), ("route_row_offset", C.c_int64),
         ("out8_amax", C.c_void_p), ("b_static", C.c_int),
+        ("force_kernel", C.c_int), ("force_width", C.c_int),
     ]
 
 
@@ -85,6 +87,7 @@ def _bind():
     lib.b200q_dequant_int4.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p,
                                        C.c_int64, C.c_int64, C.c_int64, C.c_int, C.c_void_p]
     lib.b200q_fp8_gemm.argtypes = [C.POINTER(GemmArgs)]
+    lib.b200q_fp8_gemm_plan.argtypes = [C.POINTER(GemmArgs), C.POINTER(C.c_int), C.POINTER(C.c_int)]
     lib.b200q_fp8_sdpa_fwd.argtypes = [C.POINTER(SdpaArgs)]
     lib.b200q_tp_reduce_bcast.argtypes = [C.c_void_p, C.POINTER(C.c_void_p), C.c_int, C.c_int, C.c_int64, C.c_int64, C.c_void_p]
     lib.b200q_gptq_repack.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64,
@@ -187,7 +190,7 @@ def cast_from_fp8(x8, out_dtype, scale=None, scale_mode=None, rows=None, cols=No
 
 
 def fp8_gemm_nt(a8, b8, out_dtype=torch.bfloat16, a_scale=None, b_scale=None, bias=None, out=None,
-                force_generic=False, route=None, b_static=False):
+                force_generic=False, route=None, b_static=False, tiles=(0, 0)):
     """out[M][N] = a8[M][K] . b8[N][K]^T with scalar (float) a_scale, per-column fp32 CUDA b_scale [N]
     (or float), optional per-column bias [N]: the projection-GEMM form, straight through the C ABI."""
     M, K = a8.shape
@@ -222,6 +225,7 @@ def fp8_gemm_nt(a8, b8, out_dtype=torch.bfloat16, a_scale=None, b_scale=None, bi
     if bias is not None:
         g.bias, g.bias_dtype, g.bias_mode = bias.data_ptr(), DTYPE[bias.dtype], BCAST_PER_COL
     g.force_generic = 1 if force_generic else 0
+    g.force_kernel, g.force_width = tiles  # testing: (GEMM_SINGLE or GEMM_PAIRS, columns)
     g.b_static = 1 if b_static else 0  # the weights are not being written: see b200q_gemm_args.b_static
     g.stream = torch.cuda.current_stream().cuda_stream
     check(lib.b200q_fp8_gemm(C.byref(g)), "b200q_fp8_gemm")

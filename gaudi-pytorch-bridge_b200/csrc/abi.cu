@@ -302,7 +302,8 @@ int b200q_dequant_int4(const int32_t* packed, const void* scale, const void* zp,
                            k_packed, static_cast<cudaStream_t>(stream));
 }
 
-int b200q_fp8_gemm(const b200q_gemm_args* a) {
+// Checks the arguments of a GEMM and fills the kernels' block; empty: there is nothing to compute.
+static int gemm_params(const b200q_gemm_args* a, GemmParams& g, bool& empty) {
   if (!a) return B200Q_ERR_BAD_ARGUMENT;
   if (a->M < 0 || a->N < 0 || a->K < 0 || a->batch < 0) return B200Q_ERR_BAD_ARGUMENT;
   if (!is_fp8(a->a_dtype) || !is_fp8(a->b_dtype) || !is_wide(a->out_dtype)) return B200Q_ERR_BAD_ARGUMENT;
@@ -313,9 +314,9 @@ int b200q_fp8_gemm(const b200q_gemm_args* a) {
   if (a->bias_mode != B200Q_BCAST_NONE && (!a->bias || !is_wide(a->bias_dtype))) return B200Q_ERR_BAD_ARGUMENT;
   if (a->D && !is_wide(a->d_dtype)) return B200Q_ERR_BAD_ARGUMENT;
   const int64_t work = a->M * a->N * a->batch;
-  if (work == 0) return B200Q_OK;
+  empty = work == 0;
+  if (empty) return B200Q_OK;
   if ((!a->out && a->route_count <= 0) || (a->K > 0 && (!a->A || !a->B))) return B200Q_ERR_BAD_ARGUMENT;
-  GemmParams g;
   g.A = a->A; g.B = a->B; g.a_dtype = a->a_dtype; g.b_dtype = a->b_dtype; g.trans_a = a->trans_a; g.trans_b = a->trans_b;
   g.M = a->M; g.N = a->N; g.K = a->K; g.lda = a->lda; g.ldb = a->ldb;
   g.batch = a->batch; g.a_batch_stride = a->a_batch_stride; g.b_batch_stride = a->b_batch_stride;
@@ -330,11 +331,22 @@ int b200q_fp8_gemm(const b200q_gemm_args* a) {
   g.swiglu = a->swiglu;
   g.out8_amax = g.out8_dtype ? a->out8_amax : nullptr;
   g.b_static = a->b_static ? 1 : 0;
+  g.force_kernel = a->force_kernel; g.force_width = a->force_width;
+  if (g.force_kernel != B200Q_GEMM_GENERIC && g.force_kernel != B200Q_GEMM_SINGLE && g.force_kernel != B200Q_GEMM_PAIRS)
+    return B200Q_ERR_BAD_ARGUMENT;
   g.route_count = a->route_count; g.route_rows = a->route_rows; g.route_row_offset = a->route_row_offset;
   for (int i = 0; i < 8; ++i) g.route_out[i] = a->route_out[i];
   if (g.route_count < 0 || g.route_count > 8) return B200Q_ERR_BAD_ARGUMENT;
   for (int i = 0; i < g.route_count; ++i)
     if (!g.route_out[i] || (reinterpret_cast<uintptr_t>(g.route_out[i]) & 15)) return B200Q_ERR_BAD_ARGUMENT;
+  return B200Q_OK;
+}
+
+int b200q_fp8_gemm(const b200q_gemm_args* a) {
+  GemmParams g;
+  bool empty = false;
+  const int checked = gemm_params(a, g, empty);
+  if (checked != B200Q_OK || empty) return checked;
   cudaStream_t st = static_cast<cudaStream_t>(a->stream);
   if (g.route_count > 0) {
     if (g.batch != 1 || a->force_generic || g.route_row_offset < 0) return B200Q_ERR_UNSUPPORTED;
@@ -368,7 +380,22 @@ int b200q_fp8_gemm(const b200q_gemm_args* a) {
       }
     }
   }
-  return gemm_generic_launch(g, st);
+  return a->force_kernel ? B200Q_ERR_UNSUPPORTED : gemm_generic_launch(g, st);
+}
+
+int b200q_fp8_gemm_plan(const b200q_gemm_args* a, int* kernel, int* width) {
+  if (!kernel || !width) return B200Q_ERR_BAD_ARGUMENT;
+  *kernel = B200Q_GEMM_GENERIC;
+  *width = 0;
+  GemmParams g;
+  bool empty = false;
+  const int checked = gemm_params(a, g, empty);
+  if (checked != B200Q_OK || empty || a->force_generic || g.batch > 1024) return checked;
+  g.batch = 1;
+  const GemmPlan plan = gemm_tcgen05_plan(g);
+  *kernel = plan.kernel;
+  *width = plan.width;
+  return B200Q_OK;
 }
 
 int b200q_gptq_repack(const int32_t* qweight, int32_t* qweight_out, int64_t K, int64_t N, const int32_t* qzeros,

@@ -48,6 +48,7 @@ struct GemmParams {
   int64_t route_rows, route_row_offset;
   float* out8_amax;  // fused output cast only: max |fp8 value written| (atomic max on the bit pattern), or null
   int b_static;      // B is not written by work still in flight: it may be read before the preceding kernel completes
+  int force_kernel, force_width;  // testing: this B200Q_GEMM_* kernel in tiles of this many columns, or B200Q_GEMM_GENERIC (0): the cheapest
 };
 
 // value in out_dtype -> fp8 byte of the fused output cast
@@ -145,6 +146,12 @@ __device__ __forceinline__ void epilogue_store_one(const GemmParams& p, int64_t 
 }
 
 int gemm_generic_launch(const GemmParams& p, cudaStream_t st);
+// What a launch runs: the kernel (B200Q_GEMM_*; generic: none of the tensor-core kernels takes it), the width of its column
+// tiles, and that of the single tiles for a device on which no CTA pair fits (0: there are none).
+struct GemmPlan {
+  int kernel, width, single_width;
+};
+GemmPlan gemm_tcgen05_plan(const GemmParams& p);
 int gemm_tcgen05_launch(const GemmParams& p, cudaStream_t st);  // returns B200Q_ERR_UNSUPPORTED if not eligible
 
 }  // namespace b200q

@@ -1027,110 +1027,123 @@ static int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K,
   return make_tma_map_2d(map, base, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, rows, K, ld, 128, kBlockK, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-// Estimated time of an M x N output in tiles of `rows` x `w`, on `units` SMs or SM pairs, per k and in columns: rounds of
-// tiles, each as long as its width and a width-independent part.  A grid of many rounds is limited by power and by L2,
-// not by its last round: an idle SM leaves its share to the others, so that it counts with its fraction.  us of pair
-// tiles of 256 / 224 / 192 / 160 / 128 / 96 / 64 columns, then of single tiles:
-//   256 x 4096 x 4096    16.9 / 15.3 / 13.9 / 12.2 / 11.1 / 10.6 / 10.1, 12.3    (M x N x K)
-//   256 x 8192 x 28672   71.5 / 66.5 / 64.0 / 60.7 / 56.6 / 80.7 / 75.9, 64.3
-//   300 x 14336 x 4096   33.8 / 30.0 / 35.1 / 31.8 / 35.5 / 34.9 / 40.8, 23.8
-//   700 x 2048 x 8192    26.7 / 24.1 / 21.3 / 19.7 / 17.0 / 15.6 / 23.3, 20.1
-//   1024 x 14336 x 4096  52.1 / 51.1 / 53.2 / 51.7 / 56.0 / 63.3 / 81.9, 57.0
-//   4096 x 14336 x 4096   167 / 182 / 210 / 219 / 242 / 275 / 323, 199
-static double tiling_cost(int64_t M, int64_t N, int rows, int w, int units) {
-  const int64_t tiles = (M + rows - 1) / rows * ((N + w - 1) / w);
-  const double rounds = (double)((tiles + units - 1) / units), spread = 1.1 * (double)tiles / units;
-  return (rounds > spread ? rounds : spread) * (w + 60);
+// Estimated ns of the output in tiles of w columns, on CTA pairs (256 rows) or single CTAs (128).  What paces a tile is the tensor
+// core (1.32 ns per column and 128 k), or a CTA's loads (its 128 rows and its own columns, 128 bytes each per 128 k, 100 GB/s and SM:
+// single tiles and narrow ones reach that first), or the epilogue, which runs beside the next tile's main loop and is exposed
+// behind the last.  Rounds of tiles; of many tiles, power and L2 go to those that still run, so that a last round counts
+// with its fraction.  The constants are a fit to 6289 sizes and forms (129-5000 x 180-23000 x 128-12400, M x N x K; both outputs,
+// accumulated, fp8, ragged, transposed), each timed in all twelve tilings: of 4827 others
+// what is taken is 0.5 % slower than the best in the geometric mean, 3 % at the 95th and 8 % at the 99th percentile.  (With a cost of
+// rounds, widths and 1 us for a pair alone: 6, 29 and 40 %, and slower than wide tiles throughout had been for 14336 columns and 256 rows.)
+// us of single tiles of 256 / 224 / 192 / 160 / 128 columns, then of pair tiles of 256 / 224 / 192 / 160 / 128 / 96 / 64, bf16 output:
+//   256 x 4096 x 4096    17.8 / 17.0 / 14.3 / 13.6 / 12.2, 16.3 / 14.5 / 13.2 / 12.0 / 10.8 / 10.0 / 9.7
+//   256 x 14336 x 4096   20.5 / 19.9 / 24.5 / 23.8 / 21.6, 18.8 / 17.8 / 22.2 / 20.4 / 18.6 / 20.9 / 23.4
+//   300 x 14336 x 4096   30.3 / 29.1 / 25.2 / 24.3 / 28.2, 27.2 / 25.5 / 28.6 / 26.6 / 28.8 / 30.9 / 37.1
+//   700 x 2048 x 8192    28.9 / 27.9 / 22.7 / 22.0 / 20.3, 25.2 / 22.4 / 20.1 / 18.6 / 16.4 / 14.8 / 22.4
+//   1300 x 8192 x 8192   78.6 / 77.4 / 80.9 / 78.5 / 88.4, 73.6 / 70.0 / 77.7 / 79.5 / 80.1 / 87.1 / 117
+//   678 x 5504 x 1536    12.1 / 15.8 / 14.8 / 13.3 / 11.7, 12.2 / 14.4 / 13.6 / 12.3 / 11.5 / 12.3 / 12.8
+//   4096 x 14336 x 4096   176 / 183 / 189 / 200 / 225, 163 / 163 / 166 / 171 / 184 / 213 / 295
+static double tiling_cost(const GemmParams& g, bool pair, int w) {
+  const int units = pair ? kNumSMs / 2 : kNumSMs, rows = pair ? 2 * kBlockX : kBlockX;
+  const double mma = 1.32 * w, loads = 1.28 * (kBlockX + (pair ? w / 2 : w));
+  const double main_loop = (double)((g.K + kBlockK - 1) / kBlockK) * (mma > loads ? mma : loads) + 1100, epilogue = 20. * w + 1350;
+  const int64_t tiles = (g.M + rows - 1) / rows * ((g.N + w - 1) / w);
+  const double rounds = (double)((tiles + units - 1) / units), spread = 1.02 * (double)tiles / units;
+  const double ns = (main_loop > epilogue ? main_loop : epilogue) * (rounds > spread ? rounds : spread) + 0.3 * epilogue;
+  return pair ? ns + 200 : 1.02 * ns;
 }
 
-int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
+GemmPlan gemm_tcgen05_plan(const GemmParams& g) {
   // eligibility: TMA-compatible strides and bases, one problem per launch.  A is K-major when
   // stored [M][K] (trans_a = 0), B when stored [N][K] (trans_b = 1); the other storage orders
   // are MN-major operands, which the tensor core reads through MN-major descriptors.
+  const GemmPlan none = {B200Q_GEMM_GENERIC, 0, 0};
   const bool a_mn = g.trans_a != 0, b_mn = g.trans_b == 0;
-  if (g.batch != 1 || g.K < 1 || (g.lda % 16) || (g.ldb % 16)) return B200Q_ERR_UNSUPPORTED;
-  if ((!a_mn || !b_mn) && (g.K % 16)) return B200Q_ERR_UNSUPPORTED;  // a K-major row must be 16-byte granular
-  if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) return B200Q_ERR_UNSUPPORTED;
-  if (g.a_scale_mode == B200Q_BCAST_FULL || g.b_scale_mode == B200Q_BCAST_FULL) return B200Q_ERR_UNSUPPORTED;
-  if (g.M <= 0 || g.N <= 0) return B200Q_ERR_UNSUPPORTED;
-  if (g.M > (1ll << 30) || g.N > (1ll << 30) || g.K > (1ll << 30)) return B200Q_ERR_UNSUPPORTED;
+  if (g.batch != 1 || g.K < 1 || (g.lda % 16) || (g.ldb % 16)) return none;
+  if ((!a_mn || !b_mn) && (g.K % 16)) return none;  // a K-major row must be 16-byte granular
+  if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 15) return none;
+  if (g.a_scale_mode == B200Q_BCAST_FULL || g.b_scale_mode == B200Q_BCAST_FULL) return none;
+  if (g.M <= 0 || g.N <= 0) return none;
+  if (g.M > (1ll << 30) || g.N > (1ll << 30) || g.K > (1ll << 30)) return none;
 
   // fused SwiGLU: CTA-pair kernel only, whole 256-column tiles, bf16 intermediate
-  if (g.swiglu && (g.M <= 128 || (g.N % 256) || a_mn || b_mn || g.out_dtype != B200Q_BF16 || g.out8_dtype != B200Q_E4M3))
-    return B200Q_ERR_UNSUPPORTED;
+  if (g.swiglu && (g.M <= 128 || (g.N % 256) || a_mn || b_mn || g.out_dtype != B200Q_BF16 || g.out8_dtype != B200Q_E4M3)) return none;
 
   // routed output: bf16 rows through the CTA-pair kernel, every 128-row block inside one route block
   const bool routed = g.route_count > 0;
   if (routed && (g.M <= 128 || g.N <= 128 || a_mn || b_mn || g.out_dtype != B200Q_BF16 || g.out8_dtype || g.swiglu || g.D ||
                  g.bias_mode == B200Q_BCAST_FULL || (g.N % 8) || (g.ldo % 8) || g.route_rows <= 0 || (g.route_rows % 128) ||
                  g.route_count > 8 || (g.M + g.route_rows - 1) / g.route_rows > g.route_count))
-    return B200Q_ERR_UNSUPPORTED;
+    return none;
 
+  // small M: weights on the lanes, tokens on the columns -- unless the tokens are MN-major (their
+  // column tile would be narrower than the 128-byte MN-major row)
+  if (g.M <= 128 && g.N >= 128 && !a_mn && !g.force_kernel) {
+    const int w = g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
+    return {B200Q_GEMM_FEW_TOKENS, w, w};
+  }
+  // The cheapest tiling.  (An MN-major B comes in boxes of 128 columns per CTA: single tiles of 256 or 128 columns, pair
+  // tiles of 256.)
+  static const bool no_pairs = std::getenv("B200Q_GEMM_NO_PAIRS") != nullptr;  // comparison switches
+  static const int pair_bn = std::getenv("B200Q_GEMM_PAIR_BN") ? std::atoi(std::getenv("B200Q_GEMM_PAIR_BN")) : 0;
+  const bool pairs_only = routed || g.swiglu;  // (only the pair kernel has these epilogues)
+  GemmPlan plan = none;
+  double best = 1e30;
+  auto consider = [&](int kernel, int w, double cost) {
+    if (g.force_kernel && (kernel != g.force_kernel || w != g.force_width)) return;
+    if (cost < best) best = cost, plan.kernel = kernel, plan.width = w;
+  };
+  for (int w : {256, 224, 192, 160, 128}) {
+    if (w > 128 && (g.N <= 128 || (b_mn && w % 128))) continue;
+    consider(B200Q_GEMM_SINGLE, w, pairs_only ? 1e30 : tiling_cost(g, false, w));
+  }
+  plan.single_width = plan.width;
+  if (g.M > 128 && g.N > 128 && !no_pairs)
+    for (int w : {256, 224, 192, 160, 128, 96, 64}) {
+      if ((routed && (w % 64)) || ((b_mn || g.swiglu) && w != 256)) continue;
+      consider(B200Q_GEMM_PAIRS, w, w == pair_bn ? 0. : tiling_cost(g, true, w));
+    }
+  return plan;
+}
+
+int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
+  const GemmPlan plan = gemm_tcgen05_plan(g);
+  if (plan.kernel == B200Q_GEMM_GENERIC) return B200Q_ERR_UNSUPPORTED;
+  const bool a_mn = g.trans_a != 0, b_mn = g.trans_b == 0;
   TcGemmParams tp;
   tp.g = g;
   tp.status = device_status_ptr();
   if (!tp.status) return B200Q_ERR_CUDA;
   tp.num_kb = (int)((g.K + kBlockK - 1) / kBlockK);
   tp.whole_rows = whole_rows_output(g);
-  // small M: weights on the lanes, tokens on the columns -- unless the tokens are MN-major (their
-  // column tile would be narrower than the 128-byte MN-major row)
-  const bool swap = g.M <= 128 && g.N >= 128 && !a_mn;
   CUtensorMap mx, my;
-  if (!swap) {
+  if (plan.kernel != B200Q_GEMM_FEW_TOKENS) {
     tp.x_rows = g.M; tp.y_rows = g.N;
     tp.a_fmt_bits = fmt_bits(g.a_dtype); tp.b_fmt_bits = fmt_bits(g.b_dtype);
     tp.x_mn = a_mn; tp.y_mn = b_mn;
-    tp.x_tiles = (int)((g.M + kBlockX - 1) / kBlockX);
     tp.x_tile_rows = kBlockX;
-    // Column-tile width: the cheapest one.  (An MN-major B operand comes in 128-column blocks: 256 or 128 only.)
-    static const int kWidths[] = {256, 224, 192, 160, 128};
-    int bn = 128;
-    double best = 1e30;
-    for (int w : kWidths) {
-      if (w > 128 && (g.N <= 128 || (b_mn && w % 128))) continue;
-      const double cost = 1.1 * tiling_cost(g.M, g.N, kBlockX, w, kNumSMs);  // (more L2 traffic than a pair's tile)
-      if (cost < best) { best = cost; bn = w; }
-    }
-    tp.y_tiles = (int)((g.N + bn - 1) / bn);
     int rc = make_map(&mx, g.A, g.M, g.K, g.lda, a_mn, kBlockX);
     if (rc) return rc;
-    // CTA pairs (256-row tiles) when there are enough rows to fill them.  An MN-major operand is a box of 128 rows x
-    // 128 k in each CTA, so an MN-major B takes 256 columns.  Both products of the backward pass of a linear layer (8000
-    // tokens, 4096 x 4096: B MN-major, then both; 64 MB of fp32 accumulated): 268 us on single CTAs, 244 on pairs.
-    static const bool no_pairs = std::getenv("B200Q_GEMM_NO_PAIRS") != nullptr;
-    if (g.M > 128 && g.N > 128 && !no_pairs) {
-      TcGemmParams pp = tp;
-      pp.x_tiles = (int)((g.M + 2 * kBlockX - 1) / (2 * kBlockX));
-      int bp = 0;  // 0: single CTAs are cheaper, for instance where a last 256-row tile would be half empty
-      static const int kPairWidths[] = {256, 224, 192, 160, 128, 96, 64};
-      static const int forced = std::getenv("B200Q_GEMM_PAIR_BN") ? std::atoi(std::getenv("B200Q_GEMM_PAIR_BN")) : 0;
-      if (routed) best = 1e30;  // (only the pair kernel has that epilogue)
-      for (int w : kPairWidths) {
-        if ((routed && (w % 64)) || (b_mn && w != 256)) continue;
-        // (a cluster's launch and its barriers take about 1 us more: 678 x 5504 x 1536 in a round of either 10.2 us on
-        // pairs, 9.1 on single CTAs; 2000 x 4096 x 1024 12.6, 11.5)
-        const double cost = w == forced ? 0. : tiling_cost(g.M, g.N, 2 * kBlockX, w, kNumSMs / 2) + 140e3 / (double)g.K;
-        if (cost < best) { best = cost; bp = w; }
+    if (plan.kernel == B200Q_GEMM_PAIRS) {
+      tp.x_tiles = (int)((g.M + 2 * kBlockX - 1) / (2 * kBlockX));
+      tp.y_tiles = (int)((g.N + plan.width - 1) / plan.width);
+      rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, plan.width / 2);
+      if (rc) return rc;
+      switch (plan.width) {
+        case 256: rc = launch_pair<256, 6>(mx, my, tp, st); break;
+        case 224: rc = launch_pair<224, 6>(mx, my, tp, st); break;
+        case 192: rc = launch_pair<192, 7>(mx, my, tp, st); break;
+        case 160: rc = launch_pair<160, 7>(mx, my, tp, st); break;
+        case 128: rc = launch_pair<128, 8>(mx, my, tp, st); break;
+        case 96: rc = launch_pair<96, 9>(mx, my, tp, st); break;
+        default: rc = launch_pair<64, 10>(mx, my, tp, st); break;
       }
-      if (g.swiglu) bp = 256;  // gate and up halves of a tile
-      if (bp) {
-        pp.y_tiles = (int)((g.N + bp - 1) / bp);
-        rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, bp / 2);
-        if (rc) return rc;
-      }
-      switch (bp) {
-        case 256: rc = launch_pair<256, 6>(mx, my, pp, st); break;
-        case 224: rc = launch_pair<224, 6>(mx, my, pp, st); break;
-        case 192: rc = launch_pair<192, 7>(mx, my, pp, st); break;
-        case 160: rc = launch_pair<160, 7>(mx, my, pp, st); break;
-        case 128: rc = launch_pair<128, 8>(mx, my, pp, st); break;
-        case 96: rc = launch_pair<96, 9>(mx, my, pp, st); break;
-        case 64: rc = launch_pair<64, 10>(mx, my, pp, st); break;
-        default: rc = B200Q_ERR_UNSUPPORTED;
-      }
-      if (rc != B200Q_ERR_UNSUPPORTED) return rc;
+      // (unsupported: no cluster of two fits on this device)
+      if (rc != B200Q_ERR_UNSUPPORTED || !plan.single_width) return rc;
     }
-    if (g.swiglu || routed) return B200Q_ERR_UNSUPPORTED;  // only the pair kernel has these epilogues
+    const int bn = plan.single_width;
+    tp.x_tiles = (int)((g.M + kBlockX - 1) / kBlockX);
+    tp.y_tiles = (int)((g.N + bn - 1) / bn);
     rc = make_map(&my, g.B, g.N, g.K, g.ldb, b_mn, bn);
     if (rc) return rc;
     switch (bn) {
@@ -1144,7 +1157,7 @@ int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
   tp.x_rows = g.N; tp.y_rows = g.M;
   tp.a_fmt_bits = fmt_bits(g.b_dtype); tp.b_fmt_bits = fmt_bits(g.a_dtype);
   tp.x_mn = b_mn; tp.y_mn = 0;
-  const int bn = g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
+  const int bn = plan.width;
   tp.y_tiles = (int)((g.M + bn - 1) / bn);
   // Tile height.  The kernel is one pass over the weight bytes, and a CTA's share of them is
   // (rounds of tiles over the SMs) x (tile rows): 14336 weight rows in 128-row tiles are 112 tiles,

@@ -247,9 +247,23 @@ typedef struct b200q_gemm_args {
    * 0 (default) = nothing is read before the preceding kernel is complete.  No counterpart in the
    * reference (a graph compiler orders its loads). */
   int b_static;
+  /* Testing (0 = the library chooses): this kernel (B200Q_GEMM_SINGLE or B200Q_GEMM_PAIRS) in tiles of force_width columns;
+   * B200Q_ERR_UNSUPPORTED where it cannot run the problem. */
+  int force_kernel, force_width;
 } b200q_gemm_args;
 
 int b200q_fp8_gemm(const b200q_gemm_args* args);
+
+/* The kernel that b200q_fp8_gemm runs for these arguments, and the width of its column tiles (0 for the generic kernel).
+ * Nothing is read through the pointers, only their alignment counts, and no GPU is needed.  Of a batch on both sides, the
+ * plan of its first item. */
+enum b200q_gemm_kernel {
+  B200Q_GEMM_GENERIC = 0,    /* CUDA cores */
+  B200Q_GEMM_FEW_TOKENS = 1, /* M <= 128: weights on the lanes of the tensor core, tokens on its columns */
+  B200Q_GEMM_SINGLE = 2,     /* 128-row tiles, one CTA each */
+  B200Q_GEMM_PAIRS = 3       /* 256-row tiles, a pair of CTAs each */
+};
+int b200q_fp8_gemm_plan(const b200q_gemm_args* args, int* kernel, int* width);
 
 /*
  * fp8_sdpa_fwd: scaled-dot-product attention forward on e4m3 tensors,

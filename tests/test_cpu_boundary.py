@@ -152,3 +152,53 @@ def test_fp8_gemm_kernels_keep_their_registers():
     kernels = re.findall(r"Compiling entry function '(\S*gemm_tcgen05\S*)'.*?\n.*?\n\s*(\d+) bytes stack frame, (\d+) bytes spill stores", report)
     assert len(kernels) == len(set(k[0] for k in kernels)) > 0
     assert [k for k in kernels if k[1:] != ("0", "0")] == []
+
+
+def _gemm_plan(M, N, K, tA=False, tB=True, **fields):
+    import ctypes
+    g = abi.GemmArgs()
+    g.A = g.B = g.out = 1 << 20  # (nothing is read)
+    g.a_dtype = g.b_dtype = abi.E4M3
+    g.M, g.N, g.K, g.batch, g.trans_a, g.trans_b, g.out_dtype = M, N, K, 1, int(tA), int(tB), abi.BF16
+    g.lda, g.ldb, g.ldo = (M + 15) // 16 * 16 if tA else K, K if tB else (N + 15) // 16 * 16, N
+    for name, value in fields.items():
+        setattr(g, name, value)
+    kernel, width = ctypes.c_int(-1), ctypes.c_int(-1)
+    rc = abi.lib.b200q_fp8_gemm_plan(ctypes.byref(g), ctypes.byref(kernel), ctypes.byref(width))
+    return rc, kernel.value, width.value
+
+
+@pytest.mark.parametrize("M,N,K,tA,tB,best", [
+    # sizes (with the best tilings that were measured) for which a cost in tile widths alone took a tiling that was 7 to 45 % slower
+    (130, 14336, 4096, False, True, [(abi.GEMM_PAIRS, 224)]), (256, 14336, 4096, False, True, [(abi.GEMM_PAIRS, 224)]),
+    (1300, 8192, 8192, False, True, [(abi.GEMM_PAIRS, 224)]),
+    (300, 28672, 8192, True, False, [(abi.GEMM_SINGLE, 256), (abi.GEMM_PAIRS, 256)]),
+    (196, 21320, 11808, True, False, [(abi.GEMM_SINGLE, 256), (abi.GEMM_PAIRS, 256)]),
+    (256, 4096, 4096, False, True, [(abi.GEMM_PAIRS, 64)]), (700, 2048, 8192, False, True, [(abi.GEMM_PAIRS, 96)]),
+    (8000, 4096, 4096, False, False, [(abi.GEMM_PAIRS, 256)]), (4096, 4096, 8000, True, False, [(abi.GEMM_PAIRS, 256)]),
+])
+def test_fp8_gemm_plan_takes_the_tiling_that_measured_best(M, N, K, tA, tB, best):
+    rc, kernel, width = _gemm_plan(M, N, K, tA, tB)
+    assert rc == 0 and (kernel, width) in best
+
+
+def test_fp8_gemm_plan_kernels():
+    assert _gemm_plan(16, 4096, 4096) == (0, abi.GEMM_FEW_TOKENS, 16)
+    assert _gemm_plan(128, 4096, 4096)[1:] == (abi.GEMM_FEW_TOKENS, 128)
+    assert _gemm_plan(129, 64, 4096)[1:] == (abi.GEMM_SINGLE, 128)
+    assert _gemm_plan(512, 512, 1000)[1:] == (abi.GEMM_GENERIC, 0)          # rows of no 16-byte pitch
+    assert _gemm_plan(512, 512, 1024, A=(1 << 20) + 8)[1:] == (abi.GEMM_GENERIC, 0)
+    assert _gemm_plan(512, 512, 1024, force_generic=1)[1:] == (abi.GEMM_GENERIC, 0)
+    for w in (64, 96, 128, 160, 192, 224, 256):
+        assert _gemm_plan(300, 400, 256, force_kernel=abi.GEMM_PAIRS, force_width=w)[1:] == (abi.GEMM_PAIRS, w)
+    # what a kernel cannot run is not taken: widths it does not have, B in boxes of 128 columns, few rows
+    for kw in (dict(force_kernel=abi.GEMM_PAIRS, force_width=32), dict(force_kernel=abi.GEMM_SINGLE, force_width=64),
+               dict(force_kernel=abi.GEMM_PAIRS, force_width=128, tB=False), dict(force_kernel=abi.GEMM_SINGLE, force_width=192, tB=False),
+               dict(force_kernel=abi.GEMM_PAIRS, force_width=64, M=128)):
+        assert _gemm_plan(kw.pop("M", 300), 400, 256, **kw) == (0, abi.GEMM_GENERIC, 0)
+    # SwiGLU and routed output: CTA pairs only, in 256 columns and in multiples of 64
+    assert _gemm_plan(300, 512, 1024, swiglu=1, out8_dtype=abi.E4M3)[1:] == (abi.GEMM_PAIRS, 256)
+    for kernel in (abi.GEMM_SINGLE, abi.GEMM_PAIRS):
+        assert _gemm_plan(300, 512, 1024, swiglu=1, out8_dtype=abi.E4M3, force_kernel=kernel, force_width=128)[1:] == (abi.GEMM_GENERIC, 0)
+    assert _gemm_plan(300, 512, 1024, swiglu=1, out8_dtype=abi.E4M3, out_dtype=abi.F32)[1:] == (abi.GEMM_GENERIC, 0)
+    assert _gemm_plan(64, 512, 1024, force_kernel=9)[0] == -1
