@@ -368,32 +368,111 @@ def test_tcgen05_mn_major_operands(ops, tA, tB, M, N, K):
     assert torch.equal(r.cpu(), ref)
 
 
-@pytest.mark.parametrize("M,N", [(129, 136), (700, 2056), (500, 4104), (1000, 2600), (760, 4088), (512, 8200), (300, 11016)])
-@pytest.mark.parametrize("K", [48, 1424])
-def test_tile_widths(ops, M, N, K):
-    """Pair tiles of 64, 96, 128, 160, 192 and 224 columns and single tiles of 160, with partial tiles in both directions, below
-    and beyond one filling of the stage rings; small integers, whose sums are exact."""
-    g = torch.Generator().manual_seed(M + N + K)
-    A = torch.randint(-4, 5, (M, K), generator=g).float()
-    B = torch.randint(-4, 5, (N, K), generator=g).float()
-    bias = torch.randint(-9, 10, (N,), generator=g).float()
-    r = torch.ops.hpu.fp8_gemm_v2(A.to(torch.float8_e4m3fn).cuda(), False, B.to(torch.float8_e4m3fn).cuda(), True, None, torch.float32,
-                                  None, None, bias.cuda())
-    assert torch.equal(r.cpu(), A @ B.t() + bias)
+_TILES = [("single", w) for w in (128, 160, 192, 224, 256)] + [("pairs", w) for w in (64, 96, 128, 160, 192, 224, 256)]
 
 
-@pytest.mark.parametrize("tA,tB", [(True, False), (True, True), (False, False)])
+def _gemm_in_tiles(kernel, width, A, tA, B, tB, od, D=None, bias=None, full_bias=None, out8=None, ldo=None):
+    """fp8_gemm through the C ABI in tiles of the given kernel and width; the plan says that it is these that run.  Returns
+    the output, and max |out| of an fp8 one."""
+    import ctypes
+    from b200_hpu_ops import abi
+    M, K = A.shape[::-1] if tA else A.shape
+    N = B.shape[0] if tB else B.shape[1]
+    g = abi.GemmArgs()
+    g.A, g.B, g.a_dtype, g.b_dtype = A.data_ptr(), B.data_ptr(), abi.DTYPE[A.dtype], abi.DTYPE[B.dtype]
+    g.trans_a, g.trans_b, g.M, g.N, g.K, g.batch = int(tA), int(tB), M, N, K, 1
+    g.lda, g.ldb = A.stride(0), B.stride(0)
+    ldo = ldo or N
+    out = torch.full((M, ldo), 77.0, device="cuda").to(out8 or od)
+    amax = torch.zeros((), device="cuda")
+    g.out, g.out_dtype, g.ldo = out.data_ptr(), abi.DTYPE[od], ldo
+    if D is not None:
+        g.D, g.d_dtype, g.ldd = D.data_ptr(), abi.DTYPE[D.dtype], D.stride(0)
+    if bias is not None:
+        g.bias, g.bias_dtype, g.bias_mode = bias.data_ptr(), abi.DTYPE[bias.dtype], abi.BCAST_PER_COL
+    if full_bias is not None:
+        g.bias, g.bias_dtype, g.bias_mode, g.bias_ld = full_bias.data_ptr(), abi.DTYPE[full_bias.dtype], abi.BCAST_FULL, full_bias.stride(0)
+    if out8 is not None:
+        g.out8_dtype, g.out8_scale_host, g.out8_amax = abi.DTYPE[out8], 0.5, amax.data_ptr()
+    g.force_kernel, g.force_width = {"single": abi.GEMM_SINGLE, "pairs": abi.GEMM_PAIRS}[kernel], width
+    g.stream = torch.cuda.current_stream().cuda_stream
+    k, w = ctypes.c_int(), ctypes.c_int()
+    assert abi.lib.b200q_fp8_gemm_plan(ctypes.byref(g), ctypes.byref(k), ctypes.byref(w)) == 0
+    assert (k.value, w.value) == (g.force_kernel, width)
+    assert abi.lib.b200q_fp8_gemm(ctypes.byref(g)) == 0
+    assert bool((out[:, N:].float() == 77.0 if out8 is None else out[:, N:].float() == torch.tensor(77.0).to(out8).float().cuda()).all())
+    return (out[:, :N] if out8 is None else out[:, :N].view(torch.uint8)), amax
+
+
+def _ints(shape, g, lo=-4, hi=5):
+    return torch.randint(lo, hi, shape, generator=g).float()
+
+
+@pytest.mark.parametrize("kernel,width", _TILES)
+def test_every_tile_width_in_every_output_form(ops, kernel, width):
+    """Every tiling of both kernels, in every form that the epilogue stores: row segments of bf16 and fp32 with and without an
+    fp32 accumulate input, 16-byte pieces (bf16 accumulate input, element-wise bias, a pitch of 8 bytes), single elements, fp8
+    with its amax.  Partial tiles in both directions, one k-block, the stage ring wrapped, and three tiles or more for each
+    CTA or pair.  Small integers, whose sums are exact (below 2^24), so that every result is the same to the bit."""
+    g = torch.Generator().manual_seed(width + len(kernel))
+    for M, N, K in [(300, 3 * width - 24, 48), (385, 2 * width + 8, 1424), (1000, 60 * width - 24, 144)]:
+        A, B = _ints((M, K), g), _ints((N, K), g)
+        D, full, bias = _ints((M, N), g, -99, 100), _ints((M, N), g, -99, 100), _ints((N,), g, -9, 10)
+        A8, B8 = A.to(FP8[N % 16 // 8]).cuda(), B.to(torch.float8_e4m3fn).cuda()
+        ref = A @ B.t()
+        for od in (torch.bfloat16, torch.float32):
+            r, _ = _gemm_in_tiles(kernel, width, A8, False, B8, True, od, bias=bias.cuda())
+            assert torch.equal(r.cpu(), (ref + bias).to(od))
+            for Dt in (torch.bfloat16, torch.float32):
+                r, _ = _gemm_in_tiles(kernel, width, A8, False, B8, True, od, D=D.to(Dt).cuda(), ldo=N + 16)
+                assert torch.equal(r.cpu(), (ref + D).to(od))
+            if M == 1000:
+                continue
+            r, _ = _gemm_in_tiles(kernel, width, A8, False, B8, True, od, D=D.cuda(), full_bias=full.to(torch.bfloat16).cuda())
+            assert torch.equal(r.cpu(), (ref + full + D).to(od))
+            for n in (N - 4, N - 5):  # rows of 8-byte and of element granularity
+                r, _ = _gemm_in_tiles(kernel, width, A8, False, B8[:n], True, od, bias=bias[:n].cuda())
+                assert torch.equal(r.cpu(), (ref + bias)[:, :n].to(od))
+            for out8 in FP8:
+                r, amax = _gemm_in_tiles(kernel, width, A8, False, B8, True, od, bias=bias.cuda(), out8=out8)
+                want, _ = O.cast_to_fp8_v2((ref + bias).to(od), torch.tensor(0.5), False, False, out8)
+                assert torch.equal(r.cpu(), want.view(torch.uint8))
+                assert amax.item() == want.float().abs().max().item()
+
+
+@pytest.mark.parametrize("tA,tB,width", [(True, True, w) for w in (64, 96, 128, 160, 192, 224, 256)] + [(False, False, 256), (True, False, 256)])
 @pytest.mark.parametrize("M,N,K", [(144, 144, 16), (272, 528, 2064), (5120, 2064, 144)])
-def test_mn_major_operands_on_cta_pairs(ops, tA, tB, M, N, K):
-    """Partial tiles of one k-block, the stage ring wrapped, several tiles for each pair; accumulated into fp32.
+def test_mn_major_operands_on_cta_pairs(ops, tA, tB, width, M, N, K):
+    """Partial tiles of one k-block, the stage ring wrapped, several tiles for each pair; accumulated into fp32, and bf16 without.
     Small integers, whose sums are exact (below 2^24), so that the result is the same to the bit."""
     g = torch.Generator().manual_seed(M + N + K)
-    A = torch.randint(-4, 5, (K, M) if tA else (M, K), generator=g).float()
-    B = torch.randint(-4, 5, (N, K) if tB else (K, N), generator=g).float()
-    D = torch.randint(-9, 10, (M, N), generator=g).float()
-    r = torch.ops.hpu.fp8_gemm_v2(A.to(torch.float8_e5m2).cuda(), tA, B.to(torch.float8_e4m3fn).cuda(), tB, D.cuda(), torch.float32,
-                                  None, None, None, True)
-    assert torch.equal(r.cpu(), (A.t() if tA else A) @ (B.t() if tB else B) + D)
+    A, B = _ints((K, M) if tA else (M, K), g), _ints((N, K) if tB else (K, N), g)
+    D = _ints((M, N), g, -9, 10)
+    A8, B8 = A.to(torch.float8_e5m2).cuda(), B.to(torch.float8_e4m3fn).cuda()
+    ref = (A.t() if tA else A) @ (B.t() if tB else B)
+    r, _ = _gemm_in_tiles("pairs", width, A8, tA, B8, tB, torch.float32, D=D.cuda())
+    assert torch.equal(r.cpu(), ref + D)
+    r, _ = _gemm_in_tiles("pairs", width, A8, tA, B8, tB, torch.bfloat16)
+    assert torch.equal(r.cpu(), ref.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("width", [64, 128, 192, 256])
+def test_accumulation_in_place(ops, width):
+    """D and out the same buffer, twice in a row: the second launch adds to what the first has stored."""
+    import ctypes
+    from b200_hpu_ops import abi
+    g = torch.Generator().manual_seed(width)
+    M, N, K = 1000, 2056, 256
+    A, B, D = _ints((M, K), g), _ints((N, K), g), _ints((M, N), g, -9, 10)
+    A8, B8, acc = A.to(FP8[1]).cuda(), B.to(FP8[1]).cuda(), D.cuda()
+    q = abi.GemmArgs()
+    q.A, q.B, q.a_dtype, q.b_dtype, q.trans_b = A8.data_ptr(), B8.data_ptr(), abi.E4M3, abi.E4M3, 1
+    q.M, q.N, q.K, q.lda, q.ldb, q.batch = M, N, K, K, K, 1
+    q.out, q.out_dtype, q.ldo, q.D, q.d_dtype, q.ldd = acc.data_ptr(), abi.F32, N, acc.data_ptr(), abi.F32, N
+    q.force_kernel, q.force_width, q.stream = abi.GEMM_PAIRS, width, torch.cuda.current_stream().cuda_stream
+    for _ in range(4):
+        assert abi.lib.b200q_fp8_gemm(ctypes.byref(q)) == 0
+    assert torch.equal(acc.cpu(), D + 4 * (A @ B.t()))
 
 
 def test_tcgen05_mn_major_k_not_multiple_of_16(ops):

@@ -214,3 +214,22 @@ def test_routed_gemm_and_reduce_bcast_on_one_device(tp, N):
     ref = O.fp8_gemm_v2(h8.cpu(), False, w8.cpu(), True, None, torch.bfloat16, torch.tensor(0.01), sb.cpu(), None, False, [1, N])
     assert O.rel_frobenius(outs[0], ref) <= 1e-2
     assert b200_hpu_ops.device_status() == 0
+
+
+@pytest.mark.parametrize("width", [64, 128, 192, 256])
+def test_routed_gemm_in_every_tile_width(width):
+    """A warp's patch is used again for each 64 columns of a tile, and for the tiles behind it (three or more for each pair):
+    the routed rows are those of the ordinary GEMM, bit for bit."""
+    from b200_hpu_ops import abi
+    T, N, K, rows, slot = 1000, 60 * width - 24, 160, 256, 128
+    g = torch.Generator(device="cuda").manual_seed(width)
+    h8 = torch.randn(T, K, device="cuda", generator=g).mul(50).clamp(-400, 400).to(torch.float8_e4m3fn)
+    w8 = torch.randn(N, K, device="cuda", generator=g).mul(50).clamp(-400, 400).to(torch.float8_e4m3fn)
+    sb = torch.rand(N, device="cuda", generator=g) * 1e-4 + 1e-4
+    stages = [torch.full((slot + rows, N), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(4)]
+    abi.fp8_gemm_nt(h8, w8, torch.bfloat16, 0.01, sb, None, route=([s.data_ptr() for s in stages], rows, slot), tiles=(abi.GEMM_PAIRS, width))
+    want = abi.fp8_gemm_nt(h8, w8, torch.bfloat16, 0.01, sb, None, tiles=(abi.GEMM_SINGLE, 128))
+    for i, s in enumerate(stages):
+        mine = want[i * rows:(i + 1) * rows]
+        assert torch.equal(s[slot:slot + len(mine)], mine)
+        assert bool((s[:slot] == 7.0).all()) and bool((s[slot + len(mine):] == 7.0).all())
