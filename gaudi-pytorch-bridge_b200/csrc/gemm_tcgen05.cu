@@ -457,6 +457,58 @@ __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_r
     }
   }
 }
+// fp32 output whose rows have no 16-byte pitch (element_output()), by elements: through the warp's patch as above, so that an
+// instruction stores (and reads of an accumulate input or element-wise bias) 16 neighbours of two rows.  An element of 32
+// rows per instruction, as epi_drain() has it, took eight epilogue warps longer than it had taken four.  us of four / eight / these
+// (M x N x K): 7803 x 12377 x 352 511 / 591 / 175, 2620 x 20922 x 448 226 / 250 / 101; accumulated 428 x 19217 x 864 274 / - / 66.  An
+// instance of its own: beside the other drains it cost those up to 10 % (registers).
+template <int BN>
+__device__ __forceinline__ void epi_drain_elements(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
+                                                   const float* cA, const float* cB, const float* cBias, uint4* patch, int lane, int half) {
+  const EpiFlags f = epi_flags<false>(g);
+  const int prow = lane >> 4, col = lane & 15;  // a lane's elements of the patch: rows prow + 2 i, column col
+  const int rows = (int)(g.M - row0 < 32 ? g.M - row0 : 32) - prow, cols = (int)(g.N - y0 < BN ? g.N - y0 : BN) - col;
+#pragma unroll 1
+  for (int c = 32 * half; c < BN; c += c & 16 ? 48 : 16) {
+    uint32_t r[16];
+    tmem_ld_32x16(t_row + c, r);
+    tmem_ld_wait();
+    float v[16];
+    epi_values<16>(r, c, e, cA, cB, cBias, f, v);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      patch[lane * 4 + (k ^ ((lane >> 1) & 3))] =
+          make_uint4(__float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]), __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3]));
+    __syncwarp();
+    const int64_t m = row0 + prow, n = y0 + c + col;
+    const int in = c < cols ? rows : 0;
+#pragma unroll 1
+    for (int i0 = 0; i0 < 16; i0 += 8) {
+      float w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        w[i] = reinterpret_cast<const float*>(patch)[(2 * (i0 + i) + prow) * 16 + 4 * ((col >> 2) ^ (i & 3)) + (col & 3)];
+      auto add = [&](const void* base, int dtype, int64_t ld) {
+        const int64_t at = (m + 2 * i0) * ld + n;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (2 * (i0 + i) < in) w[i] += ld_out_typed(base, dtype, at + 2 * i * ld);
+      };
+      if (g.bias_mode == B200Q_BCAST_FULL) add(g.bias, g.bias_dtype, g.bias_ld);
+      if (g.D) add(g.D, g.d_dtype, g.ldd);
+      float* out = static_cast<float*>(g.out) + (m + 2 * i0) * g.ldo + n;
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (2 * (i0 + i) < in) out[2 * i * g.ldo] = w[i];
+    }
+    __syncwarp();
+  }
+}
+
+static bool element_output(const GemmParams& g) {
+  return g.out_dtype == B200Q_F32 && !g.out8_dtype && (g.ldo % 4 || (reinterpret_cast<uintptr_t>(g.out) & 15));
+}
+
 // Outputs that epi_drain_rows() takes: 16-byte aligned rows of whole 16-byte pieces.
 static bool whole_rows_output(const GemmParams& g) {
   if (g.out8_dtype || g.swiglu || g.route_count > 0 || g.bias_mode == B200Q_BCAST_FULL || (reinterpret_cast<uintptr_t>(g.out) & 15)) return false;
@@ -517,7 +569,7 @@ __device__ __forceinline__ void epi_drain_swiglu(const GemmParams& g, uint32_t t
   }
 }
 
-template <int BN, int STAGES, bool SWAP, int KPS, int EW>
+template <int BN, int STAGES, bool SWAP, int KPS, int EW, bool ELEMENTS = false>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const TcGemmParams p) {
@@ -708,9 +760,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       if constexpr (!SWAP) {
-        if (p.whole_rows)
-          epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias,
-                             reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128, lane, half);
+        uint4* patch = reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256 + half * 128;
+        if constexpr (ELEMENTS)
+          epi_drain_elements<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, patch, lane, half);
+        else if (p.whole_rows)
+          epi_drain_rows<BN, EW>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, patch, lane, half);
         else
           epi_drain<BN, SWAP, EW>(g, t_row, er, y0, cA, cB, cBias, half);
       } else {
@@ -763,7 +817,7 @@ struct PairSmem {
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
 };
 
-template <int BN, int STAGES, int EW>
+template <int BN, int STAGES, int EW, bool ELEMENTS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                          const TcGemmParams p) {
@@ -899,7 +953,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
       uint4* patch = reinterpret_cast<uint4*>(smem + L::kPatchOffset) + q * 256;
       // (SwiGLU and routed output are bf16 epilogues: four warps, so that a quarter's 4 KB patch is one warp's)
-      if (EW == 4 && BN == 256 && g.swiglu) {
+      if constexpr (ELEMENTS) {
+        epi_drain_elements<BN>(g, t_row, er, x0 + q * 32, y0, cA, cB, cBias, patch + half * 128, lane, half);
+      } else if (EW == 4 && BN == 256 && g.swiglu) {
         epi_drain_swiglu(g, t_row, er, y0, cA, cB, cBias);
       } else if (EW == 4 && BN % 64 == 0 && g.route_count > 0) {
         if constexpr (EW == 4 && BN % 64 == 0)
@@ -931,13 +987,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
   }
 }
 
-template <int BN, int STAGES, int EW>
+template <int BN, int STAGES, int EW, bool ELEMENTS = false>
 static int launch_pair_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = PairSmem<BN, STAGES>;
   constexpr int smem = L::kTotal + 1024, kPairThreads = 64 + 32 * EW;
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
-  auto kern = gemm_tcgen05_pair_kernel<BN, STAGES, EW>;
+  auto kern = gemm_tcgen05_pair_kernel<BN, STAGES, EW, ELEMENTS>;
   // per device, once: raise the dynamic shared-memory limit and ask how many CTA pairs can be
   // resident at once (a pair needs both SMs of a TPC); -1 = pairs not available on this device
   static std::atomic<int> resident_pairs[kMaxDevices];
@@ -972,7 +1028,8 @@ static int launch_pair_ew(const CUtensorMap& mx, const CUtensorMap& my, const Tc
 
 template <int BN, int STAGES>
 static int launch_pair(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
-  return tp.g.out_dtype == B200Q_F32 ? launch_pair_ew<BN, STAGES, 8>(mx, my, tp, st) : launch_pair_ew<BN, STAGES, 4>(mx, my, tp, st);
+  if (tp.g.out_dtype != B200Q_F32) return launch_pair_ew<BN, STAGES, 4>(mx, my, tp, st);
+  return element_output(tp.g) ? launch_pair_ew<BN, STAGES, 8, true>(mx, my, tp, st) : launch_pair_ew<BN, STAGES, 8>(mx, my, tp, st);
 }
 
 // ------------------------------------------------------------------------ host side
@@ -983,14 +1040,14 @@ int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k
                          CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-template <int BN, int STAGES, bool SWAP, int KPS, int EW>
+template <int BN, int STAGES, bool SWAP, int KPS, int EW, bool ELEMENTS = false>
 static int launch_cfg_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   using L = SmemLayout<BN, STAGES, KPS>;
   constexpr int kThreads = 64 + 32 * EW;
   constexpr int smem = L::kTotal + 1024;  // slack for the manual 1024-byte alignment
   static_assert(smem <= 227 * 1024, "shared memory budget");
   static_assert(smem > 116 * 1024, "one CTA per SM: two CTAs must never contend for TMEM");
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, SWAP, KPS, EW>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, SWAP, KPS, EW, ELEMENTS>;
   static std::atomic<int> configured[kMaxDevices];
   const int dev = current_device_index();
   if (dev < 0) return B200Q_ERR_CUDA;
@@ -1014,7 +1071,9 @@ static int launch_cfg_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcG
 template <int BN, int STAGES, bool SWAP, int KPS = 1>
 static int launch_cfg(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
   if constexpr (!SWAP)
-    if (tp.g.out_dtype == B200Q_F32) return launch_cfg_ew<BN, STAGES, SWAP, KPS, 8>(mx, my, tp, st);
+    if (tp.g.out_dtype == B200Q_F32)
+      return element_output(tp.g) ? launch_cfg_ew<BN, STAGES, SWAP, KPS, 8, true>(mx, my, tp, st)
+                                  : launch_cfg_ew<BN, STAGES, SWAP, KPS, 8>(mx, my, tp, st);
   return launch_cfg_ew<BN, STAGES, SWAP, KPS, 4>(mx, my, tp, st);
 }
 

@@ -433,6 +433,8 @@ def test_every_tile_width_in_every_output_form(ops, kernel, width):
             for n in (N - 4, N - 5):  # rows of 8-byte and of element granularity
                 r, _ = _gemm_in_tiles(kernel, width, A8, False, B8[:n], True, od, bias=bias[:n].cuda())
                 assert torch.equal(r.cpu(), (ref + bias)[:, :n].to(od))
+                r, _ = _gemm_in_tiles(kernel, width, A8, False, B8[:n], True, od, D=D[:, :n].contiguous().cuda(), ldo=n + 3)
+                assert torch.equal(r.cpu(), (ref + D)[:, :n].to(od))
             for out8 in FP8:
                 r, amax = _gemm_in_tiles(kernel, width, A8, False, B8, True, od, bias=bias.cuda(), out8=out8)
                 want, _ = O.cast_to_fp8_v2((ref + bias).to(od), torch.tensor(0.5), False, False, out8)
