@@ -303,7 +303,7 @@ int b200q_dequant_int4(const int32_t* packed, const void* scale, const void* zp,
 }
 
 // Checks the arguments of a GEMM and fills the kernels' block; empty: there is nothing to compute.
-static int gemm_params(const b200q_gemm_args* a, GemmParams& g, bool& empty) {
+static int gemm_params(const b200q_gemm_args* a, GemmParams& g, GemmTiles& tiles, bool& empty) {
   if (!a) return B200Q_ERR_BAD_ARGUMENT;
   if (a->M < 0 || a->N < 0 || a->K < 0 || a->batch < 0) return B200Q_ERR_BAD_ARGUMENT;
   if (!is_fp8(a->a_dtype) || !is_fp8(a->b_dtype) || !is_wide(a->out_dtype)) return B200Q_ERR_BAD_ARGUMENT;
@@ -331,8 +331,8 @@ static int gemm_params(const b200q_gemm_args* a, GemmParams& g, bool& empty) {
   g.swiglu = a->swiglu;
   g.out8_amax = g.out8_dtype ? a->out8_amax : nullptr;
   g.b_static = a->b_static ? 1 : 0;
-  g.force_kernel = a->force_kernel; g.force_width = a->force_width;
-  if (g.force_kernel != B200Q_GEMM_GENERIC && g.force_kernel != B200Q_GEMM_SINGLE && g.force_kernel != B200Q_GEMM_PAIRS)
+  tiles = {a->force_kernel, a->force_width};
+  if (tiles.kernel != B200Q_GEMM_GENERIC && tiles.kernel != B200Q_GEMM_SINGLE && tiles.kernel != B200Q_GEMM_PAIRS)
     return B200Q_ERR_BAD_ARGUMENT;
   g.route_count = a->route_count; g.route_rows = a->route_rows; g.route_row_offset = a->route_row_offset;
   for (int i = 0; i < 8; ++i) g.route_out[i] = a->route_out[i];
@@ -344,22 +344,23 @@ static int gemm_params(const b200q_gemm_args* a, GemmParams& g, bool& empty) {
 
 int b200q_fp8_gemm(const b200q_gemm_args* a) {
   GemmParams g;
+  GemmTiles tiles;
   bool empty = false;
-  const int checked = gemm_params(a, g, empty);
+  const int checked = gemm_params(a, g, tiles, empty);
   if (checked != B200Q_OK || empty) return checked;
   cudaStream_t st = static_cast<cudaStream_t>(a->stream);
   if (g.route_count > 0) {
     if (g.batch != 1 || a->force_generic || g.route_row_offset < 0) return B200Q_ERR_UNSUPPORTED;
-    return gemm_tcgen05_launch(g, st);  // B200Q_ERR_UNSUPPORTED when the shape has no routed kernel
+    return gemm_tcgen05_launch(g, tiles, st);  // B200Q_ERR_UNSUPPORTED when the shape has no routed kernel
   }
   if (g.swiglu) {
     if (g.out8_dtype != B200Q_E4M3) return B200Q_ERR_BAD_ARGUMENT;
     if (g.batch != 1 || g.D || g.trans_a || !g.trans_b || a->force_generic) return B200Q_ERR_UNSUPPORTED;
-    return gemm_tcgen05_launch(g, st);  // B200Q_ERR_UNSUPPORTED when the shape has no fused kernel
+    return gemm_tcgen05_launch(g, tiles, st);  // B200Q_ERR_UNSUPPORTED when the shape has no fused kernel
   }
   if (!a->force_generic) {
     if (g.batch == 1) {
-      int rc = gemm_tcgen05_launch(g, st);
+      int rc = gemm_tcgen05_launch(g, tiles, st);
       if (rc != B200Q_ERR_UNSUPPORTED) return rc;
     } else if (g.batch <= 1024) {
       // batched problems: one tensor-core launch per batch item (same eligibility for all of them)
@@ -373,7 +374,7 @@ int b200q_fp8_gemm(const b200q_gemm_args* a) {
         if (g.bias_mode == B200Q_BCAST_FULL)
           gb.bias = static_cast<const uint8_t*>(g.bias) + b * g.bias_batch_stride * elem(g.bias_dtype);
         if (g.D) gb.D = static_cast<const uint8_t*>(g.D) + b * g.d_batch_stride * elem(g.d_dtype);
-        int rc = gemm_tcgen05_launch(gb, st);
+        int rc = gemm_tcgen05_launch(gb, tiles, st);
         if (rc == B200Q_ERR_UNSUPPORTED && b == 0) break;  // not eligible: the generic kernel takes the whole batch
         if (rc != B200Q_OK) return rc;
         if (b == g.batch - 1) return B200Q_OK;
@@ -388,11 +389,12 @@ int b200q_fp8_gemm_plan(const b200q_gemm_args* a, int* kernel, int* width) {
   *kernel = B200Q_GEMM_GENERIC;
   *width = 0;
   GemmParams g;
+  GemmTiles tiles;
   bool empty = false;
-  const int checked = gemm_params(a, g, empty);
+  const int checked = gemm_params(a, g, tiles, empty);
   if (checked != B200Q_OK || empty || a->force_generic || g.batch > 1024) return checked;
   g.batch = 1;
-  const GemmPlan plan = gemm_tcgen05_plan(g);
+  const GemmPlan plan = gemm_tcgen05_plan(g, tiles);
   *kernel = plan.kernel;
   *width = plan.width;
   return B200Q_OK;

@@ -48,7 +48,6 @@ struct GemmParams {
   int64_t route_rows, route_row_offset;
   float* out8_amax;  // fused output cast only: max |fp8 value written| (atomic max on the bit pattern), or null
   int b_static;      // B is not written by work still in flight: it may be read before the preceding kernel completes
-  int force_kernel, force_width;  // testing: this B200Q_GEMM_* kernel in tiles of this many columns, or B200Q_GEMM_GENERIC (0): the cheapest
 };
 
 // value in out_dtype -> fp8 byte of the fused output cast
@@ -151,7 +150,12 @@ int gemm_generic_launch(const GemmParams& p, cudaStream_t st);
 struct GemmPlan {
   int kernel, width, single_width;
 };
-GemmPlan gemm_tcgen05_plan(const GemmParams& p);
-int gemm_tcgen05_launch(const GemmParams& p, cudaStream_t st);  // returns B200Q_ERR_UNSUPPORTED if not eligible
+// A tiling asked for (testing): this kernel in tiles of this many columns; 0: the cheapest.  (Not in GemmParams, which is a kernel
+// argument: eight bytes more there took the host 0.3 us longer per launch, linear layer of one token 15.1 -> 15.6 us.)
+struct GemmTiles {
+  int kernel, width;
+};
+GemmPlan gemm_tcgen05_plan(const GemmParams& p, GemmTiles tiles);
+int gemm_tcgen05_launch(const GemmParams& p, GemmTiles tiles, cudaStream_t st);  // returns B200Q_ERR_UNSUPPORTED if not eligible
 
 }  // namespace b200q

@@ -1112,7 +1112,7 @@ static double tiling_cost(const GemmParams& g, bool pair, int w) {
   return pair ? ns + 200 : 1.02 * ns;
 }
 
-GemmPlan gemm_tcgen05_plan(const GemmParams& g) {
+GemmPlan gemm_tcgen05_plan(const GemmParams& g, GemmTiles tiles) {
   // eligibility: TMA-compatible strides and bases, one problem per launch.  A is K-major when
   // stored [M][K] (trans_a = 0), B when stored [N][K] (trans_b = 1); the other storage orders
   // are MN-major operands, which the tensor core reads through MN-major descriptors.
@@ -1137,7 +1137,7 @@ GemmPlan gemm_tcgen05_plan(const GemmParams& g) {
 
   // small M: weights on the lanes, tokens on the columns -- unless the tokens are MN-major (their
   // column tile would be narrower than the 128-byte MN-major row)
-  if (g.M <= 128 && g.N >= 128 && !a_mn && !g.force_kernel) {
+  if (g.M <= 128 && g.N >= 128 && !a_mn && !tiles.kernel) {
     const int w = g.M <= 16 ? 16 : g.M <= 32 ? 32 : g.M <= 64 ? 64 : 128;
     return {B200Q_GEMM_FEW_TOKENS, w, w};
   }
@@ -1149,7 +1149,7 @@ GemmPlan gemm_tcgen05_plan(const GemmParams& g) {
   GemmPlan plan = none;
   double best = 1e30;
   auto consider = [&](int kernel, int w, double cost) {
-    if (g.force_kernel && (kernel != g.force_kernel || w != g.force_width)) return;
+    if (tiles.kernel && (kernel != tiles.kernel || w != tiles.width)) return;
     if (cost < best) best = cost, plan.kernel = kernel, plan.width = w;
   };
   for (int w : {256, 224, 192, 160, 128}) {
@@ -1165,8 +1165,8 @@ GemmPlan gemm_tcgen05_plan(const GemmParams& g) {
   return plan;
 }
 
-int gemm_tcgen05_launch(const GemmParams& g, cudaStream_t st) {
-  const GemmPlan plan = gemm_tcgen05_plan(g);
+int gemm_tcgen05_launch(const GemmParams& g, GemmTiles tiles, cudaStream_t st) {
+  const GemmPlan plan = gemm_tcgen05_plan(g, tiles);
   if (plan.kernel == B200Q_GEMM_GENERIC) return B200Q_ERR_UNSUPPORTED;
   const bool a_mn = g.trans_a != 0, b_mn = g.trans_b == 0;
   TcGemmParams tp;
