@@ -53,7 +53,7 @@ struct TcGemmParams {
 
 // KPS = k-blocks per ring stage.  A stage is KPS sub-stages [X tile][Y tile] of one k-block each;
 // the barrier handshake (full / empty) is per stage.
-template <int BN, int STAGES, int KPS = 1>
+template <int BN, int STAGES, bool SWAP, int KPS>
 struct SmemLayout {
   static constexpr int kXBytes = kBlockX * kBlockK;
   static constexpr int kYBytes = BN * kBlockK;
@@ -63,7 +63,7 @@ struct SmemLayout {
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;  // per accumulator: col scale A, col scale B, col bias
   static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // epilogue warps x 2 KB (whole-row output)
-  static constexpr int kPatchBytes = BN >= 128 && KPS == 1 ? 4 * 4096 : 0;
+  static constexpr int kPatchBytes = SWAP ? 0 : 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
   static constexpr int kTotal = kBarOffset + kNumBars * 8 + 16;
@@ -573,7 +573,7 @@ template <int BN, int STAGES, bool SWAP, int KPS, int EW, bool ELEMENTS = false>
 __global__ void __launch_bounds__(64 + 32 * EW, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const TcGemmParams p) {
-  using L = SmemLayout<BN, STAGES, KPS>;
+  using L = SmemLayout<BN, STAGES, SWAP, KPS>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // dynamic shared memory is only guaranteed 16-byte aligned: round up to the swizzle atom
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1042,7 +1042,7 @@ int make_operand_map(CUtensorMap* map, const void* base, int64_t rows, int64_t k
 
 template <int BN, int STAGES, bool SWAP, int KPS, int EW, bool ELEMENTS = false>
 static int launch_cfg_ew(const CUtensorMap& mx, const CUtensorMap& my, const TcGemmParams& tp, cudaStream_t st) {
-  using L = SmemLayout<BN, STAGES, KPS>;
+  using L = SmemLayout<BN, STAGES, SWAP, KPS>;
   constexpr int kThreads = 64 + 32 * EW;
   constexpr int smem = L::kTotal + 1024;  // slack for the manual 1024-byte alignment
   static_assert(smem <= 227 * 1024, "shared memory budget");
