@@ -31,10 +31,6 @@ using namespace ptx;
 constexpr int kBlockX = 128;  // rows of the lane-side operand per tile (UMMA M)
 constexpr int kBlockK = 128;  // bytes (= fp8 elements) of K per ring stage: one swizzle row
 constexpr int kUmmaK = 32;
-// Epilogue warps, EW: one or two for each quarter of the TMEM lanes; two take turns with 32-column groups of a tile.  fp32
-// outputs have two, since of few k their epilogue sets the pace (linear layer's backward pass, 8000 x 4096 x 4096: 238 -> 231
-// us; see epi_drain_rows()), the others one: a gate/up GEMM of 8192 x 57344 x 8192, limited by power, took 3195 us with
-// two and 3110 with one.
 
 enum { kErrProducer = 101, kErrMma = 102, kErrMmaTmem = 103, kErrEpilogue = 104 };
 
@@ -62,7 +58,7 @@ struct SmemLayout {
   static_assert(kSubBytes % 1024 == 0, "swizzled tiles need 1024-byte alignment");
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;  // per accumulator: col scale A, col scale B, col bias
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // epilogue warps x 2 KB (whole-row output)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 2 KB for each of eight epilogue warps (epi_drain_rows())
   static constexpr int kPatchBytes = SWAP ? 0 : 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
@@ -70,6 +66,11 @@ struct SmemLayout {
 };
 
 // ---------------------------------------------------------------------------- epilogue pieces
+// Epilogue warps, EW: one or two for each quarter of the TMEM lanes; two take turns with 32-column groups of a tile.  fp32
+// outputs have two, since of few k their epilogue sets the pace (linear layer's backward pass, 8000 x 4096 x 4096: 238 -> 231
+// us; see epi_drain_rows()), the others one: a gate/up GEMM of 8192 x 57344 x 8192, limited by power, took 3195 us with
+// two and 3110 with one.
+
 // Per-thread (lane-side) and per-column epilogue operands of one tile.  Scales multiply in the
 // order (acc * sa) * sb; a scalar or lane-side scale lives in rA / rB, a column-side one in
 // shared memory (cA / cB), the other factor is 1.
@@ -374,19 +375,25 @@ __device__ __forceinline__ void epi_drain_routed(const GemmParams& g, uint32_t t
 }
 
 // fp32 output, with or without an fp32 accumulate input, or bf16 output without one, in 64-byte row segments: what a
-// thread computes for its row goes through a 2 KB patch of its warp (four 16-byte pieces per row, XOR-swizzled so that
-// neither side has bank conflicts), so that a load or store instruction covers eight rows of 64 bytes instead of 16 bytes
-// of 32 rows.  The accumulate input of the warp's next 32 columns is on its way while a group is finished.  Of few k it is
-// the epilogue that sets the pace; accumulated 4352 x 4992 x 498 (M x N x K) / plain fp32 8192 x 8192 x 640, us: 82 / - with 16-byte
-// pieces of 32 rows, 61 / 99 with four warps and 128-byte segments, 55 / 79 with eight warps.  Asking for the accumulate
-// input's lines of the next tile as far as L2 did not help (71).  (whole_rows_output() says for which outputs.)
+// thread computes for its row goes through a 2 KB patch of its warp (four 16-byte pieces per row, XOR-swizzled: eight lanes of
+// either side touch eight different groups of four banks), so that a load or store instruction covers eight rows of
+// 64 bytes instead of 16 bytes of 32 rows.  The accumulate input of a warp's next 32 columns is asked for behind the last
+// store of this group, so that it arrives under the next group's TMEM load, scaling and patch; that of a tile's first
+// group has nothing to hide under.  Of few k it is the epilogue that sets the pace; accumulated 4352 x 4992 x 498
+// (M x N x K) / plain fp32 8192 x 8192 x 640, us: 82 / - with 16-byte pieces of 32 rows, 61 / 99 with four warps and 128-byte
+// segments, 55 / 79 with eight warps.  Asking for the accumulate input's lines of the next tile as far as L2 did not help
+// (71).  The patch takes a ring stage from 224 and 160 columns: outputs that do not use it are no slower for it (pair tiles of 224
+// columns with a stage less, accumulated bf16 and element-wise bias 0.97-0.98 of the time before, fp8 0.99).
+// (The counter of shared-memory bank conflicts rose with it, 2.0 to 3.4 M in the 4096 x 14336 x 4096 product; the pattern
+// above has none, and what else it counts is not known.)  whole_rows_output() says for which outputs.
 template <int BN, int EW>
 __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
                                                const float* cA, const float* cB, const float* cBias, uint4* patch, int lane, int half) {
   const EpiFlags f = epi_flags<false>(g);
   const int prow = lane >> 2, piece = lane & 3;  // a lane's rows of the patch: prow + 8 k
   constexpr int kPiece = EW == 8 ? 4 : 8;        // columns in 16 bytes
-  // the lane's rows and columns inside the output, counted from its own first ones (in 32 bits: the fp32 form has no register to spare)
+  // the lane's rows and columns inside the output, counted from its own first ones (in 32 bits: the fp32 form has no register
+  // to spare)
   const int rows = (int)(g.M - row0 < 32 ? g.M - row0 : 32) - prow;
   const int cols = (int)(g.N - y0 < BN ? g.N - y0 : BN) - kPiece * piece;
   uint4* put = patch + lane * 4;
@@ -747,9 +754,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       float* cB = cA + BN;
       float* cBias = cB + BN;
       const EpiRow er = epi_stage_operands<BN, SWAP, EW>(g, x_end, p.y_rows, x0 + q * 32 + lane, y0, et, cA, cB, cBias);
-      // One warp waits for the accumulator (polling costs power and issue slots) and says whether to stop; the others meet it at the barrier, behind which the
-      // operands staged above can be read too.  A word per accumulator: a warp has read one before it lets the next
-      // but one be written.
+      // One warp waits for the accumulator (polling costs power and issue slots) and says whether to stop; the others meet
+      // it at the barrier, behind which the operands staged above can be read too.  A word per accumulator: a warp has
+      // read one before it lets the next but one be written.
       if (et < 32) {
         mbar_wait(bar_tfull + 8 * acc, acc_phase, abort_flag, p.status, kErrEpilogue, 128);
         __syncwarp();
@@ -802,7 +809,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 // into shared memory than two independent 128 x BN tiles, which is what bounds the
 // single-CTA kernel.  Barrier traffic: both producers' TMA bytes complete on the even CTA's
 // "full" barrier; tcgen05.commit (multicast to both CTAs) releases ring stages and publishes
-// accumulators; both CTAs' epilogue threads arrive on the even CTA's "accumulator free" barrier.
+// accumulators; the epilogue warps of both CTAs arrive on the even CTA's "accumulator free" barrier, once each.
 template <int BN, int STAGES>
 struct PairSmem {
   static constexpr int kXBytes = kBlockX * kBlockK;
@@ -810,7 +817,7 @@ struct PairSmem {
   static constexpr int kStageBytes = kXBytes + kYBytes;
   static constexpr int kRing = STAGES * kStageBytes;
   static constexpr int kEpiFloats = 2 * 3 * BN;
-  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // epilogue warps x 2 KB (whole-row output; routed output: 4 x 4 KB)
+  static constexpr int kPatchOffset = kRing + kEpiFloats * 4;  // 2 KB for each of eight epilogue warps (routed output: 4 KB of four)
   static constexpr int kPatchBytes = 4 * 4096;
   static constexpr int kBarOffset = kPatchOffset + kPatchBytes;
   static constexpr int kNumBars = 2 * STAGES + 4;
