@@ -384,7 +384,7 @@ __device__ __forceinline__ void epi_drain_routed(const GemmParams& g, uint32_t t
 // segments, 55 / 79 with eight warps.  Asking for the accumulate input's lines of the next tile as far as L2 did not help
 // (71).  The patch takes a ring stage from 224 and 160 columns: outputs that do not use it are no slower for it (pair tiles of 224
 // columns with a stage less, accumulated bf16 and element-wise bias 0.97-0.98 of the time before, fp8 0.99).
-// (The counter of shared-memory bank conflicts rose with it, 2.0 to 3.4 M in the 4096 x 14336 x 4096 product; the pattern
+// (The counter of shared-memory bank conflicts rose with it, 2.0 to 3.2 M in the 4096 x 14336 x 4096 product; the pattern
 // above has none, and what else it counts is not known.)  whole_rows_output() says for which outputs.
 template <int BN, int EW>
 __device__ __forceinline__ void epi_drain_rows(const GemmParams& g, uint32_t t_row, const EpiRow& e, int64_t row0, int64_t y0,
